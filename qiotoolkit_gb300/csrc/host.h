@@ -40,6 +40,12 @@ struct DevBuf
   template <class T> T* as() const { return (T*)ptr; }
 };
 
+// Host to device, finished on return.  A plain cudaMemcpy from pageable memory
+// may return while its last part is still on the way to the device, ordered
+// on the legacy stream only; kernels of non-blocking streams (the server's,
+// a caller's) would not wait for it.
+void h2d(void* dst, const void* src, size_t bytes, const char* what);
+
 void ensure_device();  // selects the device, uploads tables once per device
 // bit-packed walker states (32 variables per word, rows of nw words) to one
 // byte per variable, `count` rows of N bytes

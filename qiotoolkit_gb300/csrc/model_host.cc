@@ -71,6 +71,13 @@ DevBuf& DevBuf::operator=(DevBuf&& o) noexcept
   return *this;
 }
 
+void h2d(void* dst, const void* src, size_t bytes, const char* what)
+{
+  if (!bytes) return;
+  cuda_check(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what);
+  cuda_check(cudaStreamSynchronize(cudaStreamLegacy), what);
+}
+
 static std::mutex g_dev_mu;
 static std::map<int, int*> g_err;
 
@@ -114,6 +121,8 @@ void ensure_device()
   int* flag = nullptr;
   cuda_check(cudaMalloc(&flag, 4), "cudaMalloc");
   cuda_check(cudaMemset(flag, 0, 4), "cudaMemset");
+  // the tables and the flag are there before any stream's kernel reads them
+  cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "sync");
   g_err[dev] = flag;
   ready.insert(dev);
 }
@@ -646,8 +655,7 @@ void HostModel::upload() const
   // end up to 16 bytes
   blob.resize(((blob.size() + 255) & ~(size_t)255) + 256);
   dmem = DevBuf(blob.size());
-  cuda_check(cudaMemcpy(dmem.ptr, blob.data(), blob.size(), cudaMemcpyHostToDevice),
-             "model upload");
+  h2d(dmem.ptr, blob.data(), blob.size(), "model upload");
   char* b = (char*)dmem.ptr;
   dev.flavor = flavor;
   dev.n_vars = (int)N;

@@ -380,13 +380,13 @@ void LaneRunner::setup(const std::vector<DevModel>& models, const std::vector<in
     meta = DevBuf(bytes);
     arena = DevBuf((size_t)std::max<long long>(total, 256));
     char* b = (char*)meta.ptr;
-    cuda_check(cudaMemcpy(b + o_m, models.data(), models.size() * sizeof(DevModel), cudaMemcpyHostToDevice), "H2D");
+    h2d(b + o_m, models.data(), models.size() * sizeof(DevModel), "H2D");
     if (!model_of.empty())
-      cuda_check(cudaMemcpy(b + o_mo, model_of.data(), model_of.size() * 4, cudaMemcpyHostToDevice), "H2D");
-    cuda_check(cudaMemcpy(b + o_off, off.data(), (size_t)G * 8, cudaMemcpyHostToDevice), "H2D");
-    cuda_check(cudaMemcpy(b + o_nv, nv.data(), (size_t)G * 4, cudaMemcpyHostToDevice), "H2D");
+      h2d(b + o_mo, model_of.data(), model_of.size() * 4, "H2D");
+    h2d(b + o_off, off.data(), (size_t)G * 8, "H2D");
+    h2d(b + o_nv, nv.data(), (size_t)G * 4, "H2D");
     if (!local_of.empty())
-      cuda_check(cudaMemcpy(b + o_lo, local_of.data(), local_of.size() * 4, cudaMemcpyHostToDevice), "H2D");
+      h2d(b + o_lo, local_of.data(), local_of.size() * 4, "H2D");
     a = LwArgs{};
     a.models = (const DevModel*)(b + o_m);
     a.model_of = model_of.empty() ? nullptr : (const int*)(b + o_mo);
@@ -2514,10 +2514,10 @@ class SABatch : public Batch
     for (int i = 0; i < R; i++) rs[i] = Pcg(master.next()).state;
     for (int k = 1; k < (int)models.size(); k++) std::copy(rs.begin(), rs.begin() + R, rs.begin() + (size_t)k * R);
     rng0 = DevBuf((size_t)W * 8);
-    cuda_check(cudaMemcpy(rng0.ptr, rs.data(), (size_t)W * 8, cudaMemcpyHostToDevice), "H2D rng");
+    h2d(rng0.ptr, rs.data(), (size_t)W * 8, "H2D rng");
     const auto& betas = views[0]->betas;
     if (steps > 0)
-      cuda_check(cudaMemcpy(P.beta, betas.data(), betas.size() * 8, cudaMemcpyHostToDevice), "H2D beta");
+      h2d(P.beta, betas.data(), betas.size() * 8, "H2D beta");
     if (lanes)
     {
       std::vector<DevModel> dm;
@@ -2581,9 +2581,9 @@ class SABatch : public Batch
       local_of[r] = r % R;
     }
     char* b = (char*)qbuf.ptr;
-    cuda_check(cudaMemcpy(b, dm.data(), n * sizeof(DevModel), cudaMemcpyHostToDevice), "H2D models");
-    cuda_check(cudaMemcpy(b + o_mo, model_of.data(), (size_t)W * 4, cudaMemcpyHostToDevice), "H2D");
-    cuda_check(cudaMemcpy(b + o_lo, local_of.data(), (size_t)W * 4, cudaMemcpyHostToDevice), "H2D");
+    h2d(b, dm.data(), n * sizeof(DevModel), "H2D models");
+    h2d(b + o_mo, model_of.data(), (size_t)W * 4, "H2D");
+    h2d(b + o_lo, local_of.data(), (size_t)W * 4, "H2D");
     d_models = (const DevModel*)b;
     d_model_of = (int*)(b + o_mo);
     d_local_of = (int*)(b + o_lo);

@@ -102,3 +102,19 @@ def test_serving_rejects_and_polls():
     assert res is not None and "solutions" in res
     srv.forget(rid)
     srv.close()
+
+
+def test_bursts_of_models_not_yet_on_the_device():
+    """Requests whose models are uploaded by the submission itself, many in
+    flight at once: a solve on its own non-blocking stream starts after its
+    model has arrived."""
+    with_server = q.Server(memory_budget_bytes=2 << 30, max_active=128)
+    params = {"seed": 5, "sweeps": 30, "restarts": 4, "beta_start": 0.1, "beta_stop": 3.0}
+    for burst in range(3):
+        insts = [I.er_ising(60 + 37 * i, 200 + 120 * i, seed=100 * burst + i) for i in range(24)]
+        rids = [with_server.submit(q.Model("ising", off=o, ids=i, coef=c), SA, params) for o, i, c in insts]
+        got = [_strip(with_server.wait(r)) for r in rids]
+        for (o, i, c), res in zip(insts[::6], got[::6]):
+            plain = q.Solver(q.Model("ising", off=o, ids=i, coef=c), SA, params).init().run().result()
+            assert _strip(plain)["solutions"] == res["solutions"]
+    with_server.close()
