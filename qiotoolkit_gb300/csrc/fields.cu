@@ -1,32 +1,59 @@
-// fields.cu -- the field-cached Metropolis sweep (sm_103a).
+// fields.cu -- the block-decided Metropolis sweep (sm_103a).
 //
-// Two warps own one walker.  The DECIDER runs the reference's ordered sweep
-// (markov/walker.h:143-153,209-229) in 32-variable windows, like the
-// windowed kernel, but it reads each variable's cost difference from a
-// cached local field instead of summing its row: the field is the
-// difference in fixed point (DevModel::fc_rec), kept exact under every flip
-// by integer shared-memory atomics on the co-members of the flipped
-// variable's terms.  A field differs from the reference's FP64 sum by less
-// than deg + 1 units, so its sign and the FP32-screened ln-table comparison
-// (markov/metropolis.h:64-104) are decided from it with a rigorous margin;
-// only inside the margin is the exact FP64 sum taken, in the reference's
-// term order.  Committed flips go to a flip log in shared memory, with the
-// contributing-incidence masks read before the flip.
+// One warp, the DECIDER, runs a walker's ordered sweep (markov/walker.h:
+// 143-153,209-229) 32 variables at a time, a variable per lane.  At a block's
+// start every lane gathers its field -- the cost difference of its flip in
+// fixed point (model_host.cc, build_fields) -- from the walker's state in
+// shared memory: the neighbours' spins (Ising models of one- and two-member
+// terms) or one byte per term that holds the literals of all its members.
 //
-// The ACCOUNTANT consumes the log in batches of up to 32 flips: every lane
-// recomputes one flip's exact FP64 cost difference from its masks (the
-// reference's order and rounding, model/ising.h:108-117, model/pubo.h:
-// 335-367), then the running cost is accumulated in flip order exactly as
-// cost_ += diff (markov/walker.h:225) and the lowest state is taken at the
-// first strict improvement (markov/walker.h:269-280) from the accountant's
-// own copy of the spins.  Neither the decisions nor the draws depend on the
-// running cost, so moving it off the decider changes nothing in the chain.
+// The block is then decided as a whole.  Lane v's decision depends on the
+// decisions of the lanes before it in two ways: through the terms it shares
+// with them (fc_in lists these with their members' lanes) and, on replayed
+// streams, through the draw it gets (the uphill lanes before it each take
+// one).  Both only look back, so the lanes iterate: decide with the accept
+// mask of the last round, vote, and decide again where a member of a lane's
+// in-block terms changed; a mask that no longer changes any lane's terms is the
+// ordered sweep's, lane by lane from the first.  A field within its rounding
+// margin of zero, a comparison inside the FP32 screen's margin or a row too
+// wide for the log's masks ends the block early: the lanes before it are
+// committed, the lane itself is tried alone with the reference's FP64 sum and
+// ln-table expression, and the rest of the block is decided after it.
 //
-// Waits between the two warps poll shared-memory counters (acquire/release)
-// with a time limit on lack of progress; on expiry the kernel raises the
-// device error flag and both warps return.
+// A second warp, the FEEDER, runs ahead of the decider: it fills a ring with
+// the walker's random draws as intervals of their ln-table values and brings
+// each block's chunk of the model (records, in-block terms) into one of four
+// shared-memory buffers by one TMA bulk copy.
+//
+// FP64 models: a third warp, the ACCOUNTANT, consumes a log of the flips in
+// batches of up to 32: every lane recomputes one flip's exact FP64 cost
+// difference (the reference's order and rounding, model/ising.h:108-117,
+// model/pubo.h:335-367), then the running cost is accumulated in flip order
+// exactly as cost_ += diff (markov/walker.h:225) and the lowest state is taken
+// at the first strict improvement (markov/walker.h:269-280) from the
+// accountant's own copy of the spins.  Neither the decisions nor the draws
+// depend on the running cost.  Integer models keep cost and lowest in the
+// decider (exact in any order).
+//
+// What bounds it: the decider's chain of dependent votes, shared-memory loads
+// and integer instructions: 1600 cycles a block on a sparse Ising model (N =
+// 1000, 64 walkers: gather 370, decisions 330, wait and publication 320, commit
+// 160), 4200 on a PUBO of 11.7 terms a variable (gather 1040, decisions 600,
+// commit 1600).  A thousand sweeps of the first take 24.7 ms, where fields kept
+// up to date by atomics took 63; 100 sweeps of 512 tempering walkers of the
+// second 62 ms, where the windowed kernel took 190.  Shared-memory atomics have no
+// place in it: one costs 26 to 44 cycles of its warp's memory queue on this
+// chip (a load 5), so a form that kept the fields up to date by atomics on
+// the co-members took 2300 to 7900 cycles a block, and gathering them anew
+// costs less than a few flips' scatter.
+//
+// Waits between the warps poll shared-memory counters (acquire/release) with a
+// time limit on lack of progress; on expiry the kernel raises the device error
+// flag and all of the walker's warps return.
 #include <algorithm>
+#include <atomic>
 #include <climits>
+#include <cmath>
 
 #include "metropolis.cuh"
 #include "qio_internal.h"
@@ -37,17 +64,57 @@ namespace fc
 {
 using namespace qio::mc;
 static const unsigned kFull = 0xffffffffu;
-static const int kCap = 512;      // tile records (16 B each) per buffer
-static const int kLog = 128;      // flip-log entries per walker (power of 2)
-static const int kCtrl = 64;      // per-walker control block
-static const int kTable = 6208;   // per-block tables (ln row 0, screen row 0, jumps)
-static const unsigned kExactF = 0x80000000u;  // log entry: exact FP64 difference
-static const unsigned kExactI = 0x40000000u;  // log entry: exact integer difference
-static const unsigned long long kTimeoutNs = 4000000000ULL;  // 4 s without progress
+static const int kMaxRows = 64;   // records per lane of a staged block, at most
+static const int kIn = 4;         // in-block entries per lane of a staged block
+static const int kLogBytes = 1024;  // flip log per walker: 64 entries of 16 bytes, pair models 256 of 4
+static const int kRing = 128;     // draw intervals per walker (power of 2)
+static const int kCtrl = 64;      // per-walker control block: mbarriers, counters
+static const int kTable = 4096;   // per block: screen row 0
+static const unsigned kExactF = 0x80000000u;   // log entry: exact FP64 difference
+// record and in-block entry flags (build_fields)
+static const uint32_t kTermMask = 0x0003FFFFu;
+static const uint32_t kShared = 0x00080000u;   // record: another member in the block
+static const uint32_t kBigTerm = 0x00100000u;  // record: more than eight members
+static const uint32_t kBigEntry = 0x40000000u; // in-block entry: the same
+static const unsigned kNoEntry = 0xffffffffu;  // no in-block entry
+static const int kMaxSmem = 227 * 1024;
+static const int kSms = 152;
+static const long long kPatience = 8000000000LL;  // cycles without progress, about 4 s
+
+// the three forms of a field (build_fields)
+enum Form
+{
+  PAIR = 0,     // Ising, terms of one or two members: spins alone
+  COUNTER = 1,  // PUBO, MaxSat: term bytes count true literals
+  PARITY = 2    // Ising with larger terms: term bytes are parities
+};
+
+// A block's chunk of the model's table (build_fields), in 8-byte words: header
+// (4: record rows | in-block entry rows << 8 | further entry rows << 16, first
+// further entry), lane data (32), in-block entries (kIn x 32 of 8 or 16 bytes), record
+// rows (of 32; term models 33, a bank's shift, as one lane's records are read
+// across too)
+template <int FM>
+struct Chunk
+{
+  static const int kLane = 4;
+  static const int kEnt = 36;
+  static const int kRec = 36 + kIn * 32 * (FM == PAIR ? 1 : 2);
+  static const int kPitch = FM == PAIR ? 32 : 33;
+};
+__host__ __device__ inline int chunk_words(bool pair, int rows)
+{
+  return 36 + kIn * 32 * (pair ? 1 : 2) + rows * (pair ? 32 : 33);
+}
+static const int kBufs = 4;  // chunk buffers per walker (a power of two)
 
 __constant__ double c_ln[1024];
-__constant__ float c_scr[3072];
-__constant__ unsigned long long c_jA[65], c_jC[65];
+// screen of the ln-table comparison per (row, bucket): y0, dy, error margin;
+// bucket 1 (log(0), never accepted) holds y0 = +inf
+__device__ float4 g_scr[1024];
+__constant__ ulonglong2 c_jump[33];
+static const unsigned long long kMult = 6364136223846793005ULL;
+static const unsigned long long kInc = 1442695040888963407ULL;
 
 // ---- shared-memory synchronisation between the two warps -----------------
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
@@ -65,15 +132,25 @@ __device__ __forceinline__ void st_release(unsigned* p, unsigned v)
                "r"(v)
                : "memory");
 }
-__device__ __forceinline__ unsigned long long now_ns()
+// A limit on waiting without progress: SM cycles from the first look (the
+// nanosecond timer takes about a thousand cycles to read).
+struct Patience
 {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void pair_sync(int id)
+  long long t0 = 0;
+  __device__ __forceinline__ void renew() { t0 = 0; }
+  __device__ __forceinline__ bool over()
+  {
+    const long long t = clock64();
+    if (t0 == 0) t0 = t;
+    return t - t0 > kPatience;
+  }
+};
+// all warps of a walker (integer models have no accountant)
+template <bool INT>
+__device__ __forceinline__ void walker_sync(int id)
 {
-  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+  if (INT) asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+  else asm volatile("bar.sync %0, 96;" ::"r"(id) : "memory");
 }
 
 // ---- TMA bulk copy of a tile of records, completion on an mbarrier --------
@@ -86,10 +163,9 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar)
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void tile_issue(uint4* dst, const uint4* src, int n, unsigned long long* bar)
+// (the buffer's reader is done: it has published that)
+__device__ __forceinline__ void tile_issue(void* dst, const void* src, unsigned bytes, unsigned long long* bar)
 {
-  const unsigned bytes = (unsigned)(n > 0 ? n : 1) * 16u;
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
   asm volatile(
@@ -115,105 +191,104 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
   return false;
 }
 
-// ---- ln-table comparison ---------------------------------------------------
-// rows 1..3 (redraws, 1 in 256 uphill attempts) stay in constant memory
-__device__ __forceinline__ const double* ln_base(const double* s_ln0, int row)
-{
-  return row ? c_ln : s_ln0;
-}
-__device__ __forceinline__ const float* scr_base(const float* s_scr0, int row)
-{
-  return row ? c_scr : s_scr0;
-}
-// value(r) < thr in FP32 with the screen's margins plus `extra` (the field's
-// own deviation from the exact threshold); 1 accept, 0 reject, -1 undecided
-__device__ __forceinline__ int screen(const float* scr, uint32_t r, int row, float thr_f, float extra)
-{
-  const int b = (int)(r & 255u);
-  if (b == 1) return 0;  // y0 = log(0): NaN, never less
-  const int k = (row * 256 + b) * 3;
-  const float y0 = scr[k], dy = scr[k + 1], ev = scr[k + 2];
-  const float dist = __fmul_rn((float)(r >> 8), 5.96046483e-08f);
-  const float value = __fmaf_rn(dist, dy, y0);
-  const float et = __fmaf_rn(fabsf(thr_f), 1.9073486328125e-06f, 1e-30f) + extra;  // 2^-19
-  if (__fadd_rn(value, ev) < __fsub_rn(thr_f, et)) return 1;
-  if (__fsub_rn(value, ev) > __fadd_rn(thr_f, et)) return 0;
-  return -1;
-}
-
-// the exact ln-table comparison (markov/metropolis.h:96-103), kept out of
-// line: the FP64 instructions stay off the common path
-__device__ __noinline__ bool exact_less(const double* ln, uint32_t r, int row, double dE, double beta)
-{
-  return lut_less_exact(ln, r, row, __dmul_rn(dE, -beta));
-}
-
-// The redraw chain of an uphill attempt whose first replayed draw had
-// bucket 0 (markov/metropolis.h:93-103): draws at positions pos, pos + 1, ...
-// Returns 1 accept / 0 reject, the draws used in *used.
-__device__ __noinline__ int redraw_chain(const unsigned long long* jA, const unsigned long long* jC,
-                                         uint64_t rs, int pos, const double* s_ln0, bool beta_inf,
-                                         double dE, double beta, int* used)
-{
-  int row = -1, b = 0, u = 0;
-  uint32_t cur = 0;
-  bool decided = false;
-  while (b == 0)
-  {
-    if (row < 3)
-    {
-      cur = pcg_out(jA[pos + u] * rs + jC[pos + u]);
-      u++;
-      b = (int)(cur & 255u);
-      row++;
-    }
-    else
-    {
-      decided = true;
-      break;
-    }
-  }
-  *used = u;
-  if (decided) return 1;
-  if (beta_inf) return 0;
-  return lut_less_exact(row ? c_ln : s_ln0, cur, row, __dmul_rn(dE, -beta)) ? 1 : 0;
-}
-
 __device__ __forceinline__ uint32_t spin_of(const uint32_t* spins, int v)
 {
   return (spins[v >> 5] >> (v & 31)) & 1u;
 }
 
+// PCG state after k further draws
+__device__ __noinline__ uint64_t jump_to(uint64_t st, uint32_t k)
+{
+  uint64_t A = kMult, C = kInc;
+  for (; k; k >>= 1)
+  {
+    if (k & 1u) st = A * st + C;
+    C = A * C + C;
+    A = A * A;
+  }
+  return st;
+}
+
+// The redraw chain of an uphill attempt (markov/metropolis.h:93-103) on the
+// stream's next draws.  Returns 1 accept / 0 reject.
+__device__ __noinline__ int draw_chain(uint64_t rs, bool beta_inf, double dE, double beta)
+{
+  int row = -1, b = 0;
+  uint32_t cur = 0;
+  while (b == 0 && row < 3)
+  {
+    cur = pcg_out(rs);
+    rs = rs * kMult + kInc;
+    b = (int)(cur & 255u);
+    row++;
+  }
+  if (b == 0) return 1;  // four zero buckets
+  if (beta_inf) return 0;
+  return lut_less_exact(c_ln, cur, row, __dmul_rn(dE, -beta)) ? 1 : 0;
+}
+
+// the same on the two 64-bit words of a counter stream's attempt
+__device__ __noinline__ int counter_chain(uint64_t key, unsigned long long ctr, bool beta_inf, double dE, double beta)
+{
+  uint64_t w = counter_draw(key, 2ULL * ctr);
+  int row = 0;
+  uint32_t cur = (uint32_t)w;
+  while ((cur & 255u) == 0u && row < 3)
+  {
+    row++;
+    if (row == 2) w = counter_draw(key, 2ULL * ctr + 1ULL);
+    cur = (row & 1) ? (uint32_t)(w >> 32) : (uint32_t)w;
+  }
+  if ((cur & 255u) == 0u) return 1;
+  if (beta_inf) return 0;
+  return lut_less_exact(c_ln, cur, row, __dmul_rn(dE, -beta)) ? 1 : 0;
+}
+
+// Term bytes (COUNTER, PARITY).  A term of up to eight members: bit i set when
+// the literal of its i-th member by variable id is true (Ising: its spin).  A
+// larger term: the count of true literals, or the parity.
+__device__ __forceinline__ bool big_term(const DevModel& m, uint32_t t)
+{
+  return __ldg(m.trow + t + 1) - __ldg(m.trow + t) > 8;
+}
+
 // Exact cost difference of flipping v (FP64 models): the reference's sum
-// over the row in ascending term id, from the current term states.
-template <int FL>
-__device__ __noinline__ double exact_dE(const DevModel& m, int v, uint32_t sv, const uint8_t* z)
+// over the row in ascending term id, from the spins (pair) or the term bytes.
+template <int FM>
+__device__ __noinline__ double exact_dE(const DevModel& m, int v, const uint32_t* spins, const uint8_t* z)
 {
   const int rb = __ldg(m.row + v), re = __ldg(m.row + v + 1);
+  const uint32_t sv = spin_of(spins, v);
   double d = 0.0;
   for (int k = rb; k < re; k++)
   {
-    const uint32_t e = __ldg(m.inc + k);
-    const uint32_t zz = z[e & ~kNegBit];
     const double c = __ldg(m.coef + k);
-    if (FL == F_PARITY) d = __dadd_rn(d, zz ? -c : c);
+    if (FM == PAIR)
+    {
+      const int u = __ldg(m.other + k);
+      const uint32_t par = sv ^ (u >= 0 ? spin_of(spins, u) : 0u);
+      d = __dadd_rn(d, par ? -c : c);
+      continue;
+    }
+    const uint32_t e = __ldg(m.inc + k);
+    uint32_t n = z[e & ~kNegBit];  // true literals, or the parity
+    if (!big_term(m, e & ~kNegBit)) n = (uint32_t)__popc(n);
+    if (FM == PARITY) d = __dadd_rn(d, (n & 1u) ? -c : c);
     else
     {
       const bool lit = ((sv ^ (e >> 31)) & 1u) != 0u;
-      if (lit ? (zz == 1u) : (zz == 0u)) d = lit ? __dadd_rn(d, c) : __dsub_rn(d, c);
+      if (n == (lit ? 1u : 0u)) d = lit ? __dadd_rn(d, c) : __dsub_rn(d, c);
     }
   }
-  return (FL == F_PARITY) ? neg2x(d) : d;
+  return (FM == COUNTER) ? d : neg2x(d);
 }
 
 // Exact cost difference from a log entry's masks (accountant): qm = the
 // contributing incidences, sm = their signs.
-template <int FL>
-__device__ __forceinline__ double dE_from_masks(const DevModel& m, int v, int deg, uint32_t qm,
-                                                uint32_t sm)
+template <int FM>
+__device__ __forceinline__ double dE_from_masks(const double* pc, int deg, uint32_t qm, uint32_t sm)
 {
-  const double* pc = m.coef + __ldg(m.row + v);
-  uint32_t q = (FL == F_PARITY) ? ((deg >= 32) ? kFull : ((1u << deg) - 1u)) : qm;
+  uint32_t q = (FM != COUNTER) ? ((deg >= 32) ? kFull : ((1u << deg) - 1u)) : qm;
   double d = 0.0;
   while (q)
   {
@@ -232,11 +307,11 @@ __device__ __forceinline__ double dE_from_masks(const DevModel& m, int v, int de
       if (k[i] >= 0)
       {
         const bool s = ((sm >> k[i]) & 1u) != 0u;
-        if (FL == F_PARITY) d = __dadd_rn(d, s ? -c[i] : c[i]);
+        if (FM != COUNTER) d = __dadd_rn(d, s ? -c[i] : c[i]);
         else d = s ? __dadd_rn(d, c[i]) : __dsub_rn(d, c[i]);
       }
   }
-  return (FL == F_PARITY) ? neg2x(d) : d;
+  return (FM == COUNTER) ? d : neg2x(d);
 }
 
 __device__ __forceinline__ int warp_scan32(int x, int lane)
@@ -260,46 +335,62 @@ __device__ __forceinline__ long long warp_scan64(long long x, int lane)
   return x;
 }
 
-// Per-walker shared-memory region.
+// Per-walker shared-memory region, sized for the launch's largest model.
+struct Shape
+{
+  int nw;    // spin words of the population
+  int mp;    // term bytes; pair models: a byte per variable
+  int rows;  // record rows of a staged block
+  bool pair;
+};
 struct Region
 {
-  unsigned long long* bars;  // 2 mbarriers
-  unsigned* head;            // log entries published by the decider
+  unsigned long long* bars;  // kBufs mbarriers
+  unsigned* head;            // log entries published by the decider (with `used`, 8 bytes)
   unsigned* tail;            // log entries consumed by the accountant
   unsigned* done;            // the decider finished the walker
-  unsigned* beat;            // decider progress (blocks processed)
-  unsigned* abort;           // a wait gave up: both warps leave
-  uint4* log;                // kLog entries
-  uint4* tiles;              // 2 x kCap records
-  int* G;                    // fields, fc_words(N)
-  uint8_t* z;                // term states, mp bytes
-  uint32_t* spins;           // nw words
-  uint32_t* aspins;          // the accountant's spins, nw words
+  unsigned* abort;           // a wait gave up: all warps leave
+  unsigned* next;            // the walker taken from the queue
+  unsigned* made;            // draws in the ring
+  unsigned* used;            // draws taken by the decider
+  unsigned* blocks;          // blocks the decider has finished (before `head`, `used`)
+  float2* ring;              // kRing screen intervals
+  uint32_t* raw;             // kRing: stream position after the draw (replay)
+  uint4* log;                // kLogBytes (FP64 models)
+  uint2* tiles;              // kBufs block chunks
+  uint8_t* z;                // term bytes; pair models: the spins, a byte each
+  uint32_t* spins;           // nw + 4 words (words of zeros after the last)
+  uint32_t* aspins;          // the accountant's spins (FP64 models), two copies for pair models
 };
 
-__host__ __device__ inline int region_bytes(int n_vars, int nw, int mp)
+__host__ __device__ inline int tile_words(const Shape& s) { return (chunk_words(s.pair, s.rows) + 1) & ~1; }
+__host__ __device__ inline int region_bytes(const Shape& s, bool integer)
 {
-  const int np = ((n_vars + 31) / 32) * 32;
-  return kCtrl + kLog * 16 + 2 * kCap * 16 + np * 4 + mp + 8 * nw;
+  return kCtrl + kRing * 12 + (integer ? 0 : kLogBytes) + kBufs * tile_words(s) * 8 + s.mp + 4 * (s.nw + 4) +
+         (integer ? 0 : 4 * (s.nw + 4) * (s.pair ? 2 : 1));
 }
 
-__device__ __forceinline__ Region carve(unsigned char* base, int n_vars, int nw, int mp)
+template <bool INT>
+__device__ __forceinline__ Region carve(unsigned char* base, const Shape& s)
 {
   Region R;
   R.bars = (unsigned long long*)base;
-  unsigned* c = (unsigned*)(base + 16);
+  unsigned* c = (unsigned*)(base + 32);
   R.head = c;
-  R.tail = c + 1;
-  R.done = c + 2;
-  R.beat = c + 3;
-  R.abort = c + 4;
-  R.log = (uint4*)(base + kCtrl);
-  R.tiles = R.log + kLog;
-  R.G = (int*)(R.tiles + 2 * kCap);
-  const int np = ((n_vars + 31) / 32) * 32;
-  R.z = (uint8_t*)(R.G + np);
-  R.spins = (uint32_t*)(R.z + mp);
-  R.aspins = R.spins + nw;
+  R.used = c + 1;
+  R.tail = c + 2;  // (tail, made: one 8-byte word)
+  R.made = c + 3;
+  R.done = c + 4;
+  R.abort = c + 5;
+  R.next = c + 6;
+  R.blocks = c + 7;
+  R.ring = (float2*)(base + kCtrl);
+  R.raw = (uint32_t*)(R.ring + kRing);
+  R.log = (uint4*)(R.raw + kRing);
+  R.tiles = (uint2*)(R.log + (INT ? 0 : kLogBytes / 16));
+  R.z = (uint8_t*)(R.tiles + kBufs * tile_words(s));
+  R.spins = (uint32_t*)(R.z + s.mp);
+  R.aspins = R.spins + s.nw + 4;
   return R;
 }
 
@@ -309,842 +400,861 @@ __device__ __forceinline__ void raise_abort(const Region& R, int* err)
   st_release(R.abort, 1u);
 }
 
-// Field of variable v from the term states and spins (fresh populations).
-template <int FL>
-__device__ __forceinline__ int field_of(const DevModel& m, int v, const uint8_t* z, const uint32_t* spins)
+// term t's byte from the spins
+template <int FM>
+__device__ __forceinline__ uint8_t term_byte(const DevModel& m, int t, const uint32_t* spins)
 {
-  const int rb = __ldg(m.row + v), re = __ldg(m.row + v + 1);
-  const uint32_t sv = spin_of(spins, v);
-  const int pack = m.fc_pack;
-  int acc = 0;
-  for (int k = rb; k < re; k++)
+  const int b = __ldg(m.trow + t), e = __ldg(m.trow + t + 1);
+  uint32_t mask = 0, n = 0;
+  for (int k = b; k < e; k++)
   {
-    const uint4 rec = __ldg(m.fc_rec + k);
-    const uint32_t zz = z[rec.x & ~kNegBit];
-    const int q = (int)rec.y;
-    if (FL == F_PARITY) acc += zz ? -q : q;
-    else
-    {
-      const uint32_t lit = (sv ^ (rec.x >> 31)) & 1u;
-      if (lit ? (zz == 1u) : (zz == 0u)) acc += (lit ? q : -q) + pack;
-    }
+    const uint32_t x = __ldg(m.tvar + k);
+    const uint32_t lit = spin_of(spins, (int)(x & ~kNegBit)) ^ (x >> 31);
+    n += lit;
+    if (e - b > 8) continue;
+    int at = 0;
+    for (int j = b; j < e; j++) at += (__ldg(m.tvar + j) & ~kNegBit) < (x & ~kNegBit);
+    mask |= lit << at;
   }
-  return acc;
+  if (e - b <= 8) return (uint8_t)mask;
+  return (uint8_t)(FM == PARITY ? n & 1u : n);
 }
 
-// change of co-member w's field when a term's state goes zo -> zn
-template <int FL>
-__device__ __forceinline__ int co_delta(uint32_t cw, uint32_t zo, uint32_t zn, int q, int pack,
-                                        const uint32_t* spins)
+// Mutable state of one walker's decider.
+struct Walk
 {
-  if (FL == F_PARITY) return zo ? 2 * q : -2 * q;  // the term's contribution changes sign
-  const uint32_t litw = (spin_of(spins, (int)(cw & 0x7FFFu)) ^ (cw >> 15)) & 1u;
-  const int qo = litw ? (zo == 1u) : (zo == 0u);
-  const int qn = litw ? (zn == 1u) : (zn == 0u);
-  return (qn - qo) * ((litw ? q : -q) + pack);
-}
-
-// Apply one incidence of a committed flip: the term's state moves, and the
-// fields of the term's other members change by the exact integer amounts.
-// Returns this incidence's bits for the flip's log masks: bit 0 = the
-// incidence contributes to the flip's cost difference, bit 1 = its sign.
-template <int FL>
-__device__ __noinline__ void apply_overflow(const DevModel& m, const Region& R, uint32_t e, uint32_t zo,
-                                            uint32_t zn, int q, int vj, int pack)
-{
-  for (int x = __ldg(m.trow + e); x < __ldg(m.trow + e + 1); x++)
-  {
-    const uint32_t tv = __ldg(m.tvar + x);
-    const uint32_t u = tv & ~kNegBit;
-    if ((int)u == vj) continue;
-    const uint32_t cw = u | ((tv & kNegBit) ? 0x8000u : 0u);
-    const int d = co_delta<FL>(cw, zo, zn, q, pack, R.spins);
-    if (d) atomicAdd(R.G + u, d);
-  }
-}
-
-template <int FL>
-__device__ __forceinline__ unsigned apply_incidence(const DevModel& m, const Region& R, const uint4 rec,
-                                                    uint32_t sv, int vj, int pack)
-{
-  // every shared-memory load before the stores: the term state and the
-  // co-members' spin words
-  const uint32_t e = rec.x & ~kNegBit;
-  const int nco = (int)(rec.w >> 16);
-  const uint32_t cws[3] = {rec.z & 0xFFFFu, rec.z >> 16, rec.w & 0xFFFFu};
-  const uint32_t zo = R.z[e];
-  uint32_t sw[3] = {0u, 0u, 0u};
-  if (FL != F_PARITY)
-  {
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-      if (i < nco) sw[i] = R.spins[(cws[i] & 0x7FFFu) >> 5];
-  }
-  const int q = (int)rec.y;
-  uint32_t zn;
-  unsigned bits;
-  if (FL == F_PARITY)
-  {
-    bits = 1u | (zo ? 2u : 0u);
-    zn = zo ^ 1u;
-  }
-  else
-  {
-    const uint32_t lit = (sv ^ (rec.x >> 31)) & 1u;
-    bits = ((lit ? (zo == 1u) : (zo == 0u)) ? 1u : 0u) | (lit << 1);
-    zn = lit ? zo - 1u : zo + 1u;
-  }
-  int d[3] = {0, 0, 0};
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-    if (i < nco && nco <= 3)
-    {
-      if (FL == F_PARITY) d[i] = zo ? 2 * q : -2 * q;  // the term's contribution changes sign
-      else
-      {
-        const uint32_t litw = ((sw[i] >> (cws[i] & 31u)) ^ (cws[i] >> 15)) & 1u;
-        const int qo = litw ? (zo == 1u) : (zo == 0u);
-        const int qn = litw ? (zn == 1u) : (zn == 0u);
-        d[i] = (qn - qo) * ((litw ? q : -q) + pack);
-      }
-    }
-  R.z[e] = (uint8_t)zn;
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-    if (d[i]) atomicAdd(R.G + (cws[i] & 0x7FFFu), d[i]);
-  // terms of more than three co-members (count 15): after the pass
-  return bits | ((nco > 3) ? 4u : 0u) | (zo << 8) | (zn << 16);
-}
-
-// The co-members of a term with more than three (read from the term lists),
-// for the incidences the pass marked; called by the whole warp after it.
-template <int FL>
-__device__ __noinline__ void apply_overflow_lane(const DevModel& m, const Region& R, bool mine, uint4 rec,
-                                                 unsigned bits, int vj, int pack)
-{
-  if (!mine) return;
-  const uint32_t e = rec.x & ~kNegBit;
-  const uint32_t zo = (bits >> 8) & 255u, zn = (bits >> 16) & 255u;
-  apply_overflow<FL>(m, R, e, zo, zn, (int)rec.y, vj, pack);
-}
-
-// Counter-stream draw of an attempt whose first byte was 0 (rare): the
-// reference's redraw loop over the two 64-bit counter words.  Returns the
-// draw and its ln-table row; *all_zero when every try came up 0.
-__device__ __noinline__ uint32_t counter_redraw(uint64_t key, unsigned long long ctr, uint64_t w0, int* row_out,
-                                               bool* all_zero)
-{
-  int row = -1, b = 0, used = 0;
-  uint32_t cur = 0;
-  *all_zero = false;
-  while (b == 0)
-  {
-    if (row < 3)
-    {
-      if (used == 0) cur = (uint32_t)w0;
-      else if (used == 1) cur = (uint32_t)(w0 >> 32);
-      else
-      {
-        const uint64_t w1 = counter_draw(key, 2ULL * ctr + 1ULL);
-        cur = used == 2 ? (uint32_t)w1 : (uint32_t)(w1 >> 32);
-      }
-      used++;
-      b = (int)(cur & 255u);
-      row++;
-    }
-    else
-    {
-      *all_zero = true;
-      break;
-    }
-  }
-  *row_out = row;
-  return cur;
-}
-
-// One wide flip (a row of more than 32 incidences): the warp over its
-// incidences, 32 at a time.  Its log entry carries the exact difference.
-template <int FL>
-__device__ __noinline__ void apply_wide(const DevModel& m, const Region& R, const uint4* tile, bool staged,
-                                        int b_q0, int rbj, int dj, uint32_t svj, int vj, int pack)
-{
-  const int lane = threadIdx.x & 31;
-  for (int k0 = 0; k0 < dj; k0 += 32)
-  {
-    const int kk = k0 + lane;
-    uint4 rec = make_uint4(0u, 0u, 0u, 0u);
-    unsigned bits = 0;
-    if (kk < dj)
-    {
-      rec = staged ? tile[rbj - b_q0 + kk] : __ldg(m.fc_rec + rbj + kk);
-      bits = apply_incidence<FL>(m, R, rec, svj, vj, pack);
-    }
-    if (bits & 4u)
-      apply_overflow<FL>(m, R, rec.x & ~kNegBit, (bits >> 8) & 255u, (bits >> 16) & 255u, (int)rec.y, vj, pack);
-  }
-}
-
-// One window round in full generality (out of line): exact differences for
-// fields inside their margin, ln-table comparisons inside the screen's
-// margin, counter draws that needed the redraw loop, the replayed redraw
-// chain of a zero bucket.  The fast path hands a round here whenever any
-// of these occurs in it; this function decides the round from scratch.
-struct RoundIo
-{
-  // in (per lane)
-  bool active;
-  int v, cursor, nvalid, bnd, g;
-  uint32_t nb, sv, pd;
-  uint64_t w0;
-  float xmargin;
-  // in (uniform)
-  uint64_t rs, key;
-  unsigned long long ctr0;
-  double beta;
-  bool beta_inf;
-  float nbeta_f, fscale;
-  // out
-  unsigned flips;
-  int draws, adv;
-  bool have_exact;
-  double dE;
-  long long idE;
+  uint64_t rs;          // replay: the stream's state at position raw0
+  uint32_t raw0;
+  uint64_t key;         // counter streams
+  unsigned taken;       // draws taken
+  unsigned long long natt, nacc, nwin;
+  long long icost, ilow;  // integer models
 };
 
-template <int FL, bool REPLAY, bool INT>
-__device__ __noinline__ void general_round(const DevModel& m, const uint8_t* z, const double* s_ln0,
-                                           const float* s_scr0, const unsigned long long* s_jA,
-                                           const unsigned long long* s_jC, RoundIo& io)
+// replay: the stream's state after the draws taken
+__device__ __forceinline__ uint64_t stream_state(const Region& R, const Walk& W)
+{
+  const uint32_t at = W.taken ? R.raw[(W.taken - 1u) & (unsigned)(kRing - 1)] : 0u;
+  return jump_to(W.rs, at - W.raw0);
+}
+
+// ---------------------------------------------------------------------------
+// The feeder.
+//
+// Draws: the ring holds the walker's draws as screen intervals [lo, hi] of
+// their ln-table values, kRing ahead of the decider at most.  Replay: the
+// stream's draws in order; a zero bucket is skipped by the attempt that meets
+// it (markov/metropolis.h:93-103: the next draw counts, one ln-table row
+// further down) and four of them accept, so an entry is what one uphill attempt
+// takes.  Counter streams: the entry of every attempt in turn.  An entry that
+// always accepts is (-inf, -inf).
+//
+// Chunks: block t's goes to buffer t % kBufs once the decider is done with
+// block t - kBufs (t counts over the warp's walkers, from `t0`).
+// ---------------------------------------------------------------------------
+template <int FM, bool REPLAY>
+__device__ __noinline__ void feed(const Region R, const float4* s_scr, const int4* desc, const uint2* table, int tile_w,
+                                  int cap, int nblocks, int total, unsigned t0, uint64_t rs, uint64_t key,
+                                  unsigned long long ctr, int n_vars, int* err)
 {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  const bool active = io.active;
-  const int v = io.v, cursor = io.cursor, bnd = io.bnd, g = io.g;
-  const uint32_t nb = io.nb, sv = io.sv;
-  const double beta = io.beta;
-  const bool beta_inf = io.beta_inf;
-  const float nbeta_f = io.nbeta_f, fscale = io.fscale;
-  bool have_exact = false, uphill = false;
-  double dE = 0.0;
-  long long idE = 0;
-  int F = 0;
-  if (INT)
+  uint64_t st = REPLAY ? c_jump[lane].x * rs + c_jump[lane].y : 0;
+  const uint64_t jA = c_jump[32].x, jC = c_jump[32].y;
+  unsigned made = 0;
+  uint32_t raw = (uint32_t)lane + 1u;  // stream position after this lane's draw
+  int carry = 0;                       // zeros at the end of the last 32 draws that await the next
+  int first = 0;                       // counter: the first variable of the coming attempts
+  int t = 0, tb = 0;                   // chunks issued; the next one's block
+  int4 d = __ldg(desc);                // ... and its descriptor
+  Patience limit;
+  unsigned last_u = 0, last_b = 0;
+  while (true)
   {
-    idE = (FL == F_PARITY) ? -2LL * (long long)g : (long long)g;
-    uphill = active && idE > 0;
-  }
-  else
-  {
-    bool need = false;
-    if (FL == F_PARITY)
+    // what the decider has done
+    const unsigned used = ld_acquire(R.used);
+    const unsigned blocks = *(volatile unsigned*)R.blocks;
+    while (t < total && t < (int)blocks + kBufs)
     {
-      F = g;
-      need = active && F <= bnd && F >= -bnd;
-      uphill = active && F < -bnd;
+      if (lane == 0)
+      {
+        const unsigned at = (t0 + (unsigned)t) % (unsigned)kBufs;
+        tile_issue(R.tiles + at * tile_w, table + d.x, (unsigned)chunk_words(FM == PAIR, min(d.y, cap)) * 8u,
+                   &R.bars[at]);
+      }
+      t++;
+      tb = tb + 1 < nblocks ? tb + 1 : 0;
+      d = __ldg(desc + tb);
+    }
+    if (made + 32u - used >= (unsigned)kRing)
+    {
+      // no room for draws (the last one taken stays: its stream position)
+      int leave = 0;
+      if (ld_acquire(R.done)) leave = 1;
+      else if (ld_acquire(R.abort)) leave = 2;
+      else if (used != last_u || blocks != last_b)
+      {
+        last_u = used;
+        last_b = blocks;
+        limit.renew();
+      }
+      else if (limit.over())
+      {
+        raise_abort(R, err);
+        leave = 2;
+      }
+      leave = __shfl_sync(kFull, leave, 0);
+      if (leave == 0) continue;
+      // given up: the copies in flight land before the region is
+      if (leave == 2 && lane == 0)
+        for (int x = max(0, t - kBufs); x < t; x++)
+        {
+          const unsigned n = t0 + (unsigned)x;
+          mbar_wait(&R.bars[n % (unsigned)kBufs], (n / (unsigned)kBufs) & 1u);
+        }
+      return;
+    }
+    uint32_t pd;
+    int row = 0, n = 32, at = lane;
+    bool put = true, always = false;
+    if (REPLAY)
+    {
+      pd = pcg_out(st);
+      st = jA * st + jC;
+      const bool zero = (pd & 255u) == 0u;
+      const unsigned Z = __ballot_sync(kFull, zero);
+      if (Z || carry)
+      {
+        int run = lane ? __clz(~(Z << (32 - lane))) : 0;  // zeros just before this draw
+        if (run == lane) run += carry;
+        row = run & 3;
+        always = zero && row == 3;
+        put = !zero || always;
+        const unsigned P = __ballot_sync(kFull, put);
+        at = __popc(P & lt);
+        n = __popc(P);
+        carry = __shfl_sync(kFull, zero ? (run + 1) & 3 : 0, 31);
+      }
     }
     else
     {
-      F = g >> 8;
-      if (active && (g & 255) == 0) have_exact = true;  // nothing contributes: +0.0
-      need = active && !have_exact && F <= bnd && F >= -bnd;
-      uphill = active && !have_exact && F > bnd;
+      const unsigned long long c = ctr + (unsigned long long)(first + lane);
+      const uint64_t w = counter_draw(key, 2ULL * c);
+      pd = (uint32_t)w;
+      if ((pd & 255u) == 0u)
+      {
+        row = 1;
+        pd = (uint32_t)(w >> 32);
+        if ((pd & 255u) == 0u)
+        {
+          const uint64_t x = counter_draw(key, 2ULL * c + 1ULL);
+          row = 2;
+          pd = (uint32_t)x;
+          if ((pd & 255u) == 0u)
+          {
+            row = 3;
+            pd = (uint32_t)(x >> 32);
+            always = (pd & 255u) == 0u;
+          }
+        }
+      }
+      first += 32;
+      if (first >= n_vars)
+      {
+        first = 0;
+        ctr += (unsigned long long)n_vars;
+      }
     }
-    if (need)
+    const float4 e = row ? g_scr[row * 256 + (int)(pd & 255u)] : s_scr[pd & 255u];
+    const float val = __fmaf_rn(__fmul_rn((float)(pd >> 8), 5.96046483e-08f), e.y, e.x);
+    if (put)
     {
-      dE = exact_dE<FL>(m, v, sv, z);
-      have_exact = true;
-      uphill = !le_zero(dE);
+      const unsigned i = (made + (unsigned)at) & (unsigned)(kRing - 1);
+      R.ring[i] = always ? make_float2(-INFINITY, -INFINITY) : make_float2(__fsub_rn(val, e.z), __fadd_rn(val, e.z));
+      if (REPLAY) R.raw[i] = raw;
     }
+    raw += 32u;
+    made += (unsigned)n;
+    __syncwarp();
+    if (lane == 0) st_release(R.made, made);
   }
-  bool acc = active && !uphill;
-  const unsigned before = lt & ~((1u << cursor) - 1u);
-  unsigned U = 0;
-  int pos = 0;
-  if (REPLAY)
+}
+
+// Waits until *p (another warp's counter; counters wrap) reaches `want`; the
+// value seen, or want - 1 when the walker is given up (abort raised, or no
+// progress within the time limit).  Lane 0 polls for the warp.
+__device__ __noinline__ unsigned wait_count(const unsigned* p, unsigned want, unsigned* abort, int* err)
+{
+  unsigned seen = want - 1u;
+  if ((threadIdx.x & 31) == 0)
   {
-    U = __ballot_sync(kFull, uphill);
-    pos = __popc(U & before);
-  }
-  auto decide = [&](uint32_t rr, int row) -> int {
-    if (beta_inf) return 0;
-    const float* sc = scr_base(s_scr0, row);
-    if (INT) return screen(sc, rr, row, __fmul_rn((float)idE, nbeta_f), 0.f);
-    if (have_exact) return screen(sc, rr, row, __fmul_rn(approx_float(dE), nbeta_f), 0.f);
-    return screen(sc, rr, row, __fmul_rn((float)F, fscale), io.xmargin);
-  };
-  uint32_t dr = 0;
-  int drow = 0;
-  bool redraw = false;
-  int dec = 1;
-  if (REPLAY)
-  {
-    const uint32_t d0 = __shfl_sync(kFull, io.pd, pos & 31);
-    if (uphill)
+    Patience limit;
+    unsigned last = 0;
+    bool any = false;
+    while (true)
     {
-      dr = d0;
-      redraw = (dr & 255u) == 0;
-      if (!redraw) dec = decide(dr, 0);
+      seen = ld_acquire(p);
+      if ((int)(seen - want) >= 0) break;
+      if (!any || seen != last)
+      {
+        any = true;
+        last = seen;
+        limit.renew();
+      }
+      if (ld_acquire(abort))
+      {
+        seen = want - 1u;
+        break;
+      }
+      if (limit.over())
+      {
+        if (err) atomicExch(err, 1);
+        st_release(abort, 1u);
+        seen = want - 1u;
+        break;
+      }
     }
   }
-  else if (uphill)
-  {
-    const uint32_t cur0 = io.pd;
-    if ((cur0 & 255u) != 0u)
-    {
-      dr = cur0;
-      dec = decide(cur0, 0);
-    }
-    else
-    {
-      bool all_zero;
-      dr = counter_redraw(io.key, io.ctr0 + (unsigned long long)v, io.w0, &drow, &all_zero);
-      dec = all_zero ? 1 : decide(dr, drow);
-    }
-  }
-  const unsigned Rm = REPLAY ? __ballot_sync(kFull, redraw) : 0u;
-  if (!INT && __any_sync(kFull, uphill && !redraw && dec < 0))
-  {
-    // exact differences for the lanes inside the margin that can still be
-    // committed: up to the first stop under the surely accepted lanes (more
-    // acceptances can only move the stop earlier)
-    const bool sure = active && (!uphill || (!redraw && dec == 1));
-    const unsigned As = __ballot_sync(kFull, sure);
-    bool cs = false;
-    if (active && lane > cursor)
-      cs = (nb & (__brev(As) >> (32 - lane)) & ((1u << (lane - cursor)) - 1u)) != 0u;
-    const unsigned stop_s = __ballot_sync(kFull, cs) | Rm;
-    const int fs = stop_s ? (__ffs(stop_s) - 1) : 32;
-    const bool cand = active && lane <= fs && !have_exact && uphill && !redraw && dec < 0;
-    if (cand)
-    {
-      dE = exact_dE<FL>(m, v, sv, z);
-      have_exact = true;
-    }
-    if (lane > fs && dec < 0) dec = 0;  // not committed this round
-  }
-  if (uphill && !redraw && dec < 0)
-    dec = exact_less(ln_base(s_ln0, drow), dr, drow, INT ? (double)idE : dE, beta) ? 1 : 0;
-  if (uphill && !redraw) acc = dec == 1;
-  const unsigned A = __ballot_sync(kFull, acc);
-  bool conf = false;
-  if (active && lane > cursor)
-    conf = (nb & (__brev(A) >> (32 - lane)) & ((1u << (lane - cursor)) - 1u)) != 0u;
-  const unsigned Cm = __ballot_sync(kFull, conf);
-  const unsigned stop = Cm | Rm;
-  int f = stop ? (__ffs(stop) - 1) : 32;
-  if (f > io.nvalid) f = io.nvalid;
-  const bool slow = REPLAY && f < io.nvalid && ((Rm >> f) & 1u) && !((Cm >> f) & 1u);
-  const unsigned commit = ((f >= 32) ? kFull : ((1u << f) - 1u)) & ~((1u << cursor) - 1u);
-  unsigned flips = A & commit;
-  int draws = REPLAY ? __popc(U & commit) : 0;
-  if (REPLAY && slow)
-  {
-    // lane f drew a zero bucket: its redraw chain (markov/metropolis.h:93-103)
-    if (!INT && lane == f && !have_exact)
-    {
-      dE = exact_dE<FL>(m, v, sv, z);
-      have_exact = true;
-    }
-    int sacc = 0, used = 0;
-    if (lane == f)
-      sacc = redraw_chain(s_jA, s_jC, io.rs, pos, s_ln0, beta_inf, INT ? (double)idE : dE, beta, &used);
-    sacc = __shfl_sync(kFull, sacc, f);
-    used = __shfl_sync(kFull, used, f);
-    if (sacc) flips |= 1u << f;
-    draws += used;
-  }
-  io.flips = flips;
-  io.draws = draws;
-  io.adv = f + (slow ? 1 : 0) - cursor;
-  io.have_exact = have_exact;
-  io.dE = dE;
-  io.idE = idE;
+  return __shfl_sync(kFull, seen, 0);
 }
 
 // ---------------------------------------------------------------------------
 // The decider: one walker's sweeps.  Returns false when a wait gave up.
-// Committed flips are logged at head + i and published to the accountant at
-// the end of each 32-variable block (a block logs at most 32 flips; the log
-// is checked for room for them when the block starts).
 //
-// A window round, common path: every lane turns the draw at stream position
-// `lane` into the screen interval [lo, hi] of the ln-table value; each
-// uphill lane takes the interval of its position (the uphill lanes before it)
-// and compares it with its threshold field * fscale +- margin.  Inside the
-// margin, the exact FP64 difference and comparison are taken (rare).  Flips
-// are applied in lane segments of 8, 16 or 32 per flip.
+// What it keeps per sweep and per block, in the order of use.  A block's
+// counters (flips logged, draws taken) are published, and the other warps'
+// looked at, where no global load is outstanding: a shared-memory release or
+// acquire waits for those (336 cycles measured against 30).
 // ---------------------------------------------------------------------------
-template <int FL, bool REPLAY, bool INT>
-__device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const Region R, const double* s_ln0, const float* s_scr0,
-                              const unsigned long long* s_jA, const unsigned long long* s_jC, int r,
-                              unsigned& phases, uint64_t& rs, unsigned long long& natt,
-                              unsigned long long& nacc, unsigned long long& nwin)
+struct Sweep
 {
-  const DevModel& m = a.m;
+  double beta, beta_next;
+  const double* betas;
+  bool beta_inf;
+  float nbeta_f, fscale, fsa;
+  unsigned long long ctr0;
+};
+
+// the constants of the sweep that starts, and the next one's beta
+template <int FM, bool INT>
+__device__ __forceinline__ void next_sweep(Sweep& S, const SweepArgs& a, double inv, int N, int k)
+{
+  const long long swp = a.sweep_base + k;
+  S.beta = S.beta_next;
+  S.beta_inf = ((unsigned long long)__double_as_longlong(S.beta) & 0x7FFFFFFFFFFFFFFFULL) == 0x7FF0000000000000ULL;
+  // thr = field * fscale approximates dE * (-beta); an infinite beta accepts
+  // nothing uphill: thr = -3e38 with no margin, from a zero scale
+  S.nbeta_f = S.beta_inf ? 0.f : -approx_float(S.beta);
+  S.fscale = INT ? S.nbeta_f : (S.beta_inf ? 0.f : (float)(S.beta * inv * (FM == COUNTER ? -1.0 : 2.0)));
+  S.fsa = INT ? 0.f : fabsf(S.fscale) * 1.0001f;
+  S.ctr0 = (unsigned long long)swp * (unsigned long long)N;
+  if (k + 1 < a.n_sweeps) S.beta_next = S.betas[(swp + 1) * a.bs_s];
+}
+
+// publishes the blocks finished, the flips logged and the draws taken (head,
+// used: one 8-byte word)
+__device__ __forceinline__ void publish(const Region& R, unsigned blocks, unsigned head, unsigned taken)
+{
+  *(volatile unsigned*)R.blocks = blocks;
+  const unsigned long long x = (unsigned long long)head | ((unsigned long long)taken << 32);
+  asm volatile("st.release.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(R.head)), "l"(x) : "memory");
+}
+
+// the other warps' counters: flips accounted, draws in the ring
+__device__ __forceinline__ void look(const Region& R, unsigned& tail, unsigned& made)
+{
+  unsigned long long x;
+  asm volatile("ld.acquire.cta.shared::cta.b64 %0, [%1];" : "=l"(x) : "r"(smem_u32(R.tail)) : "memory");
+  tail = __shfl_sync(kFull, (unsigned)x, 0);
+  made = __shfl_sync(kFull, (unsigned)(x >> 32), 0);
+}
+
+// waits for room for 32 flips in the log and 32 draws in the ring
+template <bool INT, int LOG>
+__device__ __noinline__ void wait_room(unsigned* tail, unsigned* made, unsigned* abort, int* err, unsigned head,
+                                      unsigned taken)
+{
+  if (!INT) wait_count(tail, head + 32u - (unsigned)LOG, abort, err);
+  wait_count(made, taken + 32u, abort, err);
+}
+
+// Running cost and first lowest of integer models over a round's flips F
+// (this lane's difference g), in lane order; `word`: the block's spins after.
+__device__ __forceinline__ void account_int(const Region& R, Walk& W, bool scan32, int g, unsigned F, int bi,
+                                            int nblocks, uint32_t* g_lsp)
+{
+  const int lane = threadIdx.x & 31;
+  const bool mine = ((F >> lane) & 1u) != 0u;
+  const int de = mine ? g : 0;
+  int low = -1;
+  if (scan32)
+  {
+    const int sum = __reduce_add_sync(kFull, de);
+    const int neg = __reduce_add_sync(kFull, min(de, 0));
+    if ((long long)neg < W.ilow - W.icost)  // the lowest prefix is at least icost + neg
+    {
+      const int pre = warp_scan32(de, lane);
+      const int mn = __reduce_min_sync(kFull, mine ? pre : INT_MAX);
+      if ((long long)mn < W.ilow - W.icost)
+      {
+        low = __ffs(__ballot_sync(kFull, mine && pre == mn)) - 1;
+        W.ilow = W.icost + mn;
+      }
+    }
+    W.icost += sum;
+  }
+  else
+  {
+    const long long pre = warp_scan64((long long)de, lane);
+    const long long ci = W.icost + pre;
+    long long mn = mine ? ci : LLONG_MAX;
+#pragma unroll
+    for (int s = 16; s; s >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, s));
+    if (mn < W.ilow)
+    {
+      low = __ffs(__ballot_sync(kFull, mine && ci == mn)) - 1;
+      W.ilow = mn;
+    }
+    W.icost += __shfl_sync(kFull, pre, 31);
+  }
+  if (low >= 0)
+  {
+    // the state at the improvement: the round's later flips undone
+    const unsigned undo = F & ~((2u << low) - 1u);
+    for (int q = lane; q < nblocks; q += 32) g_lsp[q] = R.spins[q] ^ (q == bi ? undo : 0u);
+  }
+}
+
+// a flip's change of a term that it shares within the block (x: in-block entry)
+template <int FM>
+__device__ __forceinline__ void flip_shared(uint8_t* z, unsigned x, uint32_t sv)
+{
+  const unsigned t = x & kTermMask, sh = (t & 3u) * 8u;
+  unsigned* word = (unsigned*)(z + (t & ~3u));
+  if (!(x & kBigEntry)) atomicXor(word, 1u << (sh + ((x >> 23) & 7u)));
+  else if (FM == PARITY) atomicXor(word, 1u << sh);
+  else if ((sv ^ (x >> 31)) & 1u) atomicSub(word, 1u << sh);
+  else atomicAdd(word, 1u << sh);
+}
+
+// Lane f's attempt alone: the reference's sum, draws and comparison.  Bit 0:
+// accepted; bit 1: it drew.
+template <int FM, bool REPLAY, bool INT>
+__device__ __noinline__ unsigned exact_attempt(const DevModel& m, int v, int g, const uint32_t* spins, const uint8_t* z,
+                                              uint64_t rs, uint64_t key, unsigned long long ctr, double beta,
+                                              double* dE_out)
+{
+  const double dE = INT ? (double)g : exact_dE<FM>(m, v, spins, z);
+  const bool inf = ((unsigned long long)__double_as_longlong(beta) & 0x7FFFFFFFFFFFFFFFULL) == 0x7FF0000000000000ULL;
+  *dE_out = dE;
+  if (le_zero(dE)) return 1u;
+  if (REPLAY) return 2u | (unsigned)draw_chain(rs, inf, dE, beta);
+  return 2u | (unsigned)counter_chain(key, ctr, inf, dE, beta);
+}
+
+template <int FM, bool REPLAY, bool INT>
+__device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel& m, const Region R, const Shape& sh, int r,
+                                              unsigned t0, Walk& W, uint32_t* g_lsp)
+{
+  constexpr int KI = kIn;  // in-block entries held in registers
+  constexpr int kLog = FM == PAIR ? kLogBytes / 4 : kLogBytes / 16;  // entries, a power of two
+  using C = Chunk<FM>;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const int N = m.n_vars;
-  const int pack = m.fc_pack;
-  uint64_t key = 0;
-  if (!REPLAY)
-    key = counter_key(a.seed + (uint32_t)(r / a.key_div), a.key_base + (unsigned long long)(r % a.key_div));
   const int nblocks = (N + 31) >> 5;
   const int total = nblocks * a.n_sweeps;
-  unsigned head = 0;       // entries written (published at block ends)
-  unsigned tail_seen = 0;  // lane 0: the accountant's count last seen
-  // per-lane row data of the next block (prefetched a block ahead)
-  auto row_data = [&](int blk, int& rb, int& deg, uint32_t& nb) {
-    const int v = (blk << 5) + lane;
-    rb = 0;
-    deg = 0;
-    nb = 0;
-    if (v < N)
-    {
-      rb = __ldg(m.row + v);
-      deg = __ldg(m.row + v + 1) - rb;
-      nb = __ldg(m.nbr + v);
-    }
-  };
-  int n_rb, n_deg;
-  uint32_t n_nb;
-  row_data(0, n_rb, n_deg, n_nb);
-  // lane 0: record range of the tile in flight (tq) and of the next one (nq),
-  // loaded a block ahead of its copy
-  int tq0 = 0, tq1 = 0, nq0 = 0, nq1 = 0;
-  auto range_of = [&](int blk, int& q0, int& q1) {
-    q0 = __ldg(m.row + (blk << 5));
-    q1 = __ldg(m.row + min((blk << 5) + 32, N));
-  };
-  if (total > 0 && lane == 0)
+  if (total <= 0) return true;
+  const bool scan32 = m.scan32 != 0;
+  const bool big = m.fc_big != 0;
+  const double inv = m.fc_inv;
+  // (read once: `m` may be the launch's parameter or lie in device memory)
+  const uint2* table = m.fc_tab;
+  const int4* descs = m.fc_desc;
+  const void* further = m.fc_in;
+  const int tile_w = tile_words(sh), cap = sh.rows;
+
+  unsigned head = 0;                // log entries written
+  unsigned acc_tail = 0, fed = 0;   // the other warps' counters when last looked at
+  Sweep S;
+  S.betas = a.beta + (long long)r * a.bs_w;
+  S.beta_next = S.betas[a.sweep_base * a.bs_s];
+
+  int k = 0, bi = -1;  // sweep and block of gb
+  for (int gb = 0; gb < total; gb++)
   {
-    range_of(0, tq0, tq1);
-    tile_issue(R.tiles, m.fc_rec + tq0, min(tq1 - tq0, kCap), &R.bars[0]);
-    if (total > 1) range_of(nblocks > 1 ? 1 : 0, nq0, nq1);
-  }
-  double beta = 0.0;
-  bool beta_inf = false;
-  float nbeta_f = 0.f, fscale = 0.f, fsa = 0.f;
-  unsigned long long ctr0 = 0;
-  // the sweep's beta, loaded a block ahead of its first use
-  const double* betas = a.beta + (long long)r * a.bs_w;
-  double beta_next = total > 0 ? betas[a.sweep_base * a.bs_s] : 0.0;
-  int k = 0, bi = 0;                              // sweep and block of gb
-  int bi2 = nblocks > 2 ? 2 : (nblocks == 2 ? 0 : 0);  // block of gb + 2
-  for (int gb = 0; gb < total; gb++, bi++)
-  {
+    bi++;
     if (bi == nblocks)
     {
       bi = 0;
       k++;
     }
-    const int buf = gb & 1;
-    if (bi == 0)
+    if (bi == 0) next_sweep<FM, INT>(S, a, inv, N, k);
+    const int nvalid = min(32, N - (bi << 5));
+    const int v = (bi << 5) + lane;
+    // this block's chunk
+    const unsigned turn = t0 + (unsigned)gb, buf = turn % (unsigned)kBufs, par = (turn / (unsigned)kBufs) & 1u;
+    if (!__all_sync(kFull, mbar_try(&R.bars[buf], par)))
     {
-      const long long swp = a.sweep_base + k;
-      beta = beta_next;
-      beta_inf = ((unsigned long long)__double_as_longlong(beta) & 0x7FFFFFFFFFFFFFFFULL) ==
-                 0x7FF0000000000000ULL;
-      nbeta_f = -approx_float(beta);
-      // thr = field * fscale approximates dE * (-beta)
-      fscale = INT ? 0.f : (float)(beta * m.fc_inv * (FL == F_PARITY ? 2.0 : -1.0));
-      fsa = fabsf(fscale) * 1.0001f;
-      ctr0 = (unsigned long long)swp * (unsigned long long)N;
-    }
-    if (bi == nblocks - 1 && gb + 1 < total) beta_next = betas[(a.sweep_base + k + 1) * a.bs_s];
-    const int i0 = bi << 5;
-    // this block's record range, then the next block's tile into the other buffer
-    const int b_q0 = __shfl_sync(kFull, tq0, 0);
-    const int b_q1 = __shfl_sync(kFull, tq1, 0);
-    if (gb + 1 < total && lane == 0)
-    {
-      tq0 = nq0;
-      tq1 = nq1;
-      tile_issue(R.tiles + (buf ^ 1) * kCap, m.fc_rec + tq0, min(tq1 - tq0, kCap), &R.bars[buf ^ 1]);
-      if (gb + 2 < total) range_of(bi2, nq0, nq1);
-    }
-    bi2 = (bi2 + 1 == nblocks) ? 0 : bi2 + 1;
-    const int rb = n_rb, deg = n_deg;
-    const uint32_t nb = n_nb;
-    if (gb + 1 < total) row_data((bi + 1 < nblocks) ? bi + 1 : 0, n_rb, n_deg, n_nb);
-    // room in the log for this block's flips
-    bool ok = true;
-    if (lane == 0 && head + 32u - tail_seen > (unsigned)kLog)
-    {
-      unsigned long long t0 = 0;
-      unsigned last = tail_seen;
-      while (true)
+      const bool landed = mbar_wait(&R.bars[buf], par);
+      if (!__all_sync(kFull, landed))
       {
-        tail_seen = ld_acquire(R.tail);
-        if (head + 32u - tail_seen <= (unsigned)kLog) break;
-        if (tail_seen != last)
-        {
-          last = tail_seen;
-          t0 = 0;
-        }
-        if (ld_acquire(R.abort))
-        {
-          ok = false;
-          break;
-        }
-        const unsigned long long t = now_ns();
-        if (t0 == 0) t0 = t;
-        else if (t - t0 > kTimeoutNs)
-        {
-          raise_abort(R, a.err);
-          ok = false;
-          break;
-        }
-        __nanosleep(64);
+        raise_abort(R, a.err);
+        return false;
       }
     }
-    const bool tile_ok = mbar_wait(&R.bars[buf], (phases >> buf) & 1u);
-    phases ^= 1u << buf;
-    if (!__all_sync(kFull, ok && tile_ok))
-    {
-      if (lane == 0)
-      {
-        if (!tile_ok) raise_abort(R, a.err);
-        // the copy in flight lands before the walker's region is given up
-        if (gb + 1 < total)
-        {
-          mbar_wait(&R.bars[buf ^ 1], (phases >> (buf ^ 1)) & 1u);
-          phases ^= 1u << (buf ^ 1);
-        }
-      }
-      __syncwarp();
-      return false;
-    }
-    const bool staged = b_q1 - b_q0 <= kCap;
-    const uint4* tile = R.tiles + buf * kCap;
+    const uint2* chunk = R.tiles + buf * tile_w;
+    // the header through shuffles, so that what depends on it is known not to
+    // divide the warp: rows, entry rows and further entry rows
+    const uint2 head0 = *chunk;
+    const unsigned sizes = __shfl_sync(kFull, head0.x, 0);
+    const int rows = (int)(sizes & 255u), ents = (int)((sizes >> 8) & 255u), xn = (int)(sizes >> 16);
+    const uint2* tile = chunk + lane;
+    const int2 own = *(const int2*)(tile + C::kLane);
+    const uint4* tent = (const uint4*)(chunk + C::kEnt) + lane;
 
-    const int v = i0 + lane;
-    const bool valid = v < N;
-    const int nvalid = min(32, N - i0);
-    uint32_t sv = valid ? spin_of(R.spins, v) : 0u;
+    const uint32_t word = R.spins[bi];  // the block's spins before its flips
+    const uint32_t sv = (word >> lane) & 1u;
+    const int deg = own.y;
     const int bnd = deg + 1;  // |field - exact| < bnd units
-    const float xmargin = INT ? 0.f : fsa * (float)(bnd + 1);
-    const unsigned head0 = head;
-    unsigned b_att = 0, b_acc = 0, b_win = 0;
+    const float xmargin = INT ? 0.f : S.fsa * (float)(bnd + 1);
 
-    // the draws of the first round (replay: stream positions 0..31)
-    uint32_t pd = 0;
-    uint64_t w0 = 0;
-    float plo = 0.f, phi = 0.f;
-    unsigned Zm = 0;
-    auto draws_for = [&](int cur) {
-      if (REPLAY) pd = pcg_out(s_jA[lane] * rs + s_jC[lane]);
-      else
-      {
-        w0 = counter_draw(key, 2ULL * (ctr0 + (unsigned long long)(i0 + lane)));
-        pd = (uint32_t)w0;
-      }
-      const int pb = (int)(pd & 255u);
-      const float* e = s_scr0 + pb * 3;
-      const float val = __fmaf_rn(__fmul_rn((float)(pd >> 8), 5.96046483e-08f), e[1], e[0]);
-      plo = pb == 1 ? INFINITY : __fsub_rn(val, e[2]);
-      phi = pb == 1 ? INFINITY : __fadd_rn(val, e[2]);
-      Zm = __ballot_sync(kFull, pb == 0);
-      (void)cur;
+    // ---- the field; term models: the row's contributing incidences (qm)
+    int base = FM == PAIR ? own.x : 0;
+    unsigned qm = 0;
+    // one record of a term model: true when the other literals are all false
+    // (COUNTER), or the parity of the other members is odd
+    auto term = [&](const uint32_t x) -> bool {
+      const uint32_t zz = R.z[x & kTermMask];
+      if (big && (x & kBigTerm))
+        return FM == COUNTER ? zz == ((sv ^ (x >> 18)) & 1u) : ((zz ^ sv) & 1u) != 0u;
+      return FM == COUNTER ? (zz & (x >> 24)) == 0u : (__popc(zz & (x >> 24)) & 1) != 0;
     };
-    if (!REPLAY) draws_for(0);  // counter draws: fixed for the block
-
-    int cursor = 0;
-    while (cursor < nvalid)
-    {
-      if (REPLAY) draws_for(0);
-      const bool active = valid && lane >= cursor;
-      const unsigned before = lt & ~((1u << cursor) - 1u);
-      const int g = active ? R.G[v] : 0;
-      // ---- fast path: the field's sign and the screened comparison
-      bool up, rare;
-      float thr, xm;
-      if (INT)
+    // a flipped variable's unshared term: its byte after
+    auto put = [&](uint32_t x, uint32_t zz, uint32_t spin) {
+      uint32_t zn = zz ^ (~(x >> 24) & 255u);
+      if (big && (x & kBigTerm)) zn = FM == PARITY ? zz ^ 1u : (((spin ^ (x >> 18)) & 1u) ? zz - 1u : zz + 1u);
+      if (!(x & kShared)) R.z[x & kTermMask] = (uint8_t)zn;
+    };
+    // (rows come in fours; the next four's records are under way meanwhile)
+    auto gather = [&](const uint2* t0) {
+      unsigned bit = 1u;
+      uint2 e[4];
+#pragma unroll
+      for (int x = 0; x < 4; x++) e[x] = rows ? t0[C::kPitch * x] : make_uint2(0u, 0u);
+      for (int i = 4; i <= rows; i += 4)
       {
-        const long long idE = (FL == F_PARITY) ? -2LL * (long long)g : (long long)g;
-        up = active && idE > 0;
-        thr = __fmul_rn((float)idE, nbeta_f);
-        xm = 0.f;
-        rare = false;
-      }
-      else if (FL == F_PARITY)
-      {
-        up = active && g < -bnd;
-        rare = active && g <= bnd && g >= -bnd;
-        thr = __fmul_rn((float)g, fscale);
-        xm = xmargin;
-      }
-      else
-      {
-        const int F = g >> 8;
-        const bool zero = (g & 255) == 0;  // nothing contributes: +0.0
-        up = active && !zero && F > bnd;
-        rare = active && !zero && F <= bnd && F >= -bnd;
-        thr = __fmul_rn((float)F, fscale);
-        xm = xmargin;
-      }
-      unsigned U = 0;
-      float lo = plo, hi = phi;
-      bool rd = false;
-      if (REPLAY)
-      {
-        U = __ballot_sync(kFull, up);
-        const int pos = __popc(U & before);
-        lo = __shfl_sync(kFull, plo, pos);
-        hi = __shfl_sync(kFull, phi, pos);
-        rd = up && ((Zm >> pos) & 1u);
-      }
-      else
-        rare = rare || (up && (pd & 255u) == 0u);
-      const float et = __fmaf_rn(fabsf(thr), 1.9073486328125e-06f, 1e-30f) + xm;  // 2^-19
-      const bool acc_u = up && !rd && !beta_inf && hi < __fsub_rn(thr, et);
-      const bool rej_u = up && !rd && (beta_inf || lo > __fadd_rn(thr, et));
-      rare = rare || (up && !rd && !acc_u && !rej_u);
-      const unsigned A = __ballot_sync(kFull, active && (!up || acc_u));
-      const unsigned Rm = __ballot_sync(kFull, rd);
-      bool conf = false;
-      if (active && lane > cursor)
-        conf = (nb & (__brev(A) >> (32 - lane)) & ((1u << (lane - cursor)) - 1u)) != 0u;
-      const unsigned Cm = __ballot_sync(kFull, conf);
-      const unsigned stop = Cm | Rm;
-      int f = stop ? (__ffs(stop) - 1) : 32;
-      if (f > nvalid) f = nvalid;
-      const unsigned commit = ((f >= 32) ? kFull : ((1u << f) - 1u)) & ~((1u << cursor) - 1u);
-      unsigned flips = A & commit;
-      int draws = REPLAY ? __popc(U & commit) : 0;
-      int adv = f - cursor;
-      bool have_exact = false;
-      double dE = 0.0;
-      long long idE = (FL == F_PARITY) ? -2LL * (long long)g : (long long)g;
-      if (!INT && FL == F_COUNTER && active && (g & 255) == 0) have_exact = true;  // dE = +0.0
-      // the general round: a field inside its margin, a comparison inside
-      // the screen's margin, a counter redraw, or a replayed zero bucket at
-      // the stop
-      const bool slow = REPLAY && f < nvalid && ((Rm >> f) & 1u) && !((Cm >> f) & 1u);
-      const bool any_rare = __any_sync(kFull, rare);
-      if (!any_rare && slow)
-      {
-        // lane f drew a zero bucket: its redraw chain (markov/metropolis.h:93-103)
-        int sacc = 0, used = 0;
-        if (lane == f)
+        uint2 f[4];
+        const uint2* t1 = t0 + C::kPitch * (i < rows ? i : 0);
+#pragma unroll
+        for (int x = 0; x < 4; x++) f[x] = t1[C::kPitch * x];
+        if (FM == PAIR)
         {
-          double d = 0.0;
-          if (!INT) d = exact_dE<FL>(m, v, sv, R.z);
-          const int pos = __popc(U & before);
-          sacc = redraw_chain(s_jA, s_jC, rs, pos, s_ln0, beta_inf, INT ? (double)idE : d, beta, &used);
-          have_exact = !INT;
-          dE = d;
-        }
-        sacc = __shfl_sync(kFull, sacc, f);
-        used = __shfl_sync(kFull, used, f);
-        if (sacc) flips |= 1u << f;
-        draws += used;
-        adv += 1;
-      }
-      if (any_rare)
-      {
-        RoundIo io;
-        io.active = active;
-        io.v = v;
-        io.cursor = cursor;
-        io.nvalid = nvalid;
-        io.bnd = bnd;
-        io.g = g;
-        io.nb = nb;
-        io.sv = sv;
-        io.pd = pd;
-        io.w0 = w0;
-        io.xmargin = xmargin;
-        io.rs = rs;
-        io.key = key;
-        io.ctr0 = ctr0;
-        io.beta = beta;
-        io.beta_inf = beta_inf;
-        io.nbeta_f = nbeta_f;
-        io.fscale = fscale;
-        general_round<FL, REPLAY, INT>(m, R.z, s_ln0, s_scr0, s_jA, s_jC, io);
-        flips = io.flips;
-        draws = io.draws;
-        adv = io.adv;
-        have_exact = io.have_exact;
-        dE = io.dE;
-        idE = io.idE;
-      }
-      const bool mine = ((flips >> lane) & 1u) != 0u;
-      const int nfl = __popc(flips);
-      // the next round's draws, ahead of the apply (independent of it)
-      if (REPLAY) rs = s_jA[draws] * rs + s_jC[draws];
-
-      if (nfl)
-      {
-        // a wide row keeps no masks: its exact difference is taken now,
-        // before the flips change the term states
-        const bool wide = mine && deg > 32;
-        if (!INT && __any_sync(kFull, wide && !have_exact))
-          if (wide && !have_exact)
-          {
-            dE = exact_dE<FL>(m, v, sv, R.z);
-            have_exact = true;
-          }
-        const int fi = __popc(flips & lt);  // this flip's index among the round's
-        // the log entry: x = v | deg << 16 | kind, y/z = masks or the difference
-        uint4 ent;
-        ent.x = (unsigned)v | ((unsigned)deg << 16);
-        ent.y = 0u;
-        ent.z = 0u;
-        ent.w = 0u;
-        if (INT)
-        {
-          ent.x |= kExactI;
-          ent.y = (unsigned)(unsigned long long)idE;
-          ent.z = (unsigned)((unsigned long long)idE >> 32);
-        }
-        else if (have_exact)
-        {
-          ent.x |= kExactF;
-          const unsigned long long bits = (unsigned long long)__double_as_longlong(dE);
-          ent.y = (unsigned)bits;
-          ent.z = (unsigned)(bits >> 32);
-        }
-        const int maxdeg = (int)__reduce_max_sync(kFull, (unsigned)(mine ? deg : 0));
-        if (maxdeg <= 32)
-        {
-          // segments of sg lanes, one flip each, pp flips per pass
-          const int lsg = maxdeg <= 8 ? 3 : (maxdeg <= 16 ? 4 : 5);
-          const int sg = 1 << lsg;
-          const int pp = 32 >> lsg;
-          const int grp = lane >> lsg;
-          const int kk = lane & (sg - 1);
-          unsigned qm = 0, sm = 0;
-          unsigned fw = flips;  // flips not yet applied
-          for (int p0 = 0; p0 < nfl; p0 += pp)
-          {
-            // the lanes of the pass's first pp flips: successive lowest bits
-            const int q0 = __ffs(fw) - 1;
-            const unsigned f1 = fw & (fw - 1);
-            const int q1 = f1 ? __ffs(f1) - 1 : q0;
-            const unsigned f2 = f1 & (f1 - 1);
-            const int q2 = f2 ? __ffs(f2) - 1 : q0;
-            const unsigned f3 = f2 & (f2 - 1);
-            const int q3 = f3 ? __ffs(f3) - 1 : q0;
-            const int j = grp == 0 ? q0 : (grp == 1 ? q1 : (grp == 2 ? q2 : q3));
-            const bool live = p0 + grp < nfl;
-            fw = (pp == 1) ? f1 : ((pp == 2) ? f2 : (f3 & (f3 - 1)));
-            const int dj = __shfl_sync(kFull, deg, j);
-            const int rbj = __shfl_sync(kFull, rb, j);
-            const uint32_t svj = __shfl_sync(kFull, sv, j);
-            unsigned bits = 0;
-            const bool act = live && kk < dj;
-            uint4 rec = make_uint4(0u, 0u, 0u, 0u);
-            if (act)
-            {
-              rec = staged ? tile[rbj - b_q0 + kk] : __ldg(m.fc_rec + rbj + kk);
-              bits = apply_incidence<FL>(m, R, rec, svj, i0 + j, pack);
-            }
-            if (__any_sync(kFull, bits & 4u))
-              apply_overflow_lane<FL>(m, R, (bits & 4u) != 0u, rec, bits, i0 + j, pack);
-            if (!INT)
-            {
-              const unsigned Bq = __ballot_sync(kFull, bits & 1u);
-              const unsigned Bs = __ballot_sync(kFull, (bits >> 1) & 1u);
-              if (mine && fi >= p0 && fi < p0 + pp)
-              {
-                const int sh = (fi - p0) << lsg;
-                const unsigned w = (sg == 32) ? kFull : ((1u << sg) - 1u);
-                qm = (Bq >> sh) & w;
-                sm = (Bs >> sh) & w;
-              }
-            }
-          }
-          if (mine && !INT && !have_exact)
-          {
-            ent.y = (FL == F_PARITY) ? 0u : qm;
-            ent.z = sm;
-          }
+#pragma unroll
+          for (int x = 0; x < 4; x++) base -= (int)R.z[e[x].x] * (int)e[x].y;
         }
         else
         {
-          // a wide flip among them (rare): one flip at a time
-          unsigned fl = flips;
-          while (fl)
+          bool t[4];
+#pragma unroll
+          for (int x = 0; x < 4; x++) t[x] = term(e[x].x);
+#pragma unroll
+          for (int x = 0; x < 4; x++)
           {
-            const int j = __ffs(fl) - 1;
-            fl &= fl - 1;
-            const int dj = __shfl_sync(kFull, deg, j);
-            const int rbj = __shfl_sync(kFull, rb, j);
-            const uint32_t svj = __shfl_sync(kFull, sv, j);
-            unsigned bits = 0;
-            if (dj <= 32)
-            {
-              uint4 rec = make_uint4(0u, 0u, 0u, 0u);
-              if (lane < dj)
-              {
-                rec = staged ? tile[rbj - b_q0 + lane] : __ldg(m.fc_rec + rbj + lane);
-                bits = apply_incidence<FL>(m, R, rec, svj, i0 + j, pack);
-              }
-              if (__any_sync(kFull, bits & 4u))
-                apply_overflow_lane<FL>(m, R, (bits & 4u) != 0u, rec, bits, i0 + j, pack);
-            }
-            else
-              apply_wide<FL>(m, R, tile, staged, b_q0, rbj, dj, svj, i0 + j, pack);
-            if (!INT)
-            {
-              const unsigned Bq = __ballot_sync(kFull, bits & 1u);
-              const unsigned Bs = __ballot_sync(kFull, (bits >> 1) & 1u);
-              if (lane == j && !have_exact)
-              {
-                ent.y = (FL == F_PARITY) ? 0u : Bq;
-                ent.z = Bs;
-              }
-            }
+            if (FM == COUNTER) base += t[x] ? (int)e[x].y : 0;
+            else base += t[x] ? -(int)e[x].y : (int)e[x].y;
+            if (!INT && t[x]) qm |= bit << x;
+          }
+          bit <<= 4;
+        }
+#pragma unroll
+        for (int x = 0; x < 4; x++) e[x] = f[x];
+      }
+    };
+    if (rows <= cap) gather(tile + C::kRec);
+    else gather(table + __ldg(descs + bi).x + C::kRec + lane);
+    if (!INT && FM != PAIR) qm &= deg >= 32 ? kFull : ((1u << deg) - 1u);  // (padding records)
+
+    // ---- the in-block terms under a given accept mask, all against the state
+    // at the block's start.  Pair models: the member's flip changes the field
+    // by c0.  Counter models: the other literals are all false when those of
+    // the members before this lane (em) are -- the flipped ones are exactly the
+    // true ones (et) -- and those after it or elsewhere were (else em = 0, et =
+    // 1: never).  Parities: c0 of the others, and of the flips in em.
+    unsigned watch = 0;  // lanes whose flips change this lane's field
+    int val[KI];
+    unsigned em[KI], et[KI];
+    unsigned elog[KI];  // term, position in the row (5 bits), position in the term (3), big
+    // further entries (rare): xn of them, in HBM
+    const size_t xat = xn ? (size_t)__shfl_sync(kFull, head0.y, 0) + lane : 0;
+    const uint2* xpair = (const uint2*)further + xat;
+    const uint4* xterm = (const uint4*)further + xat;
+    unsigned done = 0;  // the block's flips so far
+    // an entry's em and et; D: flips whose bytes are written already
+    auto entry = [&](const uint4& e, unsigned D, unsigned& mm, unsigned& mt) {
+      const uint32_t zz = R.z[e.x & kTermMask];
+      const int n = (e.x & kBigEntry) ? (int)zz : __popc(zz);
+      const uint32_t M = e.y & lt, L = (word ^ e.z) & M;  // members before this lane, their true literals
+      // the other true literals, as of the block's start
+      const int o = n - (int)(sv ^ (e.x >> 31)) - (__popc(M & D) - 2 * __popc(L & D));
+      mm = M;
+      mt = FM == COUNTER ? L : (unsigned)o & 1u;
+      if (FM == COUNTER && o != __popc(L))
+      {
+        mm = 0u;
+        mt = 1u;
+      }
+    };
+    auto holds = [&](unsigned A, unsigned mm, unsigned mt) -> bool {
+      return FM == COUNTER ? (A & mm) == mt : ((mt ^ (unsigned)__popc(A & mm)) & 1u) != 0u;
+    };
+#pragma unroll
+    for (int i = 0; i < KI; i++)
+    {
+      if (FM == PAIR)
+      {
+        const uint2 e = tile[C::kEnt + 32 * i];
+        em[i] = e.x;
+        val[i] = (word & e.x) ? (int)e.y : -(int)e.y;
+        watch |= e.x;
+      }
+      else
+      {
+        const uint4 e = tent[32 * i];
+        entry(e, 0u, em[i], et[i]);
+        val[i] = (int)e.w;
+        elog[i] = e.x;
+        watch |= e.y & lt;
+        if (e.y == 0u) elog[i] = kNoEntry;
+      }
+    }
+    for (int i = 0; i < xn; i++) watch |= FM == PAIR ? __ldg(xpair + 32 * i).x : (__ldg(&xterm[32 * i].y) & lt);
+
+    // ---- the other warps: room for this block's flips and draws
+    auto room = [&]() -> bool {
+      return (INT || (int)(head + 32u - (unsigned)kLog - acc_tail) <= 0) && (int)(fed - (W.taken + 32u)) >= 0;
+    };
+    if (!room())
+    {
+      look(R, acc_tail, fed);
+      if (!room())
+      {
+        wait_room<INT, kLog>(R.tail, R.made, R.abort, a.err, head, W.taken);
+        look(R, acc_tail, fed);
+        if (!room()) return false;
+      }
+    }
+    const uint32_t negs = (uint32_t)own.x;  // term models: the row's negated literals
+
+    // ---- rounds: one, unless a lane has to be tried alone
+    float2 iv0 = make_float2(0.f, 0.f);
+    if (!REPLAY) iv0 = R.ring[(W.taken + (unsigned)lane) & (unsigned)(kRing - 1)];
+    int cursor = 0;
+    while (true)
+    {
+      const bool active = lane >= cursor && lane < nvalid;
+      const unsigned before = lt & ~((1u << cursor) - 1u);
+      // ---- decisions: iterate until no lane's in-block members change
+      unsigned A = done, U = 0;
+      int g = 0;
+      bool rare = false;
+      while (true)
+      {
+        int h = base;
+#pragma unroll
+        for (int i = 0; i < KI; i++)
+        {
+          if (FM == PAIR) h += (A & em[i]) ? val[i] : 0;
+          else if (FM == COUNTER) h += holds(A, em[i], et[i]) ? val[i] : 0;
+          else h += holds(A, em[i], et[i]) ? -val[i] : val[i];
+        }
+        for (int i = 0; i < xn; i++)
+        {
+          if (FM == PAIR)
+          {
+            const uint2 e = __ldg(xpair + 32 * i);
+            h += (A & e.x) ? ((word & e.x) ? (int)e.y : -(int)e.y) : 0;
+          }
+          else
+          {
+            const uint4 e = __ldg(xterm + 32 * i);
+            unsigned mm, mt;
+            entry(e, done, mm, mt);
+            const bool on = holds(A, mm, mt);
+            if (FM == COUNTER) h += on ? (int)e.w : 0;
+            else h += on ? -(int)e.w : (int)e.w;
           }
         }
-        __syncwarp();
-        if (mine)
+        // the field in the variable's own direction, its sign and threshold
+        bool up;
+        float x;
+        if (INT)
         {
-          R.log[(head + (unsigned)fi) & (unsigned)(kLog - 1)] = ent;
-          // the flipped variable's own field changes sign (the same terms
-          // contribute, with the other sign); the count stays
-          const int gv = R.G[v];
-          R.G[v] = pack ? (-gv + 2 * (gv & 255)) : -gv;
-          sv ^= 1u;
+          g = FM == COUNTER ? (sv ? h : -h) : (sv ? 2 * h : -2 * h);  // the cost difference
+          up = active && g > 0;
+          x = (float)g;
+          rare = false;
         }
-        if (lane == 0) R.spins[i0 >> 5] ^= flips;
-        __syncwarp();
-        head += (unsigned)nfl;
+        else if (FM == COUNTER)
+        {
+          const int fd = sv ? (h >> 8) : -(h >> 8);
+          const bool zero = (h & 255) == 0;  // nothing contributes: +0.0
+          up = active && !zero && fd > bnd;
+          rare = active && !zero && (unsigned)(fd + bnd) <= (unsigned)(2 * bnd);
+          x = (float)fd;
+        }
+        else
+        {
+          g = sv ? -h : h;
+          up = active && g < -bnd;
+          rare = active && (unsigned)(g + bnd) <= (unsigned)(2 * bnd);
+          x = (float)g;
+        }
+        // (an infinite beta: below every draw but an always accepting one)
+        const float thr = S.beta_inf ? -3e38f : __fmul_rn(x, S.fscale);
+        const float et = S.beta_inf ? 0.f : __fmaf_rn(fabsf(thr), 1.9073486328125e-06f, 1e-30f) + xmargin;  // 2^-19
+        float2 iv = iv0;
+        if (REPLAY)
+        {
+          U = __ballot_sync(kFull, up);
+          iv = R.ring[(W.taken + (unsigned)__popc(U & before)) & (unsigned)(kRing - 1)];
+        }
+        const bool yes = iv.y < __fsub_rn(thr, et);
+        const bool no = iv.x > __fadd_rn(thr, et);
+        rare = rare || (up && !yes && !no);
+        const bool acc = active && !rare && (!up || yes);
+        if (!INT && FM != PAIR) rare = rare || (acc && deg > 32);  // its masks do not fit the log
+        const unsigned An = __ballot_sync(kFull, acc) | done;
+        const unsigned diff = An ^ A;
+        A = An;
+        if (!__any_sync(kFull, (diff & watch) != 0u)) break;
       }
-      b_att += (unsigned)adv;
-      b_acc += (unsigned)nfl;
-      b_win++;
-      cursor += adv;
-    }
-    natt += b_att;
-    nacc += b_acc;
-    nwin += b_win;
-    // publish the block's flips
-    if (head != head0)
-    {
-      __threadfence_block();
+
+      // ---- what is committed: all, or the lanes before the first rare one, or
+      // that one alone
+      const unsigned Rm = __ballot_sync(kFull, rare);
+      unsigned F = A & ~done;
+      bool exact = false, last = true;
+      double dE = 0.0;
+      if (Rm == 0u)
+      {
+        if (REPLAY) W.taken += (unsigned)__popc(U);
+      }
+      else
+      {
+        const int f = __ffs(Rm) - 1;
+        if (f > cursor)
+        {
+          F &= (1u << f) - 1u;
+          if (REPLAY) W.taken += (unsigned)__popc(U & ((1u << f) - 1u));
+          cursor = f;
+        }
+        else
+        {
+          const uint64_t rs = REPLAY ? stream_state(R, W) : 0;
+          unsigned res = 0;
+          if (lane == f)
+            res = exact_attempt<FM, REPLAY, INT>(m, v, g, R.spins, R.z, rs, W.key, S.ctr0 + (unsigned long long)v,
+                                                 S.beta, &dE);
+          res = __shfl_sync(kFull, res, f);
+          exact = true;
+          F = (res & 1u) << f;
+          if (REPLAY) W.taken += res >> 1;
+          cursor = f + 1;
+        }
+        last = cursor >= nvalid;
+      }
+      const bool mine = ((F >> lane) & 1u) != 0u;
+      const unsigned at = (head + (unsigned)__popc(F & lt)) & (unsigned)(kLog - 1);
+      const unsigned all = done | F;
+      if (FM == PAIR)
+      {
+        if (!INT && mine) ((uint32_t*)R.log)[at] = (uint32_t)v;
+        if (mine) R.z[v] = (uint8_t)(sv ^ 1u);
+      }
+      else if (F)
+      {
+        // ---- the flips' log masks and term bytes.  In-block terms: their bits
+        // under the final mask (an exact attempt's entry has no masks).
+        unsigned lm = qm;
+        auto log_bit = [&](unsigned x, bool on) {
+          if (x == kNoEntry) return;
+          const uint32_t bit = 1u << ((x >> 18) & 31u);
+          lm = on ? lm | bit : lm & ~bit;
+        };
+        if (!INT)
+        {
+#pragma unroll
+          for (int i = 0; i < KI; i++) log_bit(elog[i], holds(A, em[i], et[i]));
+          for (int i = 0; i < xn && !exact; i++)
+          {
+            const uint4 e = __ldg(xterm + 32 * i);
+            unsigned mm, mt;
+            entry(e, done, mm, mt);
+            if (e.y) log_bit(e.x, holds(A, mm, mt));
+          }
+          __syncwarp();  // the bytes have been read
+        }
+        // Terms of one member in the block: plain stores, the byte is this
+        // block's alone.  The warp over the flips' records, sixteen lanes to a
+        // flip, eight flips' loads under way at a time.
+        auto flips = [&](const uint2* t0) {
+          const int half = lane >> 4, sub = lane & 15;
+          unsigned fl = F;
+          while (fl)
+          {
+            uint32_t x[4], zz[4];
+            int jj[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+            {
+              const int j0 = fl ? __ffs(fl) - 1 : -1;
+              fl &= fl - 1u;
+              const int j1 = fl ? __ffs(fl) - 1 : -1;
+              fl &= fl - 1u;
+              jj[i] = half ? j1 : j0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[i] = jj[i] >= 0 && sub < rows ? t0[C::kPitch * sub + (jj[i] - lane)].x : kShared;
+#pragma unroll
+            for (int i = 0; i < 4; i++) zz[i] = R.z[x[i] & kTermMask];
+#pragma unroll
+            for (int i = 0; i < 4; i++) put(x[i], zz[i], (word >> (jj[i] & 31)) & 1u);
+            for (int at = 16 + sub; at < rows; at += 16)
+            {
+#pragma unroll
+              for (int i = 0; i < 4; i++) x[i] = jj[i] >= 0 ? t0[C::kPitch * at + (jj[i] - lane)].x : kShared;
+#pragma unroll
+              for (int i = 0; i < 4; i++) zz[i] = R.z[x[i] & kTermMask];
+#pragma unroll
+              for (int i = 0; i < 4; i++) put(x[i], zz[i], (word >> (jj[i] & 31)) & 1u);
+            }
+          }
+        };
+        if (rows <= cap) flips(tile + C::kRec);
+        else flips(table + __ldg(descs + bi).x + C::kRec + lane);
+        // Terms of several: every flip changes its own bit (or the count by
+        // one), in any order.
+#pragma unroll
+        for (int i = 0; i < KI; i++)
+          if (i < ents && mine && elog[i] != kNoEntry) flip_shared<FM>(R.z, elog[i], sv);
+        for (int i = 0; i < xn; i++)
+        {
+          const uint4 e = __ldg(xterm + 32 * i);
+          if (mine && e.y) flip_shared<FM>(R.z, e.x, sv);
+        }
+        if (!INT && mine)
+        {
+          uint4 ent;
+          ent.x = (unsigned)v | ((unsigned)deg << 16) | (exact ? kExactF : 0u);
+          const unsigned long long bits = (unsigned long long)__double_as_longlong(dE);
+          // COUNTER: the sign is the literal; PARITY: the term's bit, the
+          // other members' parity and the own spin
+          ent.y = exact ? (unsigned)bits : lm;
+          ent.z = exact ? (unsigned)(bits >> 32) : (FM == COUNTER ? (sv ? ~negs : negs) : (sv ? ~lm : lm));
+          ent.w = 0u;
+          R.log[at] = ent;
+        }
+      }
       __syncwarp();
+      R.spins[bi] = word ^ all;  // (every lane the same word)
+      __syncwarp();
+      if (INT && F) account_int(R, W, scan32, g, F, bi, nblocks, g_lsp);
+      const unsigned nfl = (unsigned)__popc(F);
+      head += nfl;
+      W.nacc += nfl;
+      W.nwin++;
+      done = all;
+      if (last) break;
     }
-    if (lane == 0)
+    if (!REPLAY) W.taken += 32u;
+    W.natt += (unsigned)nvalid;
+    publish(R, (unsigned)gb + 1u, head, W.taken);
+    if (REPLAY && (gb & 0xFFFF) == 0xFFFF)
     {
-      if (head != head0) st_release(R.head, head);
-      st_release(R.beat, (unsigned)gb + 1u);
+      // stream positions are 32-bit: move their origin along
+      W.rs = stream_state(R, W);
+      W.raw0 = W.taken ? R.raw[(W.taken - 1u) & (unsigned)(kRing - 1)] : 0u;
     }
   }
   return true;
 }
 
-// ---------------------------------------------------------------------------
-// The accountant: running cost, lowest cost and lowest state from the log.
-// ---------------------------------------------------------------------------
-template <int FL, bool INT>
-__device__ __forceinline__ bool account(const SweepArgs& a, const Region R, double& cost, double& low, long long& icost,
-                        long long& ilow, uint32_t* g_lsp)
+// The running cost over n flips (lane i < n: the i-th difference d) without a
+// chain of FP64 adds, each 64 cycles of its scheduler's FP64 unit.  While the
+// cost stays inside one binade it is a whole number C of its last place u, and
+// fl(cost + d) = (C + rint(d / u)) u unless d / u lies halfway between whole
+// numbers (then the sum's parity decides): so the rounded steps are a prefix
+// sum of integers.  Every prefix has to stay strictly between 2^52 and 2^53 in
+// magnitude, where the sum before rounding lies in the binade too.  False
+// (nothing changed): a tie, a step out of the binade, or a cost or difference
+// that is zero, subnormal or not finite -- the caller adds one by one.
+__device__ __forceinline__ bool cost_prefix(double d, int n, double& cost, long long& klow, double& low, int& lowpos)
 {
-  const DevModel& m = a.m;
+  const int lane = threadIdx.x & 31;
+  const unsigned long long cb = (unsigned long long)__double_as_longlong(cost);
+  const int ce = (int)((cb >> 52) & 0x7FFu);
+  const unsigned long long kOne = 1ULL << 52;
+  const long long cm = (long long)((cb & (kOne - 1)) | kOne);
+  const long long C = (long long)cb < 0 ? -cm : cm;
+  const unsigned long long db = (unsigned long long)__double_as_longlong(d);
+  const int de = (int)((db >> 52) & 0x7FFu);
+  const unsigned long long dm = (db & (kOne - 1)) | kOne;
+  const int sh = ce - de;
+  bool ok = ce != 0 && ce != 0x7FF;
+  long long D = 0;
+  if (lane < n && (db << 1) != 0ULL)
+  {
+    ok = ok && de != 0 && de != 0x7FF && sh >= 0;  // (|D| < 2^53: no sum overflows)
+    if (ok && sh <= 53)
+    {
+      if (sh > 0)
+      {
+        const unsigned long long rem = dm & ((1ULL << sh) - 1ULL), half = 1ULL << (sh - 1);
+        ok = rem != half;
+        D = (long long)((dm >> sh) + (rem > half ? 1ULL : 0ULL));
+      }
+      else D = (long long)dm;
+      if ((long long)db < 0) D = -D;
+    }
+  }
+  const long long P = C + warp_scan64(D, lane);
+  const long long mag = C < 0 ? -P : P;
+  ok = ok && mag > (long long)kOne && mag < (long long)(kOne << 1);
+  if (!__all_sync(kFull, ok)) return false;
+  long long mn = P;  // (lanes past n repeat the last prefix)
+#pragma unroll
+  for (int s = 16; s; s >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, s));
+  auto value = [&](long long x) -> double {
+    const unsigned long long a = (unsigned long long)(x < 0 ? -x : x) & (kOne - 1);
+    return __longlong_as_double((long long)(((x < 0 ? 1ULL : 0ULL) << 63) | ((unsigned long long)ce << 52) | a));
+  };
+  const double vmin = value(mn);
+  const long long km = order_key(vmin);
+  if (km < klow)
+  {
+    klow = km;
+    low = vmin;
+    lowpos = __ffs(__ballot_sync(kFull, P == mn)) - 1;
+  }
+  cost = value(__shfl_sync(kFull, P, 31));
+  return true;
+}
+
+// ---------------------------------------------------------------------------
+// The accountant (FP64 models): running cost, lowest cost and lowest state
+// from the log.
+// ---------------------------------------------------------------------------
+template <int FM>
+__device__ __noinline__ bool account(const SweepArgs& a, const DevModel& m, const Region R, double& cost,
+                                        double& low, uint32_t* g_lsp)
+{
+  constexpr int kLog = FM == PAIR ? kLogBytes / 4 : kLogBytes / 16;
   const int lane = threadIdx.x & 31;
   const int nw = a.p.nw;
+  const int* row = m.row;
+  const double* coef = m.coef;
+  const int* other = m.other;
   unsigned tail = 0;
   long long klow = order_key(low);
   while (true)
@@ -1154,8 +1264,8 @@ __device__ __forceinline__ bool account(const SweepArgs& a, const Region R, doub
     int fin = 0;
     if (lane == 0)
     {
-      unsigned long long t0 = 0;
-      unsigned last_h = tail, last_b = ld_acquire(R.beat);
+      Patience limit;
+      unsigned last_h = tail, last_u = ld_acquire(R.used);
       while (true)
       {
         h = ld_acquire(R.head);
@@ -1171,22 +1281,20 @@ __device__ __forceinline__ bool account(const SweepArgs& a, const Region R, doub
           fin = 2;
           break;
         }
-        const unsigned b = ld_acquire(R.beat);
-        if (h != last_h || b != last_b)
+        const unsigned u = ld_acquire(R.used);
+        if (h != last_h || u != last_u)
         {
           last_h = h;
-          last_b = b;
-          t0 = 0;
+          last_u = u;
+          limit.renew();
         }
-        const unsigned long long t = now_ns();
-        if (t0 == 0) t0 = t;
-        else if (t - t0 > kTimeoutNs)
+        if (limit.over())
         {
           raise_abort(R, a.err);
           fin = 2;
           break;
         }
-        __nanosleep(128);
+        __nanosleep(20);
       }
     }
     h = __shfl_sync(kFull, h, 0);
@@ -1194,19 +1302,56 @@ __device__ __forceinline__ bool account(const SweepArgs& a, const Region R, doub
     if (fin == 2) return false;
     while (h != tail)
     {
-      const int n = (int)min(32u, h - tail);
+      int n = (int)min(32u, h - tail);
       int v = 0;
       double d = 0.0;
-      long long id = 0;
-      if (lane < n)
+      if (FM == PAIR)
+      {
+        // Flips of one sweep, in index order: a neighbour below the flip has
+        // its spin after the batch, one above it its spin before.
+        uint32_t* after = R.aspins + nw + 4;
+        if (lane < n) v = (int)((const uint32_t*)R.log)[(tail + (unsigned)lane) & (unsigned)(kLog - 1)];
+        const int prev = __shfl_up_sync(kFull, v, 1);
+        const unsigned wrap = __ballot_sync(kFull, lane > 0 && lane < n && v <= prev);
+        if (wrap) n = __ffs(wrap) - 1;
+        if (lane < n) atomicXor(after + (v >> 5), 1u << (v & 31));
+        __syncwarp();
+        if (lane < n)
+        {
+          const uint32_t sv = spin_of(R.aspins, v);
+          const int q1 = __ldg(row + v + 1);
+          for (int q = __ldg(row + v); q < q1; q += 8)
+          {
+            // eight loads in flight ahead of the dependent adds
+            double c[8];
+            int u[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+            {
+              u[i] = q + i < q1 ? __ldg(other + q + i) : -1;
+              c[i] = q + i < q1 ? __ldg(coef + q + i) : 0.0;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+            {
+              const uint32_t su = u[i] < 0 ? 0u : spin_of(u[i] < v ? after : R.aspins, u[i]);
+              if (sv ^ su) c[i] = -c[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+              if (q + i < q1) d = __dadd_rn(d, c[i]);
+          }
+          d = neg2x(d);
+        }
+      }
+      else if (lane < n)
       {
         const uint4 ent = R.log[(tail + (unsigned)lane) & (unsigned)(kLog - 1)];
         v = (int)(ent.x & 0x7FFFu);
         const int deg = (int)((ent.x >> 16) & 255u);
-        const unsigned long long bits = (unsigned long long)ent.y | ((unsigned long long)ent.z << 32);
-        if (INT) id = (long long)bits;
-        else if (ent.x & kExactF) d = __longlong_as_double((long long)bits);
-        else d = dE_from_masks<FL>(m, v, deg, ent.y, ent.z);
+        if (ent.x & kExactF)
+          d = __longlong_as_double((long long)((unsigned long long)ent.y | ((unsigned long long)ent.z << 32)));
+        else d = dE_from_masks<FM>(coef + __ldg(row + v), deg, ent.y, ent.z);
       }
       __syncwarp();
       tail += (unsigned)n;
@@ -1214,21 +1359,7 @@ __device__ __forceinline__ bool account(const SweepArgs& a, const Region R, doub
       // running cost in flip order (markov/walker.h:225) and the first
       // strict improvement of the lowest (markov/walker.h:269-280)
       int lowpos = -1;
-      if (INT)
-      {
-        const long long pre = warp_scan64(lane < n ? id : 0LL, lane);
-        const long long ci = icost + pre;
-        long long mn = lane < n ? ci : LLONG_MAX;
-#pragma unroll
-        for (int s = 16; s; s >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, s));
-        if (mn < ilow)
-        {
-          lowpos = __ffs(__ballot_sync(kFull, lane < n && ci == mn)) - 1;
-          ilow = mn;
-        }
-        icost += __shfl_sync(kFull, pre, 31);
-      }
-      else
+      if (!cost_prefix(d, n, cost, klow, low, lowpos))
       {
         double dn = __shfl_sync(kFull, d, 0);
         for (int i = 0; i < n; i++)
@@ -1260,178 +1391,266 @@ __device__ __forceinline__ bool account(const SweepArgs& a, const Region R, doub
   }
 }
 
-template <int FL, bool REPLAY, bool INT>
-__global__ void __launch_bounds__(256, 1) fc_sweep_kernel(SweepArgs a, int wpc)
+// copy n 16-byte words, four in flight per thread
+__device__ __noinline__ void copy16(uint4* dst, const uint4* src, int n, int t, int nt)
+{
+  int q = t;
+  for (; q + 3 * nt < n; q += 4 * nt)
+  {
+    const uint4 x0 = src[q], x1 = src[q + nt], x2 = src[q + 2 * nt], x3 = src[q + 3 * nt];
+    dst[q] = x0;
+    dst[q + nt] = x1;
+    dst[q + 2 * nt] = x2;
+    dst[q + 3 * nt] = x3;
+  }
+  for (; q < n; q += nt) dst[q] = src[q];
+}
+
+// A walker's warps: decider, feeder and, for FP64 models, accountant (warp w of
+// the block: role w / wpc of walker slot w % wpc, so that a block's deciders
+// lie on different schedulers).  Walker slot s of block b takes stream s *
+// gridDim + b: neighbouring streams (tempering: the hottest, which come first)
+// lie on different SMs.
+template <int FM, bool REPLAY, bool INT>
+__global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __grid_constant__ SweepArgs a, int wpc,
+                                                                     Shape sh)
 {
   extern __shared__ __align__(128) unsigned char smem[];
-  double* s_ln0 = (double*)smem;                                  // 2048 B
-  float* s_scr0 = (float*)(smem + 2048);                          // 3072 B
-  unsigned long long* s_jA = (unsigned long long*)(smem + 5120);  // 520 B
-  unsigned long long* s_jC = s_jA + 65;                            // 520 B
-  for (int t = threadIdx.x; t < 256; t += blockDim.x) s_ln0[t] = c_ln[t];
-  for (int t = threadIdx.x; t < 768; t += blockDim.x) s_scr0[t] = c_scr[t];
-  for (int t = threadIdx.x; t < 65; t += blockDim.x)
-  {
-    s_jA[t] = c_jA[t];
-    s_jC[t] = c_jC[t];
-  }
+  float4* s_scr = (float4*)smem;
+  for (int t = threadIdx.x; t < 256; t += blockDim.x) s_scr[t] = g_scr[t];
   __syncthreads();
 
+  constexpr int kRoles = INT ? 2 : 3;
   const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  const bool decider = wib < wpc;
-  const int ws = decider ? wib : wib - wpc;  // walker slot in the block
-  const int ws0 = blockIdx.x * wpc + ws;
-  if (ws0 >= a.n_streams) return;
-  const int w = a.order ? a.order[ws0] : ws0;
-  const DevModel& m = a.m;
-  const int N = m.n_vars;
-  const int nw = a.p.nw, mp = a.p.mp;
-  const int np = ((N + 31) / 32) * 32;
-  unsigned char* base = smem + kTable + (size_t)ws * region_bytes(N, nw, mp);
-  const Region R = carve(base, N, nw, mp);
+  // the warp's index through a shuffle: the compiler then knows that the roles
+  // below do not divide a warp, and puts no convergence check around every
+  // vote and shuffle (those took more than half of the decider's time)
+  const int wib = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
+  const int role = wib / wpc;  // 0 decider, 1 feeder, 2 accountant
+  const int ws = wib - role * wpc;
+  const bool decider = role == 0;
+  const int ws0 = ws * (int)gridDim.x + (int)blockIdx.x;
+  const bool queued = a.queue != nullptr;
+  if (!queued && ws0 >= a.n_streams) return;
+  const int w = queued ? 0 : (a.order ? a.order[ws0] : ws0);
+  unsigned char* base = smem + kTable + (size_t)ws * region_bytes(sh, INT);
+  const Region R = carve<INT>(base, sh);
   const int bar_id = 1 + ws;
-  if (decider && lane == 0)
-  {
-    mbar_init(&R.bars[0]);
-    mbar_init(&R.bars[1]);
-  }
-  uint64_t rs = (REPLAY && decider) ? a.rng[w] : 0;
-  unsigned phases = 0u;  // mbarrier phase bits of the two tile buffers, kept across walkers
+  const int me = role * 32 + lane, nme = kRoles * 32;  // thread of the walker
+  // (the feeder's own barriers; the first walker_sync below shows them to the decider)
+  if (role == 1 && lane == 0)
+    for (int i = 0; i < kBufs; i++) mbar_init(&R.bars[i]);
+  uint64_t rs = (REPLAY && !queued) ? a.rng[w] : 0;
+  unsigned t0 = 0;  // chunks of the walkers before this one
 
-  for (int r = w; r < a.n_walkers; r += a.n_streams)
+  int r = w;
+  while (true)
   {
+    if (queued)
+    {
+      if (decider && lane == 0) *R.next = (unsigned)atomicAdd(a.queue, 1);
+      walker_sync<INT>(bar_id);
+      r = __shfl_sync(kFull, (int)*(volatile unsigned*)R.next, 0);
+    }
+    if (r >= a.n_walkers) break;
+    const DevModel& m = queued ? a.models[a.model_of[r]] : a.m;
+    const int N = m.n_vars;
     const int slot = a.slot_of ? a.slot_of[r] : r;
-    uint32_t* g_spins = a.p.spins + (size_t)slot * nw;
-    uint8_t* g_ts = a.p.tstate + (size_t)slot * mp;
-    int* g_field = a.field + (size_t)slot * np;
-    if (decider)
+    uint32_t* g_spins = a.p.spins + (size_t)slot * a.p.nw;
+    uint8_t* g_ts = a.p.tstate + (size_t)slot * a.p.mp;
+    const int zwords = FM == PAIR ? 0 : (m.n_terms + 15) >> 4;  // 16-byte words
+    if (queued && REPLAY) rs = a.rng[r];
+    if (decider && lane == 0)
     {
-      if (lane == 0)
-      {
-        *R.head = 0u;
-        *R.tail = 0u;
-        *R.done = 0u;
-        *R.beat = 0u;
-        *R.abort = 0u;
-      }
-      for (int q = lane; q < mp / 4; q += 32) ((uint32_t*)R.z)[q] = ((const uint32_t*)g_ts)[q];
-      for (int q = lane; q < nw; q += 32) R.spins[q] = g_spins[q];
-      if (a.field_valid)
-        for (int q = lane; q < np / 4; q += 32) ((int4*)R.G)[q] = ((const int4*)g_field)[q];
+      *R.head = 0u;
+      *R.tail = 0u;
+      *R.done = 0u;
+      *R.abort = 0u;
+      *R.made = 0u;
+      *R.used = 0u;
+      *R.blocks = 0u;
     }
-    pair_sync(bar_id);
-    if (!a.field_valid)
+    copy16((uint4*)R.spins, (const uint4*)g_spins, a.p.nw >> 2, me, nme);
+    if (me < 4) R.spins[a.p.nw + me] = 0u;
+    if (!INT) copy16((uint4*)R.aspins, (const uint4*)g_spins, a.p.nw >> 2, me, nme);
+    if (!INT && FM == PAIR) copy16((uint4*)(R.aspins + a.p.nw + 4), (const uint4*)g_spins, a.p.nw >> 2, me, nme);
+    // term bytes: as the last launch left them, or from the spins
+    if (FM != PAIR && a.terms_valid) copy16((uint4*)R.z, (const uint4*)g_ts, zwords, me, nme);
+    walker_sync<INT>(bar_id);
+    if (FM != PAIR && !a.terms_valid)
     {
-      // fields from the state: both warps
-      for (int v = (decider ? 0 : 32) + lane; v < N; v += 64) R.G[v] = field_of<FL>(m, v, R.z, R.spins);
+      for (int t = me; t < m.n_terms; t += nme) R.z[t] = term_byte<FM>(m, t, R.spins);
+      walker_sync<INT>(bar_id);
     }
-    if (!decider)
-      for (int q = lane; q < nw; q += 32) R.aspins[q] = R.spins[q];
-    pair_sync(bar_id);
+    if (FM == PAIR)
+    {
+      for (int v = me; v < ((N + 31) & ~31); v += nme) R.z[v] = (uint8_t)spin_of(R.spins, v);
+      walker_sync<INT>(bar_id);
+    }
 
-    bool ok;
+    uint64_t key = 0;
+    if (!REPLAY)
+    {
+      const long long lr = queued ? a.local_of[r] : r;
+      key = counter_key(a.seed + (uint32_t)(lr / a.key_div), a.key_base + (unsigned long long)(lr % a.key_div));
+    }
+    uint32_t* g_lsp = a.p.lspins + (size_t)r * a.p.nw;
     if (decider)
     {
-      unsigned long long natt = 0, nacc = 0, nwin = 0;
-      ok = decide_sweeps<FL, REPLAY, INT>(a, R, s_ln0, s_scr0, s_jA, s_jC, r, phases, rs, natt, nacc,
-                                          nwin);
-      if (lane == 0) st_release(R.done, 1u);
-      pair_sync(bar_id);
-      if (ok && !*(volatile unsigned*)R.abort)
+      Walk W;
+      W.natt = W.nacc = W.nwin = 0;
+      W.icost = W.ilow = 0;
+      W.rs = rs;
+      W.raw0 = 0;
+      W.key = key;
+      W.taken = 0;
+      if (INT)
       {
-        for (int q = lane; q < mp / 4; q += 32) ((uint32_t*)g_ts)[q] = ((const uint32_t*)R.z)[q];
-        for (int q = lane; q < nw; q += 32) g_spins[q] = R.spins[q];
-        for (int q = lane; q < np / 4; q += 32) ((int4*)g_field)[q] = ((const int4*)R.G)[q];
-        if (lane == 0)
+        W.icost = (long long)a.p.cost[slot];
+        W.ilow = (long long)a.p.lowest[r];
+      }
+      const bool ok = decide_sweeps<FM, REPLAY, INT>(a, m, R, sh, r, t0, W, g_lsp);
+      if (lane == 0) st_release(R.done, 1u);
+      if (REPLAY) rs = stream_state(R, W);
+      walker_sync<INT>(bar_id);
+      if (ok && !*(volatile unsigned*)R.abort && lane == 0)
+      {
+        a.p.attempts[r] += W.natt;
+        a.p.accepts[r] += W.nacc;
+        a.p.step_att[r] += W.natt;
+        a.p.step_acc[r] += W.nacc;
+        if (a.p.windows) a.p.windows[r] += W.nwin;
+        if (queued && REPLAY) a.rng[r] = rs;
+        if (INT)
         {
-          a.p.attempts[r] += natt;
-          a.p.accepts[r] += nacc;
-          a.p.step_att[r] += natt;
-          a.p.step_acc[r] += nacc;
-          if (a.p.windows) a.p.windows[r] += nwin;
+          a.p.cost[slot] = (double)W.icost;
+          const double nlow = (double)W.ilow;
+          if (a.p.lowtag && nlow < a.p.lowest[r]) a.p.lowtag[r] = a.tag;
+          a.p.lowest[r] = nlow;
         }
       }
+    }
+    else if (role == 1)
+    {
+      feed<FM, REPLAY>(R, s_scr, m.fc_desc, m.fc_tab, tile_words(sh), sh.rows, (N + 31) >> 5,
+                       ((N + 31) >> 5) * a.n_sweeps, t0, rs, key,
+                       (unsigned long long)a.sweep_base * (unsigned long long)N, N, a.err);
+      walker_sync<INT>(bar_id);
     }
     else
     {
       double cost = a.p.cost[slot], low = a.p.lowest[r];
-      long long icost = INT ? (long long)cost : 0, ilow = INT ? (long long)low : 0;
-      ok = account<FL, INT>(a, R, cost, low, icost, ilow, a.p.lspins + (size_t)r * nw);
-      pair_sync(bar_id);
+      const bool ok = account<FM>(a, m, R, cost, low, g_lsp);
+      walker_sync<INT>(bar_id);
       if (ok && !*(volatile unsigned*)R.abort && lane == 0)
       {
-        a.p.cost[slot] = INT ? (double)icost : cost;
-        const double nlow = INT ? (double)ilow : low;
-        if (a.p.lowtag && nlow < a.p.lowest[r]) a.p.lowtag[r] = a.tag;
-        a.p.lowest[r] = nlow;
+        a.p.cost[slot] = cost;
+        if (a.p.lowtag && low < a.p.lowest[r]) a.p.lowtag[r] = a.tag;
+        a.p.lowest[r] = low;
       }
     }
     if (*(volatile unsigned*)R.abort) return;
-    pair_sync(bar_id);  // the region is reused by the next walker
+    t0 += (unsigned)(((N + 31) >> 5) * a.n_sweeps);
+    copy16((uint4*)g_spins, (const uint4*)R.spins, a.p.nw >> 2, me, nme);
+    if (FM != PAIR && !queued) copy16((uint4*)g_ts, (const uint4*)R.z, zwords, me, nme);
+    walker_sync<INT>(bar_id);  // the region is reused by the next walker
+    if (!queued)
+    {
+      r += a.n_streams;
+      // a stream that serves several walkers goes on where the last one ended
+      if (REPLAY && r < a.n_walkers)
+      {
+        if (decider && lane == 0) a.rng[w] = rs;
+        __threadfence_block();
+        walker_sync<INT>(bar_id);
+        rs = *(volatile uint64_t*)(a.rng + w);
+      }
+    }
   }
-  if (REPLAY && decider && lane == 0) a.rng[w] = rs;
+  if (REPLAY && !queued && decider && lane == 0) a.rng[w] = rs;
 }
 
-template <int FL, bool R, bool I>
-static cudaError_t go(const SweepArgs& a, cudaStream_t s, int wpc, int smem)
+template <int FM, bool R, bool I>
+static cudaError_t go(const SweepArgs& a, cudaStream_t s, int wpc, const Shape& sh)
 {
-  auto k = fc_sweep_kernel<FL, R, I>;
-  static int configured = -1;
-  if (smem > 48 * 1024 && configured < smem)
+  auto k = fc_sweep_kernel<FM, R, I>;
+  const int smem = kTable + wpc * region_bytes(sh, I);
+  const int threads = (I ? 64 : 96) * wpc;
+  static std::atomic<int> configured{48 * 1024};
+  if (smem > configured.load())
   {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
-    configured = smem;
+    configured = kMaxSmem;
   }
-  const int blocks = (a.n_streams + wpc - 1) / wpc;
-  if (blocks > 0) k<<<blocks, 64 * wpc, smem, s>>>(a, wpc);
+  int blocks = (a.n_streams + wpc - 1) / wpc;
+  if (a.queue)
+  {
+    // persistent: as many blocks as stay resident, the queue feeds them
+    int per_sm = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
+    if (e != cudaSuccess) return e;
+    blocks = std::max(1, std::min((a.n_walkers + wpc - 1) / wpc, std::max(1, per_sm) * kSms));
+  }
+  if (blocks > 0) k<<<blocks, threads, smem, s>>>(a, wpc, sh);
   return cudaGetLastError();
 }
 
-template <int FL>
-static cudaError_t go_fl(const SweepArgs& a, cudaStream_t s, int wpc, int smem)
+template <int FM>
+static cudaError_t go_fm(const SweepArgs& a, cudaStream_t s, int wpc, const Shape& sh)
 {
   const bool I = a.m.int_mode != 0;
-  if (a.replay) return I ? go<FL, true, true>(a, s, wpc, smem) : go<FL, true, false>(a, s, wpc, smem);
-  return I ? go<FL, false, true>(a, s, wpc, smem) : go<FL, false, false>(a, s, wpc, smem);
+  if (a.replay) return I ? go<FM, true, true>(a, s, wpc, sh) : go<FM, true, false>(a, s, wpc, sh);
+  return I ? go<FM, false, true>(a, s, wpc, sh) : go<FM, false, false>(a, s, wpc, sh);
+}
+
+// a walker's region for a model in a population of these strides
+static Shape shape_of(const DevModel& m, int nw, int mp)
+{
+  Shape s;
+  s.pair = m.flavor == F_PARITY && m.pair_only;
+  s.nw = nw;
+  s.mp = s.pair ? nw * 32 : mp;
+  s.rows = std::min(kMaxRows, m.fc_rows);
+  // a state that leaves less room: smaller tiles (larger blocks read HBM)
+  while (s.rows > 4 && kTable + region_bytes(s, m.int_mode != 0) > kMaxSmem) s.rows -= 4;
+  return s;
 }
 }  // namespace fc
 
-static const int kFcMaxSmem = 227 * 1024;
-static const int kSms = 152;
-
-int64_t fc_words(int n_vars) { return ((int64_t)(n_vars + 31) / 32) * 32; }
-
 bool fc_fits(const DevModel& m, int nw, int mp)
 {
-  if (!m.fc_rec || m.sweep_size != m.n_vars || m.n_vars <= 0) return false;
+  if (!m.fc_desc || m.sweep_size != m.n_vars || m.n_vars <= 0) return false;
   if (!(m.flavor == F_PARITY || m.flavor == F_COUNTER)) return false;
-  return fc::kTable + fc::region_bytes(m.n_vars, nw, mp) <= kFcMaxSmem;
+  return fc::kTable + fc::region_bytes(fc::shape_of(m, nw, mp), m.int_mode != 0) <= fc::kMaxSmem;
 }
 
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s)
 {
-  if (!fc_fits(a.m, a.p.nw, a.p.mp) || !a.field) return cudaErrorInvalidValue;
-  const int per = fc::region_bytes(a.m.n_vars, a.p.nw, a.p.mp);
-  const int wmax = std::min(4, (kFcMaxSmem - fc::kTable) / per);
+  if (!fc_fits(a.m, a.p.nw, a.p.mp)) return cudaErrorInvalidValue;
+  const fc::Shape sh = fc::shape_of(a.m, a.p.nw, a.p.mp);
+  const int per = fc::region_bytes(sh, a.m.int_mode != 0);
+  const int wmax = std::min(a.m.int_mode ? 8 : 4, (fc::kMaxSmem - fc::kTable) / per);
   // spread the walkers over the SMs: as few per block as fills them
-  int wpc = (a.n_streams + kSms - 1) / kSms;
+  int wpc = (a.n_streams + fc::kSms - 1) / fc::kSms;
   wpc = std::max(1, std::min(wpc, wmax));
-  const int smem = fc::kTable + wpc * per;
-  switch (a.m.flavor)
-  {
-    case F_PARITY: return fc::go_fl<F_PARITY>(a, s, wpc, smem);
-    default: return fc::go_fl<F_COUNTER>(a, s, wpc, smem);
-  }
+  if (a.m.flavor == F_COUNTER) return fc::go_fm<fc::COUNTER>(a, s, wpc, sh);
+  return a.m.pair_only ? fc::go_fm<fc::PAIR>(a, s, wpc, sh) : fc::go_fm<fc::PARITY>(a, s, wpc, sh);
 }
 
 void fc_upload(const double* ln, const float* scr, const unsigned long long* jA,
                const unsigned long long* jC)
 {
   cudaMemcpyToSymbol(fc::c_ln, ln, 1024 * sizeof(double));
-  cudaMemcpyToSymbol(fc::c_scr, scr, 3072 * sizeof(float));
-  cudaMemcpyToSymbol(fc::c_jA, jA, 65 * sizeof(unsigned long long));
-  cudaMemcpyToSymbol(fc::c_jC, jC, 65 * sizeof(unsigned long long));
+  float4 t[1024];
+  for (int i = 0; i < 1024; i++)
+  {
+    t[i] = make_float4(scr[3 * i], scr[3 * i + 1], scr[3 * i + 2], 0.f);
+    if ((i & 255) == 1) t[i].x = INFINITY;  // log(0): never accepted
+  }
+  cudaMemcpyToSymbol(fc::g_scr, t, sizeof t);
+  ulonglong2 j[33];
+  for (int i = 0; i < 33; i++) j[i] = make_ulonglong2(jA[i], jC[i]);
+  cudaMemcpyToSymbol(fc::c_jump, j, sizeof j);
 }
 }  // namespace qio

@@ -75,8 +75,11 @@ struct HostModel
   std::vector<int> rec_i;     // 2 ints per incidence (integer mode)
   std::vector<double> rec_f;  // 2 doubles per incidence: (other as bits, coef)
   std::vector<unsigned int> rec_p;  // other << 8 | coefficient, when |coef| <= 127
-  // field-cached sweep records (16 bytes per incidence; see DevModel::fc_rec)
-  std::vector<uint32_t> fc_rec;
+  // block-decided sweep tables (see DevModel::fc_desc; empty: not eligible)
+  std::vector<int> fc_desc;
+  std::vector<uint32_t> fc_tab, fc_in;
+  int fc_rows = 0;
+  bool fc_big = false;
   int fc_S = 0;
   bool fc_pack = false;
   // level schedule (levels.cu): entries grouped by level, their offsets
@@ -219,8 +222,7 @@ class Solver
   bool smem_state = true;  // walker state in shared memory when it fits
   int kernel = 0;          // sweep kernel: 0 auto, 1 one walker per warp, 2 one walker per lane,
                            // 3 level schedule (one walker per warp, counter streams),
-                           // 4 cached local fields (two warps per walker)
-  bool auto_fields = true;  // "auto" may pick the cached-field sweep (the server's solves do not)
+                           // 4 block-decided (two or three warps per walker)
   // CUDA-event pairs around sweep launches (profile mode)
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_events;
   size_t prof_used = 0;

@@ -1,5 +1,6 @@
 // model_host.cc -- model construction and upload, schedules, device setup.
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -353,22 +354,28 @@ static void build_near(HostModel& m)
     }
 }
 
-// Records of the field-cached sweep.  The local field of a variable is the
-// sum, over its contributing incidences, of the coefficients in fixed point
-// q = round(c * 2^S): Ising, every incidence, +q for a term whose parity bit
-// is clear and -q otherwise (the cost difference is -2 times the sum);
-// counter models, the incidences whose term the flip would switch, +q when
-// the variable's literal is true and -q otherwise.  S is the largest scale
-// with 2^S * max_v sum_row |c| <= 2^30 (2^22 when the field also carries the
-// count of contributing incidences in its low 8 bits), so a field never
-// overflows and differs from the reference's FP64 sum by less than deg + 1
-// units.  Integer models use S = 0: the field is then the exact difference.
+// Tables of the block-decided sweep (fields.cu).  A variable's field H_v is its
+// flip's cost difference, up to its own spin's sign, in fixed point q =
+// round(c * 2^S):
+//   pair-only Ising: H_v = sum of q over its one-member terms plus, over its
+//     two-member terms, q * (1 - 2 s_u) with u the other member; the cost
+//     difference of flipping v is -2 (1 - 2 s_v) H_v;
+//   Ising with larger terms: the same with the parity of the term's other
+//     members in place of s_u;
+//   counter models: H_v = sum over the terms none of whose other literals is
+//     true of +q (v's literal plain) or -q (negated); the cost difference is
+//     H_v when s_v is true and -H_v otherwise.
+// S is the largest scale with 2^S * max_v sum_row |c| <= 2^30 (2^22 when the
+// field also carries the number of contributing terms in its low 8 bits), so
+// a field never overflows and differs from the reference's FP64 sum by less
+// than deg + 1 units.  Integer models use S = 0: the field is then exact.
 // Eligible: Ising with the term cache or counter models, fewer than 32766
-// variables, rows of at most 255 incidences.
+// variables and 2^18 terms, rows of at most 255 incidences.
 static void build_fields(HostModel& m)
 {
-  m.fc_rec.clear();
+  m.fc_desc.clear();
   if (!(m.flavor == F_PARITY || m.flavor == F_COUNTER) || m.N == 0 || m.N >= 32766) return;
+  if (!m.pair_only && m.M >= (1 << 18)) return;  // (a term's byte would not fit shared memory)
   double amax = 0;
   for (int64_t v = 0; v < m.N; v++)
   {
@@ -387,29 +394,101 @@ static void build_fields(HostModel& m)
     m.fc_S = amax > 0 ? top - e : 0;
     if (m.fc_S < -900 || m.fc_S > 900) return;  // 2^-S must stay a normal double
   }
-  m.fc_rec.assign((size_t)m.K * 4, 0u);
-  for (int64_t v = 0; v < m.N; v++)
-    for (int q = m.row[v]; q < m.row[v + 1]; q++)
+  auto fixed = [&](int q) -> int {
+    long long f = m.int_mode ? (long long)m.coef_i[q] : std::llrint(std::ldexp(m.coef[q], m.fc_S));
+    return (int)(m.fc_pack ? f * 256 : f);
+  };
+  const bool pair = m.pair_only;
+  const int nb = (int)((m.N + 31) / 32);
+  const int KI = 4;  // fields.cu: entries per lane of a block's chunk
+  const int ew = pair ? 2 : 4, pitch = pair ? 32 : 33;  // 32-bit words of an entry, records of a row
+  const size_t ent_at = 8 + 64;                         // 32-bit words before a chunk's entries
+  const size_t rec_at = ent_at + (size_t)KI * 32 * ew;  // ... and its records
+  m.fc_desc.assign((size_t)nb * 4, 0);
+  m.fc_tab.clear();
+  m.fc_in.clear();
+  m.fc_rows = 0;
+  m.fc_big = false;
+  for (int b = 0; b < nb; b++)
+  {
+    const int v0 = b * 32, v1 = (int)std::min<int64_t>(m.N, v0 + 32);
+    int* d = &m.fc_desc[(size_t)b * 4];
+    int rows = 0, kin = 0;
+    for (int v = v0; v < v1; v++) rows = std::max(rows, m.row[v + 1] - m.row[v]);
+    rows = (rows + 3) & ~3;
+    m.fc_rows = std::max(m.fc_rows, rows);
+    const size_t at = m.fc_tab.size();
+    d[0] = (int)(at / 2);
+    d[1] = rows;
+    m.fc_tab.resize(at + ((rec_at + (size_t)rows * pitch * 2 + 3) & ~(size_t)3), 0u);
+    uint32_t* tab = &m.fc_tab[at];
+    if (!pair)  // padding records: a flip leaves them alone
+      for (size_t r = 0; r < (size_t)rows * pitch; r++) tab[rec_at + 2 * r] = 1u << 19;
+    std::vector<std::array<uint32_t, 4>> in[32];
+    for (int l = 0; l < 32; l++)
     {
-      const uint32_t t = m.inc[q] & ~kNegBit;
-      long long fq = m.int_mode ? (long long)m.coef_i[q] : std::llrint(std::ldexp(m.coef[q], m.fc_S));
-      if (m.fc_pack) fq *= 256;
-      uint32_t co[3] = {0xFFFFu, 0xFFFFu, 0xFFFFu};
-      int nco = 0;
-      for (int j = m.trow[t]; j < m.trow[t + 1]; j++)
+      const int v = v0 + l;
+      const int deg = v < v1 ? m.row[v + 1] - m.row[v] : 0;
+      int sum = 0;        // pair: all coefficients (spins all up)
+      uint32_t negs = 0;  // else: the row's negated literals
+      for (int k = 0; k < deg; k++)
       {
-        const uint32_t u = m.tvar[j] & ~kNegBit;
-        if ((int64_t)u == v) continue;
-        if (nco < 3) co[nco] = u | ((m.tvar[j] & kNegBit) ? 0x8000u : 0u);
-        nco++;
+        const int q = m.row[v] + k;
+        const uint32_t t = m.inc[q] & ~kNegBit, vneg = m.inc[q] >> 31;
+        const int f = fixed(q);
+        const int tb = m.trow[t], te = m.trow[t + 1];
+        const bool big = te - tb > 8;
+        // members by id: the variable's position, and the others in the block
+        uint32_t pos = 0, mates = 0, neg = 0;
+        for (int j = tb; j < te; j++)
+        {
+          const uint32_t u = m.tvar[j] & ~kNegBit;
+          if ((int)u < v) pos++;
+          if ((int)u == v || (int)u < v0 || (int)u >= v0 + 32) continue;
+          mates |= 1u << (u - v0);
+          if (m.tvar[j] & kNegBit) neg |= 1u << (u - v0);
+        }
+        uint32_t* r = tab + rec_at + ((size_t)k * pitch + l) * 2;
+        if (pair)
+        {
+          const int u = m.other[q];
+          sum += f;
+          if (u < 0) continue;
+          r[0] = (uint32_t)u;
+          r[1] = (uint32_t)(2 * f);
+          if (mates && u < v) in[l].push_back({mates, (uint32_t)(2 * f), 0, 0});
+          continue;
+        }
+        const int val = m.flavor == F_PARITY ? f : (vneg ? -f : f) + (m.fc_pack ? 1 : 0);
+        if (big) pos = 0;
+        r[0] = t | (vneg << 18) | (mates ? 1u << 19 : 0u) | (big ? 1u << 20 : 0u) |
+               (big ? 0u : (~(1u << pos) & 255u) << 24);
+        r[1] = mates ? 0u : (uint32_t)val;  // (a shared term's value is in its in-block entry)
+        if (k < 32) negs |= vneg << k;
+        m.fc_big = m.fc_big || big;
+        if (mates)
+          in[l].push_back({t | ((uint32_t)(k & 31) << 18) | (pos << 23) | (big ? 0x40000000u : 0u) | (vneg << 31),
+                           mates, neg, (uint32_t)val});
       }
-      if (nco > 3) nco = 15;
-      uint32_t* r = &m.fc_rec[(size_t)q * 4];
-      r[0] = m.inc[q];
-      r[1] = (uint32_t)(int32_t)fq;
-      r[2] = co[0] | (co[1] << 16);
-      r[3] = co[2] | ((uint32_t)nco << 16);
+      tab[8 + 2 * l] = pair ? (uint32_t)sum : negs;
+      tab[8 + 2 * l + 1] = (uint32_t)deg;
+      kin = std::max(kin, (int)in[l].size());
     }
+    for (int l = 0; l < 32; l++)
+      for (size_t k = 0; k < in[l].size() && k < (size_t)KI; k++)
+        memcpy(tab + ent_at + (k * 32 + l) * ew, in[l][k].data(), ew * 4);
+    tab[0] = (uint32_t)rows | (uint32_t)std::min(kin, KI) << 8;
+    if (kin > KI)
+    {
+      const size_t more = m.fc_in.size() / ew;
+      tab[0] |= (uint32_t)(kin - KI) << 16;
+      tab[1] = (uint32_t)more;
+      m.fc_in.resize(m.fc_in.size() + (size_t)(kin - KI) * 32 * ew, 0u);
+      for (int l = 0; l < 32; l++)
+        for (size_t k = KI; k < in[l].size(); k++)
+          memcpy(&m.fc_in[(more + (k - KI) * 32 + l) * ew], in[l][k].data(), ew * 4);
+    }
+  }
 }
 
 // Integer mode: every coefficient is an integer of magnitude <= 2^20 and the
@@ -493,7 +572,6 @@ std::unique_ptr<HostModel> build_model(int kind, int64_t n_terms,
                         : 1.0 / m->max_coupling;
   build_nbr(*m);
   detect_int_mode(*m);
-  build_fields(*m);
   if (m->flavor == F_PARITY || m->flavor == F_COUNTER) build_near(*m);
   if (m->flavor == F_PARITY)
   {
@@ -548,6 +626,7 @@ std::unique_ptr<HostModel> build_model(int kind, int64_t n_terms,
       }
     }
   }
+  build_fields(*m);
   return m;
 }
 
@@ -650,7 +729,7 @@ void HostModel::upload() const
          o_cf = put(blob, coef_f), o_near = put(blob, near), o_oth = put(blob, other),
          o_ri = put(blob, rec_i), o_rf = put(blob, rec_f), o_rp = put(blob, rec_p),
          o_lo = put(blob, lv_off), o_le = put(blob, lv_ent), o_lp = put(blob, lv_pos),
-         o_fc = put(blob, fc_rec);
+         o_ft = put(blob, fc_tab), o_fd = put(blob, fc_desc), o_fi = put(blob, fc_in);
   // 256 bytes of tail padding: bulk copies of incidence ranges round their
   // end up to 16 bytes
   blob.resize(((blob.size() + 255) & ~(size_t)255) + 256);
@@ -693,7 +772,11 @@ void HostModel::upload() const
   dev.n_levels = lv_ok ? n_levels : 0;
   dev.lv_recs = lv_ok ? lv_recs : 0;
   dev.lv_d8 = lv_d8 ? 1 : 0;
-  dev.fc_rec = fc_rec.empty() ? nullptr : (const uint4*)(b + o_fc);
+  dev.fc_desc = fc_desc.empty() ? nullptr : (const int4*)(b + o_fd);
+  dev.fc_tab = (const uint2*)(b + o_ft);
+  dev.fc_in = (const void*)(b + o_fi);
+  dev.fc_rows = fc_rows;
+  dev.fc_big = fc_big ? 1 : 0;
   dev.fc_S = fc_S;
   dev.fc_pack = fc_pack ? 1 : 0;
   dev.fc_inv = std::ldexp(1.0, -fc_S);

@@ -84,12 +84,29 @@ struct DevModel
   const uint32_t* tvar;    // K  members (| kNegBit for negated literals)
   const double* tcost;     // n_terms
   const int* tcost_i;      // n_terms
-  // field-cached sweep (fields.cu): one 16-byte record per incidence, in
-  // row order: x = inc (term | kNegBit), y = the coefficient in fixed point
-  // (round(c * 2^fc_S), shifted left 8 when fc_pack), z = co-members 0 and 1,
-  // w = co-member 2 | count << 16 (count 15: more than three, read trow /
-  // tvar); a co-member is id | 0x8000 for a negated literal, 0xFFFF none
-  const uint4* fc_rec;     // K, or null when the model does not qualify
+  // block-decided sweep (fields.cu), blocks of 32 variables, a lane each.
+  // Block b's chunk begins at 8-byte word fc_desc[b].x of fc_tab:
+  //   header, 32 bytes: record rows, in-block entry rows (at most four), first
+  //     further entry in fc_in, further entry rows;
+  //   lane data, 8 bytes: (pair-only Ising: sum of the variable's fixed-point
+  //     coefficients; else its row's negated literals; degree);
+  //   in-block entries, four per lane (entry i of lane l at 32 i + l), one per
+  //     term with other members in the block (pair: with an earlier one): pair,
+  //     8 bytes, (that member's lane, 2q); else 16 bytes, (term | row position
+  //     << 18 | member position << 23 | more than eight members << 30 | negated
+  //     literal << 31, the members' lanes, their negated ones, the record's
+  //     second word);
+  //   records, fc_desc[b].y rows (a multiple of four), 8 bytes, in row order:
+  //     record k of lane l at 32 k + l (not pair: 33 k + l): pair (other member,
+  //     2q); else (term | negated literal << 18 | another member in the block <<
+  //     19 | more than eight members << 20 | the byte's bits of the other
+  //     members << 24, what the term adds to the field when it contributes).
+  // Zeros pad all of them.  Further entries lie in fc_in, rows of 32.
+  const int4* fc_desc;     // or null when the model does not qualify
+  const uint2* fc_tab;
+  const void* fc_in;
+  int fc_rows;             // most records per lane of a block
+  int fc_big;              // a term has more than eight members
   int fc_S;                // fixed-point scale exponent
   int fc_pack;             // FP64 counter models: field = fixed << 8 | count
   double fc_inv;           // 2^-fc_S
@@ -135,11 +152,10 @@ struct SweepArgs
   int smem_state;       // stage spins + term state in shared memory
   int* err;             // device error flag (a bounded wait gave up)
   long long tag;        // written to p.lowtag[walker] when its lowest drops
-  // field-cached sweep: per slot the fixed-point local field of every
-  // variable (fc_words(N) ints), kept between launches; null selects the
-  // windowed kernel.  field_valid = 0: rebuild the fields from the state.
-  int* field;
-  int field_valid;
+  // block-decided sweep: 1 selects it; terms_valid = 1: the term bytes are as
+  // its last launch on this population left them (0: made from the spins)
+  int fields;
+  int terms_valid;
   // batches (windowed kernel): walker r runs models[model_of[r]] with the
   // counter key of walker local_of[r] of its own solve; with `queue` set,
   // each warp takes walkers from the counter *queue (reset to 0 before the
@@ -154,7 +170,7 @@ struct SweepArgs
   // multiple of 8; 0: launch_sweep sizes it to the model's largest block,
   // at most 640, 768 for integer models); larger blocks are read from HBM
   int tile_cap;
-  // field-cached sweep: stream w runs walker order[w] (null: walker w); set
+  // block-decided sweep: stream w runs walker order[w] (null: walker w); set
   // only with one walker per stream.  Tempering puts its hottest replicas
   // first, so that their long chains start in the first wave of blocks.
   const int* order;
@@ -184,9 +200,8 @@ cudaError_t launch_sweep(const SweepArgs& a, cudaStream_t s, int warps_per_block
 // one warp's walker state (term bytes, spins, lowest) fits shared memory
 // beside the windowed kernel's tables and tiles (required by batch queues)
 bool sweep_state_fits(const SweepArgs& a);
-// field-cached sweep (fields.cu): ints of one slot's fields, and whether the
-// kernel can run this model with this population layout
-int64_t fc_words(int n_vars);
+// block-decided sweep (fields.cu): whether it can run this model with this
+// population layout
 bool fc_fits(const DevModel& m, int nw, int mp);
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s);
 cudaError_t launch_eval_cost(const DevModel& m, int n_states,

@@ -191,18 +191,9 @@ struct Population
   uint64_t* rng = nullptr;
   int* slot_of = nullptr;
   double* beta = nullptr;
-  // cached local fields of the field-cached sweep, per slot; fvalid: they
-  // match the slots' states (false after anything else changed the states)
-  DevBuf fbuf;
-  int* field = nullptr;
-  bool fvalid = false;
-
-  void ensure_fields(int64_t N)
-  {
-    if (field) return;
-    fbuf = DevBuf((size_t)n * (size_t)fc_words((int)N) * 4);
-    field = (int*)fbuf.ptr;
-  }
+  // the term bytes are the block-decided sweep's own (fields.cu), as its last
+  // launch left them (false after anything else set the states)
+  bool tvalid = false;
 
   void alloc(const HostModel& m, int slots, int streams, bool need_slots,
              int64_t n_beta)
@@ -480,15 +471,16 @@ bool levels_for(const Solver& s, const HostModel& m)
   return !s.replay && levels_eligible(m) && m.N >= 4096;
 }
 
-// The field-cached sweep: Ising with the term cache or counter models
-// (PUBO, MaxSat with full sweeps) whose walker state, fields and record tiles
-// fit a block's shared memory.  auto: Ising models (1.47x the windowed kernel
-// on the 1000-spin sparse SA workload); counter models keep the windowed
-// kernel, which measured 4 % faster on the 4096-variable PUBO tempering
-// workload; "fields" forces it, "warp" keeps the windowed kernel.
+// The block-decided sweep (fields.cu): Ising with the term cache or counter
+// models (PUBO, MaxSat with full sweeps) whose walker state and block chunks
+// fit a block's shared memory.  auto: wherever it runs.  20 sweeps, this
+// kernel against the windowed one (ms): sparse Ising N = 1000, 64 walkers 0.64
+// / 2.37; PUBO N = 4096, 64 walkers 5.5 / 21.1, 8192 walkers 114 / 239; 3-SAT
+// N = 1000, 64 walkers 1.25 / 2.95, 8192 walkers 20.1 / 22.1.  "warp" keeps the
+// windowed kernel.
 bool fields_for(const Solver& s, const HostModel& m, const Population& P, bool full_maxsat_sweep)
 {
-  const bool ok = !m.empty() && !m.fc_rec.empty() && s.smem_state &&
+  const bool ok = !m.empty() && !m.fc_desc.empty() && s.smem_state &&
                   fc_fits(m.device_view(full_maxsat_sweep), P.pop.nw, P.pop.mp);
   if (s.kernel == 4)
   {
@@ -498,7 +490,7 @@ bool fields_for(const Solver& s, const HostModel& m, const Population& P, bool f
               "and walker state that fits shared memory");
     return true;
   }
-  return s.kernel == 0 && s.auto_fields && ok && m.flavor == F_PARITY;
+  return s.kernel == 0 && ok;
 }
 
 // beta as Metropolis::set_beta / set_temperature store it
@@ -628,16 +620,11 @@ class SimulatedAnnealing : public Solver
     levels = levels_for(*this, *model);
     lanes = !levels && lanes_for(*this, *model, restarts);
     fields = !levels && !lanes && fields_for(*this, *model, P, full_maxsat_sweep);
-    if (fields)
-    {
-      P.ensure_fields(model->N);
-      P.fvalid = false;
-      device_bytes = (int64_t)(P.buf.bytes + P.fbuf.bytes);
-    }
+    P.tvalid = false;
     used_kernel = levels ? 3 : (lanes ? 2 : (fields ? 8 : 1));
     // the lane and level sweeps work from the spins and rebuild the term
-    // bytes when they finish
-    a.skip_terms = (levels || lanes) ? 1 : 0;
+    // bytes when they finish; the field-cached sweep makes its own
+    a.skip_terms = (levels || lanes || fields) ? 1 : 0;
     cuda_check(launch_init(a, st), "init kernel");
     launches++;
     if (levels && !lvlog.buf.ptr) device_bytes += (int64_t)lvlog.ensure(R, step_limit, *model, P.pop.nw);
@@ -707,10 +694,10 @@ class SimulatedAnnealing : public Solver
     {
       a.sweep_base = base;
       a.n_sweeps = (int)n;
-      a.field = fields ? P.field : nullptr;
-      a.field_valid = P.fvalid ? 1 : 0;
+      a.fields = fields ? 1 : 0;
+      a.terms_valid = P.tvalid ? 1 : 0;
       cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
-      P.fvalid = fields;
+      P.tvalid = fields;
     }
     prof_end(st);
     launches++;
@@ -1039,14 +1026,10 @@ class ParallelTempering : public Solver
     a.seed = seed;
     a.key_base = 0;
     a.key_div = T();
-    cuda_check(launch_init(a, st), "init kernel");
     fields = fields_for(*this, *model, P, full_maxsat_sweep);
-    if (fields)
-    {
-      P.ensure_fields(model->N);
-      device_bytes += (int64_t)P.fbuf.bytes;
-    }
-    P.fvalid = false;
+    a.skip_terms = fields ? 1 : 0;  // the field-cached sweep makes its own term bytes
+    cuda_check(launch_init(a, st), "init kernel");
+    P.tvalid = false;
     used_kernel = fields ? 8 : 1;
     cuda_check(cudaStreamSynchronize(st), "sync");
     // the sweep/swap loop keeps its own copies of the stream so that a
@@ -1104,13 +1087,13 @@ class ParallelTempering : public Solver
     {
       a.sweep_base = s * spr;
       a.tag = s;  // the step, for the time order of equal lowest costs
-      a.field = fields ? P.field : nullptr;
+      a.fields = fields ? 1 : 0;
       a.order = fields ? hot_first : nullptr;
-      a.field_valid = P.fvalid ? 1 : 0;
+      a.terms_valid = P.tvalid ? 1 : 0;
       prof_begin(st);
       cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
       prof_end(st);
-      P.fvalid = fields;
+      P.tvalid = fields;
       sw.step = s;
       cuda_check(launch_pt_swap(sw, st), "swap kernel");
       launches += 2;
@@ -1188,11 +1171,11 @@ class ParallelTempering : public Solver
     {
       a.sweep_base = step_pos * spr;
       a.tag = step_pos;
-      a.field = fields ? P.field : nullptr;
+      a.fields = fields ? 1 : 0;
       a.order = fields ? hot_first : nullptr;
-      a.field_valid = P.fvalid ? 1 : 0;
+      a.terms_valid = P.tvalid ? 1 : 0;
       cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
-      P.fvalid = fields;
+      P.tvalid = fields;
       sw.step = step_pos;
       cuda_check(launch_pt_swap(sw, st), "swap kernel");
       launches += 2;

@@ -1,0 +1,84 @@
+"""Edges of the block-decided sweep (csrc/fields.cu) against the oracle, bit for
+bit (GPU required): variables around a block of 32, a walker's last and only
+block, terms inside one block and across its border, more in-block terms per
+lane than a chunk holds, terms of more members than a byte's bits or a record's
+fields, rows wider than a staged block, draws that no attempt takes (an
+infinite beta), more walkers than fit the chip at once, and sweeps cut into
+launches of one."""
+import numpy as np
+import pytest
+
+import qiotoolkit_gb300 as q
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+SA = "simulatedannealing.qiotoolkit"
+
+
+def terms(n, sizes, count, seed, span=None, integer=False, hub=0):
+    """`count` terms of the given sizes over n variables, each within a run of
+    `span` ids; `hub` further terms on variable n // 2; every variable in one."""
+    rng = np.random.default_rng(seed)
+    out = [[v] for v in range(n)]
+    for _ in range(count):
+        k = min(int(rng.choice(sizes)), n)
+        lo = 0 if span is None else int(rng.integers(0, max(1, n - span + 1)))
+        hi = n if span is None else min(n, lo + max(span, k))
+        out.append(sorted((lo + rng.choice(hi - lo, min(k, hi - lo), replace=False)).tolist()))
+    for _ in range(hub):
+        out.append(sorted({n // 2, *rng.choice(n, 2, replace=False).tolist()}))
+    out = sorted({tuple(t) for t in out})
+    coef = rng.choice([-2.0, -1.0, 1.0, 3.0], len(out)) if integer else rng.normal(size=len(out))
+    return O.flatten_terms([(float(c), list(t)) for c, t in zip(coef, out)])
+
+
+def clauses(n, seed, **kw):
+    """The same with random signs, ids from 1 and positive weights."""
+    off, ids, coef = terms(n, seed=seed, **kw)
+    sign = np.random.default_rng(seed + 1).choice([-1, 1], len(ids))
+    return off, (np.asarray(ids) + 1) * sign, np.abs(coef)
+
+
+CASES = {  # kind, instance, restarts, beta_stop
+    **{f"pair_{n}": ("ising", lambda n=n: terms(n, [2], 3 * n, n), 5, 3.0) for n in (2, 31, 32, 33, 64, 65)},
+    **{f"pubo_{n}": ("pubo", lambda n=n: terms(n, [2, 3, 4], 4 * n, n), 5, 3.0) for n in (4, 32, 33, 97)},
+    "pair_dense_block": ("ising", lambda: terms(70, [2], 700, 1, span=36, integer=True), 6, 2.0),
+    "pair_wide_rows": ("ising", lambda: terms(200, [2], 300, 2, hub=150), 6, 2.0),
+    "parity_block": ("ising", lambda: terms(90, [3, 4], 400, 3, span=40), 6, 3.0),
+    "parity_large": ("ising", lambda: terms(120, [2, 5, 9, 12], 300, 4), 6, 3.0),
+    "parity_large_int": ("ising", lambda: terms(120, [2, 6, 10], 300, 5, span=48, integer=True), 6, 3.0),
+    "pubo_block": ("pubo", lambda: terms(80, [2, 3, 5], 500, 6, span=34), 6, 3.0),
+    "pubo_block_int": ("pubo", lambda: terms(80, [2, 3, 6], 500, 7, span=34, integer=True), 6, 3.0),
+    "pubo_large": ("pubo", lambda: terms(130, [1, 4, 7, 9, 14], 400, 8), 6, 3.0),
+    "pubo_wide_rows": ("pubo", lambda: terms(260, [2, 3], 500, 9, hub=180), 6, 3.0),
+    "sat_signs": ("maxsat", lambda: clauses(75, 10, sizes=[2, 3, 5], count=400, span=38), 6, 3.0),
+    "sat_large": ("maxsat", lambda: clauses(100, 11, sizes=[3, 9, 11], count=300, integer=True), 6, 3.0),
+    "cold": ("ising", lambda: terms(100, [2], 300, 12), 4, np.inf),
+    "cold_pubo": ("pubo", lambda: terms(100, [2, 3], 300, 13), 4, np.inf),
+    "waves": ("pubo", lambda: terms(60, [2, 3], 150, 14), 1300, 2.0),
+}
+
+
+@pytest.mark.parametrize("mode", ["replay", "counter"])
+@pytest.mark.parametrize("name", list(CASES))
+def test_block_sweep_edges(name, mode):
+    kind, make, restarts, stop = CASES[name]
+    inst = make()
+    g = q.Model(kind, off=inst[0], ids=inst[1], coef=inst[2])
+    o = O.Model(kind, off=inst[0], ids=inst[1], coef=inst[2])
+    temps = np.isinf(stop)  # a temperature of zero
+    params = {"seed": 3, "sweeps": 25, "restarts": restarts, "rng_mode": mode, "kernel": "fields",
+              "maxsat_full_sweep": True, "cost_limit": -1e300}
+    if restarts > 100:
+        del params["cost_limit"]  # one launch for all sweeps
+    sched = ("linear", 2.0, 0.0) if temps else ("linear", 0.1, stop)
+    params.update({"schedule": {"type": "linear", "initial": 2.0, "final": 0.0}} if temps else
+                  {"beta_start": 0.1, "beta_stop": stop})
+    s = q.Solver(g, SA, {"params": params}).init().run()
+    assert s.stats().sweep_kernel == 8
+    r = O.run(o, "sa", seed=3, step_limit=25, restarts=restarts, sched=sched, use_inverse=not temps,
+              rng_mode=mode, threads=8, full_maxsat_sweep=True)
+    out = s.replicas()
+    for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
+        np.testing.assert_array_equal(out[key], getattr(r, key), err_msg=key)
