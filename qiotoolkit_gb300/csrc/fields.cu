@@ -1625,7 +1625,7 @@ bool fc_fits(const DevModel& m, int nw, int mp)
   return fc::kTable + fc::region_bytes(fc::shape_of(m, nw, mp), m.int_mode != 0) <= fc::kMaxSmem;
 }
 
-cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s)
+cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb)
 {
   if (!fc_fits(a.m, a.p.nw, a.p.mp)) return cudaErrorInvalidValue;
   const fc::Shape sh = fc::shape_of(a.m, a.p.nw, a.p.mp);
@@ -1633,6 +1633,7 @@ cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s)
   const int wmax = std::min(a.m.int_mode ? 8 : 4, (fc::kMaxSmem - fc::kTable) / per);
   // spread the walkers over the SMs: as few per block as fills them
   int wpc = (a.n_streams + fc::kSms - 1) / fc::kSms;
+  if (a.queue) wpc = std::min(wpc, wpb);
   wpc = std::max(1, std::min(wpc, wmax));
   if (a.m.flavor == F_COUNTER) return fc::go_fm<fc::COUNTER>(a, s, wpc, sh);
   return a.m.pair_only ? fc::go_fm<fc::PAIR>(a, s, wpc, sh) : fc::go_fm<fc::PARITY>(a, s, wpc, sh);

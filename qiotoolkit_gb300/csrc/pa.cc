@@ -422,7 +422,7 @@ class PopulationAnnealing : public Solver
     R = 0;
     // lanes need independent streams per walker: counter mode only
     levels = levels_for(*this, *model);
-    lanes = !levels && !replay && lanes_for(*this, *model, (int64_t)target_pop);
+    lanes = !levels && !replay && lanes_for(*this, *model, (int64_t)target_pop, false);
     if (replay && kernel == 2) fail(1, "parameter `kernel`: \"lanes\" needs \"rng_mode\": \"counter\" here");
     used_kernel = levels ? 3 : (lanes ? 2 : 1);
     init_population(st);

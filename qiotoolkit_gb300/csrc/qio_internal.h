@@ -203,7 +203,8 @@ bool sweep_state_fits(const SweepArgs& a);
 // block-decided sweep (fields.cu): whether it can run this model with this
 // population layout
 bool fc_fits(const DevModel& m, int nw, int mp);
-cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s);
+// (wpb: walkers per block of a queued launch, at most)
+cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb);
 cudaError_t launch_eval_cost(const DevModel& m, int n_states,
                              const uint32_t* spins, int nw, double* out,
                              cudaStream_t s);

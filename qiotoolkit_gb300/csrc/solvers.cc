@@ -403,9 +403,17 @@ void LaneRunner::setup(const std::vector<DevModel>& models, const std::vector<in
 // The lane kernel runs Ising models whose terms have one or two members.
 bool lanes_eligible(const HostModel& m) { return m.flavor == F_PARITY && m.pair_only; }
 
-// kernel choice: one walker per lane when there are enough walkers to fill
-// warps of 32 many times over (or when asked for)
-bool lanes_for(const Solver& s, const HostModel& m, int64_t walkers)
+// Kernel choice: one walker per lane when asked for, or when there are so many
+// walkers that the lane kernel's time, the same up to some tens of thousands of
+// them, is the shortest.  Measured, 20 sweeps (ms), lanes against the
+// block-decided sweep (`blocks`: it runs the model) -- sparse Ising N = 64: 4.2
+// / 8.4 at 65536 walkers, 1.5 / 2.1 at 16384, 1.4 / 0.56 at 4096; N = 1000: 66 /
+// 73, 23 / 18, 22 / 4.7; integer N = 1000: 23 / 36, 15 / 9.3, 15 / 2.7 -- and
+// against the windowed sweep: N = 1000 22 / 9.9 at 4096, 23 / 34 at 16384;
+// cubic lattice of 4096 76 / 19 at 1024, 77 / 73 at 4096, 86 / 255 at 16384.
+static int64_t lane_walkers(bool blocks) { return blocks ? 24576 : 4096; }
+
+bool lanes_for(const Solver& s, const HostModel& m, int64_t walkers, bool blocks)
 {
   if (s.kernel == 2)
   {
@@ -414,7 +422,8 @@ bool lanes_for(const Solver& s, const HostModel& m, int64_t walkers)
     return true;
   }
   if (s.kernel == 1 || s.kernel == 3) return false;
-  return lanes_eligible(m) && walkers >= 1024;
+  if (s.kernel == 4) return !blocks && lanes_eligible(m) && walkers >= 1024;
+  return lanes_eligible(m) && walkers >= lane_walkers(blocks);
 }
 
 // The level kernel runs integer pair-only Ising models whose level schedule
@@ -478,10 +487,14 @@ bool levels_for(const Solver& s, const HostModel& m)
 // / 2.37; PUBO N = 4096, 64 walkers 5.5 / 21.1, 8192 walkers 114 / 239; 3-SAT
 // N = 1000, 64 walkers 1.25 / 2.95, 8192 walkers 20.1 / 22.1.  "warp" keeps the
 // windowed kernel.
+bool fields_run(const Solver& s, const HostModel& m, const Population& P, bool full_maxsat_sweep)
+{
+  return !m.empty() && !m.fc_desc.empty() && s.smem_state &&
+         fc_fits(m.device_view(full_maxsat_sweep), P.pop.nw, P.pop.mp);
+}
 bool fields_for(const Solver& s, const HostModel& m, const Population& P, bool full_maxsat_sweep)
 {
-  const bool ok = !m.empty() && !m.fc_desc.empty() && s.smem_state &&
-                  fc_fits(m.device_view(full_maxsat_sweep), P.pop.nw, P.pop.mp);
+  const bool ok = fields_run(s, m, P, full_maxsat_sweep);
   if (s.kernel == 4)
   {
     if (!ok)
@@ -618,7 +631,7 @@ class SimulatedAnnealing : public Solver
     a.key_base = 0;
     a.key_div = (long long)1 << 40;
     levels = levels_for(*this, *model);
-    lanes = !levels && lanes_for(*this, *model, restarts);
+    lanes = !levels && lanes_for(*this, *model, restarts, fields_run(*this, *model, P, full_maxsat_sweep));
     fields = !levels && !lanes && fields_for(*this, *model, P, full_maxsat_sweep);
     P.tvalid = false;
     used_kernel = levels ? 3 : (lanes ? 2 : (fields ? 8 : 1));
@@ -2405,7 +2418,15 @@ class SABatch : public Batch
     int first, last;
     const HostModel* model;  // any member (flavour and coefficient kind)
     int max_block_inc;       // the members' largest 32-variable block
+    int fc_rows;             // the same of the block-decided sweep's record rows
+    bool fields;             // runs on the block-decided sweep
   };
+  // members of a group share the kernel's instance
+  int kind(const HostModel& m) const
+  {
+    const bool f = !lanes && block_decided(m);
+    return m.flavor * 8 + (m.int_mode ? 4 : 0) + (f ? 2 : 0) + (f && m.pair_only ? 1 : 0);
+  }
   std::vector<Group> groups;
   DevBuf qbuf;  // DevModel per instance, model_of, local_of, one queue counter per group
   const DevModel* d_models = nullptr;
@@ -2461,6 +2482,12 @@ class SABatch : public Batch
     lanes = eligible && kernel != 1;
   }
 
+  // the block-decided sweep runs the model's walkers in this population
+  bool block_decided(const HostModel& m) const
+  {
+    return smem && kernel != 1 && !m.fc_desc.empty() && fc_fits(m.device_view(full_sweep), P.pop.nw, P.pop.mp);
+  }
+
   int n_instances() const override { return (int)models.size(); }
 
   void prepare(cudaStream_t st)
@@ -2476,9 +2503,20 @@ class SABatch : public Batch
     P.alloc_sizes(N, M, W, W, false, std::max<int64_t>(1, steps));
     // every model on the device before any capture (uploads allocate)
     for (auto* m : models) m->device_view(full_sweep);
+    // One walker per lane instead of the block-decided sweep's queue: for very
+    // many walkers (lane_walkers), and for batches of small models, which are
+    // a few ms either way and keep the kernel that their plan reports (96
+    // instances of 64 to 8000 spins, 16 walkers each, 100 sweeps: 518 ms on
+    // lanes, 162 on the windowed kernel's queue, 37 on this one's).
+    if (lanes && kernel != 2)
+    {
+      bool blocks = true;
+      for (auto* m : models) blocks = blocks && block_decided(*m);
+      lanes = !blocks || (kernel != 4 && (N < 352 || W >= lane_walkers(true)));
+    }
     order.resize(models.size());
     for (size_t i = 0; i < models.size(); i++) order[i] = (int)i;
-    auto kind_of = [&](int x) { return models[x]->flavor * 2 + (models[x]->int_mode ? 1 : 0); };
+    auto kind_of = [&](int x) { return kind(*models[x]); };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
       if (kind_of(x) != kind_of(y)) return kind_of(x) < kind_of(y);
       return models[x]->N > models[y]->N;
@@ -2519,9 +2557,10 @@ class SABatch : public Batch
     prepared = true;
   }
 
-  // The windowed kernel's queue plan: groups of one flavour and coefficient
-  // kind whose walker state fits a warp's shared memory; otherwise (or with
-  // `smem_state` off) one launch per instance.
+  // The queue plan: groups of one flavour and coefficient kind on the
+  // block-decided sweep, else on the windowed kernel where their walker state
+  // fits a warp's shared memory; otherwise (or with `smem_state` off) one launch
+  // per instance.
   void plan_queue()
   {
     groups.clear();
@@ -2531,14 +2570,15 @@ class SABatch : public Batch
       const HostModel* m = models[order[k]];
       const int first = (int)k * R;
       const int mb = m->device_view(full_sweep).max_block_inc;
-      if (groups.empty() || groups.back().model->flavor != m->flavor ||
-          groups.back().model->int_mode != m->int_mode)
-        groups.push_back({first, first + R, m, mb});
+      if (groups.empty() || kind(*groups.back().model) != kind(*m))
+        groups.push_back({first, first + R, m, mb, m->fc_rows, block_decided(*m)});
       else
       {
         groups.back().last = first + R;
         groups.back().max_block_inc = std::max(groups.back().max_block_inc, mb);
+        groups.back().fc_rows = std::max(groups.back().fc_rows, m->fc_rows);
       }
+      if (groups.back().fields) continue;
       SweepArgs a{};
       a.m = m->device_view(full_sweep);
       a.m.max_block_inc = groups.back().max_block_inc;
@@ -2600,6 +2640,8 @@ class SABatch : public Batch
     a.local_of = d_local_of + G.first;
     a.queue = d_queue + g;
     a.m.max_block_inc = G.max_block_inc;  // tiles sized for the group's largest block
+    a.m.fc_rows = G.fc_rows;
+    a.fields = G.fields ? 1 : 0;
     cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
   }
 
@@ -2639,7 +2681,8 @@ class SABatch : public Batch
       a.seed = seed;
       a.key_base = 0;
       a.key_div = (long long)1 << 40;
-      a.skip_terms = (lanes && n_sweeps > 0) ? 1 : 0;  // the lane store rebuilds them
+      // the lane store rebuilds them; the block-decided sweep makes its own
+      a.skip_terms = n_sweeps > 0 && (lanes || (queued && block_decided(*models[i]))) ? 1 : 0;
       cuda_check(launch_init(a, st), "init kernel");
       n_launch++;
     }

@@ -82,3 +82,25 @@ def test_block_sweep_edges(name, mode):
     out = s.replicas()
     for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
         np.testing.assert_array_equal(out[key], getattr(r, key), err_msg=key)
+
+
+@pytest.mark.parametrize("mode", ["replay", "counter"])
+@pytest.mark.parametrize("kernel", ["auto", "fields"])
+def test_batches_of_every_form(kernel, mode):
+    """One queue per kind of model (pair, many-body and counter models, integer
+    and FP64), small and large models behind one another on a walker's slot:
+    every instance equals its plain windowed solve."""
+    models = [q.Model("ising", off=t[0], ids=t[1], coef=t[2]) for t in (
+        terms(400, [2], 900, 21), terms(33, [2], 60, 22), terms(380, [2], 800, 23, integer=True),
+        terms(90, [2, 3, 4], 200, 24), terms(64, [2, 9], 150, 25, integer=True))]
+    models += [q.Model("pubo", off=t[0], ids=t[1], coef=t[2]) for t in (
+        terms(200, [2, 3, 4], 600, 26), terms(40, [2, 3], 100, 27, hub=40), terms(70, [2, 10], 90, 28, integer=True))]
+    params = {"seed": 6, "sweeps": 12, "restarts": 9, "beta_start": 0.1, "beta_stop": 2.0, "rng_mode": mode}
+    b = q.Batch(models, SA, {"params": dict(params, kernel=kernel)}).run()
+    first = [b.result(i)["solutions"] for i in range(len(models))]
+    for i, m in enumerate(models):
+        plain = q.Solver(m, SA, {"params": dict(params, kernel="warp")}).init().run().result()
+        assert first[i] == plain["solutions"], i
+    assert [b.run().result(i)["solutions"] for i in range(len(models))] == first
+    pairs = q.Batch(models[:2], SA, {"params": dict(params, kernel=kernel)}).run()
+    assert pairs.stats().kernel == 1 and [pairs.result(i)["solutions"] for i in range(2)] == first[:2]
