@@ -56,6 +56,7 @@
 #include <cmath>
 
 #include "metropolis.cuh"
+#include "ordered_sum.cuh"
 #include "qio_internal.h"
 
 namespace qio
@@ -106,7 +107,7 @@ __host__ __device__ inline int chunk_words(bool pair, int rows)
 {
   return 36 + kIn * 32 * (pair ? 1 : 2) + rows * (pair ? 32 : 33);
 }
-static const int kBufs = 4;  // chunk buffers per walker (a power of two)
+static const int kBufs = 4;  // chunk buffers per walker, at most (Shape::bufs)
 
 __constant__ double c_ln[1024];
 // screen of the ln-table comparison per (row, bucket): y0, dy, error margin;
@@ -341,6 +342,7 @@ struct Shape
   int nw;    // spin words of the population
   int mp;    // term bytes; pair models: a byte per variable
   int rows;  // record rows of a staged block
+  int bufs;  // chunk buffers: kBufs, or one less where another walker then fits
   bool pair;
 };
 struct Region
@@ -357,7 +359,7 @@ struct Region
   float2* ring;              // kRing screen intervals
   uint32_t* raw;             // kRing: stream position after the draw (replay)
   uint4* log;                // kLogBytes (FP64 models)
-  uint2* tiles;              // kBufs block chunks
+  uint2* tiles;              // the block chunks
   uint8_t* z;                // term bytes; pair models: the spins, a byte each
   uint32_t* spins;           // nw + 4 words (words of zeros after the last)
   uint32_t* aspins;          // the accountant's spins (FP64 models), two copies for pair models
@@ -366,7 +368,7 @@ struct Region
 __host__ __device__ inline int tile_words(const Shape& s) { return (chunk_words(s.pair, s.rows) + 1) & ~1; }
 __host__ __device__ inline int region_bytes(const Shape& s, bool integer)
 {
-  return kCtrl + kRing * 12 + (integer ? 0 : kLogBytes) + kBufs * tile_words(s) * 8 + s.mp + 4 * (s.nw + 4) +
+  return kCtrl + kRing * 12 + (integer ? 0 : kLogBytes) + s.bufs * tile_words(s) * 8 + s.mp + 4 * (s.nw + 4) +
          (integer ? 0 : 4 * (s.nw + 4) * (s.pair ? 2 : 1));
 }
 
@@ -388,7 +390,7 @@ __device__ __forceinline__ Region carve(unsigned char* base, const Shape& s)
   R.raw = (uint32_t*)(R.ring + kRing);
   R.log = (uint4*)(R.raw + kRing);
   R.tiles = (uint2*)(R.log + (INT ? 0 : kLogBytes / 16));
-  R.z = (uint8_t*)(R.tiles + kBufs * tile_words(s));
+  R.z = (uint8_t*)(R.tiles + s.bufs * tile_words(s));
   R.spins = (uint32_t*)(R.z + s.mp);
   R.aspins = R.spins + s.nw + 4;
   return R;
@@ -449,12 +451,12 @@ __device__ __forceinline__ uint64_t stream_state(const Region& R, const Walk& W)
 // takes.  Counter streams: the entry of every attempt in turn.  An entry that
 // always accepts is (-inf, -inf).
 //
-// Chunks: block t's goes to buffer t % kBufs once the decider is done with
-// block t - kBufs (t counts over the warp's walkers, from `t0`).
+// Chunks: block t's goes to buffer t % bufs once the decider is done with
+// block t - bufs (t counts over the warp's walkers, from `t0`).
 // ---------------------------------------------------------------------------
 template <int FM, bool REPLAY>
 __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int4* desc, const uint2* table, int tile_w,
-                                  int cap, int nblocks, int total, unsigned t0, uint64_t rs, uint64_t key,
+                                  int cap, int bufs, int nblocks, int total, unsigned t0, uint64_t rs, uint64_t key,
                                   unsigned long long ctr, int n_vars, int* err)
 {
   const int lane = threadIdx.x & 31;
@@ -474,11 +476,11 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
     // what the decider has done
     const unsigned used = ld_acquire(R.used);
     const unsigned blocks = *(volatile unsigned*)R.blocks;
-    while (t < total && t < (int)blocks + kBufs)
+    while (t < total && t < (int)blocks + bufs)
     {
       if (lane == 0)
       {
-        const unsigned at = (t0 + (unsigned)t) % (unsigned)kBufs;
+        const unsigned at = (t0 + (unsigned)t) % (unsigned)bufs;
         tile_issue(R.tiles + at * tile_w, table + d.x, (unsigned)chunk_words(FM == PAIR, min(d.y, cap)) * 8u,
                    &R.bars[at]);
       }
@@ -507,10 +509,10 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
       if (leave == 0) continue;
       // given up: the copies in flight land before the region is
       if (leave == 2 && lane == 0)
-        for (int x = max(0, t - kBufs); x < t; x++)
+        for (int x = max(0, t - bufs); x < t; x++)
         {
           const unsigned n = t0 + (unsigned)x;
-          mbar_wait(&R.bars[n % (unsigned)kBufs], (n / (unsigned)kBufs) & 1u);
+          mbar_wait(&R.bars[n % (unsigned)bufs], (n / (unsigned)bufs) & 1u);
         }
       return;
     }
@@ -774,6 +776,7 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   const void* further = m.fc_in;
   const int tile_w = tile_words(sh), cap = sh.rows;
 
+  unsigned buf = t0 % (unsigned)sh.bufs, par = (t0 / (unsigned)sh.bufs) & 1u;  // the coming chunk's buffer and phase
   unsigned head = 0;                // log entries written
   unsigned acc_tail = 0, fed = 0;   // the other warps' counters when last looked at
   Sweep S;
@@ -793,7 +796,6 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
     const int nvalid = min(32, N - (bi << 5));
     const int v = (bi << 5) + lane;
     // this block's chunk
-    const unsigned turn = t0 + (unsigned)gb, buf = turn % (unsigned)kBufs, par = (turn / (unsigned)kBufs) & 1u;
     if (!__all_sync(kFull, mbar_try(&R.bars[buf], par)))
     {
       const bool landed = mbar_wait(&R.bars[buf], par);
@@ -804,6 +806,12 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
       }
     }
     const uint2* chunk = R.tiles + buf * tile_w;
+    buf++;
+    if (buf == (unsigned)sh.bufs)
+    {
+      buf = 0;
+      par ^= 1u;
+    }
     // the header through shuffles, so that what depends on it is known not to
     // divide the warp: rows, entry rows and further entry rows
     const uint2 head0 = *chunk;
@@ -1180,56 +1188,23 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   return true;
 }
 
-// The running cost over n flips (lane i < n: the i-th difference d) without a
-// chain of FP64 adds, each 64 cycles of its scheduler's FP64 unit.  While the
-// cost stays inside one binade it is a whole number C of its last place u, and
-// fl(cost + d) = (C + rint(d / u)) u unless d / u lies halfway between whole
-// numbers (then the sum's parity decides): so the rounded steps are a prefix
-// sum of integers.  Every prefix has to stay strictly between 2^52 and 2^53 in
-// magnitude, where the sum before rounding lies in the binade too.  False
-// (nothing changed): a tie, a step out of the binade, or a cost or difference
-// that is zero, subnormal or not finite -- the caller adds one by one.
+// The running cost over n flips (lane i < n: the i-th difference d) as a prefix
+// sum of whole numbers (ordered_sum.cuh).  False (nothing changed): a difference
+// for which that does not do -- the caller adds one by one.
 __device__ __forceinline__ bool cost_prefix(double d, int n, double& cost, long long& klow, double& low, int& lowpos)
 {
   const int lane = threadIdx.x & 31;
-  const unsigned long long cb = (unsigned long long)__double_as_longlong(cost);
-  const int ce = (int)((cb >> 52) & 0x7FFu);
-  const unsigned long long kOne = 1ULL << 52;
-  const long long cm = (long long)((cb & (kOne - 1)) | kOne);
-  const long long C = (long long)cb < 0 ? -cm : cm;
-  const unsigned long long db = (unsigned long long)__double_as_longlong(d);
-  const int de = (int)((db >> 52) & 0x7FFu);
-  const unsigned long long dm = (db & (kOne - 1)) | kOne;
-  const int sh = ce - de;
-  bool ok = ce != 0 && ce != 0x7FF;
+  int ce;
+  const long long C = osum::scaled(cost, ce);
   long long D = 0;
-  if (lane < n && (db << 1) != 0ULL)
-  {
-    ok = ok && de != 0 && de != 0x7FF && sh >= 0;  // (|D| < 2^53: no sum overflows)
-    if (ok && sh <= 53)
-    {
-      if (sh > 0)
-      {
-        const unsigned long long rem = dm & ((1ULL << sh) - 1ULL), half = 1ULL << (sh - 1);
-        ok = rem != half;
-        D = (long long)((dm >> sh) + (rem > half ? 1ULL : 0ULL));
-      }
-      else D = (long long)dm;
-      if ((long long)db < 0) D = -D;
-    }
-  }
-  const long long P = C + warp_scan64(D, lane);
-  const long long mag = C < 0 ? -P : P;
-  ok = ok && mag > (long long)kOne && mag < (long long)(kOne << 1);
-  if (!__all_sync(kFull, ok)) return false;
+  bool ok = ce != 0 && ce != 0x7FF;
+  if (ok && lane < n) ok = osum::step_of(d, ce, D);
+  const long long P = C + osum::prefix(D);
+  if (!__all_sync(kFull, ok && osum::inside(C, P))) return false;
   long long mn = P;  // (lanes past n repeat the last prefix)
 #pragma unroll
   for (int s = 16; s; s >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, s));
-  auto value = [&](long long x) -> double {
-    const unsigned long long a = (unsigned long long)(x < 0 ? -x : x) & (kOne - 1);
-    return __longlong_as_double((long long)(((x < 0 ? 1ULL : 0ULL) << 63) | ((unsigned long long)ce << 52) | a));
-  };
-  const double vmin = value(mn);
+  const double vmin = osum::unscaled(mn, ce);
   const long long km = order_key(vmin);
   if (km < klow)
   {
@@ -1237,7 +1212,7 @@ __device__ __forceinline__ bool cost_prefix(double d, int n, double& cost, long 
     low = vmin;
     lowpos = __ffs(__ballot_sync(kFull, P == mn)) - 1;
   }
-  cost = value(__shfl_sync(kFull, P, 31));
+  cost = osum::unscaled(__shfl_sync(kFull, P, 31), ce);
   return true;
 }
 
@@ -1532,7 +1507,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     }
     else if (role == 1)
     {
-      feed<FM, REPLAY>(R, s_scr, m.fc_desc, m.fc_tab, tile_words(sh), sh.rows, (N + 31) >> 5,
+      feed<FM, REPLAY>(R, s_scr, m.fc_desc, m.fc_tab, tile_words(sh), sh.rows, sh.bufs, (N + 31) >> 5,
                        ((N + 31) >> 5) * a.n_sweeps, t0, rs, key,
                        (unsigned long long)a.sweep_base * (unsigned long long)N, N, a.err);
       walker_sync<INT>(bar_id);
@@ -1550,7 +1525,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
       }
     }
     if (*(volatile unsigned*)R.abort) return;
-    t0 += (unsigned)(((N + 31) >> 5) * a.n_sweeps);
+    t0 = (t0 + (unsigned)(((N + 31) >> 5) * a.n_sweeps)) % (unsigned)(2 * sh.bufs);  // buffer and phase
     copy16((uint4*)g_spins, (const uint4*)R.spins, a.p.nw >> 2, me, nme);
     if (FM != PAIR && !queued) copy16((uint4*)g_ts, (const uint4*)R.z, zwords, me, nme);
     walker_sync<INT>(bar_id);  // the region is reused by the next walker
@@ -1612,6 +1587,7 @@ static Shape shape_of(const DevModel& m, int nw, int mp)
   s.nw = nw;
   s.mp = s.pair ? nw * 32 : mp;
   s.rows = std::min(kMaxRows, m.fc_rows);
+  s.bufs = kBufs;
   // a state that leaves less room: smaller tiles (larger blocks read HBM)
   while (s.rows > 4 && kTable + region_bytes(s, m.int_mode != 0) > kMaxSmem) s.rows -= 4;
   return s;
@@ -1628,9 +1604,20 @@ bool fc_fits(const DevModel& m, int nw, int mp)
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb)
 {
   if (!fc_fits(a.m, a.p.nw, a.p.mp)) return cudaErrorInvalidValue;
-  const fc::Shape sh = fc::shape_of(a.m, a.p.nw, a.p.mp);
-  const int per = fc::region_bytes(sh, a.m.int_mode != 0);
-  const int wmax = std::min(a.m.int_mode ? 8 : 4, (fc::kMaxSmem - fc::kTable) / per);
+  fc::Shape sh = fc::shape_of(a.m, a.p.nw, a.p.mp);
+  const bool I = a.m.int_mode != 0;
+  auto fit = [&](int bufs) {
+    sh.bufs = bufs;
+    return std::min(I ? 8 : 4, (fc::kMaxSmem - fc::kTable) / fc::region_bytes(sh, I));
+  };
+  // Three chunk buffers where four would cost a wave of blocks: 512 tempering
+  // walkers of a 4096-variable PUBO, 100 sweeps: 61.3 ms at three walkers a block
+  // with four buffers, 43.7 at four with three.  Otherwise four: the third covers
+  // the copy's latency only just.
+  const int w3 = fit(fc::kBufs - 1), w4 = fit(fc::kBufs);
+  auto waves = [&](int w) { return (a.n_streams + w * fc::kSms - 1) / (w * fc::kSms); };
+  const int wmax = waves(w3) < waves(w4) ? w3 : w4;
+  if (wmax != w4) sh.bufs = fc::kBufs - 1;
   // spread the walkers over the SMs: as few per block as fills them
   int wpc = (a.n_streams + fc::kSms - 1) / fc::kSms;
   if (a.queue) wpc = std::min(wpc, wpb);

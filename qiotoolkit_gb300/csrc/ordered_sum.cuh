@@ -1,0 +1,110 @@
+// ordered_sum.cuh -- FP64 sums in the reference's order without its chain of
+// adds.
+//
+// An FP64 add takes 64 cycles of a scheduler's unit on this chip and waits for
+// the one before it, so 32 values added in order take a warp 2100 cycles (and
+// warps on one scheduler share the unit).  While the running sum c stays inside
+// one binade it is a whole number C of its last place u, and fl(c + d) = (C +
+// rint(d / u)) u unless d / u lies halfway between whole numbers (the sum's
+// parity decides then): so its roundings are a prefix sum of integers.  Every
+// prefix has to stay strictly between 2^52 and 2^53 in magnitude, where the sum
+// before rounding lies in the binade too.  Where one does not -- a tie, a step
+// out of the binade, a sum or value that is zero, subnormal or not finite -- the
+// values before it are taken and that one is added as it is.
+#pragma once
+#include <cstdint>
+
+namespace qio
+{
+namespace osum
+{
+static const unsigned long long kOne = 1ULL << 52;
+
+// the sum c as a whole number of its last place, and its exponent field
+__device__ __forceinline__ long long scaled(double c, int& ce)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(c);
+  ce = (int)((b >> 52) & 0x7FFu);
+  const long long m = (long long)((b & (kOne - 1)) | kOne);
+  return (long long)b < 0 ? -m : m;
+}
+__device__ __forceinline__ double unscaled(long long x, int ce)
+{
+  const unsigned long long a = (unsigned long long)(x < 0 ? -x : x) & (kOne - 1);
+  return __longlong_as_double((long long)(((x < 0 ? 1ULL : 0ULL) << 63) | ((unsigned long long)ce << 52) | a));
+}
+// rint(d / u) for a sum of exponent field ce; false: not to be had this way
+__device__ __forceinline__ bool step_of(double d, int ce, long long& D)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+  D = 0;
+  if ((b << 1) == 0ULL) return true;
+  const int de = (int)((b >> 52) & 0x7FFu), sh = ce - de;
+  if (de == 0 || de == 0x7FF || sh < 0) return false;  // (|D| < 2^53: no sum of 32 overflows)
+  if (sh > 53) return true;
+  const unsigned long long m = (b & (kOne - 1)) | kOne;
+  if (sh > 0)
+  {
+    const unsigned long long rem = m & ((1ULL << sh) - 1ULL), half = 1ULL << (sh - 1);
+    if (rem == half) return false;
+    D = (long long)((m >> sh) + (rem > half ? 1ULL : 0ULL));
+  }
+  else D = (long long)m;
+  if ((long long)b < 0) D = -D;
+  return true;
+}
+// P, of the sign of C, is a prefix inside C's binade
+__device__ __forceinline__ bool inside(long long C, long long P)
+{
+  const long long mag = C < 0 ? -P : P;
+  return mag > (long long)kOne && mag < (long long)(kOne << 1);
+}
+__device__ __forceinline__ long long prefix(long long x)
+{
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1)
+  {
+    const long long y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= d) x += y;
+  }
+  return x;
+}
+
+// c plus the values of the lanes in `keep`, lane by lane; the same c on all
+// lanes
+__device__ __forceinline__ void add_lanes(double v, unsigned keep, double& c)
+{
+  const unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  // three prefixes at most (a sum near zero changes its binade often)
+  for (int round = 0; round < 3 && __popc(keep) > 4; round++)
+  {
+    int ce;
+    const long long C = scaled(c, ce);
+    const bool mine = ((keep >> lane) & 1u) != 0u;
+    long long D = 0;
+    bool ok = true;
+    if (ce == 0 || ce == 0x7FF) ok = false;
+    else if (mine) ok = step_of(v, ce, D);
+    const long long P = C + prefix(D);
+    const unsigned bad = __ballot_sync(kAll, mine && !(ok && inside(C, P)));
+    if (bad == 0u)
+    {
+      c = unscaled(__shfl_sync(kAll, P, 31), ce);
+      return;
+    }
+    const int f = __ffs(bad) - 1;
+    if (f > 0 && ce != 0 && ce != 0x7FF) c = unscaled(__shfl_sync(kAll, P, f - 1), ce);
+    c = __dadd_rn(c, __shfl_sync(kAll, v, f));
+    keep &= ~((2u << f) - 1u);
+  }
+  while (keep)
+  {
+    const int j = __ffs(keep) - 1;
+    keep &= keep - 1;
+    c = __dadd_rn(c, __shfl_sync(kAll, v, j));
+  }
+}
+}  // namespace osum
+}  // namespace qio
