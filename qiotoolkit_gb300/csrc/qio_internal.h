@@ -205,6 +205,8 @@ bool sweep_state_fits(const SweepArgs& a);
 bool fc_fits(const DevModel& m, int nw, int mp);
 // (wpb: walkers per block of a queued launch, at most)
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb);
+// state bytes [n][n_vars] to spin words [n][nw]
+cudaError_t launch_pack_states(const uint8_t* states, long long n, int n_vars, int nw, uint32_t* words, cudaStream_t s);
 cudaError_t launch_eval_cost(const DevModel& m, int n_states,
                              const uint32_t* spins, int nw, double* out,
                              cudaStream_t s);
