@@ -121,62 +121,75 @@ __device__ __forceinline__ uint32_t spin_of(const uint32_t* spins, int v)
   return (spins[v >> 5] >> (v & 31)) & 1u;
 }
 
-// Value of term t under `spins` for the full cost (calculate_cost) and a
-// skip flag for counter models (terms that do not contribute are skipped,
-// as the reference does, rather than added as 0).
+// Four terms of a lane, t0 + 32 u + lane: their state bytes (written to ts unless
+// it is null), and their values; the loads of the four overlap.
 template <int FL, bool INT>
-__device__ __forceinline__ void term_value(const DevModel& m,
-                                           const uint32_t* spins, int t,
-                                           double& val, long long& ival,
-                                           bool& skip)
+__device__ __forceinline__ void four_terms(const DevModel& m, const uint32_t* spins, uint8_t* ts, int t0, int lane,
+                                           double (&v)[4], long long& isum, bool (&skip)[4])
 {
-  int b = m.trow[t], e = m.trow[t + 1];
-  if (FL == F_PARITY || FL == F_PLAIN_ISING)
+  constexpr int U = 4;
+  constexpr bool PAR = FL == F_PARITY || FL == F_PLAIN_ISING;
+  const int M = m.n_terms;
+  int b[U], e[U];
+  uint32_t acc[U];
+#pragma unroll
+  for (int u = 0; u < U; u++)
   {
-    uint32_t par = 0;
-    for (int k = b; k < e; k++) par ^= spin_of(spins, (int)(m.tvar[k] & ~kNegBit));
-    skip = false;
-    if (INT) ival = par ? -(long long)m.tcost_i[t] : (long long)m.tcost_i[t];
-    else val = par ? -m.tcost[t] : m.tcost[t];
+    const int t = t0 + u * 32 + lane;
+    b[u] = t < M ? __ldg(m.trow + t) : 0;
+    e[u] = t < M ? __ldg(m.trow + t + 1) : 0;
+    acc[u] = 0;
   }
-  else
+  // the members of the four terms, position by position
+  for (int k = 0;; k++)
   {
-    // counter: number of true literals; the term contributes when it is 0
-    int cnt = 0;
-    for (int k = b; k < e; k++)
-    {
-      uint32_t x = m.tvar[k];
-      cnt += (int)(spin_of(spins, (int)(x & ~kNegBit)) ^ (x >> 31));
-    }
-    skip = cnt != 0;
-    if (INT) ival = skip ? 0 : (long long)m.tcost_i[t];
-    else val = skip ? 0.0 : m.tcost[t];
+    bool more = false;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (b[u] + k < e[u])
+      {
+        const uint32_t x = __ldg(m.tvar + b[u] + k);
+        const uint32_t sx = spin_of(spins, (int)(x & ~kNegBit));
+        if (PAR) acc[u] ^= sx;
+        else acc[u] += sx ^ (x >> 31);
+        more = more || b[u] + k + 1 < e[u];
+      }
+    if (!more) break;
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++)
+  {
+    const int t = t0 + u * 32 + lane;
+    v[u] = 0.0;
+    skip[u] = true;
+    if (t >= M) continue;
+    if (ts && (FL == F_PARITY || FL == F_COUNTER)) ts[t] = (uint8_t)acc[u];
+    // parity: the term's sign; counter: the term counts when no literal is true
+    skip[u] = PAR ? false : acc[u] != 0;
+    if (INT) isum += skip[u] ? 0 : (PAR && acc[u] ? -(long long)m.tcost_i[t] : (long long)m.tcost_i[t]);
+    else v[u] = skip[u] ? 0.0 : (PAR && acc[u] ? -m.tcost[t] : m.tcost[t]);
   }
 }
 
-// Sum of term values by one warp: lanes evaluate 32 terms in parallel; the
-// FP64 sum runs sequentially in term order (bit-identical to a loop), the
-// integer sum (exact in any order) as per-lane partial sums and a reduction.
+// Term state bytes (written to ts unless it is null) and the cost of a state
+// by one warp.  FP64 values are added in term order (bit-identical to a loop),
+// integers per lane and reduced.
 template <int FL, bool INT>
-__device__ void warp_cost(const DevModel& m, const uint32_t* spins, int lane,
-                          double& cost, long long& icost)
+__device__ void warp_terms_cost(const DevModel& m, const uint32_t* spins, uint8_t* ts, int lane,
+                                double& cost, long long& icost)
 {
   double c = 0.0;
   long long ic = 0;
-  for (int t0 = 0; t0 < m.n_terms; t0 += 32)
+  for (int t0 = 0; t0 < m.n_terms; t0 += 128)
   {
-    int t = t0 + lane;
-    double v = 0.0;
-    long long iv = 0;
-    bool skip = true;
-    if (t < m.n_terms) term_value<FL, INT>(m, spins, t, v, iv, skip);
-    if (INT)
+    double v[4];
+    bool skip[4];
+    four_terms<FL, INT>(m, spins, ts, t0, lane, v, ic, skip);
+    if (!INT)
     {
-      // integer sums are exact in any order: per-lane partial sums
-      if (!skip) ic += iv;
-      continue;
+#pragma unroll
+      for (int u = 0; u < 4; u++) osum::add_lanes(v[u], __ballot_sync(kFull, !skip[u]), c);
     }
-    osum::add_lanes(v, __ballot_sync(kFull, !skip), c);
   }
   if (INT)
   {
@@ -187,74 +200,57 @@ __device__ void warp_cost(const DevModel& m, const uint32_t* spins, int lane,
   icost = ic;
 }
 
-// Term state bytes (written to ts unless it is null) and the cost of a state
-// by one warp in a single pass over the terms; each lane takes four terms at
-// a time so that their loads overlap.  FP64 values are added in term order
-// (bit-identical to a loop), integers per lane and reduced.
-template <int FL, bool INT>
-__device__ void warp_terms_cost(const DevModel& m, const uint32_t* spins, uint8_t* ts, int lane,
-                                double& cost, long long& icost)
+// The same by a block of four warps; the result on thread 0.  A warp alone
+// waits for three dependent loads a term (1.5 M cycles for 20000 terms), so
+// integer models spread the terms over all warps, and FP64 models have three
+// warps evaluate 384 terms into shared memory while the first adds up the 384
+// before them.  Initialising 512 walkers of 20000 FP64 terms 794 to 531 us, 1024
+// of 32768 integer terms 909 to 240 us.
+struct CostBuf
 {
-  constexpr int U = 4;
-  constexpr bool PAR = FL == F_PARITY || FL == F_PLAIN_ISING;
+  double v[2][384];
+  unsigned keep[2][12];
+};
+template <int FL, bool INT>
+__device__ void block_terms_cost(const DevModel& m, const uint32_t* spins, uint8_t* ts, CostBuf& buf, double& cost,
+                                 long long& icost)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double c = 0.0;
   long long ic = 0;
-  const int M = m.n_terms;
-  for (int t0 = 0; t0 < M; t0 += 32 * U)
-  {
-    int b[U], e[U];
-    uint32_t acc[U];
-#pragma unroll
-    for (int u = 0; u < U; u++)
-    {
-      const int t = t0 + u * 32 + lane;
-      b[u] = t < M ? __ldg(m.trow + t) : 0;
-      e[u] = t < M ? __ldg(m.trow + t + 1) : 0;
-      acc[u] = 0;
-    }
-    // the members of the four terms, position by position
-    for (int k = 0;; k++)
-    {
-      bool more = false;
-#pragma unroll
-      for (int u = 0; u < U; u++)
-        if (b[u] + k < e[u])
-        {
-          const uint32_t x = __ldg(m.tvar + b[u] + k);
-          const uint32_t sx = spin_of(spins, (int)(x & ~kNegBit));
-          if (PAR) acc[u] ^= sx;
-          else acc[u] += sx ^ (x >> 31);
-          more = more || b[u] + k + 1 < e[u];
-        }
-      if (!more) break;
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++)
-    {
-      const int t = t0 + u * 32 + lane;
-      double v = 0.0;
-      long long iv = 0;
-      bool skip = true;
-      if (t < M)
-      {
-        if (ts && (FL == F_PARITY || FL == F_COUNTER)) ts[t] = (uint8_t)acc[u];
-        // parity: the term's sign; counter: the term counts when no literal is true
-        skip = PAR ? false : acc[u] != 0;
-        if (INT) iv = skip ? 0 : (PAR && acc[u] ? -(long long)m.tcost_i[t] : (long long)m.tcost_i[t]);
-        else v = skip ? 0.0 : (PAR && acc[u] ? -m.tcost[t] : m.tcost[t]);
-      }
-      if (INT)
-      {
-        if (!skip) ic += iv;
-        continue;
-      }
-      osum::add_lanes(v, __ballot_sync(kFull, !skip), c);
-    }
-  }
+  double v[4];
+  bool skip[4];
   if (INT)
   {
+    for (int t0 = warp * 128; t0 < m.n_terms; t0 += 512) four_terms<FL, INT>(m, spins, ts, t0, lane, v, ic, skip);
 #pragma unroll
     for (int d = 16; d; d >>= 1) ic += __shfl_xor_sync(kFull, ic, d);
+    if (lane == 0) buf.v[0][warp] = __longlong_as_double(ic);
+    __syncthreads();
+    ic = 0;
+    for (int i = 0; i < 4; i++) ic += __double_as_longlong(buf.v[0][i]);
+  }
+  else
+  {
+    const int chunks = (m.n_terms + 383) / 384;
+    for (int k = 0; k <= chunks; k++)
+    {
+      if (warp > 0 && k < chunks)
+      {
+        four_terms<FL, INT>(m, spins, ts, k * 384 + (warp - 1) * 128, lane, v, ic, skip);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+        {
+          const int b = (warp - 1) * 4 + u;
+          buf.v[k & 1][b * 32 + lane] = v[u];
+          const unsigned keep = __ballot_sync(kFull, !skip[u]);
+          if (lane == 0) buf.keep[k & 1][b] = keep;
+        }
+      }
+      if (warp == 0 && k > 0)
+        for (int b = 0; b < 12; b++) osum::add_lanes(buf.v[(k - 1) & 1][b * 32 + lane], buf.keep[(k - 1) & 1][b], c);
+      __syncthreads();
+    }
   }
   cost = c;
   icost = ic;
@@ -286,9 +282,9 @@ __device__ __forceinline__ uint8_t term_state(const DevModel& m,
 template <int FL, bool INT>
 __global__ void __launch_bounds__(128) init_kernel(InitArgs a)
 {
-  const int lane = threadIdx.x & 31;
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= a.n_walkers) return;
+  __shared__ CostBuf buf;
+  const int lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int w = blockIdx.x;  // a block per walker
   const DevModel& m = a.m;
   const int N = m.n_vars;
   const int nwd = (N + 31) >> 5;
@@ -305,68 +301,57 @@ __global__ void __launch_bounds__(128) init_kernel(InitArgs a)
     key = counter_key(a.seed + (uint32_t)(w / a.key_div),
                       a.key_base + (unsigned long long)(w % a.key_div));
   uint64_t rs = replay ? a.rng[w] : 0;
-  for (int q0 = 0; q0 < nwd; q0 += 32)
+  if (var_uniform && !a.given)
   {
-    int q = q0 + lane;
-    uint32_t word = 0;
-    if (a.given)
+    // MaxSat: a word per warp, a variable per lane
+    for (int q = tid >> 5; q < nwd; q += 4)
     {
-      if (q < nwd)
+      const int v = q * 32 + lane;
+      bool bit = false;
+      if (v < N)
+      {
+        if (replay)
+        {
+          uint64_t s0 = jump_any(rs, 2ULL * (unsigned long long)v);
+          uint32_t d0 = pcg_out(s0);
+          uint32_t d1 = pcg_out(s0 * kMult + kInc);
+          bit = canonical(d0, d1) < 0.5;
+        }
+        else
+          bit = (counter_draw(key, kInitCounterBase + (unsigned long long)v) >> 63) == 0;
+      }
+      const unsigned word = __ballot_sync(kFull, bit);
+      if (lane == 0) spins[q] = word;
+    }
+  }
+  else
+    for (int q = tid; q < nwd; q += 128)
+    {
+      uint32_t word = 0;
+      if (a.given)
+      {
         for (int b = 0; b < 32; b++)
         {
           int v = q * 32 + b;
           if (v < N && a.given[(size_t)w * N + v]) word |= 1u << b;
         }
-    }
-    else if (!var_uniform)
-    {
-      if (q < nwd)
-      {
-        if (replay) word = pcg_out(jump_any(rs, (unsigned long long)q));
-        else word = (uint32_t)counter_draw(key, kInitCounterBase + (unsigned long long)q);
       }
-    }
-    else
-    {
-      // MaxSat: bit b of word q0+j is variable 32*(q0+j)+b; lanes take one
-      // variable each, 32 words per pass
-      for (int j = 0; j < 32 && q0 + j < nwd; j++)
-      {
-        int v = (q0 + j) * 32 + lane;
-        bool bit = false;
-        if (v < N)
-        {
-          if (replay)
-          {
-            uint64_t s0 = jump_any(rs, 2ULL * (unsigned long long)v);
-            uint32_t d0 = pcg_out(s0);
-            uint32_t d1 = pcg_out(s0 * kMult + kInc);
-            bit = canonical(d0, d1) < 0.5;
-          }
-          else
-            bit = (counter_draw(key, kInitCounterBase + (unsigned long long)v) >> 63) == 0;
-        }
-        unsigned bw = __ballot_sync(kFull, bit);
-        if (lane == j) word = bw;
-      }
-    }
-    if (q < nwd)
-    {
+      else if (replay) word = pcg_out(jump_any(rs, (unsigned long long)q));
+      else word = (uint32_t)counter_draw(key, kInitCounterBase + (unsigned long long)q);
       if (q == nwd - 1 && (N & 31)) word &= (1u << (N & 31)) - 1u;
       spins[q] = word;
     }
-  }
-  for (int q = nwd + lane; q < a.p.nw; q += 32) spins[q] = 0;
-  if (replay && lane == 0)
+  for (int q = nwd + tid; q < a.p.nw; q += 128) spins[q] = 0;
+  __syncthreads();  // (and every thread has read the walker's stream)
+  if (replay && tid == 0)
     a.rng[w] = jump_any(rs, var_uniform ? 2ULL * (unsigned long long)N
                                         : (unsigned long long)nwd);
-  __syncwarp();
   double cost;
   long long icost;
-  warp_terms_cost<FL, INT>(m, spins, a.skip_terms ? nullptr : ts, lane, cost, icost);
+  block_terms_cost<FL, INT>(m, spins, a.skip_terms ? nullptr : ts, buf, cost, icost);
   if (INT) cost = (double)icost;
-  for (int q = lane; q < a.p.nw; q += 32) lsp[q] = spins[q];
-  if (lane == 0)
+  for (int q = tid; q < a.p.nw; q += 128) lsp[q] = spins[q];
+  if (tid == 0)
   {
     a.p.cost[slot] = cost;
     a.p.lowest[w] = cost;
@@ -386,16 +371,15 @@ __global__ void __launch_bounds__(128) init_kernel(InitArgs a)
 // Evaluation kernels for the per-state contract.
 // ---------------------------------------------------------------------------
 template <int FL, bool INT>
-__global__ void eval_cost_kernel(DevModel m, int n, const uint32_t* spins,
+__global__ void __launch_bounds__(128) eval_cost_kernel(DevModel m, int n, const uint32_t* spins,
                                  int nw, double* out)
 {
-  const int lane = threadIdx.x & 31;
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= n) return;
+  __shared__ CostBuf buf;
+  const int w = blockIdx.x;  // a block per state
   double c;
   long long ic;
-  warp_cost<FL, INT>(m, spins + (size_t)w * nw, lane, c, ic);
-  if (lane == 0) out[w] = INT ? (double)ic : c;
+  block_terms_cost<FL, INT>(m, spins + (size_t)w * nw, nullptr, buf, c, ic);
+  if (threadIdx.x == 0) out[w] = INT ? (double)ic : c;
 }
 
 // State bytes (nonzero: set) to spin words, a warp per four words: bounded by
@@ -1490,9 +1474,7 @@ void upload_tables(int)
 template <int FL, bool INT>
 static void init_dispatch(const InitArgs& a, cudaStream_t s)
 {
-  const int wpb = 4;
-  int blocks = (a.n_walkers + wpb - 1) / wpb;
-  if (blocks > 0) init_kernel<FL, INT><<<blocks, 32 * wpb, 0, s>>>(a);
+  if (a.n_walkers > 0) init_kernel<FL, INT><<<a.n_walkers, 128, 0, s>>>(a);
 }
 
 cudaError_t launch_init(const InitArgs& a, cudaStream_t s)
@@ -1520,8 +1502,7 @@ template <int FL, bool I>
 static void cost_dispatch(const DevModel& m, int n, const uint32_t* sp, int nw,
                           double* out, cudaStream_t s)
 {
-  int blocks = (n + 3) / 4;
-  if (blocks > 0) eval_cost_kernel<FL, I><<<blocks, 128, 0, s>>>(m, n, sp, nw, out);
+  if (n > 0) eval_cost_kernel<FL, I><<<n, 128, 0, s>>>(m, n, sp, nw, out);
 }
 
 cudaError_t launch_eval_cost(const DevModel& m, int n, const uint32_t* sp,
@@ -1610,7 +1591,7 @@ __global__ void eval_cost_noalloc_kernel(DevModel m, int n, const uint8_t* state
   __syncwarp();
   double c;
   long long ic;
-  warp_cost<FL, INT>(m, sp, lane, c, ic);
+  warp_terms_cost<FL, INT>(m, sp, nullptr, lane, c, ic);
   if (lane == 0) out[w] = INT ? (double)ic : c;
 }
 
