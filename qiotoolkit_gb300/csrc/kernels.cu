@@ -14,6 +14,7 @@
 // The result is the reference's trajectory, evaluated up to 32-wide.
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 
 #include "exp_cr.cuh"
 #include "ordered_sum.cuh"
@@ -925,8 +926,8 @@ cudaError_t launch_ssmc_walk(const SsmcArgs& a, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------------------
-// Quantum Monte Carlo: one warp per restart, lanes over its slices (slice k
-// on lane k % 32).  For each variable v of the ordered sweep: every slice
+// Quantum Monte Carlo, any number of slices: one warp per restart, lanes over
+// its slices (slice k on lane k % 32).  For each variable v of the ordered sweep: every slice
 // computes its difference and, for k > 0 with the same value of v as slice
 // k-1, its bond (a uniform() below bond_prob); each run of bonded slices
 // (slice 0 and every unbonded slice start one) sums its differences in slice
@@ -1070,6 +1071,510 @@ __global__ void __launch_bounds__(128) qmc_kernel(QmcArgs a)
     }
     __syncwarp();
   }
+}
+
+// Quantum Monte Carlo of up to 32 slices, two warps to a restart, a lane to a
+// slice.  Variable v's values are one word w[v] (bit k: slice k) in shared
+// memory, so that a term's parities, or whether any other literal is true, take
+// one word operation a member for all slices, lane j taking the row's j-th
+// incidence.  Rows do not depend on the state: their loads run up to four
+// variables ahead.
+//
+// The first warp decides.  The differences' FP64 adds (68 cycles each, one after
+// another) and those of a run's sum (up to 31 more) are not on its way: it sums
+// in FP32, over the runs by one prefix sum, with a bound on its error, and only
+// where sign or comparison lie inside that does it sum as the reference does
+// (exact_run_sum).  Integer models sum exactly.  The second warp gets a word of
+// flips a variable, keeps its own w, and takes the exact differences of the
+// flipped slices into their costs and lowest.
+//
+// What bounds it: the decider's chain of loads, votes and shuffles a variable.
+// N = 1000, 3000 couplings, 16 restarts of 32 slices, 50 sweeps: 145.4 ms with a
+// lane per slice on spins, costs and streams in HBM, 94 with w, costs and
+// streams on the chip and every sum in FP64, @@ here.
+namespace qs
+{
+static const int kRing = 512;  // flip words, a power of two
+static const long long kPatience = 8000000000LL;  // cycles without progress
+struct Sync
+{
+  unsigned head, tail, abort, pad;
+};
+__device__ __forceinline__ unsigned acquire(const unsigned* p)
+{
+  unsigned v;
+  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void release(unsigned* p, unsigned v)
+{
+  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+}
+// waits until *p (counters wrap) reaches `want`; false: given up
+__device__ __noinline__ bool wait_for(const unsigned* p, unsigned want, unsigned* abort, int* err, unsigned& seen)
+{
+  unsigned ok = 1;
+  if ((threadIdx.x & 31) == 0)
+  {
+    const long long t0 = clock64();
+    while (true)
+    {
+      seen = acquire(p);
+      if ((int)(seen - want) >= 0) break;
+      if (acquire(abort) || clock64() - t0 > kPatience)
+      {
+        if (err) atomicExch(err, 1);
+        release(abort, 1u);
+        ok = 0;
+        break;
+      }
+    }
+  }
+  seen = __shfl_sync(kFull, seen, 0);
+  return __shfl_sync(kFull, ok, 0) != 0u;
+}
+
+// A variable's row, lane j holding its j-th incidence (the first 32), loaded
+// ahead: bounds four variables before, incidence and coefficient three, the
+// term's bounds two, its first four members one.  CT: the coefficients' type.
+template <int FL, bool PAIR, class CT>
+struct Rows
+{
+  static constexpr bool PAR = FL == F_PARITY || FL == F_PLAIN_ISING;
+  struct Row { int b, e; };
+  struct Inc { uint32_t x; CT c; };
+  struct Term { int b, e; };
+  struct Mem { uint32_t x[4]; };
+  const int *row, *other, *trow;
+  const uint32_t *inc, *tvar;
+  const CT* coef;
+  int SW, lane, ahead;
+  Row r0, r1, r2, r3, r4;
+  Inc i0, i1, i2, i3;
+  Term t0, t1, t2;
+  Mem f0, f1;
+
+  __device__ __forceinline__ Row load_row(int v) const { return {__ldg(row + v), __ldg(row + v + 1)}; }
+  __device__ __forceinline__ Inc load_inc(Row t, int at) const
+  {
+    Inc o{0u, (CT)0};
+    if (t.b + at < t.e)
+    {
+      o.x = PAIR ? (uint32_t)__ldg(other + t.b + at) : __ldg(inc + t.b + at);
+      o.c = __ldg(coef + t.b + at);
+    }
+    return o;
+  }
+  __device__ __forceinline__ Term load_term(Row t, int at, const Inc& o) const
+  {
+    if (PAIR || t.b + at >= t.e) return {0, 0};
+    const int x = (int)(o.x & ~kNegBit);
+    return {__ldg(trow + x), __ldg(trow + x + 1)};
+  }
+  __device__ __forceinline__ Mem load_mem(const Term& t) const
+  {
+    Mem o;
+#pragma unroll
+    for (int i = 0; i < 4; i++) o.x[i] = !PAIR && t.b + i < t.e ? __ldg(tvar + t.b + i) : 0u;
+    return o;
+  }
+  __device__ __forceinline__ int next(int v) const { return v + 1 < SW ? v + 1 : 0; }
+  __device__ __forceinline__ void start(const DevModel& m, const CT* c, int l)
+  {
+    row = m.row, other = m.other, trow = m.trow, inc = m.inc, tvar = m.tvar, coef = c;
+    SW = m.sweep_size, lane = l;
+    const int v1 = next(0), v2 = next(v1), v3 = next(v2);
+    ahead = next(v3);
+    r0 = load_row(0), r1 = load_row(v1), r2 = load_row(v2), r3 = load_row(v3);
+    i0 = load_inc(r0, lane), i1 = load_inc(r1, lane), i2 = load_inc(r2, lane);
+    t0 = load_term(r0, lane, i0), t1 = load_term(r1, lane, i1);
+    f0 = load_mem(t0);
+  }
+  // the loads that run ahead of the variable in turn
+  __device__ __forceinline__ void issue()
+  {
+    r4 = load_row(ahead);
+    i3 = load_inc(r3, lane);
+    t2 = load_term(r2, lane, i2);
+    f1 = load_mem(t1);
+  }
+  __device__ __forceinline__ void shift()
+  {
+    r0 = r1, r1 = r2, r2 = r3, r3 = r4;
+    i0 = i1, i1 = i2, i2 = i3;
+    t0 = t1, t1 = t2;
+    f0 = f1;
+    ahead = next(ahead);
+  }
+  __device__ __forceinline__ int degree() const { return __shfl_sync(kFull, r0.e - r0.b, 0); }
+  // incidences j0 .. j0 + 31 of variable v, for all slices: the terms' parities,
+  // or the slices in which another literal is true; the coefficients, negated
+  // where v's literal is
+  __device__ __forceinline__ void take(int v, int deg, int j0, const uint32_t* w, uint32_t& on, CT& c) const
+  {
+    Inc o = i0;
+    Term t = t0;
+    Mem f = f0;
+    if (j0)
+    {
+      o = load_inc(r0, j0 + lane);
+      t = load_term(r0, j0 + lane, o);
+      f = load_mem(t);
+    }
+    on = 0u;
+    c = o.c;
+    if (j0 + lane >= deg) return;
+    if (PAIR)
+    {
+      on = w[v] ^ ((int)o.x >= 0 ? w[o.x] : 0u);
+      return;
+    }
+    for (int i = 0; i < t.e - t.b; i++)
+    {
+      const uint32_t x = i == 0 ? f.x[0] : i == 1 ? f.x[1] : i == 2 ? f.x[2] : i == 3 ? f.x[3] : __ldg(tvar + t.b + i);
+      const int u = (int)(x & ~kNegBit);
+      if (PAR) on ^= w[u];
+      else if (u != v) on |= w[u] ^ ((x & kNegBit) ? kFull : 0u);
+    }
+    if (!PAR && (o.x & kNegBit)) c = -c;
+  }
+};
+
+// The slice's exact difference of flipping v, times_minus2 taken (Ising); the
+// sum in row order
+template <int FL, bool INT, bool PAIR, class CT>
+__device__ __forceinline__ double exact_dif(const Rows<FL, PAIR, CT>& R, int v, const uint32_t* w)
+{
+  constexpr bool PAR = FL == F_PARITY || FL == F_PLAIN_ISING;
+  const uint32_t sv = (w[v] >> R.lane) & 1u;
+  const int deg = R.degree();
+  double d = 0.0;
+  int id = 0;
+  for (int j0 = 0; j0 < deg; j0 += 32)
+  {
+    uint32_t on;
+    CT c;
+    R.take(v, deg, j0, w, on, c);
+    const int n = min(32, deg - j0);
+#pragma unroll 4
+    for (int j = 0; j < n; j++)
+    {
+      const uint32_t b = (__shfl_sync(kFull, on, j) >> R.lane) & 1u;
+      const CT x = __shfl_sync(kFull, c, j);
+      if (INT)
+      {
+        if (PAR) id += b ? -(int)x : (int)x;
+        else if (!b) id += sv ? (int)x : -(int)x;
+      }
+      else if (PAR) d = __dadd_rn(d, b ? -(double)x : (double)x);
+      else if (!b) d = __dadd_rn(d, sv ? (double)x : -(double)x);
+    }
+  }
+  if (INT) return (double)(PAR ? -2ll * id : (long long)id);
+  return PAR ? times_minus2(d) : d;
+}
+
+// Rare: a run's sum (lanes first .. end - 1, on its first) as the reference adds
+// it
+template <int FL, bool PAIR>
+__device__ __noinline__ double exact_run_sum(const DevModel& m, int v, const uint32_t* w, bool head, int end)
+{
+  const int lane = threadIdx.x & 31;
+  Rows<FL, PAIR, double> R;
+  R.row = m.row, R.other = m.other, R.trow = m.trow, R.inc = m.inc, R.tvar = m.tvar, R.coef = m.coef;
+  R.SW = m.sweep_size, R.lane = lane;
+  R.r0 = R.load_row(v);
+  R.i0 = R.load_inc(R.r0, lane);
+  R.t0 = R.load_term(R.r0, lane, R.i0);
+  R.f0 = R.load_mem(R.t0);
+  const double dif = exact_dif<FL, false, PAIR, double>(R, v, w);
+  double sum = dif;
+  for (int i = 1; __any_sync(kFull, head && lane + i < end); i++)
+  {
+    const double d = __shfl_down_sync(kFull, dif, i);
+    if (head && lane + i < end) sum = __dadd_rn(sum, d);
+  }
+  return sum;
+}
+}  // namespace qs
+
+template <int FL, bool INT, bool PAIR>
+__global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ QmcArgs a)
+{
+  using namespace qs;
+  constexpr bool PAR = FL == F_PARITY || FL == F_PLAIN_ISING;
+  extern __shared__ uint32_t qmem[];
+  __shared__ Sync sync;
+  __shared__ uint32_t ring[kRing];
+  const DevModel& m = a.m;
+  // (through a shuffle: known to be the same on all lanes)
+  const int role = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0);
+  const int lane = threadIdx.x & 31, r = blockIdx.x;
+  const int P = a.trotter, N = m.n_vars, SW = m.sweep_size, nw = a.p.nw, nwd = (N + 31) >> 5;
+  uint32_t* w = qmem + (role ? N : 0);  // each warp's own
+  const bool mine = lane < P;
+  const int slot = r * P + (mine ? lane : 0);
+  uint32_t* g_spins = a.p.spins + (size_t)slot * nw;
+  if (threadIdx.x == 0) sync.head = sync.tail = sync.abort = 0u;
+  for (int q = 0; q < nwd; q++)
+  {
+    const uint32_t x = mine ? g_spins[q] : 0u;
+    uint32_t out = 0;
+#pragma unroll
+    for (int b = 0; b < 32; b++)
+    {
+      const unsigned y = __ballot_sync(kFull, (x >> b) & 1u);
+      if (lane == b) out = y;
+    }
+    if (q * 32 + lane < N) w[q * 32 + lane] = out;
+  }
+  __syncthreads();
+
+  if (role == 1)
+  {
+    // ---- the accountant
+    double cost = a.p.cost[slot], low = a.low[r];
+    unsigned long long acc_n = 0;
+    unsigned tail = 0, seen = 0;
+    using CT = typename std::conditional<INT, int, double>::type;
+    Rows<FL, PAIR, CT> R;
+    if constexpr (INT) R.start(m, m.coef_i, lane);
+    else R.start(m, m.coef, lane);
+    for (int st = 0; st < a.n_steps; st++)
+    {
+      for (int v = 0; v < SW; v++)
+      {
+        if (seen == tail)
+        {
+          if (lane == 0) release(&sync.tail, tail);
+          if (!wait_for(&sync.head, tail + 1u, &sync.abort, a.err, seen)) return;
+        }
+        R.issue();
+        const uint32_t F = __shfl_sync(kFull, ring[tail & (kRing - 1u)], 0);
+        if (F)
+        {
+          const double d = exact_dif<FL, INT, PAIR, CT>(R, v, w);
+          if ((F >> lane) & 1u)
+          {
+            cost = __dadd_rn(cost, d);
+            acc_n++;
+          }
+          __syncwarp();
+          if (lane == 0) w[v] ^= F;
+          __syncwarp();
+        }
+        tail++;
+        R.shift();
+      }
+      // save_lowest: the first lowest slice
+      double bc = cost;
+      int bk = mine ? lane : INT_MAX;
+#pragma unroll
+      for (int sh = 16; sh; sh >>= 1)
+      {
+        const double oc = __shfl_xor_sync(kFull, bc, sh);
+        const int ok = __shfl_xor_sync(kFull, bk, sh);
+        if (ok != INT_MAX && (bk == INT_MAX || oc < bc || (oc == bc && ok < bk)))
+        {
+          bc = oc;
+          bk = ok;
+        }
+      }
+      if (__any_sync(kFull, bc < low))
+      {
+        low = bc;
+        for (int q = 0; q < nwd; q++)
+        {
+          const int v = q * 32 + lane;
+          const unsigned y = __ballot_sync(kFull, v < N && ((w[min(v, N - 1)] >> bk) & 1u));
+          if (lane == 0) a.low_spins[(size_t)r * nw + q] = y;
+        }
+      }
+    }
+    for (int q = 0; q < nwd; q++)
+    {
+      uint32_t x = 0;
+      for (int b = 0; b < 32 && q * 32 + b < N; b++) x |= ((w[q * 32 + b] >> lane) & 1u) << b;
+      if (mine) g_spins[q] = x;
+    }
+    if (mine)
+    {
+      a.p.cost[slot] = cost;
+      a.p.accepts[slot] += acc_n;
+      a.p.attempts[slot] += (unsigned long long)SW * (unsigned long long)a.n_steps;
+    }
+    if (lane == 0) a.low[r] = low;
+    return;
+  }
+
+  // ---- the decider
+  uint64_t rs = a.replay ? a.rng[slot] : 0;
+  const uint64_t key = a.replay ? 0 : counter_key(a.seed, (uint64_t)slot);
+  // the 64 random bits of one uniform() (qmc_bits)
+  auto bits = [&](unsigned long long ctr) -> unsigned long long {
+    if (!a.replay) return counter_draw(key, ctr);
+    const uint32_t d0 = pcg_out(rs);
+    rs = rs * kMult + kInc;
+    const uint32_t d1 = pcg_out(rs);
+    rs = rs * kMult + kInc;
+    return ((unsigned long long)d1 << 32) | d0;
+  };
+  using CT = typename std::conditional<INT, int, float>::type;
+  Rows<FL, PAIR, CT> R;
+  if constexpr (INT) R.start(m, m.coef_i, lane);
+  else R.start(m, m.coef_f, lane);
+  unsigned head = 0, tail = 0;
+  for (int st = 0; st < a.n_steps; st++)
+  {
+    const long long S = a.step_base + st;
+    const double be = a.beta_eff[S];
+    const float bef = (float)be;
+    const unsigned long long blim = a.bond_lim[S];
+    const bool ball = a.bond_all[S] != 0;
+    for (int v = 0; v < SW; v++)
+    {
+      R.issue();
+      const unsigned long long c = 2ull * ((unsigned long long)S * (unsigned long long)N + (unsigned long long)v);
+      const uint32_t word = w[v];
+      const uint32_t sv = (word >> lane) & 1u;
+      // ---- the slices' differences; `mag`: the sum of their terms' magnitudes
+      float fd = 0.f, mag = 0.f;
+      int id = 0;
+      const int deg = R.degree();
+      for (int j0 = 0; j0 < deg; j0 += 32)
+      {
+        uint32_t on;
+        CT cj;
+        R.take(v, deg, j0, w, on, cj);
+        const int n = min(32, deg - j0);
+#pragma unroll 4
+        for (int j = 0; j < n; j++)
+        {
+          const uint32_t b = (__shfl_sync(kFull, on, j) >> lane) & 1u;
+          const CT x = __shfl_sync(kFull, cj, j);
+          if (INT)
+          {
+            if (PAR) id += b ? -(int)x : (int)x;
+            else id += b ? 0 : (sv ? (int)x : -(int)x);
+          }
+          else
+          {
+            if (PAR) fd += b ? -(float)x : (float)x;
+            else fd += b ? 0.f : (sv ? (float)x : -(float)x);
+            mag += fabsf((float)x);
+          }
+        }
+      }
+      if (PAR)
+      {
+        fd *= -2.f;
+        mag *= 2.f;
+      }
+      // ---- bonds to the slice before, on equal values
+      bool bonded = false;
+      if (mine && lane > 0 && !(((word ^ (word << 1)) >> lane) & 1u))
+      {
+        const unsigned long long x = bits(c);
+        bonded = a.replay ? (ball || x < blim) : ((x >> 11) < blim);
+      }
+      const unsigned B = __ballot_sync(kFull, bonded);
+      const bool first = mine && !bonded;
+      // ---- every run's sum, on its first slice
+      const unsigned above = ~B & ~((2u << lane) - 1u);
+      const int end = min(P, above ? __ffs(above) - 1 : 32);
+      float s, e;
+      bool up, amb = false;
+      double sum = 0.0;
+      bool have = false;  // `sum` is the reference's
+      if (INT)
+      {
+        long long x = PAR ? -2ll * id : (long long)id;
+        const long long own = x;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+        {
+          const long long y = __shfl_up_sync(kFull, x, d);
+          if (lane >= d) x += y;
+        }
+        const long long t = __shfl_sync(kFull, x, end - 1) - x + own;
+        sum = (double)t;
+        s = (float)sum;
+        e = 0.f;
+        up = first && t > 0;
+        have = true;
+      }
+      else
+      {
+        float x = fd;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+        {
+          const float y = __shfl_up_sync(kFull, x, d);
+          if (lane >= d) x += y;
+        }
+        s = __shfl_sync(kFull, x, end - 1) - x + fd;
+        // A difference is off by (deg + 2) 2^-24 of mag, a prefix of 32 of them
+        // by that and six more roundings of 32 mag, their difference by twice
+        // the latter.
+        e = mag * (float)(512 + 40 * (deg + 2)) * 0x1p-24f + 1e-30f;
+        const bool dn = s + e < 0.99e-11f;
+        up = first && s - e > 1.01e-11f;
+        amb = first && !dn && !up;
+        if (__any_sync(kFull, amb))
+        {
+          sum = exact_run_sum<FL, PAIR>(m, v, w, first, end);
+          have = true;
+          if (amb) up = !(sum < 10E-12);
+        }
+      }
+      bool ok = first;
+      unsigned long long ub = 0;
+      amb = false;
+      if (up)
+      {
+        ub = bits(c + 1);
+        // (the screen of qmc_kernel, with the sum's error)
+        const float uf = (float)(uint32_t)(ub >> 40) * 0x1p-24f;
+        const float xf = -bef * s, ef = expf(xf), de = bef * e;
+        const float te = ef * ((fabsf(xf) + 2.0f) * 0x1p-20f + 1.1f * de);
+        amb = !(de < 0.03f);
+        ok = uf + 0x1p-23f < ef - te;
+        amb = amb || !(ok || uf - 0x1p-23f > ef + te);
+      }
+      if (__any_sync(kFull, amb))
+      {
+        if (!INT && !have) sum = exact_run_sum<FL, PAIR>(m, v, w, first, end);
+        if (amb)
+        {
+          const double u = qmc_uniform(a, ub);
+          const double x = exp(__dmul_rn(-be, sum));
+          if (fabs(u - x) <= 1e-15 * x) atomicAdd(a.near_ties, 1ULL);
+          ok = u < x;
+        }
+      }
+      // ---- a run flips as its first slice decides
+      const unsigned H = __ballot_sync(kFull, first), A = __ballot_sync(kFull, ok);
+      const unsigned at = H & ((2u << lane) - 1u);
+      const unsigned F = __ballot_sync(kFull, mine && ((A >> (31 - __clz(at))) & 1u));
+      if (lane == 0)
+      {
+        w[v] = word ^ F;
+        ring[head & (kRing - 1u)] = F;
+      }
+      __syncwarp();
+      head++;
+      R.shift();
+      if ((head & 31u) == 0u)
+      {
+        if (lane == 0) release(&sync.head, head);
+        if (head - tail > (unsigned)kRing - 32u &&
+            !wait_for(&sync.tail, head - (unsigned)kRing + 32u, &sync.abort, a.err, tail))
+          return;
+      }
+    }
+  }
+  if (lane == 0) release(&sync.head, head);
+  if (mine && a.replay) a.rng[slot] = rs;
 }
 
 // Level-parallel QMC sweeps for counter streams (positional draws): one
@@ -1259,6 +1764,19 @@ cudaError_t launch_qmc_levels(const QmcArgs& a, cudaStream_t s)
 template <int FL, bool I>
 static cudaError_t qmc_dispatch(const QmcArgs& a, cudaStream_t s)
 {
+  // a slice per lane where there are lanes and the variables' words fit
+  const size_t words = (size_t)a.m.n_vars * 8;
+  if (a.trotter <= 32 && words <= 200 * 1024)
+  {
+    auto k = FL == F_PARITY && a.m.pair_only ? qmc_sliced_kernel<FL, I, FL == F_PARITY> : qmc_sliced_kernel<FL, I, false>;
+    if (words > 44 * 1024)
+    {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)words);
+      if (e != cudaSuccess) return e;
+    }
+    k<<<a.restarts, 64, words, s>>>(a);
+    return cudaGetLastError();
+  }
   const size_t per_warp = (size_t)a.trotter * 8 + (((size_t)a.trotter * 2 + 7) & ~(size_t)7);
   const int blocks = (a.restarts + 3) / 4;
   const size_t smem = 4 * per_warp;

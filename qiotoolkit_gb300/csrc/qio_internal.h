@@ -402,6 +402,7 @@ struct QmcArgs
   double* low;               // per restart: lowest cost of its slices
   uint32_t* low_spins;       // per restart: that slice's spins (p.nw words)
   unsigned long long* near_ties;  // exp() within 1e-15 of its uniform draw
+  int* err;                  // set when a bounded wait gave up
   // level schedule (counter streams only): variables lv_var[lv_off[t] ..
   // lv_off[t+1]) share no term and follow all their lower-index neighbours'
   // levels; dlog holds each slice's flip differences of a sweep (restarts *

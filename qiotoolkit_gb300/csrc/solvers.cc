@@ -1703,6 +1703,7 @@ class QuantumMonteCarlo : public Solver
     a.low = d_low;
     a.low_spins = d_lspins;
     a.near_ties = d_ties;
+    a.err = device_error_flag();
     a.n_levels = n_levels;
     a.lv_off = d_lv_off;
     a.lv_var = d_lv_var;
