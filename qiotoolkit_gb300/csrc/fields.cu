@@ -4,14 +4,14 @@
 // 143-153,209-229) 32 variables at a time, a variable per lane.  At a block's
 // start every lane gathers its field -- the cost difference of its flip in
 // fixed point (model_host.cc, build_fields) -- from the walker's state in
-// shared memory: the neighbours' spins (Ising models of one- and two-member
-// terms) or one byte per term that holds the literals of all its members.
+// shared memory: a byte per literal of the terms' other members (Ising models of
+// one- and two-member terms: per spin), or one per wide term.
 //
 // The block is then decided as a whole.  Lane v's decision depends on the
 // decisions of the lanes before it in two ways: through the terms it shares
-// with them (fc_in lists these with their members' lanes) and, on replayed
-// streams, through the draw it gets (the uphill lanes before it each take
-// one).  Both only look back, so the lanes iterate: decide with the accept
+// with them (in-block entries list these with their members' lanes) and, on
+// replayed streams, through the draw it gets (the uphill lanes before it each
+// take one).  Both only look back, so the lanes iterate: decide with the accept
 // mask of the last round, vote, and decide again where a member of a lane's
 // in-block terms changed; a mask that no longer changes any lane's terms is the
 // ordered sweep's, lane by lane from the first.  A field within its rounding
@@ -22,30 +22,33 @@
 //
 // A second warp, the FEEDER, runs ahead of the decider: it fills a ring with
 // the walker's random draws as intervals of their ln-table values and brings
-// each block's chunk of the model (records, in-block terms) into one of four
-// shared-memory buffers by one TMA bulk copy.
+// each block's chunk of the model (records, in-block entries) into one of three
+// or four shared-memory buffers by one TMA bulk copy.
 //
 // FP64 models: a third warp, the ACCOUNTANT, consumes a log of the flips in
 // batches of up to 32: every lane recomputes one flip's exact FP64 cost
 // difference (the reference's order and rounding, model/ising.h:108-117,
-// model/pubo.h:335-367), then the running cost is accumulated in flip order
-// exactly as cost_ += diff (markov/walker.h:225) and the lowest state is taken
-// at the first strict improvement (markov/walker.h:269-280) from the
-// accountant's own copy of the spins.  Neither the decisions nor the draws
-// depend on the running cost.  Integer models keep cost and lowest in the
-// decider (exact in any order).
+// model/pubo.h:335-367) from the spins (pair-only Ising) or from the masks of
+// the contributing terms that the decider gathered beside the field, then the
+// running cost is accumulated in flip order exactly as cost_ += diff
+// (markov/walker.h:225) and the lowest state is taken at the first strict
+// improvement (markov/walker.h:269-280) from the accountant's own copy of the
+// spins.  Neither the decisions nor the draws depend on the running cost.
+// Integer models keep cost and lowest in the decider (exact in any order).
 //
 // What bounds it: the decider's chain of dependent votes, shared-memory loads
-// and integer instructions: 1600 cycles a block on a sparse Ising model (N =
-// 1000, 64 walkers: gather 370, decisions 330, wait and publication 320, commit
-// 160), 4200 on a PUBO of 11.7 terms a variable (gather 1040, decisions 600,
-// commit 1600).  A thousand sweeps of the first take 24.7 ms, where fields kept
-// up to date by atomics took 63; 100 sweeps of 512 tempering walkers of the
-// second 62 ms, where the windowed kernel took 190.  Shared-memory atomics have no
-// place in it: one costs 26 to 44 cycles of its warp's memory queue on this
-// chip (a load 5), so a form that kept the fields up to date by atomics on
-// the co-members took 2300 to 7900 cycles a block, and gathering them anew
-// costs less than a few flips' scatter.
+// and integer instructions, about five cycles each: 1650 cycles a block on a
+// sparse Ising model (N = 1000, 64 walkers: gather 400, decisions 340, commit
+// 165), 3600 on a PUBO of 11.7 terms a variable, four walkers an SM (gather
+// 1360, decisions 640, commit 360), 3000 on 3-SAT.  Measured on the way (ms:
+// 1000 sweeps of the first / 100 of 512 tempering walkers of the second / 200 of
+// 64 of the third): fields kept up to date by shared-memory atomics, 26 to 44
+// cycles of the warp's memory queue each where a load takes 5, 40 / 93 / -; the
+// windowed kernel 63 / 190 / 45; gathered from a byte per term, which every flip
+// has to write, 24.6 / 43.7 / 17.6; from literals, where a flip writes two bytes,
+// 24.9 / 35.6 / 13.1; the same with the accountant finding the contributing terms
+// itself, a row a lane, 25.6 / 59 / 15.8 (its scattered loads take the memory
+// pipe from the deciders), or a row a warp, 39 / 147 / 32.
 //
 // Waits between the warps poll shared-memory counters (acquire/release) with a
 // time limit on lack of progress; on expiry the kernel raises the device error
@@ -65,19 +68,15 @@ namespace fc
 {
 using namespace qio::mc;
 static const unsigned kFull = 0xffffffffu;
-static const int kMaxRows = 64;   // records per lane of a staged block, at most
 static const int kIn = 4;         // in-block entries per lane of a staged block
 static const int kLogBytes = 1024;  // flip log per walker: 64 entries of 16 bytes, pair models 256 of 4
 static const int kRing = 128;     // draw intervals per walker (power of 2)
 static const int kCtrl = 64;      // per-walker control block: mbarriers, counters
 static const int kTable = 4096;   // per block: screen row 0
+static const uint32_t kWideMask = 0x0003FFFFu;  // wide term of a record or entry
+static const uint32_t kNoWide = 0x40000000u;    // wide record: padding
+static const uint32_t kSharedWide = 0x20000000u;  // an entry holds its value
 static const unsigned kExactF = 0x80000000u;   // log entry: exact FP64 difference
-// record and in-block entry flags (build_fields)
-static const uint32_t kTermMask = 0x0003FFFFu;
-static const uint32_t kShared = 0x00080000u;   // record: another member in the block
-static const uint32_t kBigTerm = 0x00100000u;  // record: more than eight members
-static const uint32_t kBigEntry = 0x40000000u; // in-block entry: the same
-static const unsigned kNoEntry = 0xffffffffu;  // no in-block entry
 static const int kMaxSmem = 227 * 1024;
 static const int kSms = 152;
 static const long long kPatience = 8000000000LL;  // cycles without progress, about 4 s
@@ -86,27 +85,18 @@ static const long long kPatience = 8000000000LL;  // cycles without progress, ab
 enum Form
 {
   PAIR = 0,     // Ising, terms of one or two members: spins alone
-  COUNTER = 1,  // PUBO, MaxSat: term bytes count true literals
-  PARITY = 2    // Ising with larger terms: term bytes are parities
+  COUNTER = 1,  // PUBO, MaxSat: a term counts when no other literal is true
+  PARITY = 2    // Ising with larger terms: the parity of the other spins
 };
 
-// A block's chunk of the model's table (build_fields), in 8-byte words: header
-// (4: record rows | in-block entry rows << 8 | further entry rows << 16, first
-// further entry), lane data (32), in-block entries (kIn x 32 of 8 or 16 bytes), record
-// rows (of 32; term models 33, a bank's shift, as one lane's records are read
-// across too)
+// A block's chunk of the model's table (DevModel::fc_desc), in 8-byte words
 template <int FM>
 struct Chunk
 {
   static const int kLane = 4;
-  static const int kEnt = 36;
-  static const int kRec = 36 + kIn * 32 * (FM == PAIR ? 1 : 2);
-  static const int kPitch = FM == PAIR ? 32 : 33;
+  static const int kEnt = FM == PAIR ? 36 : 68;
+  static const int kRec = kEnt + kIn * 32 * (FM == PAIR ? 1 : 2);
 };
-__host__ __device__ inline int chunk_words(bool pair, int rows)
-{
-  return 36 + kIn * 32 * (pair ? 1 : 2) + rows * (pair ? 32 : 33);
-}
 static const int kBufs = 4;  // chunk buffers per walker, at most (Shape::bufs)
 
 __constant__ double c_ln[1024];
@@ -117,7 +107,7 @@ __constant__ ulonglong2 c_jump[33];
 static const unsigned long long kMult = 6364136223846793005ULL;
 static const unsigned long long kInc = 1442695040888963407ULL;
 
-// ---- shared-memory synchronisation between the two warps -----------------
+// ---- shared-memory synchronisation between a walker's warps -------------
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
 {
   unsigned v;
@@ -245,47 +235,71 @@ __device__ __noinline__ int counter_chain(uint64_t key, unsigned long long ctr, 
   return lut_less_exact(c_ln, cur, row, __dmul_rn(dE, -beta)) ? 1 : 0;
 }
 
-// Term bytes (COUNTER, PARITY).  A term of up to eight members: bit i set when
-// the literal of its i-th member by variable id is true (Ising: its spin).  A
-// larger term: the count of true literals, or the parity.
-__device__ __forceinline__ bool big_term(const DevModel& m, uint32_t t)
-{
-  return __ldg(m.trow + t + 1) - __ldg(m.trow + t) > 8;
-}
-
-// Exact cost difference of flipping v (FP64 models): the reference's sum
-// over the row in ascending term id, from the spins (pair) or the term bytes.
+// Exact cost difference of flipping v (FP64 models), row entries q .. qe - 1: the
+// reference's sum over the row in ascending term id (model/ising.h:108-117, model/pubo.h:335-367).
+// Members below v have their spins in `after`, the others in `before`.
 template <int FM>
-__device__ __noinline__ double exact_dE(const DevModel& m, int v, const uint32_t* spins, const uint8_t* z)
+__device__ __forceinline__ double exact_dE(const DevModel& m, int v, int q, int qe, const uint32_t* before,
+                                           const uint32_t* after)
 {
-  const int rb = __ldg(m.row + v), re = __ldg(m.row + v + 1);
-  const uint32_t sv = spin_of(spins, v);
+  const uint32_t sv = spin_of(before, v);
+  auto spin = [&](int u) -> uint32_t { return spin_of(u < v ? after : before, u); };
+  auto lit = [&](uint32_t x) -> uint32_t {
+    x &= 0xFFFFu;
+    return x == 0xFFFFu ? 0u : spin((int)(x >> 1)) ^ (x & 1u);
+  };
+  constexpr int U = 4;  // loads in flight ahead of the dependent adds
   double d = 0.0;
-  for (int k = rb; k < re; k++)
+  for (; q < qe; q += U)
   {
-    const double c = __ldg(m.coef + k);
-    if (FM == PAIR)
+    double c[U];
+    uint2 o[U];
+    uint32_t on[U];
+#pragma unroll
+    for (int i = 0; i < U; i++)
     {
-      const int u = __ldg(m.other + k);
-      const uint32_t par = sv ^ (u >= 0 ? spin_of(spins, u) : 0u);
-      d = __dadd_rn(d, par ? -c : c);
-      continue;
+      const bool in = q + i < qe;
+      if (FM == PAIR) o[i] = make_uint2(in ? (uint32_t)__ldg(m.other + q + i) : 0xffffffffu, 0u);
+      else o[i] = in ? __ldg(m.fc_oth + q + i) : make_uint2(0xffffffffu, 0xffffu);
+      c[i] = in ? __ldg(m.coef + q + i) : 0.0;
     }
-    const uint32_t e = __ldg(m.inc + k);
-    uint32_t n = z[e & ~kNegBit];  // true literals, or the parity
-    if (!big_term(m, e & ~kNegBit)) n = (uint32_t)__popc(n);
-    if (FM == PARITY) d = __dadd_rn(d, (n & 1u) ? -c : c);
-    else
+#pragma unroll
+    for (int i = 0; i < U; i++)
     {
-      const bool lit = ((sv ^ (e >> 31)) & 1u) != 0u;
-      if (n == (lit ? 1u : 0u)) d = lit ? __dadd_rn(d, c) : __dsub_rn(d, c);
+      if (FM == PAIR)
+      {
+        on[i] = (int)o[i].x < 0 ? 0u : spin((int)o[i].x);
+        continue;
+      }
+      const uint32_t a = lit(o[i].x), b = lit(o[i].x >> 16), e = lit(o[i].y);
+      on[i] = FM == COUNTER ? (a | b | e) : (a ^ b ^ e);
+      if (o[i].y & (1u << 17))
+      {
+        // a wide term: its members
+        const int t = (int)(__ldg(m.inc + q + i) & ~kNegBit);
+        for (int k = __ldg(m.trow + t), e1 = __ldg(m.trow + t + 1); k < e1; k++)
+        {
+          const uint32_t x = __ldg(m.tvar + k);
+          const int u = (int)(x & ~kNegBit);
+          if (u == v) continue;
+          if (FM == COUNTER) on[i] |= spin(u) ^ (x >> 31);
+          else on[i] ^= spin(u);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < U; i++)
+    {
+      if (q + i >= qe) continue;
+      if (FM != COUNTER) d = __dadd_rn(d, (sv ^ on[i]) ? -c[i] : c[i]);
+      else if (!on[i]) d = (sv ^ (o[i].y >> 16)) & 1u ? __dadd_rn(d, c[i]) : __dsub_rn(d, c[i]);
     }
   }
-  return (FM == COUNTER) ? d : neg2x(d);
+  return FM == COUNTER ? d : neg2x(d);
 }
 
-// Exact cost difference from a log entry's masks (accountant): qm = the
-// contributing incidences, sm = their signs.
+// Exact cost difference from a log entry's masks (accountant): COUNTER: qm = the
+// contributing incidences, sm = their signs; PARITY: all contribute.
 template <int FM>
 __device__ __forceinline__ double dE_from_masks(const double* pc, int deg, uint32_t qm, uint32_t sm)
 {
@@ -339,10 +353,10 @@ __device__ __forceinline__ long long warp_scan64(long long x, int lane)
 // Per-walker shared-memory region, sized for the launch's largest model.
 struct Shape
 {
-  int nw;    // spin words of the population
-  int mp;    // term bytes; pair models: a byte per variable
-  int rows;  // record rows of a staged block
-  int bufs;  // chunk buffers: kBufs, or one less where another walker then fits
+  int nw;     // spin words of the population
+  int zb;     // literal bytes and wide terms' bytes; pair models: a byte per variable
+  int words;  // 8-byte words of a staged chunk (larger blocks read their records from HBM)
+  int bufs;   // chunk buffers: kBufs, or one less where another walker then fits
   bool pair;
 };
 struct Region
@@ -360,15 +374,14 @@ struct Region
   uint32_t* raw;             // kRing: stream position after the draw (replay)
   uint4* log;                // kLogBytes (FP64 models)
   uint2* tiles;              // the block chunks
-  uint8_t* z;                // term bytes; pair models: the spins, a byte each
+  uint8_t* z;                // literals, a byte each, then the wide terms'; pair models: spins
   uint32_t* spins;           // nw + 4 words (words of zeros after the last)
   uint32_t* aspins;          // the accountant's spins (FP64 models), two copies for pair models
 };
 
-__host__ __device__ inline int tile_words(const Shape& s) { return (chunk_words(s.pair, s.rows) + 1) & ~1; }
 __host__ __device__ inline int region_bytes(const Shape& s, bool integer)
 {
-  return kCtrl + kRing * 12 + (integer ? 0 : kLogBytes) + s.bufs * tile_words(s) * 8 + s.mp + 4 * (s.nw + 4) +
+  return kCtrl + kRing * 12 + (integer ? 0 : kLogBytes) + s.bufs * s.words * 8 + s.zb + 4 * (s.nw + 4) +
          (integer ? 0 : 4 * (s.nw + 4) * (s.pair ? 2 : 1));
 }
 
@@ -390,8 +403,8 @@ __device__ __forceinline__ Region carve(unsigned char* base, const Shape& s)
   R.raw = (uint32_t*)(R.ring + kRing);
   R.log = (uint4*)(R.raw + kRing);
   R.tiles = (uint2*)(R.log + (INT ? 0 : kLogBytes / 16));
-  R.z = (uint8_t*)(R.tiles + s.bufs * tile_words(s));
-  R.spins = (uint32_t*)(R.z + s.mp);
+  R.z = (uint8_t*)(R.tiles + s.bufs * s.words);
+  R.spins = (uint32_t*)(R.z + s.zb);
   R.aspins = R.spins + s.nw + 4;
   return R;
 }
@@ -402,24 +415,30 @@ __device__ __forceinline__ void raise_abort(const Region& R, int* err)
   st_release(R.abort, 1u);
 }
 
-// term t's byte from the spins
+// The bytes that the gather reads, from the spins, by thread `me` of `n`: pair
+// models the spins; else the literals (one more is false) and the wide terms'
 template <int FM>
-__device__ __forceinline__ uint8_t term_byte(const DevModel& m, int t, const uint32_t* spins)
+__device__ __noinline__ void make_bytes(const DevModel& m, uint8_t* z, const uint32_t* spins, int nw, int me, int n)
 {
-  const int b = __ldg(m.trow + t), e = __ldg(m.trow + t + 1);
-  uint32_t mask = 0, n = 0;
-  for (int k = b; k < e; k++)
+  for (int v = me; v < 32 * nw; v += n)
   {
-    const uint32_t x = __ldg(m.tvar + k);
-    const uint32_t lit = spin_of(spins, (int)(x & ~kNegBit)) ^ (x >> 31);
-    n += lit;
-    if (e - b > 8) continue;
-    int at = 0;
-    for (int j = b; j < e; j++) at += (__ldg(m.tvar + j) & ~kNegBit) < (x & ~kNegBit);
-    mask |= lit << at;
+    const uint32_t s = spin_of(spins, v);
+    if (FM == PAIR) z[v] = (uint8_t)s;
+    else ((uint16_t*)z)[v] = (uint16_t)(s | (s ^ 1u) << 8);
   }
-  if (e - b <= 8) return (uint8_t)mask;
-  return (uint8_t)(FM == PARITY ? n & 1u : n);
+  if (FM == PAIR) return;
+  if (me < 16) z[64 * nw + me] = (uint8_t)(me & 1);
+  for (int i = me; i < m.fc_wide; i += n)
+  {
+    const int t = __ldg(m.fc_wterm + i);
+    uint32_t c = 0;
+    for (int k = __ldg(m.trow + t), e = __ldg(m.trow + t + 1); k < e; k++)
+    {
+      const uint32_t x = __ldg(m.tvar + k);
+      c += spin_of(spins, (int)(x & ~kNegBit)) ^ (FM == COUNTER ? x >> 31 : 0u);
+    }
+    z[64 * nw + 16 + i] = (uint8_t)(FM == PARITY ? c & 1u : c);
+  }
 }
 
 // Mutable state of one walker's decider.
@@ -481,7 +500,7 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
       if (lane == 0)
       {
         const unsigned at = (t0 + (unsigned)t) % (unsigned)bufs;
-        tile_issue(R.tiles + at * tile_w, table + d.x, (unsigned)chunk_words(FM == PAIR, min(d.y, cap)) * 8u,
+        tile_issue(R.tiles + at * tile_w, table + d.x, (unsigned)min(d.y, cap) * 8u,
                    &R.bars[at]);
       }
       t++;
@@ -506,7 +525,11 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
         leave = 2;
       }
       leave = __shfl_sync(kFull, leave, 0);
-      if (leave == 0) continue;
+      if (leave == 0)
+      {
+        __nanosleep(100);  // (its polls would take the decider's turns at shared memory)
+        continue;
+      }
       // given up: the copies in flight land before the region is
       if (leave == 2 && lane == 0)
         for (int x = max(0, t - bufs); x < t; x++)
@@ -727,26 +750,25 @@ __device__ __forceinline__ void account_int(const Region& R, Walk& W, bool scan3
   }
 }
 
-// a flip's change of a term that it shares within the block (x: in-block entry)
+// a flip's change of a wide term's byte, v's literal `lit` before it (several
+// lanes may hold the term, or its word's other bytes)
 template <int FM>
-__device__ __forceinline__ void flip_shared(uint8_t* z, unsigned x, uint32_t sv)
+__device__ __forceinline__ void flip_wide(uint8_t* zw, unsigned t, uint32_t lit)
 {
-  const unsigned t = x & kTermMask, sh = (t & 3u) * 8u;
-  unsigned* word = (unsigned*)(z + (t & ~3u));
-  if (!(x & kBigEntry)) atomicXor(word, 1u << (sh + ((x >> 23) & 7u)));
-  else if (FM == PARITY) atomicXor(word, 1u << sh);
-  else if ((sv ^ (x >> 31)) & 1u) atomicSub(word, 1u << sh);
+  const unsigned sh = (t & 3u) * 8u;
+  unsigned* word = (unsigned*)(zw + (t & ~3u));
+  if (FM == PARITY) atomicXor(word, 1u << sh);
+  else if (lit) atomicSub(word, 1u << sh);
   else atomicAdd(word, 1u << sh);
 }
 
 // Lane f's attempt alone: the reference's sum, draws and comparison.  Bit 0:
 // accepted; bit 1: it drew.
 template <int FM, bool REPLAY, bool INT>
-__device__ __noinline__ unsigned exact_attempt(const DevModel& m, int v, int g, const uint32_t* spins, const uint8_t* z,
-                                              uint64_t rs, uint64_t key, unsigned long long ctr, double beta,
-                                              double* dE_out)
+__device__ __noinline__ unsigned exact_attempt(const DevModel& m, int v, int g, const uint32_t* spins, uint64_t rs,
+                                              uint64_t key, unsigned long long ctr, double beta, double* dE_out)
 {
-  const double dE = INT ? (double)g : exact_dE<FM>(m, v, spins, z);
+  const double dE = INT ? (double)g : exact_dE<FM>(m, v, __ldg(m.row + v), __ldg(m.row + v + 1), spins, spins);
   const bool inf = ((unsigned long long)__double_as_longlong(beta) & 0x7FFFFFFFFFFFFFFFULL) == 0x7FF0000000000000ULL;
   *dE_out = dE;
   if (le_zero(dE)) return 1u;
@@ -760,6 +782,7 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
 {
   constexpr int KI = kIn;  // in-block entries held in registers
   constexpr int kLog = FM == PAIR ? kLogBytes / 4 : kLogBytes / 16;  // entries, a power of two
+  constexpr bool MASKS = !INT && FM != PAIR;  // the log needs the row's masks, and weights carry row positions
   using C = Chunk<FM>;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -768,13 +791,13 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   const int total = nblocks * a.n_sweeps;
   if (total <= 0) return true;
   const bool scan32 = m.scan32 != 0;
-  const bool big = m.fc_big != 0;
   const double inv = m.fc_inv;
   // (read once: `m` may be the launch's parameter or lie in device memory)
   const uint2* table = m.fc_tab;
   const int4* descs = m.fc_desc;
   const void* further = m.fc_in;
-  const int tile_w = tile_words(sh), cap = sh.rows;
+  const int cap = sh.words;
+  uint8_t* zw = R.z + 64 * sh.nw + 16;  // the wide terms' bytes
 
   unsigned buf = t0 % (unsigned)sh.bufs, par = (t0 / (unsigned)sh.bufs) & 1u;  // the coming chunk's buffer and phase
   unsigned head = 0;                // log entries written
@@ -787,12 +810,11 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   for (int gb = 0; gb < total; gb++)
   {
     bi++;
-    if (bi == nblocks)
+    if (bi == nblocks || gb == 0)
     {
       bi = 0;
-      k++;
+      next_sweep<FM, INT>(S, a, inv, N, k++);
     }
-    if (bi == 0) next_sweep<FM, INT>(S, a, inv, N, k);
     const int nvalid = min(32, N - (bi << 5));
     const int v = (bi << 5) + lane;
     // this block's chunk
@@ -805,20 +827,27 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
         return false;
       }
     }
-    const uint2* chunk = R.tiles + buf * tile_w;
+    const uint2* chunk = R.tiles + buf * cap;
     buf++;
-    if (buf == (unsigned)sh.bufs)
-    {
-      buf = 0;
-      par ^= 1u;
-    }
+    par ^= buf == (unsigned)sh.bufs ? 1u : 0u;
+    buf = buf == (unsigned)sh.bufs ? 0u : buf;
     // the header through shuffles, so that what depends on it is known not to
     // divide the warp: rows, entry rows and further entry rows
     const uint2 head0 = *chunk;
-    const unsigned sizes = __shfl_sync(kFull, head0.x, 0);
-    const int rows = (int)(sizes & 255u), ents = (int)((sizes >> 8) & 255u), xn = (int)(sizes >> 16);
+    const unsigned h0 = __shfl_sync(kFull, head0.x, 0);
+    const unsigned h1 = __shfl_sync(kFull, head0.y, 0);
+    const int n0 = (int)(h0 & 127u) * 4, n1 = FM == PAIR ? 0 : (int)((h0 >> 7) & 255u) * 2;
+    const int n2 = FM == PAIR ? 0 : (int)((h0 >> 15) & 255u) * 2, n3 = FM == PAIR ? 0 : (int)(h1 & 255u);
+    const int ents = (int)((h0 >> 23) & 7u), xn = (int)(h1 >> 8);
+    const bool staged = C::kRec + 32 * (n0 + n1 + n2 + n3) + 16 * n2 <= cap;
     const uint2* tile = chunk + lane;
-    const int2 own = *(const int2*)(tile + C::kLane);
+    int4 own;  // field, degree, negated literals, terms of v alone
+    if (FM == PAIR)
+    {
+      const int2 x = *(const int2*)(tile + C::kLane);
+      own = make_int4(x.x, x.y, 0, 0);
+    }
+    else own = *((const int4*)(chunk + C::kLane) + lane);
     const uint4* tent = (const uint4*)(chunk + C::kEnt) + lane;
 
     const uint32_t word = R.spins[bi];  // the block's spins before its flips
@@ -827,61 +856,92 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
     const int bnd = deg + 1;  // |field - exact| < bnd units
     const float xmargin = INT ? 0.f : S.fsa * (float)(bnd + 1);
 
-    // ---- the field; term models: the row's contributing incidences (qm)
-    int base = FM == PAIR ? own.x : 0;
-    unsigned qm = 0;
-    // one record of a term model: true when the other literals are all false
-    // (COUNTER), or the parity of the other members is odd
-    auto term = [&](const uint32_t x) -> bool {
-      const uint32_t zz = R.z[x & kTermMask];
-      if (big && (x & kBigTerm))
-        return FM == COUNTER ? zz == ((sv ^ (x >> 18)) & 1u) : ((zz ^ sv) & 1u) != 0u;
-      return FM == COUNTER ? (zz & (x >> 24)) == 0u : (__popc(zz & (x >> 24)) & 1) != 0;
-    };
-    // a flipped variable's unshared term: its byte after
-    auto put = [&](uint32_t x, uint32_t zz, uint32_t spin) {
-      uint32_t zn = zz ^ (~(x >> 24) & 255u);
-      if (big && (x & kBigTerm)) zn = FM == PARITY ? zz ^ 1u : (((spin ^ (x >> 18)) & 1u) ? zz - 1u : zz + 1u);
-      if (!(x & kShared)) R.z[x & kTermMask] = (uint8_t)zn;
-    };
-    // (rows come in fours; the next four's records are under way meanwhile)
-    auto gather = [&](const uint2* t0) {
-      unsigned bit = 1u;
-      uint2 e[4];
-#pragma unroll
-      for (int x = 0; x < 4; x++) e[x] = rows ? t0[C::kPitch * x] : make_uint2(0u, 0u);
-      for (int i = 4; i <= rows; i += 4)
+    // ---- the field: the lane's value less the weights of the records whose
+    // op is 1.  Rows come in fours (one literal) and twos; the next ones'
+    // records are under way meanwhile.
+    int base = own.x;
+    unsigned qm = (unsigned)own.w;  // COUNTER: the incidences that contribute; PARITY: those of odd parity
+    auto op = [](uint32_t x, uint32_t y) -> uint32_t { return FM == COUNTER ? (x | y) : (x ^ y); };
+    // a record's op (0 or 1) and weight into field and mask
+    auto put = [&](uint32_t on, uint32_t w) {
+      if (MASKS)
       {
-        uint2 f[4];
-        const uint2* t1 = t0 + C::kPitch * (i < rows ? i : 0);
+        base -= (int)on * (int)(w & ~255u);
+        if ((FM == COUNTER) != (on != 0u)) qm |= __funnelshift_l(0u, 1u, w);
+      }
+      else base -= (int)on * (int)w;
+    };
+    auto gather = [&](const uint2* t0) {
+      {
+        uint2 e[4];
 #pragma unroll
-        for (int x = 0; x < 4; x++) f[x] = t1[C::kPitch * x];
-        if (FM == PAIR)
+        for (int x = 0; x < 4; x++) e[x] = n0 ? t0[32 * x] : make_uint2(0u, 0u);
+        for (int i = 4; i <= n0; i += 4)
         {
+          uint2 f[4];
+          const uint2* t1 = t0 + 32 * (i < n0 ? i : 0);
 #pragma unroll
-          for (int x = 0; x < 4; x++) base -= (int)R.z[e[x].x] * (int)e[x].y;
+          for (int x = 0; x < 4; x++) f[x] = t1[32 * x];
+#pragma unroll
+          for (int x = 0; x < 4; x++) put(R.z[e[x].x], e[x].y);
+#pragma unroll
+          for (int x = 0; x < 4; x++) e[x] = f[x];
         }
-        else
+      }
+      if (FM == PAIR) return;
+      t0 += 32 * n0;
+      if (n1)
+      {
+        uint2 e0 = t0[0], e1 = t0[32];
+        for (int i = 2; i <= n1; i += 2)
         {
-          bool t[4];
-#pragma unroll
-          for (int x = 0; x < 4; x++) t[x] = term(e[x].x);
-#pragma unroll
-          for (int x = 0; x < 4; x++)
-          {
-            if (FM == COUNTER) base += t[x] ? (int)e[x].y : 0;
-            else base += t[x] ? -(int)e[x].y : (int)e[x].y;
-            if (!INT && t[x]) qm |= bit << x;
-          }
-          bit <<= 4;
+          const uint2* t1 = t0 + 32 * (i < n1 ? i : 0);
+          const uint2 f0 = t1[0], f1 = t1[32];
+          const uint32_t a0 = R.z[e0.x & 0xFFFFu], b0 = R.z[e0.x >> 16], a1 = R.z[e1.x & 0xFFFFu], b1 = R.z[e1.x >> 16];
+          put(op(a0, b0), e0.y);
+          put(op(a1, b1), e1.y);
+          e0 = f0;
+          e1 = f1;
         }
-#pragma unroll
-        for (int x = 0; x < 4; x++) e[x] = f[x];
+        t0 += 32 * n1;
+      }
+      if (n2)
+      {
+        const uint32_t* c0 = (const uint32_t*)(t0 - lane + 32 * n2) + lane;  // the third literals
+        uint2 e0 = t0[0], e1 = t0[32];
+        uint32_t k0 = c0[0], k1 = c0[32];
+        for (int i = 2; i <= n2; i += 2)
+        {
+          const int nx = i < n2 ? i : 0;
+          const uint2 f0 = t0[32 * nx], f1 = t0[32 * nx + 32];
+          const uint32_t g0 = c0[32 * nx], g1 = c0[32 * nx + 32];
+          const uint32_t a0 = R.z[e0.x & 0xFFFFu], b0 = R.z[e0.x >> 16], d0 = R.z[k0];
+          const uint32_t a1 = R.z[e1.x & 0xFFFFu], b1 = R.z[e1.x >> 16], d1 = R.z[k1];
+          put(op(op(a0, b0), d0), e0.y);
+          put(op(op(a1, b1), d1), e1.y);
+          e0 = f0;
+          e1 = f1;
+          k0 = g0;
+          k1 = g1;
+        }
+        t0 += 48 * n2;
+      }
+      // wide terms: the true literals but for the own, or the others' parity
+      for (int i = 0; i < n3; i++)
+      {
+        const uint2 e = t0[32 * i];
+        const uint32_t zz = zw[e.x & kWideMask];
+        const uint32_t on = FM == COUNTER ? (zz != ((sv ^ (e.x >> 31)) & 1u) ? 1u : 0u) : ((zz ^ sv) & 1u);
+        if (!(e.x & (kNoWide | kSharedWide))) put(on, e.y);
       }
     };
-    if (rows <= cap) gather(tile + C::kRec);
-    else gather(table + __ldg(descs + bi).x + C::kRec + lane);
-    if (!INT && FM != PAIR) qm &= deg >= 32 ? kFull : ((1u << deg) - 1u);  // (padding records)
+    const uint2* far = table;  // (not staged) the records
+    if (staged) gather(tile + C::kRec);
+    else
+    {
+      far = table + __ldg(descs + bi).x + C::kRec + lane;
+      gather(far);
+    }
 
     // ---- the in-block terms under a given accept mask, all against the state
     // at the block's start.  Pair models: the member's flip changes the field
@@ -891,23 +951,28 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
     // 1: never).  Parities: c0 of the others, and of the flips in em.
     unsigned watch = 0;  // lanes whose flips change this lane's field
     int val[KI];
+    unsigned bit[KI];  // its place in the mask
     unsigned em[KI], et[KI];
-    unsigned elog[KI];  // term, position in the row (5 bits), position in the term (3), big
     // further entries (rare): xn of them, in HBM
-    const size_t xat = xn ? (size_t)__shfl_sync(kFull, head0.y, 0) + lane : 0;
+    const size_t xat = xn ? (size_t)__shfl_sync(kFull, chunk[1].x, 0) + lane : 0;
     const uint2* xpair = (const uint2*)further + xat;
     const uint4* xterm = (const uint4*)further + xat;
     unsigned done = 0;  // the block's flips so far
     // an entry's em and et; D: flips whose bytes are written already
     auto entry = [&](const uint4& e, unsigned D, unsigned& mm, unsigned& mt) {
-      const uint32_t zz = R.z[e.x & kTermMask];
-      const int n = (e.x & kBigEntry) ? (int)zz : __popc(zz);
-      const uint32_t M = e.y & lt, L = (word ^ e.z) & M;  // members before this lane, their true literals
-      // the other true literals, as of the block's start
-      const int o = n - (int)(sv ^ (e.x >> 31)) - (__popc(M & D) - 2 * __popc(L & D));
+      const uint32_t M = e.x, L = (word ^ e.y) & M;  // members before this lane, their true literals
+      const bool wide = FM != PAIR && (e.z >> 18) == 0x3FFFu;
+      uint32_t o;  // the other members: whether a literal is true, or their parity
+      if (!wide) o = op(R.z[e.z & 0xFFFFu], R.z[e.z >> 16]);
+      else
+      {
+        const uint32_t zz = zw[e.z & kWideMask], lit = (sv ^ (e.y >> lane)) & 1u;
+        if (FM == COUNTER) o = (int)zz - (int)lit != __popc((L ^ D) & M) ? 1u : 0u;
+        else o = (zz ^ sv ^ (uint32_t)__popc((word ^ D) & M)) & 1u;
+      }
       mm = M;
-      mt = FM == COUNTER ? L : (unsigned)o & 1u;
-      if (FM == COUNTER && o != __popc(L))
+      mt = FM == COUNTER ? L : (o ^ (uint32_t)__popc(word & M)) & 1u;
+      if (FM == COUNTER && o)
       {
         mm = 0u;
         mt = 1u;
@@ -919,6 +984,10 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
 #pragma unroll
     for (int i = 0; i < KI; i++)
     {
+      em[i] = bit[i] = 0u;
+      et[i] = 1u;
+      val[i] = 0;
+      if (FM != PAIR && i >= 2 && ents <= 2) continue;  // (most blocks have two at most)
       if (FM == PAIR)
       {
         const uint2 e = tile[C::kEnt + 32 * i];
@@ -930,13 +999,12 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
       {
         const uint4 e = tent[32 * i];
         entry(e, 0u, em[i], et[i]);
-        val[i] = (int)e.w;
-        elog[i] = e.x;
-        watch |= e.y & lt;
-        if (e.y == 0u) elog[i] = kNoEntry;
+        val[i] = MASKS ? (int)(e.w & ~255u) : (int)e.w;
+        bit[i] = MASKS && e.x ? __funnelshift_l(0u, 1u, e.w) : 0u;
+        watch |= e.x;
       }
     }
-    for (int i = 0; i < xn; i++) watch |= FM == PAIR ? __ldg(xpair + 32 * i).x : (__ldg(&xterm[32 * i].y) & lt);
+    for (int i = 0; i < xn; i++) watch |= FM == PAIR ? __ldg(xpair + 32 * i).x : __ldg(&xterm[32 * i].x);
 
     // ---- the other warps: room for this block's flips and draws
     auto room = [&]() -> bool {
@@ -952,7 +1020,6 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
         if (!room()) return false;
       }
     }
-    const uint32_t negs = (uint32_t)own.x;  // term models: the row's negated literals
 
     // ---- rounds: one, unless a lane has to be tried alone
     float2 iv0 = make_float2(0.f, 0.f);
@@ -963,18 +1030,26 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
       const bool active = lane >= cursor && lane < nvalid;
       const unsigned before = lt & ~((1u << cursor) - 1u);
       // ---- decisions: iterate until no lane's in-block members change
-      unsigned A = done, U = 0;
+      unsigned A = done, U = 0, lm = 0;
       int g = 0;
       bool rare = false;
       while (true)
       {
         int h = base;
+        lm = qm;
 #pragma unroll
         for (int i = 0; i < KI; i++)
         {
-          if (FM == PAIR) h += (A & em[i]) ? val[i] : 0;
-          else if (FM == COUNTER) h += holds(A, em[i], et[i]) ? val[i] : 0;
-          else h += holds(A, em[i], et[i]) ? -val[i] : val[i];
+          if (FM != PAIR && i >= 2 && ents <= 2) continue;
+          if (FM == PAIR)
+          {
+            h += (A & em[i]) ? val[i] : 0;
+            continue;
+          }
+          const bool on = holds(A, em[i], et[i]);
+          if (FM == COUNTER) h += on ? val[i] : 0;
+          else h += on ? -val[i] : val[i];
+          if (MASKS && on) lm |= bit[i];
         }
         for (int i = 0; i < xn; i++)
         {
@@ -988,9 +1063,11 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
             const uint4 e = __ldg(xterm + 32 * i);
             unsigned mm, mt;
             entry(e, done, mm, mt);
-            const bool on = holds(A, mm, mt);
-            if (FM == COUNTER) h += on ? (int)e.w : 0;
-            else h += on ? -(int)e.w : (int)e.w;
+            const bool on = e.x && holds(A, mm, mt);
+            const int w = MASKS ? (int)(e.w & ~255u) : (int)e.w;
+            if (FM == COUNTER) h += on ? w : 0;
+            else h += on ? -w : w;
+            if (MASKS && on) lm |= __funnelshift_l(0u, 1u, e.w);
           }
         }
         // the field in the variable's own direction, its sign and threshold
@@ -1006,13 +1083,14 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
         else if (FM == COUNTER)
         {
           const int fd = sv ? (h >> 8) : -(h >> 8);
-          const bool zero = (h & 255) == 0;  // nothing contributes: +0.0
+          const bool zero = lm == 0u;  // nothing contributes: +0.0
           up = active && !zero && fd > bnd;
           rare = active && !zero && (unsigned)(fd + bnd) <= (unsigned)(2 * bnd);
           x = (float)fd;
         }
         else
         {
+          if (FM == PARITY) h >>= 8;
           g = sv ? -h : h;
           up = active && g < -bnd;
           rare = active && (unsigned)(g + bnd) <= (unsigned)(2 * bnd);
@@ -1031,7 +1109,7 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
         const bool no = iv.x > __fadd_rn(thr, et);
         rare = rare || (up && !yes && !no);
         const bool acc = active && !rare && (!up || yes);
-        if (!INT && FM != PAIR) rare = rare || (acc && deg > 32);  // its masks do not fit the log
+        if (MASKS) rare = rare || (acc && deg > 32);  // its masks do not fit the log
         const unsigned An = __ballot_sync(kFull, acc) | done;
         const unsigned diff = An ^ A;
         A = An;
@@ -1062,12 +1140,12 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
           const uint64_t rs = REPLAY ? stream_state(R, W) : 0;
           unsigned res = 0;
           if (lane == f)
-            res = exact_attempt<FM, REPLAY, INT>(m, v, g, R.spins, R.z, rs, W.key, S.ctr0 + (unsigned long long)v,
-                                                 S.beta, &dE);
+            res = exact_attempt<FM, REPLAY, INT>(m, v, g, R.spins, rs, W.key, S.ctr0 + (unsigned long long)v, S.beta,
+                                                 &dE);
           res = __shfl_sync(kFull, res, f);
-          exact = true;
           F = (res & 1u) << f;
           if (REPLAY) W.taken += res >> 1;
+          exact = true;
           cursor = f + 1;
         }
         last = cursor >= nvalid;
@@ -1075,93 +1153,39 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
       const bool mine = ((F >> lane) & 1u) != 0u;
       const unsigned at = (head + (unsigned)__popc(F & lt)) & (unsigned)(kLog - 1);
       const unsigned all = done | F;
-      if (FM == PAIR)
+      if (!INT && mine)
       {
-        if (!INT && mine) ((uint32_t*)R.log)[at] = (uint32_t)v;
-        if (mine) R.z[v] = (uint8_t)(sv ^ 1u);
-      }
-      else if (F)
-      {
-        // ---- the flips' log masks and term bytes.  In-block terms: their bits
-        // under the final mask (an exact attempt's entry has no masks).
-        unsigned lm = qm;
-        auto log_bit = [&](unsigned x, bool on) {
-          if (x == kNoEntry) return;
-          const uint32_t bit = 1u << ((x >> 18) & 31u);
-          lm = on ? lm | bit : lm & ~bit;
-        };
-        if (!INT)
+        if (FM == PAIR) ((uint32_t*)R.log)[at] = (uint32_t)v;
+        else
         {
-#pragma unroll
-          for (int i = 0; i < KI; i++) log_bit(elog[i], holds(A, em[i], et[i]));
-          for (int i = 0; i < xn && !exact; i++)
-          {
-            const uint4 e = __ldg(xterm + 32 * i);
-            unsigned mm, mt;
-            entry(e, done, mm, mt);
-            if (e.y) log_bit(e.x, holds(A, mm, mt));
-          }
-          __syncwarp();  // the bytes have been read
-        }
-        // Terms of one member in the block: plain stores, the byte is this
-        // block's alone.  The warp over the flips' records, sixteen lanes to a
-        // flip, eight flips' loads under way at a time.
-        auto flips = [&](const uint2* t0) {
-          const int half = lane >> 4, sub = lane & 15;
-          unsigned fl = F;
-          while (fl)
-          {
-            uint32_t x[4], zz[4];
-            int jj[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-            {
-              const int j0 = fl ? __ffs(fl) - 1 : -1;
-              fl &= fl - 1u;
-              const int j1 = fl ? __ffs(fl) - 1 : -1;
-              fl &= fl - 1u;
-              jj[i] = half ? j1 : j0;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) x[i] = jj[i] >= 0 && sub < rows ? t0[C::kPitch * sub + (jj[i] - lane)].x : kShared;
-#pragma unroll
-            for (int i = 0; i < 4; i++) zz[i] = R.z[x[i] & kTermMask];
-#pragma unroll
-            for (int i = 0; i < 4; i++) put(x[i], zz[i], (word >> (jj[i] & 31)) & 1u);
-            for (int at = 16 + sub; at < rows; at += 16)
-            {
-#pragma unroll
-              for (int i = 0; i < 4; i++) x[i] = jj[i] >= 0 ? t0[C::kPitch * at + (jj[i] - lane)].x : kShared;
-#pragma unroll
-              for (int i = 0; i < 4; i++) zz[i] = R.z[x[i] & kTermMask];
-#pragma unroll
-              for (int i = 0; i < 4; i++) put(x[i], zz[i], (word >> (jj[i] & 31)) & 1u);
-            }
-          }
-        };
-        if (rows <= cap) flips(tile + C::kRec);
-        else flips(table + __ldg(descs + bi).x + C::kRec + lane);
-        // Terms of several: every flip changes its own bit (or the count by
-        // one), in any order.
-#pragma unroll
-        for (int i = 0; i < KI; i++)
-          if (i < ents && mine && elog[i] != kNoEntry) flip_shared<FM>(R.z, elog[i], sv);
-        for (int i = 0; i < xn; i++)
-        {
-          const uint4 e = __ldg(xterm + 32 * i);
-          if (mine && e.y) flip_shared<FM>(R.z, e.x, sv);
-        }
-        if (!INT && mine)
-        {
+          const unsigned long long bits = (unsigned long long)__double_as_longlong(dE);
+          const unsigned negs = (unsigned)own.z;
           uint4 ent;
           ent.x = (unsigned)v | ((unsigned)deg << 16) | (exact ? kExactF : 0u);
-          const unsigned long long bits = (unsigned long long)__double_as_longlong(dE);
-          // COUNTER: the sign is the literal; PARITY: the term's bit, the
-          // other members' parity and the own spin
+          // COUNTER: the sign is the literal; PARITY: the term's, the other
+          // members' parity and the own spin
           ent.y = exact ? (unsigned)bits : lm;
           ent.z = exact ? (unsigned)(bits >> 32) : (FM == COUNTER ? (sv ? ~negs : negs) : (sv ? ~lm : lm));
           ent.w = 0u;
           R.log[at] = ent;
+        }
+      }
+      if (FM == PAIR)
+      {
+        if (mine) R.z[v] = (uint8_t)(sv ^ 1u);
+      }
+      else if (F)
+      {
+        if (!INT && xn) __syncwarp();  // (entries have been read)
+        if (mine) ((uint16_t*)R.z)[v] = (uint16_t)((sv ^ 1u) | sv << 8);
+        if (n3 && mine)
+        {
+          const uint2* t3 = (staged ? tile + C::kRec : far) + 32 * (n0 + n1) + 48 * n2;
+          for (int i = 0; i < n3; i++)
+          {
+            const uint32_t x = t3[32 * i].x;
+            if (!(x & kNoWide)) flip_wide<FM>(zw, x & kWideMask, (sv ^ (x >> 31)) & 1u);
+          }
         }
       }
       __syncwarp();
@@ -1224,14 +1248,25 @@ template <int FM>
 __device__ __noinline__ bool account(const SweepArgs& a, const DevModel& m, const Region R, double& cost,
                                         double& low, uint32_t* g_lsp)
 {
-  constexpr int kLog = FM == PAIR ? kLogBytes / 4 : kLogBytes / 16;
   const int lane = threadIdx.x & 31;
   const int nw = a.p.nw;
-  const int* row = m.row;
-  const double* coef = m.coef;
-  const int* other = m.other;
+  constexpr int kLog = FM == PAIR ? kLogBytes / 4 : kLogBytes / 16;
   unsigned tail = 0;
   long long klow = order_key(low);
+  // the coming batch's entries and row bounds, in the lanes below `ready`: their
+  // loads run beside the sum over the batch before
+  int v = 0, q0 = 0, q1 = 0, ready = 0;
+  uint4 ent = make_uint4(0u, 0u, 0u, 0u);
+  auto fetch = [&](unsigned at) {
+    if (FM == PAIR) v = (int)((const uint32_t*)R.log)[at & (unsigned)(kLog - 1)];
+    else
+    {
+      ent = R.log[at & (unsigned)(kLog - 1)];
+      v = (int)(ent.x & 0x7FFFu);
+    }
+    q0 = __ldg(m.row + v);
+    q1 = __ldg(m.row + v + 1);
+  };
   while (true)
   {
     // wait for a batch (16 entries, or whatever is left once the decider is done)
@@ -1278,59 +1313,33 @@ __device__ __noinline__ bool account(const SweepArgs& a, const DevModel& m, cons
     while (h != tail)
     {
       int n = (int)min(32u, h - tail);
-      int v = 0;
       double d = 0.0;
+      if (lane < n && lane >= ready) fetch(tail + (unsigned)lane);
       if (FM == PAIR)
       {
-        // Flips of one sweep, in index order: a neighbour below the flip has
-        // its spin after the batch, one above it its spin before.
+        // Flips of one sweep, in index order: a member below the flip has its
+        // spin after the batch, one above it its spin before.
         uint32_t* after = R.aspins + nw + 4;
-        if (lane < n) v = (int)((const uint32_t*)R.log)[(tail + (unsigned)lane) & (unsigned)(kLog - 1)];
         const int prev = __shfl_up_sync(kFull, v, 1);
         const unsigned wrap = __ballot_sync(kFull, lane > 0 && lane < n && v <= prev);
         if (wrap) n = __ffs(wrap) - 1;
         if (lane < n) atomicXor(after + (v >> 5), 1u << (v & 31));
         __syncwarp();
-        if (lane < n)
-        {
-          const uint32_t sv = spin_of(R.aspins, v);
-          const int q1 = __ldg(row + v + 1);
-          for (int q = __ldg(row + v); q < q1; q += 8)
-          {
-            // eight loads in flight ahead of the dependent adds
-            double c[8];
-            int u[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-            {
-              u[i] = q + i < q1 ? __ldg(other + q + i) : -1;
-              c[i] = q + i < q1 ? __ldg(coef + q + i) : 0.0;
-            }
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-            {
-              const uint32_t su = u[i] < 0 ? 0u : spin_of(u[i] < v ? after : R.aspins, u[i]);
-              if (sv ^ su) c[i] = -c[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-              if (q + i < q1) d = __dadd_rn(d, c[i]);
-          }
-          d = neg2x(d);
-        }
+        if (lane < n) d = exact_dE<FM>(m, v, q0, q1, R.aspins, after);
       }
       else if (lane < n)
       {
-        const uint4 ent = R.log[(tail + (unsigned)lane) & (unsigned)(kLog - 1)];
-        v = (int)(ent.x & 0x7FFFu);
         const int deg = (int)((ent.x >> 16) & 255u);
         if (ent.x & kExactF)
           d = __longlong_as_double((long long)((unsigned long long)ent.y | ((unsigned long long)ent.z << 32)));
-        else d = dE_from_masks<FM>(coef + __ldg(row + v), deg, ent.y, ent.z);
+        else d = dE_from_masks<FM>(m.coef + q0, deg, ent.y, ent.z);
       }
       __syncwarp();
       tail += (unsigned)n;
       if (lane == 0) st_release(R.tail, tail);
+      const int fv = v;  // this batch's
+      ready = (int)min(32u, h - tail);
+      if (lane < ready) fetch(tail + (unsigned)lane);
       // running cost in flip order (markov/walker.h:225) and the first
       // strict improvement of the lowest (markov/walker.h:269-280)
       int lowpos = -1;
@@ -1352,14 +1361,14 @@ __device__ __noinline__ bool account(const SweepArgs& a, const DevModel& m, cons
         }
       }
       // the accountant's spins, and the lowest state at lowpos
-      if (lane < n && lane <= lowpos) atomicXor(R.aspins + (v >> 5), 1u << (v & 31));
+      if (lane < n && lane <= lowpos) atomicXor(R.aspins + (fv >> 5), 1u << (fv & 31));
       __syncwarp();
       if (lowpos >= 0)
       {
         for (int q = lane; q < nw; q += 32) g_lsp[q] = R.aspins[q];
         __syncwarp();
       }
-      if (lane < n && lane > lowpos) atomicXor(R.aspins + (v >> 5), 1u << (v & 31));
+      if (lane < n && lane > lowpos) atomicXor(R.aspins + (fv >> 5), 1u << (fv & 31));
       __syncwarp();
     }
     if (fin == 1) return true;
@@ -1432,8 +1441,6 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     const int N = m.n_vars;
     const int slot = a.slot_of ? a.slot_of[r] : r;
     uint32_t* g_spins = a.p.spins + (size_t)slot * a.p.nw;
-    uint8_t* g_ts = a.p.tstate + (size_t)slot * a.p.mp;
-    const int zwords = FM == PAIR ? 0 : (m.n_terms + 15) >> 4;  // 16-byte words
     if (queued && REPLAY) rs = a.rng[r];
     if (decider && lane == 0)
     {
@@ -1449,19 +1456,9 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     if (me < 4) R.spins[a.p.nw + me] = 0u;
     if (!INT) copy16((uint4*)R.aspins, (const uint4*)g_spins, a.p.nw >> 2, me, nme);
     if (!INT && FM == PAIR) copy16((uint4*)(R.aspins + a.p.nw + 4), (const uint4*)g_spins, a.p.nw >> 2, me, nme);
-    // term bytes: as the last launch left them, or from the spins
-    if (FM != PAIR && a.terms_valid) copy16((uint4*)R.z, (const uint4*)g_ts, zwords, me, nme);
     walker_sync<INT>(bar_id);
-    if (FM != PAIR && !a.terms_valid)
-    {
-      for (int t = me; t < m.n_terms; t += nme) R.z[t] = term_byte<FM>(m, t, R.spins);
-      walker_sync<INT>(bar_id);
-    }
-    if (FM == PAIR)
-    {
-      for (int v = me; v < ((N + 31) & ~31); v += nme) R.z[v] = (uint8_t)spin_of(R.spins, v);
-      walker_sync<INT>(bar_id);
-    }
+    make_bytes<FM>(m, R.z, R.spins, a.p.nw, me, nme);
+    walker_sync<INT>(bar_id);
 
     uint64_t key = 0;
     if (!REPLAY)
@@ -1507,7 +1504,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     }
     else if (role == 1)
     {
-      feed<FM, REPLAY>(R, s_scr, m.fc_desc, m.fc_tab, tile_words(sh), sh.rows, sh.bufs, (N + 31) >> 5,
+      feed<FM, REPLAY>(R, s_scr, m.fc_desc, m.fc_tab, sh.words, sh.words, sh.bufs, (N + 31) >> 5,
                        ((N + 31) >> 5) * a.n_sweeps, t0, rs, key,
                        (unsigned long long)a.sweep_base * (unsigned long long)N, N, a.err);
       walker_sync<INT>(bar_id);
@@ -1527,7 +1524,6 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     if (*(volatile unsigned*)R.abort) return;
     t0 = (t0 + (unsigned)(((N + 31) >> 5) * a.n_sweeps)) % (unsigned)(2 * sh.bufs);  // buffer and phase
     copy16((uint4*)g_spins, (const uint4*)R.spins, a.p.nw >> 2, me, nme);
-    if (FM != PAIR && !queued) copy16((uint4*)g_ts, (const uint4*)R.z, zwords, me, nme);
     walker_sync<INT>(bar_id);  // the region is reused by the next walker
     if (!queued)
     {
@@ -1579,32 +1575,35 @@ static cudaError_t go_fm(const SweepArgs& a, cudaStream_t s, int wpc, const Shap
   return I ? go<FM, false, true>(a, s, wpc, sh) : go<FM, false, false>(a, s, wpc, sh);
 }
 
-// a walker's region for a model in a population of these strides
-static Shape shape_of(const DevModel& m, int nw, int mp)
+// a walker's region for a model in a population of this stride
+static Shape shape_of(const DevModel& m, int nw)
 {
   Shape s;
   s.pair = m.flavor == F_PARITY && m.pair_only;
   s.nw = nw;
-  s.mp = s.pair ? nw * 32 : mp;
-  s.rows = std::min(kMaxRows, m.fc_rows);
+  s.zb = s.pair ? nw * 32 : (64 * nw + 16 + m.fc_wide + 15) & ~15;
+  s.words = m.fc_words;
   s.bufs = kBufs;
-  // a state that leaves less room: smaller tiles (larger blocks read HBM)
-  while (s.rows > 4 && kTable + region_bytes(s, m.int_mode != 0) > kMaxSmem) s.rows -= 4;
+  // a state that leaves less room: smaller tiles (larger blocks read their
+  // records from HBM)
+  const int least = Chunk<COUNTER>::kRec;
+  const int room = (kMaxSmem - kTable - region_bytes(s, m.int_mode != 0)) / (8 * kBufs);
+  if (room < 0) s.words = std::max(least, (s.words + room - 1) & ~1);
   return s;
 }
 }  // namespace fc
 
-bool fc_fits(const DevModel& m, int nw, int mp)
+bool fc_fits(const DevModel& m, int nw)
 {
   if (!m.fc_desc || m.sweep_size != m.n_vars || m.n_vars <= 0) return false;
   if (!(m.flavor == F_PARITY || m.flavor == F_COUNTER)) return false;
-  return fc::kTable + fc::region_bytes(fc::shape_of(m, nw, mp), m.int_mode != 0) <= fc::kMaxSmem;
+  return fc::kTable + fc::region_bytes(fc::shape_of(m, nw), m.int_mode != 0) <= fc::kMaxSmem;
 }
 
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb)
 {
-  if (!fc_fits(a.m, a.p.nw, a.p.mp)) return cudaErrorInvalidValue;
-  fc::Shape sh = fc::shape_of(a.m, a.p.nw, a.p.mp);
+  if (!fc_fits(a.m, a.p.nw)) return cudaErrorInvalidValue;
+  fc::Shape sh = fc::shape_of(a.m, a.p.nw);
   const bool I = a.m.int_mode != 0;
   auto fit = [&](int bufs) {
     sh.bufs = bufs;

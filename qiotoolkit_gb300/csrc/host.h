@@ -77,9 +77,9 @@ struct HostModel
   std::vector<unsigned int> rec_p;  // other << 8 | coefficient, when |coef| <= 127
   // block-decided sweep tables (see DevModel::fc_desc; empty: not eligible)
   std::vector<int> fc_desc;
-  std::vector<uint32_t> fc_tab, fc_in;
-  int fc_rows = 0;
-  bool fc_big = false;
+  std::vector<uint32_t> fc_tab, fc_in, fc_oth;
+  std::vector<int> fc_wide;
+  int fc_words = 0;
   int fc_S = 0;
   bool fc_pack = false;
   // level schedule (levels.cu): entries grouped by level, their offsets

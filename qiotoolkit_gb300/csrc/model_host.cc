@@ -1,6 +1,5 @@
 // model_host.cc -- model construction and upload, schedules, device setup.
 #include <algorithm>
-#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -9,6 +8,7 @@
 #include <map>
 #include <mutex>
 #include <set>
+#include <unordered_map>
 
 #include "host.h"
 
@@ -141,7 +141,7 @@ static void build_graph(HostModel& m, int64_t n_terms, const int64_t* off,
   if (n_terms <= 0)
     fail(1, "parameter `terms`: size must be greater than 0, found 0");
   const bool merge = (m.kind == K_PUBO || m.kind == K_PUBO_PLAIN);
-  std::map<int32_t, int> name_to_id;
+  std::unordered_map<int32_t, int> name_to_id;
   std::vector<std::vector<int>> members;
   std::vector<std::vector<int>> node_edges;
   m.min_loc = INT32_MAX;
@@ -357,23 +357,29 @@ static void build_near(HostModel& m)
 // Tables of the block-decided sweep (fields.cu).  A variable's field H_v is its
 // flip's cost difference, up to its own spin's sign, in fixed point q =
 // round(c * 2^S):
-//   pair-only Ising: H_v = sum of q over its one-member terms plus, over its
-//     two-member terms, q * (1 - 2 s_u) with u the other member; the cost
-//     difference of flipping v is -2 (1 - 2 s_v) H_v;
-//   Ising with larger terms: the same with the parity of the term's other
-//     members in place of s_u;
+//   Ising: H_v = sum over v's terms of q, negated where the product of the other
+//     members' spins is; the cost difference of flipping v is -2 (1 - 2 s_v) H_v;
 //   counter models: H_v = sum over the terms none of whose other literals is
 //     true of +q (v's literal plain) or -q (negated); the cost difference is
 //     H_v when s_v is true and -H_v otherwise.
-// S is the largest scale with 2^S * max_v sum_row |c| <= 2^30 (2^22 when the
-// field also carries the number of contributing terms in its low 8 bits), so
+// S is the largest scale with 2^S * max_v sum_row |c| <= 2^30 (2^22 when a
+// weight also carries its term's row position in its low 8 bits), so
 // a field never overflows and differs from the reference's FP64 sum by less
 // than deg + 1 units.  Integer models use S = 0: the field is then exact.
+//
+// A term is kept as its other members' literals: literal 2u + 1 is u negated, 2N
+// none (false).  Terms of more than four members are wide: the sweep keeps a
+// byte for each (true literals, or the parity).
 // Eligible: Ising with the term cache or counter models, fewer than 32766
 // variables and 2^18 terms, rows of at most 255 incidences.
 static void build_fields(HostModel& m)
 {
   m.fc_desc.clear();
+  m.fc_tab.clear();
+  m.fc_in.clear();
+  m.fc_oth.clear();
+  m.fc_wide.clear();
+  m.fc_words = 0;
   if (!(m.flavor == F_PARITY || m.flavor == F_COUNTER) || m.N == 0 || m.N >= 32766) return;
   if (!m.pair_only && m.M >= (1 << 18)) return;  // (a term's byte would not fit shared memory)
   double amax = 0;
@@ -384,7 +390,7 @@ static void build_fields(HostModel& m)
     for (int q = m.row[v]; q < m.row[v + 1]; q++) s += std::fabs(m.coef[q]);
     amax = std::max(amax, s);
   }
-  m.fc_pack = !m.int_mode && m.flavor == F_COUNTER;
+  m.fc_pack = !m.int_mode && !m.pair_only;
   if (m.int_mode) m.fc_S = 0;
   else
   {
@@ -394,99 +400,191 @@ static void build_fields(HostModel& m)
     m.fc_S = amax > 0 ? top - e : 0;
     if (m.fc_S < -900 || m.fc_S > 900) return;  // 2^-S must stay a normal double
   }
-  auto fixed = [&](int q) -> int {
+  // (sums of these wrap as the device's do; what they end in does not)
+  auto fixed = [&](int q) -> uint32_t {
     long long f = m.int_mode ? (long long)m.coef_i[q] : std::llrint(std::ldexp(m.coef[q], m.fc_S));
-    return (int)(m.fc_pack ? f * 256 : f);
+    return (uint32_t)(int)(m.fc_pack ? f * 256 : f);
   };
-  const bool pair = m.pair_only;
+  const bool pair = m.pair_only, ising = m.flavor == F_PARITY;
   const int nb = (int)((m.N + 31) / 32);
   const int KI = 4;  // fields.cu: entries per lane of a block's chunk
-  const int ew = pair ? 2 : 4, pitch = pair ? 32 : 33;  // 32-bit words of an entry, records of a row
-  const size_t ent_at = 8 + 64;                         // 32-bit words before a chunk's entries
+  const int ew = pair ? 2 : 4;                          // 32-bit words of an entry
+  const size_t ent_at = 8 + (pair ? 64 : 128);          // 32-bit words before a chunk's entries
   const size_t rec_at = ent_at + (size_t)KI * 32 * ew;  // ... and its records
+  const uint32_t none = (uint32_t)(2 * m.N);
+  std::vector<int> wide_of;  // term -> wide term, or -1
+  if (!pair)
+  {
+    wide_of.assign((size_t)m.M, -1);
+    for (int64_t t = 0; t < m.M; t++)
+      if (m.trow[t + 1] - m.trow[t] > 4)
+      {
+        wide_of[t] = (int)m.fc_wide.size();
+        m.fc_wide.push_back((int)t);
+      }
+    m.fc_oth.assign((size_t)m.K * 2, 0);
+  }
   m.fc_desc.assign((size_t)nb * 4, 0);
-  m.fc_tab.clear();
-  m.fc_in.clear();
-  m.fc_rows = 0;
-  m.fc_big = false;
+  struct Rec { uint32_t lit[3]; uint32_t val; };
+  struct Entry { uint32_t w[4]; };
+  std::vector<Rec> rec[32][3];  // by number of others
+  std::vector<Entry> in[32], wide[32];
+  m.fc_tab.reserve((size_t)m.K * 3 + (size_t)nb * rec_at);
   for (int b = 0; b < nb; b++)
   {
     const int v0 = b * 32, v1 = (int)std::min<int64_t>(m.N, v0 + 32);
-    int* d = &m.fc_desc[(size_t)b * 4];
-    int rows = 0, kin = 0;
-    for (int v = v0; v < v1; v++) rows = std::max(rows, m.row[v + 1] - m.row[v]);
-    rows = (rows + 3) & ~3;
-    m.fc_rows = std::max(m.fc_rows, rows);
-    const size_t at = m.fc_tab.size();
-    d[0] = (int)(at / 2);
-    d[1] = rows;
-    m.fc_tab.resize(at + ((rec_at + (size_t)rows * pitch * 2 + 3) & ~(size_t)3), 0u);
-    uint32_t* tab = &m.fc_tab[at];
-    if (!pair)  // padding records: a flip leaves them alone
-      for (size_t r = 0; r < (size_t)rows * pitch; r++) tab[rec_at + 2 * r] = 1u << 19;
-    std::vector<std::array<uint32_t, 4>> in[32];
+    for (int l = 0; l < 32; l++)
+    {
+      for (auto& r : rec[l]) r.clear();
+      in[l].clear();
+      wide[l].clear();
+    }
+    uint32_t base[32] = {}, degree[32] = {}, negs[32] = {}, alone[32] = {};
+    int rows[4] = {}, kin = 0;
     for (int l = 0; l < 32; l++)
     {
       const int v = v0 + l;
       const int deg = v < v1 ? m.row[v + 1] - m.row[v] : 0;
-      int sum = 0;        // pair: all coefficients (spins all up)
-      uint32_t negs = 0;  // else: the row's negated literals
+      degree[l] = (uint32_t)deg;
       for (int k = 0; k < deg; k++)
       {
         const int q = m.row[v] + k;
-        const uint32_t t = m.inc[q] & ~kNegBit, vneg = m.inc[q] >> 31;
-        const int f = fixed(q);
-        const int tb = m.trow[t], te = m.trow[t + 1];
-        const bool big = te - tb > 8;
-        // members by id: the variable's position, and the others in the block
-        uint32_t pos = 0, mates = 0, neg = 0;
-        for (int j = tb; j < te; j++)
-        {
-          const uint32_t u = m.tvar[j] & ~kNegBit;
-          if ((int)u < v) pos++;
-          if ((int)u == v || (int)u < v0 || (int)u >= v0 + 32) continue;
-          mates |= 1u << (u - v0);
-          if (m.tvar[j] & kNegBit) neg |= 1u << (u - v0);
-        }
-        uint32_t* r = tab + rec_at + ((size_t)k * pitch + l) * 2;
+        const uint32_t f = fixed(q);
         if (pair)
         {
           const int u = m.other[q];
-          sum += f;
+          base[l] += f;
           if (u < 0) continue;
-          r[0] = (uint32_t)u;
-          r[1] = (uint32_t)(2 * f);
-          if (mates && u < v) in[l].push_back({mates, (uint32_t)(2 * f), 0, 0});
+          rec[l][0].push_back({{(uint32_t)u, 0, 0}, 2u * f});
+          if (u >= v0 && u < v) in[l].push_back({{1u << (u - v0), 2u * f, 0, 0}});
           continue;
         }
-        const int val = m.flavor == F_PARITY ? f : (vneg ? -f : f) + (m.fc_pack ? 1 : 0);
-        if (big) pos = 0;
-        r[0] = t | (vneg << 18) | (mates ? 1u << 19 : 0u) | (big ? 1u << 20 : 0u) |
-               (big ? 0u : (~(1u << pos) & 255u) << 24);
-        r[1] = mates ? 0u : (uint32_t)val;  // (a shared term's value is in its in-block entry)
-        if (k < 32) negs |= vneg << k;
-        m.fc_big = m.fc_big || big;
-        if (mates)
-          in[l].push_back({t | ((uint32_t)(k & 31) << 18) | (pos << 23) | (big ? 0x40000000u : 0u) | (vneg << 31),
-                           mates, neg, (uint32_t)val});
+        const uint32_t t = m.inc[q] & ~kNegBit, vneg = m.inc[q] >> 31;
+        const uint32_t val = ising ? f : (vneg ? 0u - f : f);
+        const uint32_t at = m.fc_pack ? (uint32_t)(k & 31) : 0u;  // the row position beside a weight
+        if (k < 32) negs[l] |= vneg << k;
+        // the other members: before this one in the block, and the rest
+        uint32_t mates = 0, neg = 0, lit[3] = {none, none, none};
+        int n = 0;
+        uint32_t rest[2] = {none, none};
+        int nrest = 0;
+        for (int j = m.trow[t]; j < m.trow[t + 1]; j++)
+        {
+          const uint32_t u = m.tvar[j] & ~kNegBit, un = ising ? 0u : m.tvar[j] >> 31;
+          if ((int)u == v) continue;
+          if (wide_of[t] < 0) lit[n++] = 2 * u + un;
+          if ((int)u >= v0 && (int)u < v)
+          {
+            mates |= 1u << (u - v0);
+            neg |= un << (u - v0);
+          }
+          else if (nrest < 2) rest[nrest++] = 2 * u + un;  // (more only without mates, or wide)
+        }
+        uint32_t* o = &m.fc_oth[(size_t)q * 2];
+        for (int i = 0; i < 3; i++) lit[i] = i < n ? lit[i] : none;
+        o[0] = (n > 0 ? lit[0] : 0xFFFFu) | (n > 1 ? lit[1] : 0xFFFFu) << 16;
+        o[1] = (n > 2 ? lit[2] : 0xFFFFu) | vneg << 16 | (wide_of[t] >= 0 ? 1u << 17 : 0u);
+        if (wide_of[t] >= 0)
+        {
+          const uint32_t w = (uint32_t)wide_of[t];
+          wide[l].push_back({{w | vneg << 31, (mates ? 0u : ising ? 2u * f : val) | at, mates ? 1u : 0u, 0}});
+          if (mates) in[l].push_back({{mates, neg | vneg << l, 0xFFFC0000u | w, val | at}});
+        }
+        else if (mates)
+        {
+          in[l].push_back({{mates, neg, rest[0] | rest[1] << 16, val | at}});
+        }
+        else if (n > 0) rec[l][n - 1].push_back({{lit[0], lit[1], lit[2]}, (ising ? 2u * f : val) | at});
+        else if (!ising) alone[l] |= 1u << (k & 31);
+        if (!mates) base[l] += val;
       }
-      tab[8 + 2 * l] = pair ? (uint32_t)sum : negs;
-      tab[8 + 2 * l + 1] = (uint32_t)deg;
       kin = std::max(kin, (int)in[l].size());
+      rows[3] = std::max(rows[3], (int)wide[l].size());
     }
+    // Rows of records of one, two and three literals (a shorter one may fill a
+    // longer one's row)
+    for (int l = 0; l < 32; l++) rows[2] = std::max(rows[2], (int)rec[l][2].size());
+    rows[2] = (rows[2] + 1) & ~1;
+    auto left = [&](int l, int c) {  // records that the longer rows leave
+      int n = 0;
+      for (int i = 2; i >= c; i--) n += (int)rec[l][i].size() - (i > c ? rows[i] : 0);
+      return n;
+    };
+    for (int l = 0; l < 32; l++) rows[1] = std::max(rows[1], left(l, 1));
+    rows[1] = (rows[1] + 1) & ~1;
+    for (int l = 0; l < 32; l++) rows[0] = std::max(rows[0], left(l, 0));
+    rows[0] = (rows[0] + 3) & ~3;
+    const size_t words = rec_at / 2 + 32 * (size_t)(rows[0] + rows[1] + rows[2] + rows[3]) + 16 * (size_t)rows[2];
+    const size_t at = m.fc_tab.size();
+    m.fc_tab.resize(at + ((2 * words + 3) & ~(size_t)3), 0u);
+    uint32_t* tab = &m.fc_tab[at];
+    m.fc_desc[(size_t)b * 4] = (int)(at / 2);
+    m.fc_desc[(size_t)b * 4 + 1] = (int)((words + 1) & ~(size_t)1);
+    m.fc_words = std::max(m.fc_words, m.fc_desc[(size_t)b * 4 + 1]);
+    tab[0] = (uint32_t)(rows[0] / 4) | (uint32_t)(rows[1] / 2) << 7 | (uint32_t)(rows[2] / 2) << 15 |
+             (uint32_t)std::min(kin, KI) << 23 | (kin > KI || rows[3] ? 1u << 31 : 0u);
+    tab[1] = (uint32_t)rows[3];
+    uint32_t* s0 = tab + rec_at;
+    uint32_t* s1 = s0 + 64 * rows[0];
+    uint32_t* s2 = s1 + 64 * rows[1];
+    uint32_t* s2c = s2 + 64 * rows[2];
+    uint32_t* s3 = s2c + 32 * rows[2];
     for (int l = 0; l < 32; l++)
+    {
+      uint32_t* own = tab + 8 + (pair ? 2 : 4) * l;
+      own[0] = base[l];
+      own[1] = degree[l];
+      if (!pair)
+      {
+        own[2] = negs[l];
+        own[3] = alone[l];
+      }
+      // (padding records have no weight, and an op that leaves the mask alone)
+      // (longest first)
+      int c = 2;
+      size_t x = 0;
+      const uint32_t pad = pair ? 0u : ising ? none : none + 1;
+      auto take = [&]() -> Rec {
+        while (c >= 0 && x == rec[l][c].size()) c--, x = 0;
+        return c >= 0 ? rec[l][c][x++] : Rec{{pad, none, none}, 0u};
+      };
+      for (int k = 0; k < rows[2]; k++)
+      {
+        const Rec r = take();
+        s2[(k * 32 + l) * 2] = r.lit[0] | r.lit[1] << 16;
+        s2[(k * 32 + l) * 2 + 1] = r.val;
+        s2c[k * 32 + l] = r.lit[2];
+      }
+      for (int k = 0; k < rows[1]; k++)
+      {
+        const Rec r = take();
+        s1[(k * 32 + l) * 2] = r.lit[0] | r.lit[1] << 16;
+        s1[(k * 32 + l) * 2 + 1] = r.val;
+      }
+      for (int k = 0; k < rows[0]; k++)
+      {
+        const Rec r = take();
+        s0[(k * 32 + l) * 2] = r.lit[0];
+        s0[(k * 32 + l) * 2 + 1] = r.val;
+      }
+      for (int k = 0; k < rows[3]; k++)
+      {
+        const bool have = (size_t)k < wide[l].size();
+        s3[(k * 32 + l) * 2] = have ? wide[l][k].w[0] | wide[l][k].w[2] << 29 : 1u << 30;
+        s3[(k * 32 + l) * 2 + 1] = have ? wide[l][k].w[1] : 0u;
+      }
       for (size_t k = 0; k < in[l].size() && k < (size_t)KI; k++)
-        memcpy(tab + ent_at + (k * 32 + l) * ew, in[l][k].data(), ew * 4);
-    tab[0] = (uint32_t)rows | (uint32_t)std::min(kin, KI) << 8;
+        memcpy(tab + ent_at + (k * 32 + l) * ew, in[l][k].w, ew * 4);
+    }
     if (kin > KI)
     {
       const size_t more = m.fc_in.size() / ew;
-      tab[0] |= (uint32_t)(kin - KI) << 16;
-      tab[1] = (uint32_t)more;
+      tab[1] |= (uint32_t)(kin - KI) << 8;
+      tab[2] = (uint32_t)more;
       m.fc_in.resize(m.fc_in.size() + (size_t)(kin - KI) * 32 * ew, 0u);
       for (int l = 0; l < 32; l++)
         for (size_t k = KI; k < in[l].size(); k++)
-          memcpy(&m.fc_in[(more + (k - KI) * 32 + l) * ew], in[l][k].data(), ew * 4);
+          memcpy(&m.fc_in[(more + (k - KI) * 32 + l) * ew], in[l][k].w, ew * 4);
     }
   }
 }
@@ -729,7 +827,8 @@ void HostModel::upload() const
          o_cf = put(blob, coef_f), o_near = put(blob, near), o_oth = put(blob, other),
          o_ri = put(blob, rec_i), o_rf = put(blob, rec_f), o_rp = put(blob, rec_p),
          o_lo = put(blob, lv_off), o_le = put(blob, lv_ent), o_lp = put(blob, lv_pos),
-         o_ft = put(blob, fc_tab), o_fd = put(blob, fc_desc), o_fi = put(blob, fc_in);
+         o_ft = put(blob, fc_tab), o_fd = put(blob, fc_desc), o_fi = put(blob, fc_in),
+         o_fo = put(blob, fc_oth), o_fw = put(blob, fc_wide);
   // 256 bytes of tail padding: bulk copies of incidence ranges round their
   // end up to 16 bytes
   blob.resize(((blob.size() + 255) & ~(size_t)255) + 256);
@@ -775,8 +874,10 @@ void HostModel::upload() const
   dev.fc_desc = fc_desc.empty() ? nullptr : (const int4*)(b + o_fd);
   dev.fc_tab = (const uint2*)(b + o_ft);
   dev.fc_in = (const void*)(b + o_fi);
-  dev.fc_rows = fc_rows;
-  dev.fc_big = fc_big ? 1 : 0;
+  dev.fc_words = fc_words;
+  dev.fc_oth = (const uint2*)(b + o_fo);
+  dev.fc_wterm = (const int*)(b + o_fw);
+  dev.fc_wide = (int)fc_wide.size();
   dev.fc_S = fc_S;
   dev.fc_pack = fc_pack ? 1 : 0;
   dev.fc_inv = std::ldexp(1.0, -fc_S);

@@ -86,29 +86,37 @@ struct DevModel
   const int* tcost_i;      // n_terms
   // block-decided sweep (fields.cu), blocks of 32 variables, a lane each.
   // Block b's chunk begins at 8-byte word fc_desc[b].x of fc_tab:
-  //   header, 32 bytes: record rows, in-block entry rows (at most four), first
-  //     further entry in fc_in, further entry rows;
-  //   lane data, 8 bytes: (pair-only Ising: sum of the variable's fixed-point
-  //     coefficients; else its row's negated literals; degree);
+  //   header, 32 bytes: rows of records of one literal / 4 | of two / 2 << 7 | of
+  //     three / 2 << 15 | in-block entry rows (at most four) << 23 | the next
+  //     word is not 0 << 31; rows of wide terms | further entry rows << 8; first
+  //     further entry in fc_in;
+  //   lane data, 8 bytes: the field with every record's op 0; degree; not pair: 16,
+  //     the row's negated literals, its terms of v alone (counter models);
   //   in-block entries, four per lane (entry i of lane l at 32 i + l), one per
-  //     term with other members in the block (pair: with an earlier one): pair,
-  //     8 bytes, (that member's lane, 2q); else 16 bytes, (term | row position
-  //     << 18 | member position << 23 | more than eight members << 30 | negated
-  //     literal << 31, the members' lanes, their negated ones, the record's
-  //     second word);
-  //   records, fc_desc[b].y rows (a multiple of four), 8 bytes, in row order:
-  //     record k of lane l at 32 k + l (not pair: 33 k + l): pair (other member,
-  //     2q); else (term | negated literal << 18 | another member in the block <<
-  //     19 | more than eight members << 20 | the byte's bits of the other
-  //     members << 24, what the term adds to the field when it contributes).
-  // Zeros pad all of them.  Further entries lie in fc_in, rows of 32.
-  const int4* fc_desc;     // or null when the model does not qualify
+  //     term with earlier members in the block: pair-only Ising, 8 bytes, (that
+  //     member's lane as a bit, 2q); else 16 bytes, (the earlier members' lanes,
+  //     the negated ones, up to two literals of the rest, 16 bits each -- or
+  //     0xFFFC0000 | wide term, and bit l of the second word the own literal's
+  //     negation --, the term's value);
+  //   rows of 32 records, of the other terms' members: one literal (literal,
+  //     weight); two (16 bits each, weight); three (the same, and the third's
+  //     rows of 32 words behind them); wide terms (term | own literal negated <<
+  //     31, weight; 1 << 30: padding; 1 << 29: an entry holds its value).
+  // Weights and values of FP64 models that are not pair-only are multiples of 256,
+  // the row position (modulo 32) beside them.  The field is the lane's value minus the weights whose op is 1: the literals'
+  // OR (counter models) or XOR.  A literal 2u + n is variable u's, negated with n
+  // = 1; 2N is false; pair-only Ising uses u itself.  Further entries lie in
+  // fc_in, rows of 32.
+  const int4* fc_desc;     // (start, 8-byte words), or null when the model does not qualify
   const uint2* fc_tab;
   const void* fc_in;
-  int fc_rows;             // most records per lane of a block
-  int fc_big;              // a term has more than eight members
+  const uint2* fc_oth;     // K (not pair-only): up to three other literals, 16 bits each (0xFFFF:
+                           // none), own literal negated << 48, wide term << 49
+  const int* fc_wterm;     // wide terms (more than four members)
+  int fc_wide;             // their number
+  int fc_words;            // 8-byte words of the largest chunk
   int fc_S;                // fixed-point scale exponent
-  int fc_pack;             // FP64 counter models: field = fixed << 8 | count
+  int fc_pack;             // FP64 models that are not pair-only: field = fixed << 8
   double fc_inv;           // 2^-fc_S
 };
 
@@ -152,10 +160,7 @@ struct SweepArgs
   int smem_state;       // stage spins + term state in shared memory
   int* err;             // device error flag (a bounded wait gave up)
   long long tag;        // written to p.lowtag[walker] when its lowest drops
-  // block-decided sweep: 1 selects it; terms_valid = 1: the term bytes are as
-  // its last launch on this population left them (0: made from the spins)
-  int fields;
-  int terms_valid;
+  int fields;           // 1: the block-decided sweep
   // batches (windowed kernel): walker r runs models[model_of[r]] with the
   // counter key of walker local_of[r] of its own solve; with `queue` set,
   // each warp takes walkers from the counter *queue (reset to 0 before the
@@ -202,7 +207,7 @@ cudaError_t launch_sweep(const SweepArgs& a, cudaStream_t s, int warps_per_block
 bool sweep_state_fits(const SweepArgs& a);
 // block-decided sweep (fields.cu): whether it can run this model with this
 // population layout
-bool fc_fits(const DevModel& m, int nw, int mp);
+bool fc_fits(const DevModel& m, int nw);
 // (wpb: walkers per block of a queued launch, at most)
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb);
 // state bytes [n][n_vars] to spin words [n][nw]

@@ -191,9 +191,6 @@ struct Population
   uint64_t* rng = nullptr;
   int* slot_of = nullptr;
   double* beta = nullptr;
-  // the term bytes are the block-decided sweep's own (fields.cu), as its last
-  // launch left them (false after anything else set the states)
-  bool tvalid = false;
 
   void alloc(const HostModel& m, int slots, int streams, bool need_slots,
              int64_t n_beta)
@@ -490,7 +487,7 @@ bool levels_for(const Solver& s, const HostModel& m)
 bool fields_run(const Solver& s, const HostModel& m, const Population& P, bool full_maxsat_sweep)
 {
   return !m.empty() && !m.fc_desc.empty() && s.smem_state &&
-         fc_fits(m.device_view(full_maxsat_sweep), P.pop.nw, P.pop.mp);
+         fc_fits(m.device_view(full_maxsat_sweep), P.pop.nw);
 }
 bool fields_for(const Solver& s, const HostModel& m, const Population& P, bool full_maxsat_sweep)
 {
@@ -633,7 +630,6 @@ class SimulatedAnnealing : public Solver
     levels = levels_for(*this, *model);
     lanes = !levels && lanes_for(*this, *model, restarts, fields_run(*this, *model, P, full_maxsat_sweep));
     fields = !levels && !lanes && fields_for(*this, *model, P, full_maxsat_sweep);
-    P.tvalid = false;
     used_kernel = levels ? 3 : (lanes ? 2 : (fields ? 8 : 1));
     // the lane and level sweeps work from the spins and rebuild the term
     // bytes when they finish; the field-cached sweep makes its own
@@ -708,9 +704,7 @@ class SimulatedAnnealing : public Solver
       a.sweep_base = base;
       a.n_sweeps = (int)n;
       a.fields = fields ? 1 : 0;
-      a.terms_valid = P.tvalid ? 1 : 0;
       cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
-      P.tvalid = fields;
     }
     prof_end(st);
     launches++;
@@ -1040,9 +1034,8 @@ class ParallelTempering : public Solver
     a.key_base = 0;
     a.key_div = T();
     fields = fields_for(*this, *model, P, full_maxsat_sweep);
-    a.skip_terms = fields ? 1 : 0;  // the field-cached sweep makes its own term bytes
+    a.skip_terms = fields ? 1 : 0;  // the block-decided sweep works from the spins
     cuda_check(launch_init(a, st), "init kernel");
-    P.tvalid = false;
     used_kernel = fields ? 8 : 1;
     cuda_check(cudaStreamSynchronize(st), "sync");
     // the sweep/swap loop keeps its own copies of the stream so that a
@@ -1102,11 +1095,9 @@ class ParallelTempering : public Solver
       a.tag = s;  // the step, for the time order of equal lowest costs
       a.fields = fields ? 1 : 0;
       a.order = fields ? hot_first : nullptr;
-      a.terms_valid = P.tvalid ? 1 : 0;
       prof_begin(st);
       cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
       prof_end(st);
-      P.tvalid = fields;
       sw.step = s;
       cuda_check(launch_pt_swap(sw, st), "swap kernel");
       launches += 2;
@@ -1186,9 +1177,7 @@ class ParallelTempering : public Solver
       a.tag = step_pos;
       a.fields = fields ? 1 : 0;
       a.order = fields ? hot_first : nullptr;
-      a.terms_valid = P.tvalid ? 1 : 0;
       cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
-      P.tvalid = fields;
       sw.step = step_pos;
       cuda_check(launch_pt_swap(sw, st), "swap kernel");
       launches += 2;
@@ -2419,7 +2408,7 @@ class SABatch : public Batch
     int first, last;
     const HostModel* model;  // any member (flavour and coefficient kind)
     int max_block_inc;       // the members' largest 32-variable block
-    int fc_rows;             // the same of the block-decided sweep's record rows
+    int fc_words, fc_wide;   // the same of the block-decided sweep's chunks and wide terms
     bool fields;             // runs on the block-decided sweep
   };
   // members of a group share the kernel's instance
@@ -2486,7 +2475,7 @@ class SABatch : public Batch
   // the block-decided sweep runs the model's walkers in this population
   bool block_decided(const HostModel& m) const
   {
-    return smem && kernel != 1 && !m.fc_desc.empty() && fc_fits(m.device_view(full_sweep), P.pop.nw, P.pop.mp);
+    return smem && kernel != 1 && !m.fc_desc.empty() && fc_fits(m.device_view(full_sweep), P.pop.nw);
   }
 
   int n_instances() const override { return (int)models.size(); }
@@ -2572,12 +2561,13 @@ class SABatch : public Batch
       const int first = (int)k * R;
       const int mb = m->device_view(full_sweep).max_block_inc;
       if (groups.empty() || kind(*groups.back().model) != kind(*m))
-        groups.push_back({first, first + R, m, mb, m->fc_rows, block_decided(*m)});
+        groups.push_back({first, first + R, m, mb, m->fc_words, (int)m->fc_wide.size(), block_decided(*m)});
       else
       {
         groups.back().last = first + R;
         groups.back().max_block_inc = std::max(groups.back().max_block_inc, mb);
-        groups.back().fc_rows = std::max(groups.back().fc_rows, m->fc_rows);
+        groups.back().fc_words = std::max(groups.back().fc_words, m->fc_words);
+        groups.back().fc_wide = std::max(groups.back().fc_wide, (int)m->fc_wide.size());
       }
       if (groups.back().fields) continue;
       SweepArgs a{};
@@ -2641,7 +2631,8 @@ class SABatch : public Batch
     a.local_of = d_local_of + G.first;
     a.queue = d_queue + g;
     a.m.max_block_inc = G.max_block_inc;  // tiles sized for the group's largest block
-    a.m.fc_rows = G.fc_rows;
+    a.m.fc_words = G.fc_words;
+    a.m.fc_wide = G.fc_wide;
     a.fields = G.fields ? 1 : 0;
     cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
   }

@@ -1339,7 +1339,7 @@ cudaError_t launch_sweep(const SweepArgs& a_in, cudaStream_t s, int wpb)
 {
   using namespace sw;
   // the block-decided sweep where the caller asks for it
-  if (a_in.fields && a_in.smem_state && fc_fits(a_in.m, a_in.p.nw, a_in.p.mp)) return launch_fc_sweep(a_in, s, wpb);
+  if (a_in.fields && a_in.smem_state && fc_fits(a_in.m, a_in.p.nw)) return launch_fc_sweep(a_in, s, wpb);
   // record tiles sized to the largest block (a batch passes its largest)
   SweepArgs a = a_in;
   if (a.tile_cap <= 0) a.tile_cap = tile_cap_for(a.m);

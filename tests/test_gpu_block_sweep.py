@@ -52,6 +52,8 @@ CASES = {  # kind, instance, restarts, beta_stop
     "pubo_block_int": ("pubo", lambda: terms(80, [2, 3, 6], 500, 7, span=34, integer=True), 6, 3.0),
     "pubo_large": ("pubo", lambda: terms(130, [1, 4, 7, 9, 14], 400, 8), 6, 3.0),
     "pubo_wide_rows": ("pubo", lambda: terms(260, [2, 3], 500, 9, hub=180), 6, 3.0),
+    "pubo_widest_rows": ("pubo", lambda: terms(600, [2], 300, 15, hub=253), 4, 3.0),
+    "sat_wide_block": ("maxsat", lambda: clauses(64, 16, sizes=[5, 6, 20], count=150, span=40), 6, 3.0),
     "sat_signs": ("maxsat", lambda: clauses(75, 10, sizes=[2, 3, 5], count=400, span=38), 6, 3.0),
     "sat_large": ("maxsat", lambda: clauses(100, 11, sizes=[3, 9, 11], count=300, integer=True), 6, 3.0),
     "cold": ("ising", lambda: terms(100, [2], 300, 12), 4, np.inf),
