@@ -2,6 +2,7 @@
 // tempering solvers, configured from the reference's params JSON.
 #include <algorithm>
 #include <array>
+#include <charconv>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -2893,18 +2894,25 @@ std::unique_ptr<Batch> make_batch(const std::vector<const HostModel*>& models, c
 // ---------------------------------------------------------------------------
 static std::string render_config(const HostModel& m, const uint8_t* s)
 {
-  std::string o = "{";
-  for (int64_t v = 0; v < m.N; v++)
-  {
-    int val;
-    if (m.kind == K_ISING || m.kind == K_ISING_PLAIN) val = s[v] ? -1 : 1;
-    else if (m.kind == K_MAXSAT) val = s[v] ? 1 : 0;
-    else val = s[v] ? 0 : 1;
-    o += (v ? "," : "") + json::quote(std::to_string(m.names[v])) + ":" + std::to_string(val);
-  }
-  for (size_t i = 0; i < m.free_vars.size(); i++)
-    o += ((m.N || i) ? "," : "") + json::quote(std::to_string(m.free_vars[i])) + ":1";
-  return o + "}";
+  // the two values' texts, after a name (names are 32-bit integers)
+  const bool ising = m.kind == K_ISING || m.kind == K_ISING_PLAIN;
+  const char* clear = ising ? "\":1," : m.kind == K_MAXSAT ? "\":0," : "\":1,";
+  const char* set = ising ? "\":-1," : m.kind == K_MAXSAT ? "\":1," : "\":0,";
+  const size_t n = (size_t)m.N + m.free_vars.size();
+  std::string o(2 + 20 * n, '\0');
+  char* p = &o[0];
+  *p++ = '{';
+  auto entry = [&](int32_t name, const char* value) {
+    *p++ = '"';
+    p = std::to_chars(p, p + 12, name).ptr;
+    while (*value) *p++ = *value++;
+  };
+  for (int64_t v = 0; v < m.N; v++) entry(m.names[v], s[v] ? set : clear);
+  for (int32_t f : m.free_vars) entry(f, "\":1,");
+  if (n) p--;  // the last comma
+  *p++ = '}';
+  o.resize((size_t)(p - &o[0]));
+  return o;
 }
 
 void Solver::best(double& cost, std::vector<uint8_t>& state)
@@ -2968,11 +2976,16 @@ std::string Solver::result_json()
     }
     for (size_t j = 0; j < k; j++) list.push_back({low[idx[j]], ls.data() + idx[j] * model->N});
     sol += ",\"cost\":" + json::number(list[0].first + model->const_cost);
-    sol += ",\"configuration\":" + render_config(*model, list[0].second);
+    const std::string first = render_config(*model, list[0].second);  // (the first solution's too)
+    sol += ",\"configuration\":" + first;
     sol += ",\"solutions\":[";
     for (size_t j = 0; j < list.size(); j++)
-      sol += (j ? "," : "") + std::string("{\"cost\":") + json::number(list[j].first + model->const_cost) +
-             ",\"configuration\":" + render_config(*model, list[j].second) + "}";
+    {
+      sol += (j ? ",{\"cost\":" : "{\"cost\":") + json::number(list[j].first + model->const_cost) +
+             ",\"configuration\":";
+      sol += j ? render_config(*model, list[j].second) : first;
+      sol += "}";
+    }
     sol += "]";
   }
   else
