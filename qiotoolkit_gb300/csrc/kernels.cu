@@ -1077,7 +1077,7 @@ __global__ void __launch_bounds__(128) qmc_kernel(QmcArgs a)
 // slice.  Variable v's values are one word w[v] (bit k: slice k) in shared
 // memory, so that a term's parities, or whether any other literal is true, take
 // one word operation a member for all slices, lane j taking the row's j-th
-// incidence.  Rows do not depend on the state: their loads run up to four
+// incidence.  Rows do not depend on the state: their copies run up to three
 // variables ahead.
 //
 // The first warp decides.  The differences' FP64 adds (68 cycles each, one after
@@ -1088,10 +1088,12 @@ __global__ void __launch_bounds__(128) qmc_kernel(QmcArgs a)
 // flips a variable, keeps its own w, and takes the exact differences of the
 // flipped slices into their costs and lowest.
 //
-// What bounds it: the decider's chain of loads, votes and shuffles a variable.
-// N = 1000, 3000 couplings, 16 restarts of 32 slices, 50 sweeps: 145.4 ms with a
-// lane per slice on spins, costs and streams in HBM, 94 with w, costs and
-// streams on the chip and every sum in FP64, @@ here.
+// What bounds it: the decider's chain of loads, votes and shuffles, 1750 cycles a
+// variable (differences 540, draws and bonds 270, runs 250, comparison 200, flips
+// 190), the accountant close behind.  N = 1000, 3000 couplings, 16 restarts of 32
+// slices, 50 sweeps: 145.4 ms with a lane per slice on spins, costs and streams in
+// HBM, 94 with w, costs and streams on the chip and every sum in FP64, 47.7 with
+// the exact sums off the way and the rows ahead in registers, 45.5 here.
 namespace qs
 {
 static const int kRing = 512;  // flip words, a power of two
@@ -1134,109 +1136,130 @@ __device__ __noinline__ bool wait_for(const unsigned* p, unsigned want, unsigned
   return __shfl_sync(kFull, ok, 0) != 0u;
 }
 
-// A variable's row, lane j holding its j-th incidence (the first 32), loaded
-// ahead: bounds four variables before, incidence and coefficient three, the
-// term's bounds two, its first four members one.  CT: the coefficients' type.
+// A variable's row, lane j having its j-th incidence (the first 32): incidence and
+// coefficient come three variables ahead, the term's bounds two, its first four
+// members one, by asynchronous copies into the lane's own slots of shared memory
+// (held in registers, moving them up a place would wait for them).  CT: the
+// coefficients' type.
+struct Slots
+{
+  uint32_t x[4][32];     // incidence, or the pair's other member
+  double c[4][32];
+  int2 t[4][32];         // its term's bounds
+  uint32_t m[2][32][4];  // members
+};
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"(BYTES)
+               : "memory");
+}
 template <int FL, bool PAIR, class CT>
 struct Rows
 {
   static constexpr bool PAR = FL == F_PARITY || FL == F_PLAIN_ISING;
   struct Row { int b, e; };
-  struct Inc { uint32_t x; CT c; };
-  struct Term { int b, e; };
-  struct Mem { uint32_t x[4]; };
   const int *row, *other, *trow;
   const uint32_t *inc, *tvar;
   const CT* coef;
+  Slots* S;
   int SW, lane, ahead;
-  Row r0, r1, r2, r3, r4;
-  Inc i0, i1, i2, i3;
-  Term t0, t1, t2;
-  Mem f0, f1;
+  unsigned turn;
+  Row r0, r1, r2, r3;
 
-  __device__ __forceinline__ Row load_row(int v) const { return {__ldg(row + v), __ldg(row + v + 1)}; }
-  __device__ __forceinline__ Inc load_inc(Row t, int at) const
-  {
-    Inc o{0u, (CT)0};
-    if (t.b + at < t.e)
-    {
-      o.x = PAIR ? (uint32_t)__ldg(other + t.b + at) : __ldg(inc + t.b + at);
-      o.c = __ldg(coef + t.b + at);
-    }
-    return o;
-  }
-  __device__ __forceinline__ Term load_term(Row t, int at, const Inc& o) const
-  {
-    if (PAIR || t.b + at >= t.e) return {0, 0};
-    const int x = (int)(o.x & ~kNegBit);
-    return {__ldg(trow + x), __ldg(trow + x + 1)};
-  }
-  __device__ __forceinline__ Mem load_mem(const Term& t) const
-  {
-    Mem o;
-#pragma unroll
-    for (int i = 0; i < 4; i++) o.x[i] = !PAIR && t.b + i < t.e ? __ldg(tvar + t.b + i) : 0u;
-    return o;
-  }
+  __device__ __forceinline__ Row load_row(int v) const { return {row[v], row[v + 1]}; }
   __device__ __forceinline__ int next(int v) const { return v + 1 < SW ? v + 1 : 0; }
-  __device__ __forceinline__ void start(const DevModel& m, const CT* c, int l)
+  __device__ __forceinline__ CT& coef_slot(unsigned t) const { return *(CT*)&S->c[t & 3u][lane]; }
+  __device__ __forceinline__ void get_inc(unsigned t, Row r) const
   {
-    row = m.row, other = m.other, trow = m.trow, inc = m.inc, tvar = m.tvar, coef = c;
-    SW = m.sweep_size, lane = l;
+    if (r.b + lane >= r.e) return;
+    copy_async<4>(&S->x[t & 3u][lane], PAIR ? (const void*)(other + r.b + lane) : (const void*)(inc + r.b + lane));
+    copy_async<sizeof(CT)>(&coef_slot(t), coef + r.b + lane);
+  }
+  __device__ __forceinline__ void get_term(unsigned t, Row r) const
+  {
+    if (PAIR || r.b + lane >= r.e) return;
+    const int* p = trow + (int)(S->x[t & 3u][lane] & ~kNegBit);
+    copy_async<4>(&S->t[t & 3u][lane].x, p);
+    copy_async<4>(&S->t[t & 3u][lane].y, p + 1);
+  }
+  __device__ __forceinline__ void get_mem(unsigned t, Row r) const
+  {
+    if (PAIR || r.b + lane >= r.e) return;
+    const int2 b = S->t[t & 3u][lane];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (b.x + i < b.y) copy_async<4>(&S->m[t & 1u][lane][i], tvar + b.x + i);
+  }
+  __device__ __forceinline__ void arrived() const
+  {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  // (rows: the row bounds in shared memory)
+  __device__ __forceinline__ void start(const DevModel& m, const CT* c, const int* rows, Slots* slots, int l)
+  {
+    row = rows, other = m.other, trow = m.trow, inc = m.inc, tvar = m.tvar, coef = c, S = slots;
+    SW = m.sweep_size, lane = l, turn = 0;
     const int v1 = next(0), v2 = next(v1), v3 = next(v2);
     ahead = next(v3);
     r0 = load_row(0), r1 = load_row(v1), r2 = load_row(v2), r3 = load_row(v3);
-    i0 = load_inc(r0, lane), i1 = load_inc(r1, lane), i2 = load_inc(r2, lane);
-    t0 = load_term(r0, lane, i0), t1 = load_term(r1, lane, i1);
-    f0 = load_mem(t0);
+    get_inc(0, r0), get_inc(1, r1), get_inc(2, r2);
+    arrived();
+    get_term(0, r0), get_term(1, r1);
+    arrived();
+    get_mem(0, r0);
   }
-  // the loads that run ahead of the variable in turn
-  __device__ __forceinline__ void issue()
+  // what the last turn fetched has come; the next turns' is sent for
+  __device__ __forceinline__ void issue() const
   {
-    r4 = load_row(ahead);
-    i3 = load_inc(r3, lane);
-    t2 = load_term(r2, lane, i2);
-    f1 = load_mem(t1);
+    arrived();
+    get_inc(turn + 3u, r3);
+    get_term(turn + 2u, r2);
+    get_mem(turn + 1u, r1);
   }
   __device__ __forceinline__ void shift()
   {
-    r0 = r1, r1 = r2, r2 = r3, r3 = r4;
-    i0 = i1, i1 = i2, i2 = i3;
-    t0 = t1, t1 = t2;
-    f0 = f1;
+    r0 = r1, r1 = r2, r2 = r3, r3 = load_row(ahead);
     ahead = next(ahead);
+    turn++;
   }
   __device__ __forceinline__ int degree() const { return __shfl_sync(kFull, r0.e - r0.b, 0); }
   // incidences j0 .. j0 + 31 of variable v, for all slices: the terms' parities,
   // or the slices in which another literal is true; the coefficients, negated
-  // where v's literal is
+  // where v's literal is; nothing past the row
   __device__ __forceinline__ void take(int v, int deg, int j0, const uint32_t* w, uint32_t& on, CT& c) const
   {
-    Inc o = i0;
-    Term t = t0;
-    Mem f = f0;
-    if (j0)
-    {
-      o = load_inc(r0, j0 + lane);
-      t = load_term(r0, j0 + lane, o);
-      f = load_mem(t);
-    }
     on = 0u;
-    c = o.c;
+    c = (CT)0;
     if (j0 + lane >= deg) return;
+    uint32_t x;
+    int2 t = make_int2(0, 0);
+    if (j0 == 0)
+    {
+      x = S->x[turn & 3u][lane];
+      c = coef_slot(turn);
+      if (!PAIR) t = S->t[turn & 3u][lane];
+    }
+    else
+    {
+      const int q = r0.b + j0 + lane;
+      x = PAIR ? (uint32_t)__ldg(other + q) : __ldg(inc + q);
+      c = __ldg(coef + q);
+      if (!PAIR) t = make_int2(__ldg(trow + (x & ~kNegBit)), __ldg(trow + (x & ~kNegBit) + 1));
+    }
     if (PAIR)
     {
-      on = w[v] ^ ((int)o.x >= 0 ? w[o.x] : 0u);
+      on = w[v] ^ ((int)x >= 0 ? w[x] : 0u);
       return;
     }
-    for (int i = 0; i < t.e - t.b; i++)
+    for (int i = 0; i < t.y - t.x; i++)
     {
-      const uint32_t x = i == 0 ? f.x[0] : i == 1 ? f.x[1] : i == 2 ? f.x[2] : i == 3 ? f.x[3] : __ldg(tvar + t.b + i);
-      const int u = (int)(x & ~kNegBit);
+      const uint32_t y = j0 == 0 && i < 4 ? S->m[turn & 1u][lane][i] : __ldg(tvar + t.x + i);
+      const int u = (int)(y & ~kNegBit);
       if (PAR) on ^= w[u];
-      else if (u != v) on |= w[u] ^ ((x & kNegBit) ? kFull : 0u);
+      else if (u != v) on |= w[u] ^ ((y & kNegBit) ? kFull : 0u);
     }
-    if (!PAR && (o.x & kNegBit)) c = -c;
+    if (!PAIR && (x & kNegBit)) c = -c;
   }
 };
 
@@ -1280,14 +1303,36 @@ template <int FL, bool PAIR>
 __device__ __noinline__ double exact_run_sum(const DevModel& m, int v, const uint32_t* w, bool head, int end)
 {
   const int lane = threadIdx.x & 31;
-  Rows<FL, PAIR, double> R;
-  R.row = m.row, R.other = m.other, R.trow = m.trow, R.inc = m.inc, R.tvar = m.tvar, R.coef = m.coef;
-  R.SW = m.sweep_size, R.lane = lane;
-  R.r0 = R.load_row(v);
-  R.i0 = R.load_inc(R.r0, lane);
-  R.t0 = R.load_term(R.r0, lane, R.i0);
-  R.f0 = R.load_mem(R.t0);
-  const double dif = exact_dif<FL, false, PAIR, double>(R, v, w);
+  const uint32_t sv = (w[v] >> lane) & 1u;
+  constexpr bool PAR = FL == F_PARITY || FL == F_PLAIN_ISING;
+  double dif = 0.0;
+  for (int q = __ldg(m.row + v), qe = __ldg(m.row + v + 1); q < qe; q++)
+  {
+    const double c = __ldg(m.coef + q);
+    uint32_t on = 0;
+    bool neg = false;
+    if (PAIR)
+    {
+      const int u = __ldg(m.other + q);
+      on = w[v] ^ (u >= 0 ? w[u] : 0u);
+    }
+    else
+    {
+      const uint32_t e = __ldg(m.inc + q);
+      neg = !PAR && (e & kNegBit) != 0u;
+      for (int k = __ldg(m.trow + (e & ~kNegBit)), ke = __ldg(m.trow + (e & ~kNegBit) + 1); k < ke; k++)
+      {
+        const uint32_t y = __ldg(m.tvar + k);
+        const int u = (int)(y & ~kNegBit);
+        if (PAR) on ^= w[u];
+        else if (u != v) on |= w[u] ^ ((y & kNegBit) ? kFull : 0u);
+      }
+    }
+    const uint32_t b = (on >> lane) & 1u;
+    if (PAR) dif = __dadd_rn(dif, b ? -c : c);
+    else if (!b) dif = __dadd_rn(dif, ((sv != 0u) != neg) ? c : -c);
+  }
+  if (PAR) dif = times_minus2(dif);
   double sum = dif;
   for (int i = 1; __any_sync(kFull, head && lane + i < end); i++)
   {
@@ -1306,12 +1351,16 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
   extern __shared__ uint32_t qmem[];
   __shared__ Sync sync;
   __shared__ uint32_t ring[kRing];
+  __shared__ __align__(16) Slots slots[2];
+  __shared__ __align__(16) uint2 pair[32];  // the decider's row: words and coefficients
   const DevModel& m = a.m;
   // (through a shuffle: known to be the same on all lanes)
   const int role = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31, r = blockIdx.x;
   const int P = a.trotter, N = m.n_vars, SW = m.sweep_size, nw = a.p.nw, nwd = (N + 31) >> 5;
   uint32_t* w = qmem + (role ? N : 0);  // each warp's own
+  int* rows = (int*)qmem + 2 * N;
+  for (int v = threadIdx.x; v <= N; v += 64) rows[v] = __ldg(m.row + v);
   const bool mine = lane < P;
   const int slot = r * P + (mine ? lane : 0);
   uint32_t* g_spins = a.p.spins + (size_t)slot * nw;
@@ -1338,8 +1387,8 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
     unsigned tail = 0, seen = 0;
     using CT = typename std::conditional<INT, int, double>::type;
     Rows<FL, PAIR, CT> R;
-    if constexpr (INT) R.start(m, m.coef_i, lane);
-    else R.start(m, m.coef, lane);
+    if constexpr (INT) R.start(m, m.coef_i, rows, &slots[1], lane);
+    else R.start(m, m.coef, rows, &slots[1], lane);
     for (int st = 0; st < a.n_steps; st++)
     {
       for (int v = 0; v < SW; v++)
@@ -1347,7 +1396,11 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
         if (seen == tail)
         {
           if (lane == 0) release(&sync.tail, tail);
-          if (!wait_for(&sync.head, tail + 1u, &sync.abort, a.err, seen)) return;
+          if (!wait_for(&sync.head, tail + 1u, &sync.abort, a.err, seen))
+          {
+            R.arrived();
+            return;
+          }
         }
         R.issue();
         const uint32_t F = __shfl_sync(kFull, ring[tail & (kRing - 1u)], 0);
@@ -1404,25 +1457,21 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
       a.p.attempts[slot] += (unsigned long long)SW * (unsigned long long)a.n_steps;
     }
     if (lane == 0) a.low[r] = low;
+    R.arrived();
     return;
   }
 
   // ---- the decider
   uint64_t rs = a.replay ? a.rng[slot] : 0;
   const uint64_t key = a.replay ? 0 : counter_key(a.seed, (uint64_t)slot);
-  // the 64 random bits of one uniform() (qmc_bits)
-  auto bits = [&](unsigned long long ctr) -> unsigned long long {
-    if (!a.replay) return counter_draw(key, ctr);
-    const uint32_t d0 = pcg_out(rs);
-    rs = rs * kMult + kInc;
-    const uint32_t d1 = pcg_out(rs);
-    rs = rs * kMult + kInc;
-    return ((unsigned long long)d1 << 32) | d0;
-  };
+  // Replay: a slice's next two uniforms take its stream's next four outputs; both
+  // are made before it is known whether it takes none, one or two.
+  const unsigned long long A2 = kMult * kMult, C2 = kMult * kInc + kInc;
+  const unsigned long long A4 = A2 * A2, C4 = A2 * C2 + C2;
   using CT = typename std::conditional<INT, int, float>::type;
   Rows<FL, PAIR, CT> R;
-  if constexpr (INT) R.start(m, m.coef_i, lane);
-  else R.start(m, m.coef_f, lane);
+  if constexpr (INT) R.start(m, m.coef_i, rows, &slots[0], lane);
+  else R.start(m, m.coef_f, rows, &slots[0], lane);
   unsigned head = 0, tail = 0;
   for (int st = 0; st < a.n_steps; st++)
   {
@@ -1446,39 +1495,66 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
         uint32_t on;
         CT cj;
         R.take(v, deg, j0, w, on, cj);
+        // through shared memory to all lanes, four at a time (nothing pads)
+        uint2 p;
+        p.x = on;
+        if (INT) p.y = (uint32_t)(int)cj;
+        else p.y = __float_as_uint((float)cj);
+        pair[lane] = p;
+        __syncwarp();
         const int n = min(32, deg - j0);
-#pragma unroll 4
-        for (int j = 0; j < n; j++)
+        for (int j = 0; j < n; j += 4)
         {
-          const uint32_t b = (__shfl_sync(kFull, on, j) >> lane) & 1u;
-          const CT x = __shfl_sync(kFull, cj, j);
-          if (INT)
+          uint2 q[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) q[i] = pair[j + i];
+#pragma unroll
+          for (int i = 0; i < 4; i++)
           {
-            if (PAR) id += b ? -(int)x : (int)x;
-            else id += b ? 0 : (sv ? (int)x : -(int)x);
-          }
-          else
-          {
-            if (PAR) fd += b ? -(float)x : (float)x;
-            else fd += b ? 0.f : (sv ? (float)x : -(float)x);
-            mag += fabsf((float)x);
+            const uint32_t b = (q[i].x >> lane) & 1u;
+            if (INT)
+            {
+              const int x = (int)q[i].y;
+              if (PAR) id += b ? -x : x;
+              else id += b ? 0 : (sv ? x : -x);
+            }
+            else
+            {
+              const float x = __uint_as_float(q[i].y);
+              if (PAR) fd += b ? -x : x;
+              else fd += b ? 0.f : (sv ? x : -x);
+              mag += fabsf(x);
+            }
           }
         }
+        __syncwarp();
       }
       if (PAR)
       {
         fd *= -2.f;
         mag *= 2.f;
       }
-      // ---- bonds to the slice before, on equal values
-      bool bonded = false;
-      if (mine && lane > 0 && !(((word ^ (word << 1)) >> lane) & 1u))
+      // ---- the draws that may be taken (qmc_bits)
+      unsigned long long x1, x2;
+      uint64_t s2 = 0, s4 = 0;
+      if (a.replay)
       {
-        const unsigned long long x = bits(c);
-        bonded = a.replay ? (ball || x < blim) : ((x >> 11) < blim);
+        s2 = A2 * rs + C2;
+        s4 = A4 * rs + C4;
+        x1 = ((unsigned long long)pcg_out(rs * kMult + kInc) << 32) | pcg_out(rs);
+        x2 = ((unsigned long long)pcg_out(s2 * kMult + kInc) << 32) | pcg_out(s2);
       }
+      else
+      {
+        x1 = counter_draw(key, c);
+        x2 = counter_draw(key, c + 1);
+      }
+      // ---- bonds to the slice before, on equal values
+      const bool equal = mine && lane > 0 && !(((word ^ (word << 1)) >> lane) & 1u);
+      const bool bonded = equal && (a.replay ? (ball || x1 < blim) : ((x1 >> 11) < blim));
       const unsigned B = __ballot_sync(kFull, bonded);
       const bool first = mine && !bonded;
+      const unsigned long long ub = a.replay && !equal ? x1 : x2;
       // ---- every run's sum, on its first slice
       const unsigned above = ~B & ~((2u << lane) - 1u);
       const int end = min(P, above ? __ffs(above) - 1 : 32);
@@ -1528,11 +1604,9 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
         }
       }
       bool ok = first;
-      unsigned long long ub = 0;
       amb = false;
       if (up)
       {
-        ub = bits(c + 1);
         // (the screen of qmc_kernel, with the sum's error)
         const float uf = (float)(uint32_t)(ub >> 40) * 0x1p-24f;
         const float xf = -bef * s, ef = expf(xf), de = bef * e;
@@ -1552,8 +1626,9 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
           ok = u < x;
         }
       }
+      rs = equal && up ? s4 : (equal || up ? s2 : rs);
       // ---- a run flips as its first slice decides
-      const unsigned H = __ballot_sync(kFull, first), A = __ballot_sync(kFull, ok);
+      const unsigned H = ~B, A = __ballot_sync(kFull, ok);
       const unsigned at = H & ((2u << lane) - 1u);
       const unsigned F = __ballot_sync(kFull, mine && ((A >> (31 - __clz(at))) & 1u));
       if (lane == 0)
@@ -1569,11 +1644,15 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
         if (lane == 0) release(&sync.head, head);
         if (head - tail > (unsigned)kRing - 32u &&
             !wait_for(&sync.tail, head - (unsigned)kRing + 32u, &sync.abort, a.err, tail))
+        {
+          R.arrived();
           return;
+        }
       }
     }
   }
   if (lane == 0) release(&sync.head, head);
+  R.arrived();
   if (mine && a.replay) a.rng[slot] = rs;
 }
 
@@ -1765,11 +1844,11 @@ template <int FL, bool I>
 static cudaError_t qmc_dispatch(const QmcArgs& a, cudaStream_t s)
 {
   // a slice per lane where there are lanes and the variables' words fit
-  const size_t words = (size_t)a.m.n_vars * 8;
+  const size_t words = ((size_t)a.m.n_vars * 3 + 1) * 4;  // two copies, the row bounds
   if (a.trotter <= 32 && words <= 200 * 1024)
   {
     auto k = FL == F_PARITY && a.m.pair_only ? qmc_sliced_kernel<FL, I, FL == F_PARITY> : qmc_sliced_kernel<FL, I, false>;
-    if (words > 44 * 1024)
+    if (words > 32 * 1024)
     {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)words);
       if (e != cudaSuccess) return e;
