@@ -828,6 +828,309 @@ __global__ void __launch_bounds__(128) tabu_kernel(TabuArgs a)
   }
 }
 
+// The same for pair-only Ising models that fit an SM's shared memory: the model
+// once a block (rows, the other members, coefficients), and per walker (a warp)
+// the differences as ordered keys, the list and both spin vectors; the hill
+// climber's differences stay in HBM.
+//
+// What bounds it: a flip's refresh -- the rows of its neighbours, added in order
+// -- and a scan's comparisons, a few instructions a variable with one vote per
+// 128; from HBM the refresh waited for four dependent loads (5500 cycles) and the
+// scan took 10500.  1216 walkers of a 1000-spin model, 200 steps: 3.78 ms from
+// HBM, 2.27 here; 4096 of 1180 spins, 60 steps, in waves: 10.9 and 9.2; 8 of 1000:
+// 2.86 and 1.88.  (With the differences and lists alone in shared memory the rows
+// fell out of the L1 cache: 3.56, and 11.8 and 2.98 for the other two.)
+struct TabuFit
+{
+  size_t model, walker;  // bytes
+  int warps;             // walkers a block, at most; 0: does not fit
+};
+static TabuFit tabu_fit(const DevModel& m, int nw)
+{
+  TabuFit f;
+  f.model = ((size_t)(m.n_vars + 1) * 4 + (size_t)m.n_inc * 4 + 15) / 16 * 16 + ((size_t)m.n_inc * (m.int_mode ? 4 : 8) + 15) / 16 * 16;
+  f.walker = (16 * (size_t)m.n_vars + 8 * (size_t)nw + 15) / 16 * 16;
+  const size_t room = 226 * 1024;
+  f.warps = f.model + f.walker > room ? 0 : (int)std::min<size_t>(8, (room - f.model) / f.walker);
+  return f;
+}
+
+template <bool INT>
+__global__ void __launch_bounds__(256, 1) tabu_pair_kernel(TabuArgs a, size_t model_bytes, size_t walker_bytes)
+{
+  using CT = typename std::conditional<INT, int, double>::type;
+  extern __shared__ __align__(16) unsigned char tmem[];
+  const DevModel& m = a.m;
+  const int N = m.n_vars, K = m.n_inc, nw = a.p.nw;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  int* row = (int*)tmem;
+  int* other = row + N + 1;
+  CT* coef = (CT*)(tmem + ((size_t)(N + 1) * 4 + (size_t)K * 4 + 15) / 16 * 16);
+  for (int q = threadIdx.x; q <= N; q += blockDim.x) row[q] = __ldg(m.row + q);
+  for (int q = threadIdx.x; q < K; q += blockDim.x)
+  {
+    other[q] = __ldg(m.other + q);
+    if constexpr (INT) coef[q] = __ldg(m.coef_i + q);
+    else coef[q] = __ldg(m.coef + q);
+  }
+  __syncthreads();
+  const int w = blockIdx.x * (blockDim.x >> 5) + wib;
+  if (w >= a.n_walkers) return;  // whole warps leave together
+  unsigned char* base = tmem + model_bytes + wib * walker_bytes;
+  unsigned long long* key = (unsigned long long*)base;  // differences (raw_key)
+  unsigned long long* tb = key + N;
+  uint32_t* sp = (uint32_t*)(tb + N);
+  uint32_t* hs = sp + nw;
+  uint32_t* g_sp = a.p.spins + (size_t)w * nw;
+  uint32_t* ls = a.p.lspins + (size_t)w * nw;
+  uint32_t* g_hs = a.hc + (size_t)w * nw;
+  uint32_t* hl = a.hc_low + (size_t)w * nw;
+  unsigned long long* g_tb = a.tabu + (size_t)w * N;
+  double* g_df = a.diff + (size_t)w * N;
+  double* hd = a.hdiff + (size_t)w * N;
+  TabuState S = a.st[w];
+  double cost = a.p.cost[w], low = a.p.lowest[w];
+  unsigned long long att = 0, acc = 0;
+  const unsigned long long tenure = a.tenures ? a.tenures[w] : a.tenure;
+
+  // invertible and ordered but for -0, which `as_key` makes +0 where it matters
+  auto raw_key = [](double x) -> unsigned long long {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+  };
+  auto of_key = [](unsigned long long k) -> double {
+    return __longlong_as_double((long long)((k >> 63) ? (k ^ 0x8000000000000000ull) : ~k));
+  };
+  auto as_key = [](unsigned long long k) -> unsigned long long {
+    return k == 0x7FFFFFFFFFFFFFFFull ? 0x8000000000000000ull : k;
+  };
+  // the difference of flipping v, terms in row order (lane_diff)
+  auto diff_of = [&](const uint32_t* s, int v) -> double {
+    const uint32_t sv = spin_of(s, v);
+    const int qe = row[v + 1];
+    double d = 0.0;
+    int id = 0;
+    for (int q = row[v]; q < qe; q += 4)
+    {
+      int o[4];
+      CT c[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+      {
+        o[u] = other[min(q + u, qe - 1)];
+        c[u] = coef[min(q + u, qe - 1)];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+      {
+        const uint32_t par = sv ^ (o[u] >= 0 ? spin_of(s, o[u]) : 0u);
+        if (q + u >= qe) continue;
+        if constexpr (INT) id += par ? -c[u] : c[u];
+        else d = __dadd_rn(d, par ? -c[u] : c[u]);
+      }
+    }
+    return INT ? (double)(-2ll * id) : times_minus2(d);
+  };
+  // i's flip: its difference and its neighbours' afresh (tabu_refresh)
+  auto refresh = [&](const uint32_t* s, int i, bool climber) {
+    const int rb = row[i], re = row[i + 1];
+    for (int q0 = rb; q0 < max(re, rb + 1); q0 += 32)
+    {
+      const int q = q0 + lane;
+      int x = q < re ? other[q] : -1;
+      // i itself on the first free lane of the first pass
+      if (q0 == rb && lane == min(re - rb, 31))
+      {
+        if (x < 0) x = i;
+        else
+        {
+          const double d = diff_of(s, i);
+          if (climber) hd[i] = d;
+          else key[i] = raw_key(d);
+        }
+      }
+      if (x >= 0)
+      {
+        const double d = diff_of(s, x);
+        if (climber) hd[x] = d;
+        else key[x] = raw_key(d);
+      }
+    }
+    __syncwarp();
+  };
+
+  warp_copy(sp, g_sp, nw, lane);
+  warp_copy(hs, g_hs, nw, lane);
+  for (int q = lane; q < N; q += 32)
+  {
+    key[q] = raw_key(S.ready ? g_df[q] : diff_of(sp, q));
+    tb[q] = g_tb[q];
+  }
+  S.ready = 1;
+  __syncwarp();
+
+  // (tabu_kernel's)
+  auto local_sweep = [&]() {
+    const double prev = S.hc_low;
+    int v0 = 0;
+    while (v0 < N)
+    {
+      const int v = v0 + lane;
+      const bool ok = v < N;
+      const double d = ok ? hd[v] : 0.0;
+      const unsigned take = __ballot_sync(kFull, ok && __double_as_longlong(d) <= 0);
+      if (!take)
+      {
+        att += (unsigned long long)min(32, N - v0);
+        v0 += 32;
+        continue;
+      }
+      const int j = __ffs(take) - 1;
+      const double dj = __shfl_sync(kFull, d, j);
+      const int i = v0 + j;
+      att += (unsigned long long)(j + 1);
+      if (lane == 0) hs[i >> 5] ^= 1u << (i & 31);
+      __syncwarp();
+      acc++;
+      S.hc_cost = __dadd_rn(S.hc_cost, dj);
+      if (S.hc_cost < S.hc_low)
+      {
+        S.hc_low = S.hc_cost;
+        warp_copy(hl, hs, nw, lane);
+      }
+      refresh(hs, i, true);
+      v0 = i + 1;
+    }
+    if (S.hc_low < prev)
+    {
+      low = S.hc_low;
+      warp_copy(ls, hl, nw, lane);
+    }
+    else
+      S.local = 0;
+  };
+
+  for (int step = 0; step < a.n_steps; step++)
+  {
+    if (S.local)
+    {
+      local_sweep();
+      continue;
+    }
+    // the scan (tabu_kernel): a difference surely below t is taken, one surely
+    // above it is not
+    const unsigned long long it = S.iter;
+    const double t = __dadd_rn(low, -cost);
+    const double e = fmax(__dmul_rn(fmax(fmax(fabs(cost), fabs(low)), fabs(t)), 0x1p-48), 0x1p-1000);
+    const unsigned long long klo = fkey(__dadd_rn(t, -e)), khi = fkey(__dadd_rn(t, e));
+    unsigned long long bk = ~0ull;
+    int bv = INT_MAX;
+    int found = -1;
+    for (int c0 = 0; c0 < N && found < 0; c0 += 128)
+    {
+      unsigned long long k[4];
+      bool may = false;
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+      {
+        const int v = c0 + 32 * u + lane;
+        const bool ok = v < N;
+        k[u] = ok ? as_key(key[v]) : ~0ull;
+        const unsigned long long x = ok ? tb[v] : ~0ull;
+        may = may || (ok && k[u] <= khi);
+        const bool better = ok && x < it && k[u] < bk;
+        bk = better ? k[u] : bk;
+        bv = better ? v : bv;
+      }
+      if (!__any_sync(kFull, may)) continue;
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+      {
+        const int v = c0 + 32 * u + lane;
+        const bool ok = v < N && found < 0;
+        unsigned take = __ballot_sync(kFull, ok && k[u] < klo);
+        const unsigned near = __ballot_sync(kFull, ok && k[u] >= klo && k[u] <= khi);
+        if (near) take |= __ballot_sync(kFull, ((near >> lane) & 1) && __dadd_rn(cost, of_key(k[u])) < low);
+        if (take && found < 0) found = c0 + 32 * u + __ffs(take) - 1;
+      }
+    }
+    if (found >= 0)
+    {
+      const int i = found;
+      const double di = of_key(key[i]);
+      __syncwarp();
+      // attempt_transition accepted it: flip, cost, lowest
+      if (lane == 0) sp[i >> 5] ^= 1u << (i & 31);
+      __syncwarp();
+      acc++;
+      cost = __dadd_rn(cost, di);
+      low = cost;
+      warp_copy(ls, sp, nw, lane);
+      if (lane == 0) tb[i] = it + tenure;
+      refresh(sp, i, false);
+      // local_search_init: a hill climber on a copy, its cost computed afresh
+      warp_copy(hs, sp, nw, lane);
+      warp_copy(hl, sp, nw, lane);
+      for (int q = lane; q < N; q += 32) hd[q] = of_key(key[q]);
+      __syncwarp();
+      double c;
+      long long ic;
+      warp_terms_cost<F_PARITY, INT>(m, hs, nullptr, lane, c, ic);
+      S.hc_cost = INT ? (double)ic : c;
+      S.hc_low = S.hc_cost;
+      S.local = 1;
+      S.incomplete += (unsigned long long)i;
+      att += (unsigned long long)(i + 1);
+      if (S.incomplete < (unsigned long long)N)
+        local_sweep();
+      else
+        S.incomplete -= (unsigned long long)N;
+    }
+    else
+    {
+      att += (unsigned long long)N;
+      // the lowest difference off the tabu list, the first on ties
+      const unsigned hi = __reduce_min_sync(kFull, (unsigned)(bk >> 32));
+      const bool h1 = (unsigned)(bk >> 32) == hi;
+      const unsigned lo = __reduce_min_sync(kFull, h1 ? (unsigned)bk : ~0u);
+      bv = __reduce_min_sync(kFull, h1 && (unsigned)bk == lo ? bv : INT_MAX);
+      if (bv != INT_MAX)
+      {
+        // Walker::apply_transition(transition, diff)
+        const double bd = of_key(key[bv]);
+        __syncwarp();
+        if (lane == 0) sp[bv >> 5] ^= 1u << (bv & 31);
+        __syncwarp();
+        cost = __dadd_rn(cost, bd);
+        if (cost < low)
+        {
+          low = cost;
+          warp_copy(ls, sp, nw, lane);
+        }
+        if (lane == 0) tb[bv] = it + tenure;
+        refresh(sp, bv, false);
+      }
+    }
+    S.iter++;
+    __syncwarp();
+  }
+  warp_copy(g_sp, sp, nw, lane);
+  warp_copy(g_hs, hs, nw, lane);
+  for (int q = lane; q < N; q += 32)
+  {
+    g_df[q] = of_key(key[q]);
+    g_tb[q] = tb[q];
+  }
+  if (lane == 0)
+  {
+    a.st[w] = S;
+    a.p.cost[w] = cost;
+    a.p.lowest[w] = low;
+    a.p.attempts[w] += att;
+    a.p.accepts[w] += acc;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Substochastic Monte Carlo walker steps.  Replay: one thread per emulated
 // OpenMP thread t of the reference, serving walkers [b_t, e_t) (libgomp's
@@ -2261,6 +2564,24 @@ cudaError_t launch_tabu(const TabuArgs& a, cudaStream_t s)
 {
   if (a.n_walkers <= 0 || a.n_steps <= 0) return cudaSuccess;
   const bool I = a.m.int_mode != 0;
+  if (a.m.flavor == F_PARITY && a.m.pair_only && a.m.sweep_size == a.m.n_vars)
+  {
+    const TabuFit f = tabu_fit(a.m, a.p.nw);
+    // as few walkers a block as the SMs need
+    const int wpb = std::min(f.warps, std::max(1, (a.n_walkers + 151) / 152));
+    if (wpb > 0)
+    {
+      const size_t smem = f.model + wpb * f.walker;
+      auto k = I ? tabu_pair_kernel<true> : tabu_pair_kernel<false>;
+      if (smem > 48 * 1024)
+      {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+      }
+      k<<<(a.n_walkers + wpb - 1) / wpb, 32 * wpb, smem, s>>>(a, f.model, f.walker);
+      return cudaGetLastError();
+    }
+  }
   switch (a.m.flavor)
   {
     case F_PARITY: I ? tabu_dispatch<F_PARITY, true>(a, s) : tabu_dispatch<F_PARITY, false>(a, s); break;

@@ -838,6 +838,7 @@ void HostModel::upload() const
   dev.flavor = flavor;
   dev.n_vars = (int)N;
   dev.n_terms = (int)M;
+  dev.n_inc = (int)K;
   dev.sweep_size = (int)N;
   dev.int_mode = int_mode ? 1 : 0;
   dev.row = (const int*)(b + o_row);

@@ -44,6 +44,7 @@ struct DevModel
   int flavor;
   int n_vars;
   int n_terms;
+  int n_inc;        // K
   int sweep_size;   // attempts per sweep (n_vars; 1 for MaxSat strict)
   int int_mode;     // coefficients are small integers
   const int* row;          // n_vars + 1
