@@ -1212,32 +1212,69 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   return true;
 }
 
-// The running cost over n flips (lane i < n: the i-th difference d) as a prefix
-// sum of whole numbers (ordered_sum.cuh).  False (nothing changed): a difference
-// for which that does not do -- the caller adds one by one.
-__device__ __forceinline__ bool cost_prefix(double d, int n, double& cost, long long& klow, double& low, int& lowpos)
+// The running cost over n flips (lane i < n: the i-th difference d), in order, as
+// prefix sums of whole numbers (ordered_sum.cuh) between the flips that need an
+// add of their own; the first lowest (lane lowpos) below klow.
+__device__ __forceinline__ void accumulate(double d, int n, double& cost, long long& klow, double& low, int& lowpos)
 {
   const int lane = threadIdx.x & 31;
-  int ce;
-  const long long C = osum::scaled(cost, ce);
-  long long D = 0;
-  bool ok = ce != 0 && ce != 0x7FF;
-  if (ok && lane < n) ok = osum::step_of(d, ce, D);
-  const long long P = C + osum::prefix(D);
-  if (!__all_sync(kFull, ok && osum::inside(C, P))) return false;
-  long long mn = P;  // (lanes past n repeat the last prefix)
-#pragma unroll
-  for (int s = 16; s; s >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, s));
-  const double vmin = osum::unscaled(mn, ce);
-  const long long km = order_key(vmin);
-  if (km < klow)
+  int start = 0;
+  // four prefixes at most (a cost near zero changes its binade often)
+  for (int round = 0; round < 4 && n - start > 4; round++)
   {
-    klow = km;
-    low = vmin;
-    lowpos = __ffs(__ballot_sync(kFull, P == mn)) - 1;
+    int ce;
+    const long long C = osum::scaled(cost, ce);
+    const bool in = lane >= start && lane < n, normal = ce != 0 && ce != 0x7FF;
+    long long D = 0;
+    bool ok = normal, tie = false;
+    if (normal && in) ok = osum::step_of(d, ce, D, tie);
+    const long long P = osum::prefix(C, D, tie);
+    const unsigned bad = __ballot_sync(kFull, in && !(ok && osum::inside(C, P)));
+    const int f = bad ? __ffs(bad) - 1 : n;
+    if (f > start)
+    {
+      const bool taken = in && lane < f;
+      long long mn = taken ? P : LLONG_MAX;
+#pragma unroll
+      for (int s = 16; s; s >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, s));
+      const double vmin = osum::unscaled(mn, ce);
+      const long long km = order_key(vmin);
+      if (km < klow)
+      {
+        klow = km;
+        low = vmin;
+        lowpos = __ffs(__ballot_sync(kFull, taken && P == mn)) - 1;
+      }
+      cost = osum::unscaled(__shfl_sync(kFull, P, f - 1), ce);
+      start = f;
+    }
+    if (f < n)
+    {
+      cost = __dadd_rn(cost, __shfl_sync(kFull, d, f));
+      const long long kc = order_key(cost);
+      if (kc < klow)
+      {
+        klow = kc;
+        low = cost;
+        lowpos = f;
+      }
+      start = f + 1;
+    }
   }
-  cost = osum::unscaled(__shfl_sync(kFull, P, 31), ce);
-  return true;
+  double dn = __shfl_sync(kFull, d, start & 31);
+  for (int i = start; i < n; i++)
+  {
+    const double di = dn;
+    dn = __shfl_sync(kFull, d, (i + 1) & 31);  // ahead of the dependent add
+    cost = __dadd_rn(cost, di);
+    const long long kc = order_key(cost);
+    if (kc < klow)
+    {
+      klow = kc;
+      low = cost;
+      lowpos = i;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1343,23 +1380,7 @@ __device__ __noinline__ bool account(const SweepArgs& a, const DevModel& m, cons
       // running cost in flip order (markov/walker.h:225) and the first
       // strict improvement of the lowest (markov/walker.h:269-280)
       int lowpos = -1;
-      if (!cost_prefix(d, n, cost, klow, low, lowpos))
-      {
-        double dn = __shfl_sync(kFull, d, 0);
-        for (int i = 0; i < n; i++)
-        {
-          const double di = dn;
-          dn = __shfl_sync(kFull, d, (i + 1) & 31);  // ahead of the dependent add
-          cost = __dadd_rn(cost, di);
-          const long long kc = order_key(cost);
-          if (kc < klow)
-          {
-            klow = kc;
-            low = cost;
-            lowpos = i;
-          }
-        }
-      }
+      accumulate(d, n, cost, klow, low, lowpos);
       // the accountant's spins, and the lowest state at lowpos
       if (lane < n && lane <= lowpos) atomicXor(R.aspins + (fv >> 5), 1u << (fv & 31));
       __syncwarp();

@@ -1550,19 +1550,18 @@ struct Rows
       c = __ldg(coef + q);
       if (!PAIR) t = make_int2(__ldg(trow + (x & ~kNegBit)), __ldg(trow + (x & ~kNegBit) + 1));
     }
-    if (PAIR)
+    if constexpr (PAIR) on = w[v] ^ ((int)x >= 0 ? w[x] : 0u);
+    else
     {
-      on = w[v] ^ ((int)x >= 0 ? w[x] : 0u);
-      return;
+      for (int i = 0; i < t.y - t.x; i++)
+      {
+        const uint32_t y = j0 == 0 && i < 4 ? S->m[turn & 1u][lane][i] : __ldg(tvar + t.x + i);
+        const int u = (int)(y & ~kNegBit);
+        if (PAR) on ^= w[u];
+        else if (u != v) on |= w[u] ^ ((y & kNegBit) ? kFull : 0u);
+      }
+      if (x & kNegBit) c = -c;
     }
-    for (int i = 0; i < t.y - t.x; i++)
-    {
-      const uint32_t y = j0 == 0 && i < 4 ? S->m[turn & 1u][lane][i] : __ldg(tvar + t.x + i);
-      const int u = (int)(y & ~kNegBit);
-      if (PAR) on ^= w[u];
-      else if (u != v) on |= w[u] ^ ((y & kNegBit) ? kFull : 0u);
-    }
-    if (!PAIR && (x & kNegBit)) c = -c;
   }
 };
 
