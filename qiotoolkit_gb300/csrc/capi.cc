@@ -381,6 +381,11 @@ qio_status qio_solver_replicas(qio_solver* s, int64_t* n, double* cost, double* 
 {
   return guard([&] {
     if (!s || !n) fail(1, "arguments must not be null");
+    if (s->s->initialized && !cost && !lowest && !attempts && !accepts && !lowest_states && !states)
+    {
+      *n = s->s->n_walkers();  // asked for the number alone: nothing to read back
+      return;
+    }
     std::vector<double> c, l;
     std::vector<uint64_t> at, ac;
     std::vector<uint8_t> ls, st;
