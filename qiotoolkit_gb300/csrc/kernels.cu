@@ -2190,6 +2190,9 @@ cudaError_t launch_qmc(const QmcArgs& a, cudaStream_t s)
 // ---------------------------------------------------------------------------
 __global__ void pt_swap_kernel(SwapArgs a)
 {
+  // launched while the sweep before it runs, and lets the next one's blocks in
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   // one warp per restart: lanes over the ladder's walkers, then over the
   // step's pairs (pairs of one parity share no walker)
   const int lane = threadIdx.x & 31;
@@ -2445,8 +2448,17 @@ cudaError_t launch_pt_swap(const SwapArgs& a, cudaStream_t s)
 {
   const int threads = 128;  // four restarts per block, a warp each
   const int blocks = (a.restarts * 32 + threads - 1) / threads;
-  if (blocks > 0) pt_swap_kernel<<<blocks, threads, 0, s>>>(a);
-  return cudaGetLastError();
+  if (blocks <= 0) return cudaGetLastError();
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, pt_swap_kernel, a);
 }
 
 // ---------------------------------------------------------------------------

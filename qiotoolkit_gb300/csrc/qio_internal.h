@@ -162,6 +162,8 @@ struct SweepArgs
   int* err;             // device error flag (a bounded wait gave up)
   long long tag;        // written to p.lowtag[walker] when its lowest drops
   int fields;           // 1: the block-decided sweep
+  int chained;          // ... launched behind a kernel of its own stream that lets it
+                        // start early (tempering's swaps)
   // batches (windowed kernel): walker r runs models[model_of[r]] with the
   // counter key of walker local_of[r] of its own solve; with `queue` set,
   // each warp takes walkers from the counter *queue (reset to 0 before the

@@ -1095,6 +1095,7 @@ class ParallelTempering : public Solver
       a.sweep_base = s * spr;
       a.tag = s;  // the step, for the time order of equal lowest costs
       a.fields = fields ? 1 : 0;
+      a.chained = 1;
       a.order = fields ? hot_first : nullptr;
       prof_begin(st);
       cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
@@ -1177,6 +1178,7 @@ class ParallelTempering : public Solver
       a.sweep_base = step_pos * spr;
       a.tag = step_pos;
       a.fields = fields ? 1 : 0;
+      a.chained = 1;
       a.order = fields ? hot_first : nullptr;
       cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
       sw.step = step_pos;
