@@ -90,7 +90,7 @@ WORKLOADS = {
     "batch_pubo": dict(desc="Batched SA on many-body models: 512 random PUBO instances, N log-uniform "
                             "in [100, 2000], 3N terms of orders 1-4 with N(0,1) FP64 coefficients, 16 "
                             "restarts each, linear beta 0.1->3.0 over 500 sweeps, one captured CUDA "
-                            "graph (the windowed kernel's persistent queue)",
+                            "graph (one persistent queue per kind of model)",
                        target="simulatedannealing.qiotoolkit"),
 }
 
