@@ -37,18 +37,18 @@
 // Integer models keep cost and lowest in the decider (exact in any order).
 //
 // What bounds it: the decider's chain of dependent votes, shared-memory loads
-// and integer instructions, about five cycles each: 1650 cycles a block on a
-// sparse Ising model (N = 1000, 64 walkers: gather 400, decisions 340, commit
-// 165), 3600 on a PUBO of 11.7 terms a variable, four walkers an SM (gather
-// 1360, decisions 640, commit 360), 3000 on 3-SAT.  Measured on the way (ms:
-// 1000 sweeps of the first / 100 of 512 tempering walkers of the second / 200 of
-// 64 of the third): fields kept up to date by shared-memory atomics, 26 to 44
-// cycles of the warp's memory queue each where a load takes 5, 40 / 93 / -; the
-// windowed kernel 63 / 190 / 45; gathered from a byte per term, which every flip
-// has to write, 24.6 / 43.7 / 17.6; from literals, where a flip writes two bytes,
-// 24.9 / 35.6 / 13.1; the same with the accountant finding the contributing terms
+// and integer instructions, about five cycles each, and its branches, ten to
+// twenty: 1300 cycles a block on a sparse Ising model (N = 1000, 64 walkers), 3500
+// on a PUBO of 11.7 terms a variable, four walkers an SM, 2400 on 3-SAT, a third
+// of it the gather, a fifth the decisions.  Measured on the way (ms: 1000 sweeps
+// of the first / 100 of 512 tempering walkers of the second / 200 of 64 of the
+// third): the windowed kernel 63 / 190 / 45; fields kept up to date by
+// shared-memory atomics, 26 to 44 cycles of the warp's memory queue each where a
+// load takes 5, 40 / 93 / -; gathered from a byte per term, which every flip has
+// to write, 24.6 / 43.7 / 17.6; from literals, where a flip writes two bytes, 24.9
+// / 35.6 / 13.1; the same with the accountant finding the contributing terms
 // itself, a row a lane, 25.6 / 59 / 15.8 (its scattered loads take the memory
-// pipe from the deciders), or a row a warp, 39 / 147 / 32.
+// pipe from the deciders), or a row a warp, 39 / 147 / 32; here 20.7 / 36.0 / 10.8.
 //
 // Waits between the warps poll shared-memory counters (acquire/release) with a
 // time limit on lack of progress; on expiry the kernel raises the device error
@@ -57,6 +57,7 @@
 #include <atomic>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 
 #include "metropolis.cuh"
 #include "ordered_sum.cuh"
@@ -801,6 +802,7 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
 
   unsigned buf = t0 % (unsigned)sh.bufs, par = (t0 / (unsigned)sh.bufs) & 1u;  // the coming chunk's buffer and phase
   unsigned head = 0;                // log entries written
+  unsigned moved = 0;               // draws taken when the stream's origin last moved
   unsigned acc_tail = 0, fed = 0;   // the other warps' counters when last looked at
   Sweep S;
   S.betas = a.beta + (long long)r * a.bs_w;
@@ -812,6 +814,13 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
     bi++;
     if (bi == nblocks || gb == 0)
     {
+      if (REPLAY && W.taken - moved > (1u << 28))
+      {
+        // stream positions are 32-bit: move their origin along
+        W.rs = stream_state(R, W);
+        W.raw0 = R.raw[(W.taken - 1u) & (unsigned)(kRing - 1)];
+        moved = W.taken;
+      }
       bi = 0;
       next_sweep<FM, INT>(S, a, inv, N, k++);
     }
@@ -840,405 +849,414 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
     const int n2 = FM == PAIR ? 0 : (int)((h0 >> 15) & 255u) * 2, n3 = FM == PAIR ? 0 : (int)(h1 & 255u);
     const int ents = (int)((h0 >> 23) & 7u), xn = (int)(h1 >> 8);
     const bool staged = C::kRec + 32 * (n0 + n1 + n2 + n3) + 16 * n2 <= cap;
-    const uint2* tile = chunk + lane;
-    int4 own;  // field, degree, negated literals, terms of v alone
-    if (FM == PAIR)
-    {
-      const int2 x = *(const int2*)(tile + C::kLane);
-      own = make_int4(x.x, x.y, 0, 0);
-    }
-    else own = *((const int4*)(chunk + C::kLane) + lane);
-    const uint4* tent = (const uint4*)(chunk + C::kEnt) + lane;
-
-    const uint32_t word = R.spins[bi];  // the block's spins before its flips
-    const uint32_t sv = (word >> lane) & 1u;
-    const int deg = own.y;
-    const int bnd = deg + 1;  // |field - exact| < bnd units
-    const float xmargin = INT ? 0.f : S.fsa * (float)(bnd + 1);
-
-    // ---- the field: the lane's value less the weights of the records whose
-    // op is 1.  Rows come in fours (one literal) and twos and are taken four or
-    // eight at a time, a load's latency being six rows' work (3-SAT, 18 rows of
-    // two: 1120 cycles a block in twos; 200 sweeps 13.1 and 12.5 ms; sparse Ising
-    // in fours and eights 24.5 and 23.4 ms).
-    int base = own.x;
-    unsigned qm = (unsigned)own.w;  // COUNTER: the incidences that contribute; PARITY: those of odd parity
-    auto op = [](uint32_t x, uint32_t y) -> uint32_t { return FM == COUNTER ? (x | y) : (x ^ y); };
-    // a record's op (0 or 1) and weight into field and mask
-    auto put = [&](uint32_t on, uint32_t w) {
-      if (MASKS)
-      {
-        base -= (int)on * (int)(w & ~255u);
-        if ((FM == COUNTER) != (on != 0u)) qm |= __funnelshift_l(0u, 1u, w);
-      }
-      else base -= (int)on * (int)w;
-    };
-    auto gather = [&](const uint2* t0) {
-      if constexpr (FM == PAIR)
-      {
-        uint2 e[8];
-        for (int i = 0; i + 8 <= n0; i += 8)
-        {
-#pragma unroll
-          for (int x = 0; x < 8; x++) e[x] = t0[32 * (i + x)];
-#pragma unroll
-          for (int x = 0; x < 8; x++) put(R.z[e[x].x], e[x].y);
-        }
-        if (n0 & 4)
-        {
-#pragma unroll
-          for (int x = 0; x < 4; x++) e[x] = t0[32 * (n0 - 4 + x)];
-#pragma unroll
-          for (int x = 0; x < 4; x++) put(R.z[e[x].x], e[x].y);
-        }
-      }
-      else
-      {
-        {
-          uint2 e[4];
-#pragma unroll
-          for (int x = 0; x < 4; x++) e[x] = n0 ? t0[32 * x] : make_uint2(0u, 0u);
-          for (int i = 4; i <= n0; i += 4)
-          {
-            uint2 f[4];
-            const uint2* t1 = t0 + 32 * (i < n0 ? i : 0);
-#pragma unroll
-            for (int x = 0; x < 4; x++) f[x] = t1[32 * x];
-#pragma unroll
-            for (int x = 0; x < 4; x++) put(R.z[e[x].x], e[x].y);
-#pragma unroll
-            for (int x = 0; x < 4; x++) e[x] = f[x];
-          }
-        }
-        t0 += 32 * n0;
-        if (n1)
-        {
-          auto two = [&](const uint2& e) { put(op(R.z[e.x & 0xFFFFu], R.z[e.x >> 16]), e.y); };
-          uint2 e[4];
-#pragma unroll
-          for (int x = 0; x < 4; x++) e[x] = t0[32 * min(x, n1 - 1)];
-          int i = 4;
-          for (; i <= n1; i += 4)
-          {
-            uint2 f[4];
-#pragma unroll
-            for (int x = 0; x < 4; x++) f[x] = t0[32 * min(i + x, n1 - 1)];
-#pragma unroll
-            for (int x = 0; x < 4; x++) two(e[x]);
-#pragma unroll
-            for (int x = 0; x < 4; x++) e[x] = f[x];
-          }
-          if (i - 4 < n1)
-          {
-            two(e[0]);
-            two(e[1]);
-          }
-          t0 += 32 * n1;
-        }
-        if (n2)
-        {
-          const uint32_t* c0 = (const uint32_t*)(t0 - lane + 32 * n2) + lane;  // the third literals
-          uint2 e0 = t0[0], e1 = t0[32];
-          uint32_t k0 = c0[0], k1 = c0[32];
-          for (int i = 2; i <= n2; i += 2)
-          {
-            const int nx = i < n2 ? i : 0;
-            const uint2 f0 = t0[32 * nx], f1 = t0[32 * nx + 32];
-            const uint32_t g0 = c0[32 * nx], g1 = c0[32 * nx + 32];
-            const uint32_t a0 = R.z[e0.x & 0xFFFFu], b0 = R.z[e0.x >> 16], d0 = R.z[k0];
-            const uint32_t a1 = R.z[e1.x & 0xFFFFu], b1 = R.z[e1.x >> 16], d1 = R.z[k1];
-            put(op(op(a0, b0), d0), e0.y);
-            put(op(op(a1, b1), d1), e1.y);
-            e0 = f0;
-            e1 = f1;
-            k0 = g0;
-            k1 = g1;
-          }
-          t0 += 48 * n2;
-        }
-        // wide terms: the true literals but for the own, or the others' parity
-        for (int i = 0; i < n3; i++)
-        {
-          const uint2 e = t0[32 * i];
-          const uint32_t zz = zw[e.x & kWideMask];
-          const uint32_t on = FM == COUNTER ? (zz != ((sv ^ (e.x >> 31)) & 1u) ? 1u : 0u) : ((zz ^ sv) & 1u);
-          if (!(e.x & (kNoWide | kSharedWide))) put(on, e.y);
-        }
-      }
-    };
-    const uint2* far = table;  // (not staged) the records
-    if (staged) gather(tile + C::kRec);
-    else
-    {
-      far = table + __ldg(descs + bi).x + C::kRec + lane;
-      gather(far);
-    }
-
-    // ---- the in-block terms under a given accept mask, all against the state
-    // at the block's start.  Pair models: the member's flip changes the field
-    // by c0.  Counter models: the other literals are all false when those of
-    // the members before this lane (em) are -- the flipped ones are exactly the
-    // true ones (et) -- and those after it or elsewhere were (else em = 0, et =
-    // 1: never).  Parities: c0 of the others, and of the flips in em.
-    unsigned watch = 0;  // lanes whose flips change this lane's field
-    int val[KI];
-    unsigned bit[KI];  // its place in the mask
-    unsigned em[KI], et[KI];
-    // further entries (rare): xn of them, in HBM
-    const size_t xat = xn ? (size_t)__shfl_sync(kFull, chunk[1].x, 0) + lane : 0;
-    const uint2* xpair = (const uint2*)further + xat;
-    const uint4* xterm = (const uint4*)further + xat;
-    unsigned done = 0;  // the block's flips so far
-    // an entry's em and et; D: flips whose bytes are written already
-    auto entry = [&](const uint4& e, unsigned D, unsigned& mm, unsigned& mt) {
-      const uint32_t M = e.x, L = (word ^ e.y) & M;  // members before this lane, their true literals
-      const bool wide = FM != PAIR && (e.z >> 18) == 0x3FFFu;
-      uint32_t o;  // the other members: whether a literal is true, or their parity
-      if (!wide) o = op(R.z[e.z & 0xFFFFu], R.z[e.z >> 16]);
-      else
-      {
-        const uint32_t zz = zw[e.z & kWideMask], lit = (sv ^ (e.y >> lane)) & 1u;
-        if (FM == COUNTER) o = (int)zz - (int)lit != __popc((L ^ D) & M) ? 1u : 0u;
-        else o = (zz ^ sv ^ (uint32_t)__popc((word ^ D) & M)) & 1u;
-      }
-      mm = M;
-      mt = FM == COUNTER ? L : (o ^ (uint32_t)__popc(word & M)) & 1u;
-      if (FM == COUNTER && o)
-      {
-        mm = 0u;
-        mt = 1u;
-      }
-    };
-    auto holds = [&](unsigned A, unsigned mm, unsigned mt) -> bool {
-      return FM == COUNTER ? (A & mm) == mt : ((mt ^ (unsigned)__popc(A & mm)) & 1u) != 0u;
-    };
-#pragma unroll
-    for (int i = 0; i < KI; i++)
-    {
-      em[i] = bit[i] = 0u;
-      et[i] = 1u;
-      val[i] = 0;
-      if (FM != PAIR && i >= 2 && ents <= 2) continue;  // (most blocks have two at most)
+    // The block itself.  SP: it has records or entries beyond its chunk, or wide
+    // terms; the other form, most blocks', has a branch less for each of these
+    // (a branch costs ten to twenty cycles of its warp): sparse Ising 23.6 and
+    // 20.7 ms with the stream's positions looked after once a sweep, 3-SAT 11.9
+    // and 10.8.
+    auto block = [&](auto sp) __attribute__((always_inline)) -> bool {
+      constexpr bool SP = decltype(sp)::value;
+      const uint2* tile = chunk + lane;
+      int4 own;  // field, degree, negated literals, terms of v alone
       if (FM == PAIR)
       {
-        const uint2 e = tile[C::kEnt + 32 * i];
-        em[i] = e.x;
-        val[i] = (word & e.x) ? (int)e.y : -(int)e.y;
-        watch |= e.x;
+        const int2 x = *(const int2*)(tile + C::kLane);
+        own = make_int4(x.x, x.y, 0, 0);
       }
+      else own = *((const int4*)(chunk + C::kLane) + lane);
+      const uint4* tent = (const uint4*)(chunk + C::kEnt) + lane;
+
+      const uint32_t word = R.spins[bi];  // the block's spins before its flips
+      const uint32_t sv = (word >> lane) & 1u;
+      const int deg = own.y;
+      const int bnd = deg + 1;  // |field - exact| < bnd units
+      const float xmargin = INT ? 0.f : S.fsa * (float)(bnd + 1);
+
+      // ---- the field: the lane's value less the weights of the records whose
+      // op is 1.  Rows come in fours (one literal) and twos and are taken four or
+      // eight at a time, a load's latency being six rows' work (3-SAT, 18 rows of
+      // two: 1120 cycles a block in twos; 200 sweeps 13.1 and 12.5 ms; sparse Ising
+      // in fours and eights 24.5 and 23.4 ms).
+      int base = own.x;
+      unsigned qm = (unsigned)own.w;  // COUNTER: the incidences that contribute; PARITY: those of odd parity
+      auto op = [](uint32_t x, uint32_t y) -> uint32_t { return FM == COUNTER ? (x | y) : (x ^ y); };
+      // a record's op (0 or 1) and weight into field and mask
+      auto put = [&](uint32_t on, uint32_t w) {
+        if (MASKS)
+        {
+          base -= (int)on * (int)(w & ~255u);
+          if ((FM == COUNTER) != (on != 0u)) qm |= __funnelshift_l(0u, 1u, w);
+        }
+        else base -= (int)on * (int)w;
+      };
+      auto gather = [&](const uint2* t0) {
+        if constexpr (FM == PAIR)
+        {
+          uint2 e[8];
+          for (int i = 0; i + 8 <= n0; i += 8)
+          {
+#pragma unroll
+            for (int x = 0; x < 8; x++) e[x] = t0[32 * (i + x)];
+#pragma unroll
+            for (int x = 0; x < 8; x++) put(R.z[e[x].x], e[x].y);
+          }
+          if (n0 & 4)
+          {
+#pragma unroll
+            for (int x = 0; x < 4; x++) e[x] = t0[32 * (n0 - 4 + x)];
+#pragma unroll
+            for (int x = 0; x < 4; x++) put(R.z[e[x].x], e[x].y);
+          }
+        }
+        else
+        {
+          {
+            uint2 e[4];
+#pragma unroll
+            for (int x = 0; x < 4; x++) e[x] = n0 ? t0[32 * x] : make_uint2(0u, 0u);
+            for (int i = 4; i <= n0; i += 4)
+            {
+              uint2 f[4];
+              const uint2* t1 = t0 + 32 * (i < n0 ? i : 0);
+#pragma unroll
+              for (int x = 0; x < 4; x++) f[x] = t1[32 * x];
+#pragma unroll
+              for (int x = 0; x < 4; x++) put(R.z[e[x].x], e[x].y);
+#pragma unroll
+              for (int x = 0; x < 4; x++) e[x] = f[x];
+            }
+          }
+          t0 += 32 * n0;
+          if (n1)
+          {
+            auto two = [&](const uint2& e) { put(op(R.z[e.x & 0xFFFFu], R.z[e.x >> 16]), e.y); };
+            uint2 e[4];
+#pragma unroll
+            for (int x = 0; x < 4; x++) e[x] = t0[32 * min(x, n1 - 1)];
+            int i = 4;
+            for (; i <= n1; i += 4)
+            {
+              uint2 f[4];
+#pragma unroll
+              for (int x = 0; x < 4; x++) f[x] = t0[32 * min(i + x, n1 - 1)];
+#pragma unroll
+              for (int x = 0; x < 4; x++) two(e[x]);
+#pragma unroll
+              for (int x = 0; x < 4; x++) e[x] = f[x];
+            }
+            if (i - 4 < n1)
+            {
+              two(e[0]);
+              two(e[1]);
+            }
+            t0 += 32 * n1;
+          }
+          if (n2)
+          {
+            const uint32_t* c0 = (const uint32_t*)(t0 - lane + 32 * n2) + lane;  // the third literals
+            uint2 e0 = t0[0], e1 = t0[32];
+            uint32_t k0 = c0[0], k1 = c0[32];
+            for (int i = 2; i <= n2; i += 2)
+            {
+              const int nx = i < n2 ? i : 0;
+              const uint2 f0 = t0[32 * nx], f1 = t0[32 * nx + 32];
+              const uint32_t g0 = c0[32 * nx], g1 = c0[32 * nx + 32];
+              const uint32_t a0 = R.z[e0.x & 0xFFFFu], b0 = R.z[e0.x >> 16], d0 = R.z[k0];
+              const uint32_t a1 = R.z[e1.x & 0xFFFFu], b1 = R.z[e1.x >> 16], d1 = R.z[k1];
+              put(op(op(a0, b0), d0), e0.y);
+              put(op(op(a1, b1), d1), e1.y);
+              e0 = f0;
+              e1 = f1;
+              k0 = g0;
+              k1 = g1;
+            }
+            t0 += 48 * n2;
+          }
+          // wide terms: the true literals but for the own, or the others' parity
+          for (int i = 0; SP && i < n3; i++)
+          {
+            const uint2 e = t0[32 * i];
+            const uint32_t zz = zw[e.x & kWideMask];
+            const uint32_t on = FM == COUNTER ? (zz != ((sv ^ (e.x >> 31)) & 1u) ? 1u : 0u) : ((zz ^ sv) & 1u);
+            if (!(e.x & (kNoWide | kSharedWide))) put(on, e.y);
+          }
+        }
+      };
+      const uint2* far = table;  // (not staged) the records
+      if (!SP || staged) gather(tile + C::kRec);
       else
       {
-        const uint4 e = tent[32 * i];
-        entry(e, 0u, em[i], et[i]);
-        val[i] = MASKS ? (int)(e.w & ~255u) : (int)e.w;
-        bit[i] = MASKS && e.x ? __funnelshift_l(0u, 1u, e.w) : 0u;
-        watch |= e.x;
+        far = table + __ldg(descs + bi).x + C::kRec + lane;
+        gather(far);
       }
-    }
-    for (int i = 0; i < xn; i++) watch |= FM == PAIR ? __ldg(xpair + 32 * i).x : __ldg(&xterm[32 * i].x);
 
-    // ---- the other warps: room for this block's flips and draws
-    auto room = [&]() -> bool {
-      return (INT || (int)(head + 32u - (unsigned)kLog - acc_tail) <= 0) && (int)(fed - (W.taken + 32u)) >= 0;
-    };
-    if (!room())
-    {
-      look(R, acc_tail, fed);
+      // ---- the in-block terms under a given accept mask, all against the state
+      // at the block's start.  Pair models: the member's flip changes the field
+      // by c0.  Counter models: the other literals are all false when those of
+      // the members before this lane (em) are -- the flipped ones are exactly the
+      // true ones (et) -- and those after it or elsewhere were (else em = 0, et =
+      // 1: never).  Parities: c0 of the others, and of the flips in em.
+      unsigned watch = 0;  // lanes whose flips change this lane's field
+      int val[KI];
+      unsigned bit[KI];  // its place in the mask
+      unsigned em[KI], et[KI];
+      // further entries (rare): xn of them, in HBM
+      const size_t xat = SP && xn ? (size_t)__shfl_sync(kFull, chunk[1].x, 0) + lane : 0;
+      const uint2* xpair = (const uint2*)further + xat;
+      const uint4* xterm = (const uint4*)further + xat;
+      unsigned done = 0;  // the block's flips so far
+      // an entry's em and et; D: flips whose bytes are written already
+      auto entry = [&](const uint4& e, unsigned D, unsigned& mm, unsigned& mt) {
+        const uint32_t M = e.x, L = (word ^ e.y) & M;  // members before this lane, their true literals
+        const bool wide = FM != PAIR && (e.z >> 18) == 0x3FFFu;
+        uint32_t o;  // the other members: whether a literal is true, or their parity
+        if (!wide) o = op(R.z[e.z & 0xFFFFu], R.z[e.z >> 16]);
+        else
+        {
+          const uint32_t zz = zw[e.z & kWideMask], lit = (sv ^ (e.y >> lane)) & 1u;
+          if (FM == COUNTER) o = (int)zz - (int)lit != __popc((L ^ D) & M) ? 1u : 0u;
+          else o = (zz ^ sv ^ (uint32_t)__popc((word ^ D) & M)) & 1u;
+        }
+        mm = M;
+        mt = FM == COUNTER ? L : (o ^ (uint32_t)__popc(word & M)) & 1u;
+        if (FM == COUNTER && o)
+        {
+          mm = 0u;
+          mt = 1u;
+        }
+      };
+      auto holds = [&](unsigned A, unsigned mm, unsigned mt) -> bool {
+        return FM == COUNTER ? (A & mm) == mt : ((mt ^ (unsigned)__popc(A & mm)) & 1u) != 0u;
+      };
+#pragma unroll
+      for (int i = 0; i < KI; i++)
+      {
+        em[i] = bit[i] = 0u;
+        et[i] = 1u;
+        val[i] = 0;
+        if (FM != PAIR && i >= 2 && ents <= 2) continue;  // (most blocks have two at most)
+        if (FM == PAIR)
+        {
+          const uint2 e = tile[C::kEnt + 32 * i];
+          em[i] = e.x;
+          val[i] = (word & e.x) ? (int)e.y : -(int)e.y;
+          watch |= e.x;
+        }
+        else
+        {
+          const uint4 e = tent[32 * i];
+          entry(e, 0u, em[i], et[i]);
+          val[i] = MASKS ? (int)(e.w & ~255u) : (int)e.w;
+          bit[i] = MASKS && e.x ? __funnelshift_l(0u, 1u, e.w) : 0u;
+          watch |= e.x;
+        }
+      }
+      if (SP)
+        for (int i = 0; i < xn; i++) watch |= FM == PAIR ? __ldg(xpair + 32 * i).x : __ldg(&xterm[32 * i].x);
+
+      // ---- the other warps: room for this block's flips and draws
+      auto room = [&]() -> bool {
+        return (INT || (int)(head + 32u - (unsigned)kLog - acc_tail) <= 0) && (int)(fed - (W.taken + 32u)) >= 0;
+      };
       if (!room())
       {
-        wait_room<INT, kLog>(R.tail, R.made, R.abort, a.err, head, W.taken);
         look(R, acc_tail, fed);
-        if (!room()) return false;
+        if (!room())
+        {
+          wait_room<INT, kLog>(R.tail, R.made, R.abort, a.err, head, W.taken);
+          look(R, acc_tail, fed);
+          if (!room()) return false;
+        }
       }
-    }
 
-    // ---- rounds: one, unless a lane has to be tried alone
-    float2 iv0 = make_float2(0.f, 0.f);
-    if (!REPLAY) iv0 = R.ring[(W.taken + (unsigned)lane) & (unsigned)(kRing - 1)];
-    int cursor = 0;
-    while (true)
-    {
-      const bool active = lane >= cursor && lane < nvalid;
-      const unsigned before = lt & ~((1u << cursor) - 1u);
-      // ---- decisions: iterate until no lane's in-block members change
-      unsigned A = done, U = 0, lm = 0;
-      int g = 0;
-      bool rare = false;
+      // ---- rounds: one, unless a lane has to be tried alone
+      float2 iv0 = make_float2(0.f, 0.f);
+      if (!REPLAY) iv0 = R.ring[(W.taken + (unsigned)lane) & (unsigned)(kRing - 1)];
+      int cursor = 0;
       while (true)
       {
-        int h = base;
-        lm = qm;
+        const bool active = lane >= cursor && lane < nvalid;
+        const unsigned before = lt & ~((1u << cursor) - 1u);
+        // ---- decisions: iterate until no lane's in-block members change
+        unsigned A = done, U = 0, lm = 0;
+        int g = 0;
+        bool rare = false;
+        while (true)
+        {
+          int h = base;
+          lm = qm;
 #pragma unroll
-        for (int i = 0; i < KI; i++)
-        {
-          if (FM != PAIR && i >= 2 && ents <= 2) continue;
-          if (FM == PAIR)
+          for (int i = 0; i < KI; i++)
           {
-            h += (A & em[i]) ? val[i] : 0;
-            continue;
+            if (FM != PAIR && i >= 2 && ents <= 2) continue;
+            if (FM == PAIR)
+            {
+              h += (A & em[i]) ? val[i] : 0;
+              continue;
+            }
+            const bool on = holds(A, em[i], et[i]);
+            if (FM == COUNTER) h += on ? val[i] : 0;
+            else h += on ? -val[i] : val[i];
+            if (MASKS && on) lm |= bit[i];
           }
-          const bool on = holds(A, em[i], et[i]);
-          if (FM == COUNTER) h += on ? val[i] : 0;
-          else h += on ? -val[i] : val[i];
-          if (MASKS && on) lm |= bit[i];
-        }
-        for (int i = 0; i < xn; i++)
-        {
-          if (FM == PAIR)
+          for (int i = 0; SP && i < xn; i++)
           {
-            const uint2 e = __ldg(xpair + 32 * i);
-            h += (A & e.x) ? ((word & e.x) ? (int)e.y : -(int)e.y) : 0;
+            if (FM == PAIR)
+            {
+              const uint2 e = __ldg(xpair + 32 * i);
+              h += (A & e.x) ? ((word & e.x) ? (int)e.y : -(int)e.y) : 0;
+            }
+            else
+            {
+              const uint4 e = __ldg(xterm + 32 * i);
+              unsigned mm, mt;
+              entry(e, done, mm, mt);
+              const bool on = e.x && holds(A, mm, mt);
+              const int w = MASKS ? (int)(e.w & ~255u) : (int)e.w;
+              if (FM == COUNTER) h += on ? w : 0;
+              else h += on ? -w : w;
+              if (MASKS && on) lm |= __funnelshift_l(0u, 1u, e.w);
+            }
+          }
+          // the field in the variable's own direction, its sign and threshold
+          bool up;
+          float x;
+          if (INT)
+          {
+            g = FM == COUNTER ? (sv ? h : -h) : (sv ? 2 * h : -2 * h);  // the cost difference
+            up = active && g > 0;
+            x = (float)g;
+            rare = false;
+          }
+          else if (FM == COUNTER)
+          {
+            const int fd = sv ? (h >> 8) : -(h >> 8);
+            const bool zero = lm == 0u;  // nothing contributes: +0.0
+            up = active && !zero && fd > bnd;
+            rare = active && !zero && (unsigned)(fd + bnd) <= (unsigned)(2 * bnd);
+            x = (float)fd;
           }
           else
           {
-            const uint4 e = __ldg(xterm + 32 * i);
-            unsigned mm, mt;
-            entry(e, done, mm, mt);
-            const bool on = e.x && holds(A, mm, mt);
-            const int w = MASKS ? (int)(e.w & ~255u) : (int)e.w;
-            if (FM == COUNTER) h += on ? w : 0;
-            else h += on ? -w : w;
-            if (MASKS && on) lm |= __funnelshift_l(0u, 1u, e.w);
+            if (FM == PARITY) h >>= 8;
+            g = sv ? -h : h;
+            up = active && g < -bnd;
+            rare = active && (unsigned)(g + bnd) <= (unsigned)(2 * bnd);
+            x = (float)g;
           }
-        }
-        // the field in the variable's own direction, its sign and threshold
-        bool up;
-        float x;
-        if (INT)
-        {
-          g = FM == COUNTER ? (sv ? h : -h) : (sv ? 2 * h : -2 * h);  // the cost difference
-          up = active && g > 0;
-          x = (float)g;
-          rare = false;
-        }
-        else if (FM == COUNTER)
-        {
-          const int fd = sv ? (h >> 8) : -(h >> 8);
-          const bool zero = lm == 0u;  // nothing contributes: +0.0
-          up = active && !zero && fd > bnd;
-          rare = active && !zero && (unsigned)(fd + bnd) <= (unsigned)(2 * bnd);
-          x = (float)fd;
-        }
-        else
-        {
-          if (FM == PARITY) h >>= 8;
-          g = sv ? -h : h;
-          up = active && g < -bnd;
-          rare = active && (unsigned)(g + bnd) <= (unsigned)(2 * bnd);
-          x = (float)g;
-        }
-        // (an infinite beta: below every draw but an always accepting one)
-        const float thr = S.beta_inf ? -3e38f : __fmul_rn(x, S.fscale);
-        const float et = S.beta_inf ? 0.f : __fmaf_rn(fabsf(thr), 1.9073486328125e-06f, 1e-30f) + xmargin;  // 2^-19
-        float2 iv = iv0;
-        if (REPLAY)
-        {
-          U = __ballot_sync(kFull, up);
-          iv = R.ring[(W.taken + (unsigned)__popc(U & before)) & (unsigned)(kRing - 1)];
-        }
-        const bool yes = iv.y < __fsub_rn(thr, et);
-        const bool no = iv.x > __fadd_rn(thr, et);
-        rare = rare || (up && !yes && !no);
-        const bool acc = active && !rare && (!up || yes);
-        if (MASKS) rare = rare || (acc && deg > 32);  // its masks do not fit the log
-        const unsigned An = __ballot_sync(kFull, acc) | done;
-        const unsigned diff = An ^ A;
-        A = An;
-        if (!__any_sync(kFull, (diff & watch) != 0u)) break;
-      }
-
-      // ---- what is committed: all, or the lanes before the first rare one, or
-      // that one alone
-      const unsigned Rm = __ballot_sync(kFull, rare);
-      unsigned F = A & ~done;
-      bool exact = false, last = true;
-      double dE = 0.0;
-      if (Rm == 0u)
-      {
-        if (REPLAY) W.taken += (unsigned)__popc(U);
-      }
-      else
-      {
-        const int f = __ffs(Rm) - 1;
-        if (f > cursor)
-        {
-          F &= (1u << f) - 1u;
-          if (REPLAY) W.taken += (unsigned)__popc(U & ((1u << f) - 1u));
-          cursor = f;
-        }
-        else
-        {
-          const uint64_t rs = REPLAY ? stream_state(R, W) : 0;
-          unsigned res = 0;
-          if (lane == f)
-            res = exact_attempt<FM, REPLAY, INT>(m, v, g, R.spins, rs, W.key, S.ctr0 + (unsigned long long)v, S.beta,
-                                                 &dE);
-          res = __shfl_sync(kFull, res, f);
-          F = (res & 1u) << f;
-          if (REPLAY) W.taken += res >> 1;
-          exact = true;
-          cursor = f + 1;
-        }
-        last = cursor >= nvalid;
-      }
-      const bool mine = ((F >> lane) & 1u) != 0u;
-      const unsigned at = (head + (unsigned)__popc(F & lt)) & (unsigned)(kLog - 1);
-      const unsigned all = done | F;
-      if (!INT && mine)
-      {
-        if (FM == PAIR) ((uint32_t*)R.log)[at] = (uint32_t)v;
-        else
-        {
-          const unsigned long long bits = (unsigned long long)__double_as_longlong(dE);
-          const unsigned negs = (unsigned)own.z;
-          uint4 ent;
-          ent.x = (unsigned)v | ((unsigned)deg << 16) | (exact ? kExactF : 0u);
-          // COUNTER: the sign is the literal; PARITY: the term's, the other
-          // members' parity and the own spin
-          ent.y = exact ? (unsigned)bits : lm;
-          ent.z = exact ? (unsigned)(bits >> 32) : (FM == COUNTER ? (sv ? ~negs : negs) : (sv ? ~lm : lm));
-          ent.w = 0u;
-          R.log[at] = ent;
-        }
-      }
-      if (FM == PAIR)
-      {
-        if (mine) R.z[v] = (uint8_t)(sv ^ 1u);
-      }
-      else if (F)
-      {
-        if (!INT && xn) __syncwarp();  // (entries have been read)
-        if (mine) ((uint16_t*)R.z)[v] = (uint16_t)((sv ^ 1u) | sv << 8);
-        if (n3 && mine)
-        {
-          const uint2* t3 = (staged ? tile + C::kRec : far) + 32 * (n0 + n1) + 48 * n2;
-          for (int i = 0; i < n3; i++)
+          // (an infinite beta: below every draw but an always accepting one)
+          const float thr = S.beta_inf ? -3e38f : __fmul_rn(x, S.fscale);
+          const float et = S.beta_inf ? 0.f : __fmaf_rn(fabsf(thr), 1.9073486328125e-06f, 1e-30f) + xmargin;  // 2^-19
+          float2 iv = iv0;
+          if (REPLAY)
           {
-            const uint32_t x = t3[32 * i].x;
-            if (!(x & kNoWide)) flip_wide<FM>(zw, x & kWideMask, (sv ^ (x >> 31)) & 1u);
+            U = __ballot_sync(kFull, up);
+            iv = R.ring[(W.taken + (unsigned)__popc(U & before)) & (unsigned)(kRing - 1)];
+          }
+          const bool yes = iv.y < __fsub_rn(thr, et);
+          const bool no = iv.x > __fadd_rn(thr, et);
+          rare = rare || (up && !yes && !no);
+          const bool acc = active && !rare && (!up || yes);
+          if (MASKS) rare = rare || (acc && deg > 32);  // its masks do not fit the log
+          const unsigned An = __ballot_sync(kFull, acc) | done;
+          const unsigned diff = An ^ A;
+          A = An;
+          if (!__any_sync(kFull, (diff & watch) != 0u)) break;
+        }
+
+        // ---- what is committed: all, or the lanes before the first rare one, or
+        // that one alone
+        const unsigned Rm = __ballot_sync(kFull, rare);
+        unsigned F = A & ~done;
+        bool exact = false, last = true;
+        double dE = 0.0;
+        if (Rm == 0u)
+        {
+          if (REPLAY) W.taken += (unsigned)__popc(U);
+        }
+        else
+        {
+          const int f = __ffs(Rm) - 1;
+          if (f > cursor)
+          {
+            F &= (1u << f) - 1u;
+            if (REPLAY) W.taken += (unsigned)__popc(U & ((1u << f) - 1u));
+            cursor = f;
+          }
+          else
+          {
+            const uint64_t rs = REPLAY ? stream_state(R, W) : 0;
+            unsigned res = 0;
+            if (lane == f)
+              res = exact_attempt<FM, REPLAY, INT>(m, v, g, R.spins, rs, W.key, S.ctr0 + (unsigned long long)v, S.beta,
+                                                   &dE);
+            res = __shfl_sync(kFull, res, f);
+            F = (res & 1u) << f;
+            if (REPLAY) W.taken += res >> 1;
+            exact = true;
+            cursor = f + 1;
+          }
+          last = cursor >= nvalid;
+        }
+        const bool mine = ((F >> lane) & 1u) != 0u;
+        const unsigned at = (head + (unsigned)__popc(F & lt)) & (unsigned)(kLog - 1);
+        const unsigned all = done | F;
+        if (!INT && mine)
+        {
+          if (FM == PAIR) ((uint32_t*)R.log)[at] = (uint32_t)v;
+          else
+          {
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(dE);
+            const unsigned negs = (unsigned)own.z;
+            uint4 ent;
+            ent.x = (unsigned)v | ((unsigned)deg << 16) | (exact ? kExactF : 0u);
+            // COUNTER: the sign is the literal; PARITY: the term's, the other
+            // members' parity and the own spin
+            ent.y = exact ? (unsigned)bits : lm;
+            ent.z = exact ? (unsigned)(bits >> 32) : (FM == COUNTER ? (sv ? ~negs : negs) : (sv ? ~lm : lm));
+            ent.w = 0u;
+            R.log[at] = ent;
           }
         }
+        if (FM == PAIR)
+        {
+          if (mine) R.z[v] = (uint8_t)(sv ^ 1u);
+        }
+        else if (F)
+        {
+          if (SP && !INT && xn) __syncwarp();  // (entries have been read)
+          if (mine) ((uint16_t*)R.z)[v] = (uint16_t)((sv ^ 1u) | sv << 8);
+          if (SP && n3 && mine)
+          {
+            const uint2* t3 = (staged ? tile + C::kRec : far) + 32 * (n0 + n1) + 48 * n2;
+            for (int i = 0; i < n3; i++)
+            {
+              const uint32_t x = t3[32 * i].x;
+              if (!(x & kNoWide)) flip_wide<FM>(zw, x & kWideMask, (sv ^ (x >> 31)) & 1u);
+            }
+          }
+        }
+        __syncwarp();
+        R.spins[bi] = word ^ all;  // (every lane the same word)
+        __syncwarp();
+        if (INT && F) account_int(R, W, scan32, g, F, bi, nblocks, g_lsp);
+        const unsigned nfl = (unsigned)__popc(F);
+        head += nfl;
+        W.nacc += nfl;
+        W.nwin++;
+        done = all;
+        if (last) break;
       }
-      __syncwarp();
-      R.spins[bi] = word ^ all;  // (every lane the same word)
-      __syncwarp();
-      if (INT && F) account_int(R, W, scan32, g, F, bi, nblocks, g_lsp);
-      const unsigned nfl = (unsigned)__popc(F);
-      head += nfl;
-      W.nacc += nfl;
-      W.nwin++;
-      done = all;
-      if (last) break;
+      return true;
+    };
+    if (!staged || xn != 0 || n3 != 0)
+    {
+      if (!block(std::true_type{})) return false;
     }
+    else if (!block(std::false_type{})) return false;
     if (!REPLAY) W.taken += 32u;
     W.natt += (unsigned)nvalid;
     publish(R, (unsigned)gb + 1u, head, W.taken);
-    if (REPLAY && (gb & 0xFFFF) == 0xFFFF)
-    {
-      // stream positions are 32-bit: move their origin along
-      W.rs = stream_state(R, W);
-      W.raw0 = W.taken ? R.raw[(W.taken - 1u) & (unsigned)(kRing - 1)] : 0u;
-    }
   }
   return true;
 }
