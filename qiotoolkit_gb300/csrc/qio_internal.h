@@ -164,7 +164,7 @@ struct SweepArgs
   int fields;           // 1: the block-decided sweep
   int chained;          // ... launched behind a kernel of its own stream that lets it
                         // start early (tempering's swaps)
-  // batches (windowed kernel): walker r runs models[model_of[r]] with the
+  // batches: walker r runs models[model_of[r]] with the
   // counter key of walker local_of[r] of its own solve; with `queue` set,
   // each warp takes walkers from the counter *queue (reset to 0 before the
   // launch) until n_walkers are taken, in index order, and keeps walker r's

@@ -633,7 +633,7 @@ class SimulatedAnnealing : public Solver
     fields = !levels && !lanes && fields_for(*this, *model, P, full_maxsat_sweep);
     used_kernel = levels ? 3 : (lanes ? 2 : (fields ? 8 : 1));
     // the lane and level sweeps work from the spins and rebuild the term
-    // bytes when they finish; the field-cached sweep makes its own
+    // bytes when they finish; the block-decided sweep works from the spins
     a.skip_terms = (levels || lanes || fields) ? 1 : 0;
     cuda_check(launch_init(a, st), "init kernel");
     launches++;
@@ -867,7 +867,7 @@ class ParallelTempering : public Solver
   std::vector<double> temps;   // sorted
   std::vector<double> betas;   // per position
   Population P;
-  bool fields = false;         // field-cached sweep
+  bool fields = false;         // block-decided sweep
   DevBuf aux;
   int* dir = nullptr;
   double *obs_acc = nullptr, *obs_cost = nullptr, *obs_dir = nullptr;
@@ -1018,7 +1018,7 @@ class ParallelTempering : public Solver
     cuda_check(cudaMemcpyAsync(P.beta, bw.data(), W * 8, cudaMemcpyHostToDevice, st), "H2D");
     cuda_check(cudaMemcpyAsync(master, ms.data(), K * 8, cudaMemcpyHostToDevice, st), "H2D");
     cuda_check(cudaMemcpyAsync(swap_key, keys.data(), K * 8, cudaMemcpyHostToDevice, st), "H2D");
-    // walkers hottest first (smallest beta; stable): the field-cached
+    // walkers hottest first (smallest beta; stable): the block-decided
     // sweep's blocks take them in this order
     std::vector<int> ord(W);
     for (int w = 0; w < W; w++) ord[w] = w;
