@@ -1034,7 +1034,8 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
         em[i] = bit[i] = 0u;
         et[i] = 1u;
         val[i] = 0;
-        if (FM != PAIR && i >= 2 && ents <= 2) continue;  // (most blocks have two at most)
+      }
+      auto take = [&](int i) {
         if (FM == PAIR)
         {
           const uint2 e = tile[C::kEnt + 32 * i];
@@ -1050,6 +1051,13 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
           bit[i] = MASKS && e.x ? __funnelshift_l(0u, 1u, e.w) : 0u;
           watch |= e.x;
         }
+      };
+      take(0);
+      take(1);
+      if (FM == PAIR || ents > 2)  // (most blocks have two at most; one branch for both: 3-SAT 10.6 and 10.3 ms)
+      {
+        take(2);
+        take(3);
       }
       if (SP)
         for (int i = 0; i < xn; i++) watch |= FM == PAIR ? __ldg(xpair + 32 * i).x : __ldg(&xterm[32 * i].x);
@@ -1085,19 +1093,23 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
         {
           int h = base;
           lm = qm;
-#pragma unroll
-          for (int i = 0; i < KI; i++)
-          {
-            if (FM != PAIR && i >= 2 && ents <= 2) continue;
+          auto apply = [&](int i) {
             if (FM == PAIR)
             {
               h += (A & em[i]) ? val[i] : 0;
-              continue;
+              return;
             }
             const bool on = holds(A, em[i], et[i]);
             if (FM == COUNTER) h += on ? val[i] : 0;
             else h += on ? -val[i] : val[i];
             if (MASKS && on) lm |= bit[i];
+          };
+          apply(0);
+          apply(1);
+          if (FM == PAIR || ents > 2)
+          {
+            apply(2);
+            apply(3);
           }
           for (int i = 0; SP && i < xn; i++)
           {
