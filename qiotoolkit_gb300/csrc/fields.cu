@@ -59,6 +59,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "block_turns.h"
 #include "metropolis.cuh"
 #include "ordered_sum.cuh"
 #include "qio_internal.h"
@@ -511,33 +512,32 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
     if (made + 32u - used >= (unsigned)kRing)
     {
       // no room for draws (the last one taken stays: its stream position)
-      int leave = 0;
-      if (ld_acquire(R.done)) leave = 1;
-      else if (ld_acquire(R.abort)) leave = 2;
-      else if (used != last_u || blocks != last_b)
+      bool leave = ld_acquire(R.done) != 0u || ld_acquire(R.abort) != 0u;
+      if (!leave)
       {
-        last_u = used;
-        last_b = blocks;
-        limit.renew();
+        if (used != last_u || blocks != last_b)
+        {
+          last_u = used;
+          last_b = blocks;
+          limit.renew();
+        }
+        else if (limit.over())
+        {
+          raise_abort(R, err);
+          leave = true;
+        }
       }
-      else if (limit.over())
-      {
-        raise_abort(R, err);
-        leave = 2;
-      }
-      leave = __shfl_sync(kFull, leave, 0);
-      if (leave == 0)
+      leave = __shfl_sync(kFull, (int)leave, 0) != 0;
+      if (!leave)
       {
         __nanosleep(100);  // (its polls would take the decider's turns at shared memory)
         continue;
       }
-      // given up: the copies in flight land before the region is
-      if (leave == 2 && lane == 0)
-        for (int x = max(0, t - bufs); x < t; x++)
-        {
-          const unsigned n = t0 + (unsigned)x;
-          mbar_wait(&R.bars[n % (unsigned)bufs], (n / (unsigned)bufs) & 1u);
-        }
+      // the copies in flight land before the region is given up
+      const unsigned n = in_flight((unsigned)t, *(volatile unsigned*)R.blocks);
+      if (lane == 0)
+        for (unsigned x = t0 + (unsigned)t - n; x != t0 + (unsigned)t; x++)
+          mbar_wait(&R.bars[x % (unsigned)bufs], (x / (unsigned)bufs) & 1u);
       return;
     }
     uint32_t pd;
