@@ -472,13 +472,13 @@ __device__ __forceinline__ uint64_t stream_state(const Region& R, const Walk& W)
 // takes.  Counter streams: the entry of every attempt in turn.  An entry that
 // always accepts is (-inf, -inf).
 //
-// Chunks: block t's goes to buffer t % bufs once the decider is done with
-// block t - bufs (t counts over the warp's walkers, from `t0`).
+// Chunks: a block's goes to the next buffer in turn (T, kept over the warp's
+// walkers) once the decider is done with the block `bufs` before.
 // ---------------------------------------------------------------------------
 template <int FM, bool REPLAY>
 __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int4* desc, const uint2* table, int tile_w,
-                                  int cap, int bufs, int nblocks, int total, unsigned t0, uint64_t rs, uint64_t key,
-                                  unsigned long long ctr, int n_vars, int* err)
+                                  int cap, Turns& turns, int n_sweeps, uint64_t rs, uint64_t key, unsigned long long ctr,
+                                  int n_vars, int* err)
 {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -488,7 +488,8 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
   uint32_t raw = (uint32_t)lane + 1u;  // stream position after this lane's draw
   int carry = 0;                       // zeros at the end of the last 32 draws that await the next
   int first = 0;                       // counter: the first variable of the coming attempts
-  int t = 0, tb = 0;                   // chunks issued; the next one's block
+  Turns T = turns;                     // the next chunk's place
+  unsigned issued = 0;                 // chunks
   int4 d = __ldg(desc);                // ... and its descriptor
   Patience limit;
   unsigned last_u = 0, last_b = 0;
@@ -497,17 +498,13 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
     // what the decider has done
     const unsigned used = ld_acquire(R.used);
     const unsigned blocks = *(volatile unsigned*)R.blocks;
-    while (t < total && t < (int)blocks + bufs)
+    while (T.sweep < n_sweeps && in_flight(issued, blocks) < (unsigned)T.bufs)
     {
       if (lane == 0)
-      {
-        const unsigned at = (t0 + (unsigned)t) % (unsigned)bufs;
-        tile_issue(R.tiles + at * tile_w, table + d.x, (unsigned)min(d.y, cap) * 8u,
-                   &R.bars[at]);
-      }
-      t++;
-      tb = tb + 1 < nblocks ? tb + 1 : 0;
-      d = __ldg(desc + tb);
+        tile_issue(R.tiles + T.buf * tile_w, table + d.x, (unsigned)min(d.y, cap) * 8u, &R.bars[T.buf]);
+      issued++;
+      T.next();
+      d = __ldg(desc + T.block);
     }
     if (made + 32u - used >= (unsigned)kRing)
     {
@@ -534,10 +531,14 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
         continue;
       }
       // the copies in flight land before the region is given up
-      const unsigned n = in_flight((unsigned)t, *(volatile unsigned*)R.blocks);
       if (lane == 0)
-        for (unsigned x = t0 + (unsigned)t - n; x != t0 + (unsigned)t; x++)
-          mbar_wait(&R.bars[x % (unsigned)bufs], (x / (unsigned)bufs) & 1u);
+      {
+        Turns U = T;
+        const unsigned n = in_flight(issued, *(volatile unsigned*)R.blocks);
+        U.back(n);
+        for (unsigned x = 0; x < n; x++, U.next_buffer()) mbar_wait(&R.bars[U.buf], U.phase);
+      }
+      turns = T;
       return;
     }
     uint32_t pd;
@@ -779,7 +780,7 @@ __device__ __noinline__ unsigned exact_attempt(const DevModel& m, int v, int g, 
 
 template <int FM, bool REPLAY, bool INT>
 __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel& m, const Region R, const Shape& sh, int r,
-                                              unsigned t0, Walk& W, uint32_t* g_lsp)
+                                              Turns& turns, Walk& W, uint32_t* g_lsp)
 {
   constexpr int KI = kIn;  // in-block entries held in registers
   constexpr int kLog = FM == PAIR ? kLogBytes / 4 : kLogBytes / 16;  // entries, a power of two
@@ -788,9 +789,9 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const int N = m.n_vars;
-  const int nblocks = (N + 31) >> 5;
-  const int total = nblocks * a.n_sweeps;
-  if (total <= 0) return true;
+  Turns T = turns;  // the coming block
+  const int nblocks = T.nblocks;
+  if (a.n_sweeps <= 0) return true;
   const bool scan32 = m.scan32 != 0;
   const double inv = m.fc_inv;
   // (read once: `m` may be the launch's parameter or lie in device memory)
@@ -800,7 +801,6 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   const int cap = sh.words;
   uint8_t* zw = R.z + 64 * sh.nw + 16;  // the wide terms' bytes
 
-  unsigned buf = t0 % (unsigned)sh.bufs, par = (t0 / (unsigned)sh.bufs) & 1u;  // the coming chunk's buffer and phase
   unsigned head = 0;                // log entries written
   unsigned moved = 0;               // draws taken when the stream's origin last moved
   unsigned acc_tail = 0, fed = 0;   // the other warps' counters when last looked at
@@ -808,12 +808,13 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   S.betas = a.beta + (long long)r * a.bs_w;
   S.beta_next = S.betas[a.sweep_base * a.bs_s];
 
-  int k = 0, bi = -1;  // sweep and block of gb
-  for (int gb = 0; gb < total; gb++)
+  unsigned finished = 0;  // blocks
+  while (true)
   {
-    bi++;
-    if (bi == nblocks || gb == 0)
+    const int bi = T.block;
+    if (bi == 0)
     {
+      if (T.sweep == a.n_sweeps) break;
       if (REPLAY && W.taken - moved > (1u << 28))
       {
         // stream positions are 32-bit: move their origin along
@@ -821,25 +822,22 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
         W.raw0 = R.raw[(W.taken - 1u) & (unsigned)(kRing - 1)];
         moved = W.taken;
       }
-      bi = 0;
-      next_sweep<FM, INT>(S, a, inv, N, k++);
+      next_sweep<FM, INT>(S, a, inv, N, T.sweep);
     }
     const int nvalid = min(32, N - (bi << 5));
     const int v = (bi << 5) + lane;
     // this block's chunk
-    if (!__all_sync(kFull, mbar_try(&R.bars[buf], par)))
+    if (!__all_sync(kFull, mbar_try(&R.bars[T.buf], T.phase)))
     {
-      const bool landed = mbar_wait(&R.bars[buf], par);
+      const bool landed = mbar_wait(&R.bars[T.buf], T.phase);
       if (!__all_sync(kFull, landed))
       {
         raise_abort(R, a.err);
         return false;
       }
     }
-    const uint2* chunk = R.tiles + buf * cap;
-    buf++;
-    par ^= buf == (unsigned)sh.bufs ? 1u : 0u;
-    buf = buf == (unsigned)sh.bufs ? 0u : buf;
+    const uint2* chunk = R.tiles + T.buf * cap;
+    T.next();
     // the header through shuffles, so that what depends on it is known not to
     // divide the warp: rows, entry rows and further entry rows
     const uint2 head0 = *chunk;
@@ -1268,8 +1266,9 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
     else if (!block(std::false_type{})) return false;
     if (!REPLAY) W.taken += 32u;
     W.natt += (unsigned)nvalid;
-    publish(R, (unsigned)gb + 1u, head, W.taken);
+    publish(R, ++finished, head, W.taken);
   }
+  turns = T;
   return true;
 }
 
@@ -1512,7 +1511,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
   if (role == 1 && lane == 0)
     for (int i = 0; i < kBufs; i++) mbar_init(&R.bars[i]);
   uint64_t rs = (REPLAY && !queued) ? a.rng[w] : 0;
-  unsigned t0 = 0;  // chunks of the walkers before this one
+  Turns turns(1, sh.bufs);
 
   int r = w;
   while (true)
@@ -1526,6 +1525,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     if (r >= a.n_walkers) break;
     const DevModel& m = queued ? a.models[a.model_of[r]] : a.m;
     const int N = m.n_vars;
+    turns.walker((N + 31) >> 5);
     const int slot = a.slot_of ? a.slot_of[r] : r;
     uint32_t* g_spins = a.p.spins + (size_t)slot * a.p.nw;
     if (queued && REPLAY) rs = a.rng[r];
@@ -1568,7 +1568,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
         W.icost = (long long)a.p.cost[slot];
         W.ilow = (long long)a.p.lowest[r];
       }
-      const bool ok = decide_sweeps<FM, REPLAY, INT>(a, m, R, sh, r, t0, W, g_lsp);
+      const bool ok = decide_sweeps<FM, REPLAY, INT>(a, m, R, sh, r, turns, W, g_lsp);
       if (lane == 0) st_release(R.done, 1u);
       if (REPLAY) rs = stream_state(R, W);
       walker_sync<INT>(bar_id);
@@ -1591,8 +1591,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     }
     else if (role == 1)
     {
-      feed<FM, REPLAY>(R, s_scr, m.fc_desc, m.fc_tab, sh.words, sh.words, sh.bufs, (N + 31) >> 5,
-                       ((N + 31) >> 5) * a.n_sweeps, t0, rs, key,
+      feed<FM, REPLAY>(R, s_scr, m.fc_desc, m.fc_tab, sh.words, sh.words, turns, a.n_sweeps, rs, key,
                        (unsigned long long)a.sweep_base * (unsigned long long)N, N, a.err);
       walker_sync<INT>(bar_id);
     }
@@ -1609,7 +1608,6 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
       }
     }
     if (*(volatile unsigned*)R.abort) return;
-    t0 = (t0 + (unsigned)(((N + 31) >> 5) * a.n_sweeps)) % (unsigned)(2 * sh.bufs);  // buffer and phase
     copy16((uint4*)g_spins, (const uint4*)R.spins, a.p.nw >> 2, me, nme);
     walker_sync<INT>(bar_id);  // the region is reused by the next walker
     if (!queued)

@@ -23,6 +23,7 @@
 #include <climits>
 #include <type_traits>
 
+#include "block_turns.h"
 #include "metropolis.cuh"
 #include "qio_internal.h"
 
@@ -1153,9 +1154,10 @@ __global__ void __launch_bounds__(256, 1) sweep2_kernel(SweepArgs a)
                           a.key_base + (unsigned long long)(lr % a.key_div));
     }
     const int nblocks = (Sz + 31) >> 5;
-    const int total_blocks = nblocks * a.n_sweeps;
+    const int n_sweeps = nblocks > 0 ? a.n_sweeps : 0;
+    fc::Turns T(nblocks, 2);
     int toff[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, tq0[2] = {0, 0}, tq1[2] = {0, 0};
-    if (staged && total_blocks > 0 && lane == 0)
+    if (staged && n_sweeps > 0 && lane == 0)
     {
       int q0 = __ldg(m.row + 0), q1 = __ldg(m.row + min(32, Sz));
       tile_issue<INT>(tile_at<INT>(tile_base, cap), cap, &bars[0], m, q0, q1, toff[0]);
@@ -1163,12 +1165,11 @@ __global__ void __launch_bounds__(256, 1) sweep2_kernel(SweepArgs a)
       tq1[0] = q1;
     }
     bool aborted = false;
-    for (int gb = 0; gb < total_blocks; gb++)
+    for (; T.sweep < n_sweeps; T.next())
     {
-      const int k = gb / nblocks;
-      const int bi = gb - k * nblocks;
-      const int buf = gb & 1;
-      const long long swp = a.sweep_base + k;
+      const int bi = T.block;
+      const int buf = (int)T.buf;
+      const long long swp = a.sweep_base + T.sweep;
       const double beta = a.beta[(long long)r * a.bs_w + swp * a.bs_s];
       const bool beta_inf =
           ((unsigned long long)__double_as_longlong(beta) & 0x7FFFFFFFFFFFFFFFULL) ==
@@ -1179,7 +1180,7 @@ __global__ void __launch_bounds__(256, 1) sweep2_kernel(SweepArgs a)
       if (staged)
       {
         // issue the next block's tile into the other buffer, then wait for ours
-        if (gb + 1 < total_blocks && lane == 0)
+        if ((bi + 1 < nblocks || T.sweep + 1 < n_sweeps) && lane == 0)
         {
           int nb = (bi + 1 < nblocks) ? bi + 1 : 0;
           int q0 = __ldg(m.row + (nb << 5)), q1 = __ldg(m.row + min((nb << 5) + 32, Sz));
