@@ -54,7 +54,6 @@
 // time limit on lack of progress; on expiry the kernel raises the device error
 // flag and all of the walker's warps return.
 #include <algorithm>
-#include <atomic>
 #include <climits>
 #include <cmath>
 #include <type_traits>
@@ -1632,13 +1631,8 @@ static cudaError_t go(const SweepArgs& a, cudaStream_t s, int wpc, const Shape& 
   auto k = fc_sweep_kernel<FM, R, I>;
   const int smem = kTable + wpc * region_bytes(sh, I);
   const int threads = (I ? 64 : 96) * wpc;
-  static std::atomic<int> configured{48 * 1024};
-  if (smem > configured.load())
-  {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    if (e != cudaSuccess) return e;
-    configured = kMaxSmem;
-  }
+  const cudaError_t allowed = allow_shared((const void*)k, smem);
+  if (allowed != cudaSuccess) return allowed;
   int blocks = (a.n_streams + wpc - 1) / wpc;
   if (a.queue)
   {

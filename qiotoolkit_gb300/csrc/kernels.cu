@@ -2116,12 +2116,8 @@ template <int FL, bool I>
 static cudaError_t qmc_level_dispatch(const QmcArgs& a, cudaStream_t s)
 {
   const size_t smem = qmc_level_smem(a.trotter, a.p.nw);
-  if (smem > 48 * 1024)
-  {
-    cudaError_t e =
-        cudaFuncSetAttribute(qmc_level_kernel<FL, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t allowed = allow_shared((const void*)qmc_level_kernel<FL, I>, (int)smem);
+  if (allowed != cudaSuccess) return allowed;
   qmc_level_kernel<FL, I><<<a.restarts, kQmcLevelWarps * 32, smem, s>>>(a);
   return cudaGetLastError();
 }
@@ -2150,22 +2146,16 @@ static cudaError_t qmc_dispatch(const QmcArgs& a, cudaStream_t s)
   if (a.trotter <= 32 && words <= 200 * 1024)
   {
     auto k = FL == F_PARITY && a.m.pair_only ? qmc_sliced_kernel<FL, I, FL == F_PARITY> : qmc_sliced_kernel<FL, I, false>;
-    if (words > 32 * 1024)
-    {
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)words);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t allowed = allow_shared((const void*)k, (int)words);
+    if (allowed != cudaSuccess) return allowed;
     k<<<a.restarts, 64, words, s>>>(a);
     return cudaGetLastError();
   }
   const size_t per_warp = (size_t)a.trotter * 8 + (((size_t)a.trotter * 2 + 7) & ~(size_t)7);
   const int blocks = (a.restarts + 3) / 4;
   const size_t smem = 4 * per_warp;
-  if (smem > 48 * 1024)
-  {
-    cudaError_t e = cudaFuncSetAttribute(qmc_kernel<FL, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t allowed = allow_shared((const void*)qmc_kernel<FL, I>, (int)smem);
+  if (allowed != cudaSuccess) return allowed;
   if (blocks > 0) qmc_kernel<FL, I><<<blocks, 128, smem, s>>>(a);
   return cudaGetLastError();
 }
@@ -2584,11 +2574,8 @@ cudaError_t launch_tabu(const TabuArgs& a, cudaStream_t s)
     {
       const size_t smem = f.model + wpb * f.walker;
       auto k = I ? tabu_pair_kernel<true> : tabu_pair_kernel<false>;
-      if (smem > 48 * 1024)
-      {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-      }
+      const cudaError_t allowed = allow_shared((const void*)k, (int)smem);
+      if (allowed != cudaSuccess) return allowed;
       k<<<(a.n_walkers + wpb - 1) / wpb, 32 * wpb, smem, s>>>(a, f.model, f.walker);
       return cudaGetLastError();
     }

@@ -426,13 +426,8 @@ static cudaError_t lw_go_k(const LwArgs& a, cudaStream_t s, int wpb)
 {
   auto k = lw::lw_sweep_kernel<R, RK, SM, KP>;
   const int bytes = SM ? wpb * a.smem_words * a.G * 4 : 0;
-  static int configured = 48 * 1024;
-  if (bytes > configured)
-  {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    configured = bytes;
-  }
+  const cudaError_t allowed = allow_shared((const void*)k, bytes);
+  if (allowed != cudaSuccess) return allowed;
   const int groups = (a.n_walkers + a.G - 1) / a.G;
   const int blocks = (groups + wpb - 1) / wpb;
   if (blocks > 0) k<<<blocks, 32 * wpb, bytes, s>>>(a);

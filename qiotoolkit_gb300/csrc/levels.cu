@@ -460,13 +460,8 @@ static cudaError_t lv_go(const LvArgs& a, int stride, cudaStream_t s)
   const long long even = ((long long)a.n_walkers + sms * waves - 1) / (sms * waves);
   const int wpb = (int)std::max(1LL, std::min<long long>(cap, even));
   const int bytes = wpb * stride * 4;
-  static int configured = 48 * 1024;
-  if (bytes > configured)
-  {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kLvSmemBytes);
-    if (e != cudaSuccess) return e;
-    configured = kLvSmemBytes;
-  }
+  const cudaError_t allowed = allow_shared((const void*)k, bytes);
+  if (allowed != cudaSuccess) return allowed;
   const int blocks = (a.n_walkers + wpb - 1) / wpb;
   k<<<blocks, 32 * wpb, bytes, s>>>(a, stride);
   return cudaGetLastError();
@@ -477,13 +472,8 @@ static cudaError_t lv_low(const LvArgs& a, cudaStream_t s)
 {
   auto k = lv::lv_lowest_kernel<D8, STAGE>;
   const int bytes = STAGE ? (int)(a.diff_stride * (D8 ? 1 : 4)) : 0;
-  static int configured = 48 * 1024;
-  if (bytes > configured)
-  {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kLvRowBytes);
-    if (e != cudaSuccess) return e;
-    configured = kLvRowBytes;
-  }
+  const cudaError_t allowed = allow_shared((const void*)k, bytes);
+  if (allowed != cudaSuccess) return allowed;
   const int blocks = (int)std::min<long long>(152LL * 4, a.n_walkers);  // persistent over the walkers
   k<<<blocks, kLvLowThreads, bytes, s>>>(a);
   return cudaGetLastError();

@@ -79,6 +79,25 @@ void h2d(void* dst, const void* src, size_t bytes, const char* what)
   cuda_check(cudaStreamSynchronize(cudaStreamLegacy), what);
 }
 
+cudaError_t allow_shared(const void* kernel, int bytes)
+{
+  if (bytes <= 32 * 1024) return cudaSuccess;  // (with the kernels' static bytes below the default limit)
+  static std::mutex mu;
+  static std::set<std::pair<int, const void*>> raised;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> g(mu);
+  if (raised.count({dev, kernel})) return cudaSuccess;
+  cudaFuncAttributes at;
+  if ((e = cudaFuncGetAttributes(&at, kernel)) != cudaSuccess) return e;
+  int most = 0;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
+  if (e == cudaSuccess) raised.insert({dev, kernel});
+  return e;
+}
+
 static std::mutex g_dev_mu;
 static std::map<int, int*> g_err;
 

@@ -203,6 +203,11 @@ struct InitArgs
 
 // ---- launchers (kernels.cu) -------------------------------------------
 void upload_tables(int device);  // ln table + PCG jump tables
+// Lets `kernel` be launched with `bytes` of dynamic shared memory.  The limit is
+// the kernel's on this device, for all threads: it goes to the most that a block
+// may have at once, as a launch's own size, set by one thread, would refuse
+// another thread's larger launch.
+cudaError_t allow_shared(const void* kernel, int bytes);
 cudaError_t launch_init(const InitArgs& a, cudaStream_t s);
 cudaError_t launch_sweep(const SweepArgs& a, cudaStream_t s, int warps_per_block);
 // one warp's walker state (term bytes, spins, lowest) fits shared memory

@@ -1274,13 +1274,8 @@ template <int FL, bool R, bool I, bool SM, bool B>
 static cudaError_t go(const SweepArgs& a, cudaStream_t s, int wpb, int smem)
 {
   auto k = sweep2_kernel<FL, R, I, SM, B>;
-  static int configured = -1;
-  if (smem > 48 * 1024 && configured < smem)
-  {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    configured = smem;
-  }
+  const cudaError_t allowed = allow_shared((const void*)k, smem);
+  if (allowed != cudaSuccess) return allowed;
   int blocks = (a.n_streams + wpb - 1) / wpb;
   if (B)
   {
