@@ -162,9 +162,7 @@ qio_status qio_model_get_info(const qio_model* model, qio_model_info* out)
     out->const_cost = m.const_cost;
     out->scale_factor = m.scale_factor;
     out->max_coupling = m.max_coupling;
-    out->device_bytes = (int64_t)(m.row.size() * 4 + m.inc.size() * 4 + m.coef.size() * 8 +
-                                  m.coef_i.size() * 4 + m.nbr.size() * 4 + m.trow.size() * 4 +
-                                  m.tvar.size() * 4 + m.tcost.size() * 8 + m.tcost_i.size() * 4);
+    out->device_bytes = (int64_t)m.device_copy_bytes();
     out->n_levels = m.n_levels;
     out->max_level_width = m.lv_width;
     out->level_kernel = levels_eligible(m) ? 1 : 0;

@@ -110,6 +110,14 @@ struct HostModel
   mutable int upload_device = -1;  // CUDA ordinal that holds dmem
 
   bool empty() const { return N == 0; }
+  // the arrays of the device copy, in its order, each on a 256-byte boundary;
+  // and its bytes, which are those of the model on the device
+  template <class F> void device_arrays(F f) const
+  {
+    f(row), f(inc), f(coef), f(coef_i), f(nbr), f(trow), f(tvar), f(tcost), f(tcost_i), f(coef_f), f(near), f(other);
+    f(rec_i), f(rec_f), f(rec_p), f(lv_off), f(lv_ent), f(lv_pos), f(fc_tab), f(fc_desc), f(fc_in), f(fc_oth), f(fc_wide);
+  }
+  size_t device_copy_bytes() const;
   void upload() const;
   const DevModel& device() const
   {

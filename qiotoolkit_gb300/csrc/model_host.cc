@@ -1,5 +1,6 @@
 // model_host.cc -- model construction and upload, schedules, device setup.
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -827,30 +828,29 @@ static void build_levels(HostModel& m)
   m.lv_ok = true;
 }
 
-template <class T>
-static size_t put(std::vector<char>& blob, const std::vector<T>& v)
+// 256 bytes of tail padding: bulk copies of incidence ranges round their end up
+// to 16 bytes
+static size_t boundary(size_t n) { return (n + 255) & ~(size_t)255; }
+size_t HostModel::device_copy_bytes() const
 {
-  size_t o = (blob.size() + 255) & ~(size_t)255;
-  blob.resize(o + v.size() * sizeof(T));
-  if (!v.empty()) memcpy(blob.data() + o, v.data(), v.size() * sizeof(T));
-  return o;
+  size_t n = 0;
+  device_arrays([&](const auto& v) { n = boundary(n) + v.size() * sizeof(v[0]); });
+  return boundary(n) + 256;
 }
 
 void HostModel::upload() const
 {
   ensure_device();
-  std::vector<char> blob;
-  size_t o_row = put(blob, row), o_inc = put(blob, inc), o_coef = put(blob, coef),
-         o_ci = put(blob, coef_i), o_nbr = put(blob, nbr), o_trow = put(blob, trow),
-         o_tvar = put(blob, tvar), o_tc = put(blob, tcost), o_tci = put(blob, tcost_i),
-         o_cf = put(blob, coef_f), o_near = put(blob, near), o_oth = put(blob, other),
-         o_ri = put(blob, rec_i), o_rf = put(blob, rec_f), o_rp = put(blob, rec_p),
-         o_lo = put(blob, lv_off), o_le = put(blob, lv_ent), o_lp = put(blob, lv_pos),
-         o_ft = put(blob, fc_tab), o_fd = put(blob, fc_desc), o_fi = put(blob, fc_in),
-         o_fo = put(blob, fc_oth), o_fw = put(blob, fc_wide);
-  // 256 bytes of tail padding: bulk copies of incidence ranges round their
-  // end up to 16 bytes
-  blob.resize(((blob.size() + 255) & ~(size_t)255) + 256);
+  std::vector<char> blob(device_copy_bytes());
+  std::array<size_t, 23> at;
+  size_t n = 0, k = 0;
+  device_arrays([&](const auto& v) {
+    at[k++] = n = boundary(n);
+    if (!v.empty()) memcpy(blob.data() + n, v.data(), v.size() * sizeof(v[0]));
+    n += v.size() * sizeof(v[0]);
+  });
+  const auto [o_row, o_inc, o_coef, o_ci, o_nbr, o_trow, o_tvar, o_tc, o_tci, o_cf, o_near, o_oth, o_ri, o_rf, o_rp,
+              o_lo, o_le, o_lp, o_ft, o_fd, o_fi, o_fo, o_fw] = at;
   dmem = DevBuf(blob.size());
   h2d(dmem.ptr, blob.data(), blob.size(), "model upload");
   char* b = (char*)dmem.ptr;

@@ -47,16 +47,7 @@ struct Request
   int64_t piece = 1;
 };
 
-int64_t model_bytes(const HostModel& m)
-{
-  return (int64_t)(m.row.size() * 4 + m.inc.size() * 4 + m.coef.size() * 8 + m.coef_i.size() * 4 +
-                   m.coef_f.size() * 4 + m.near.size() * 8 + m.nbr.size() * 4 + m.trow.size() * 4 +
-                   m.tvar.size() * 4 + m.tcost.size() * 8 + m.tcost_i.size() * 4 + m.other.size() * 4 +
-                   m.rec_i.size() * 4 + m.rec_f.size() * 8 + m.rec_p.size() * 4 + m.lv_off.size() * 4 +
-                   m.lv_ent.size() * 4 + m.lv_pos.size() * 4 + 19 * 256);
-}
-
-// device bytes of a solve: the model blob and the walker population
+// device bytes of a solve: the model's device copy and the walker population
 int64_t footprint_of(const HostModel& m, const Solver& s)
 {
   const int64_t W = std::max<int64_t>(1, s.n_walkers());
@@ -81,7 +72,7 @@ int64_t footprint_of(const HostModel& m, const Solver& s)
   int64_t extra = 0;
   if (s.target() == "substochasticmontecarlo.cpu") extra = W * (per + 12) + nw * 4;
   if (s.target() == "quantummontecarlo.qiotoolkit") extra = steps * 17 + W * (8 + nw * 4);
-  return model_bytes(m) + W * per + steps * 8 + W * 64 + lv + tabu + extra + 64 * 1024;
+  return (int64_t)m.device_copy_bytes() + W * per + steps * 8 + W * 64 + lv + tabu + extra + 64 * 1024;
 }
 }  // namespace
 
