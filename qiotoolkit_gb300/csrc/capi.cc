@@ -188,7 +188,8 @@ qio_status qio_model_destroy(qio_model* model)
 }
 
 // Device scratch of a per-state call: the states' spin words, `extra` bytes
-// after them, and room for the states' own bytes, 256 MB of them at a time.
+// after them, and room for the states' own bytes, 256 MB of them at a time.  A
+// device without that room gets words packed on the host.
 struct StateScratch
 {
   int nw;
@@ -200,12 +201,32 @@ struct StateScratch
     words = ((size_t)n * nw * 4 + 255) & ~(size_t)255;
     extra = (extra + 255) & ~(size_t)255;
     chunk = std::min<size_t>((size_t)n, std::max<size_t>(1, ((size_t)256 << 20) / (size_t)std::max<int64_t>(1, m.N)));
-    buf = DevBuf(words + extra + chunk * (size_t)m.N);
     at = words + extra;
+    try
+    {
+      buf = DevBuf(at + chunk * (size_t)m.N);
+    }
+    catch (const Error& e)
+    {
+      if (e.status != 2) throw;
+      cudaGetLastError();  // (the refused allocation)
+      chunk = 0;
+      buf = DevBuf(at);
+    }
   }
   char* after() const { return (char*)buf.ptr + words; }
-  void pack(const HostModel& m, int64_t n, const uint8_t* states, cudaStream_t s) const
+  // (a host copy of the words lives as long as this object)
+  void pack(const HostModel& m, int64_t n, const uint8_t* states, cudaStream_t s)
   {
+    if (!chunk && m.N)
+    {
+      host.assign((size_t)n * nw, 0);
+      for (int64_t q = 0; q < n; q++)
+        for (int64_t v = 0; v < m.N; v++)
+          if (states[q * m.N + v]) host[q * nw + v / 32] |= 1u << (v % 32);
+      cuda_check(cudaMemcpyAsync(buf.ptr, host.data(), host.size() * 4, cudaMemcpyHostToDevice, s), "H2D");
+      return;
+    }
     uint8_t* bytes = (uint8_t*)buf.ptr + at;
     for (size_t q = 0; q < (size_t)n; q += chunk)
     {
@@ -217,6 +238,7 @@ struct StateScratch
 
  private:
   size_t at;
+  std::vector<uint32_t> host;
 };
 
 qio_status qio_states_cost(const qio_model* model, int64_t n, const uint8_t* states,
