@@ -88,8 +88,12 @@ __device__ __forceinline__ void add_lanes(double v, unsigned keep, double& c)
 {
   const unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  // three prefixes at most (a sum near zero changes its binade often)
-  for (int round = 0; round < 3 && __popc(keep) > 4; round++)
+  // Three prefixes at most, and none after one that took eight values or fewer: a
+  // sum near zero changes its binade often, and a prefix costs as much as eight
+  // adds.  Initial costs of 8 walkers, terms of both signs (us): 256 Ising terms 65
+  // and 62, 1024 PUBO terms 91 and 71, 4096 147 and 120.
+  bool worth = true;
+  for (int round = 0; round < 3 && worth && __popc(keep) > 4; round++)
   {
     int ce;
     const long long C = scaled(c, ce);
@@ -108,6 +112,7 @@ __device__ __forceinline__ void add_lanes(double v, unsigned keep, double& c)
     const int f = __ffs(bad) - 1;
     if (f > 0 && ce != 0 && ce != 0x7FF) c = unscaled(__shfl_sync(kAll, P, f - 1), ce);
     c = __dadd_rn(c, __shfl_sync(kAll, v, f));
+    worth = __popc(keep & ((2u << f) - 1u)) > 8;
     keep &= ~((2u << f) - 1u);
   }
   while (keep)
