@@ -280,12 +280,14 @@ __device__ __forceinline__ uint8_t term_state(const DevModel& m,
 // get_random_binary_state (model/ising.h:23-41, model/pubo.h:16-34) or the
 // MaxSat per-variable uniform() < 0.5 (model/max_sat.h:144-150).
 // ---------------------------------------------------------------------------
-template <int FL, bool INT>
+// WPW: warps per walker, 4 (a block) or 1 (four walkers a block).
+template <int FL, bool INT, int WPW>
 __global__ void __launch_bounds__(128) init_kernel(InitArgs a)
 {
-  __shared__ CostBuf buf;
-  const int lane = threadIdx.x & 31, tid = threadIdx.x;
-  const int w = blockIdx.x;  // a block per walker
+  const int lane = threadIdx.x & 31, tid = WPW == 1 ? lane : (int)threadIdx.x;  // thread of the walker
+  constexpr int T = 32 * WPW;
+  const int w = WPW == 1 ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)blockIdx.x;
+  if (w >= a.n_walkers) return;
   const DevModel& m = a.m;
   const int N = m.n_vars;
   const int nwd = (N + 31) >> 5;
@@ -305,7 +307,7 @@ __global__ void __launch_bounds__(128) init_kernel(InitArgs a)
   if (var_uniform && !a.given)
   {
     // MaxSat: a word per warp, a variable per lane
-    for (int q = tid >> 5; q < nwd; q += 4)
+    for (int q = tid >> 5; q < nwd; q += WPW)
     {
       const int v = q * 32 + lane;
       bool bit = false;
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(128) init_kernel(InitArgs a)
     }
   }
   else
-    for (int q = tid; q < nwd; q += 128)
+    for (int q = tid; q < nwd; q += T)
     {
       uint32_t word = 0;
       if (a.given)
@@ -342,16 +344,23 @@ __global__ void __launch_bounds__(128) init_kernel(InitArgs a)
       if (q == nwd - 1 && (N & 31)) word &= (1u << (N & 31)) - 1u;
       spins[q] = word;
     }
-  for (int q = nwd + tid; q < a.p.nw; q += 128) spins[q] = 0;
-  __syncthreads();  // (and every thread has read the walker's stream)
+  for (int q = nwd + tid; q < a.p.nw; q += T) spins[q] = 0;
+  // (and every thread has read the walker's stream)
+  if (WPW == 1) __syncwarp();
+  else __syncthreads();
   if (replay && tid == 0)
     a.rng[w] = jump_any(rs, var_uniform ? 2ULL * (unsigned long long)N
                                         : (unsigned long long)nwd);
   double cost;
   long long icost;
-  block_terms_cost<FL, INT>(m, spins, a.skip_terms ? nullptr : ts, buf, cost, icost);
+  if constexpr (WPW == 1) warp_terms_cost<FL, INT>(m, spins, a.skip_terms ? nullptr : ts, lane, cost, icost);
+  else
+  {
+    __shared__ CostBuf buf;
+    block_terms_cost<FL, INT>(m, spins, a.skip_terms ? nullptr : ts, buf, cost, icost);
+  }
   if (INT) cost = (double)icost;
-  for (int q = tid; q < a.p.nw; q += 128) lsp[q] = spins[q];
+  for (int q = tid; q < a.p.nw; q += T) lsp[q] = spins[q];
   if (tid == 0)
   {
     a.p.cost[slot] = cost;
@@ -2366,7 +2375,15 @@ void upload_tables(int)
 template <int FL, bool INT>
 static void init_dispatch(const InitArgs& a, cudaStream_t s)
 {
-  if (a.n_walkers > 0) init_kernel<FL, INT><<<a.n_walkers, 128, 0, s>>>(a);
+  if (a.n_walkers <= 0) return;
+  // A block shortens one walker's chain of loads and sums; with few terms, or warps
+  // enough on the chip, its idle lanes and waits cost more.  Initialising by block
+  // and by warp (us): integer Ising of 4096 terms, 256 walkers 58 and 100, 4096 92
+  // and 114, 65536 810 and 772, of 512 terms, 4096 walkers 66 and 62; FP64 PUBO of
+  // 128 terms, 65536 walkers 472 and 356, of 4096, 256 walkers 180 and 217, 4096
+  // 364 and 341.
+  if (a.m.n_terms > 512 && a.n_walkers < (INT ? 8192 : 2048)) init_kernel<FL, INT, 4><<<a.n_walkers, 128, 0, s>>>(a);
+  else init_kernel<FL, INT, 1><<<(a.n_walkers + 3) / 4, 128, 0, s>>>(a);
 }
 
 cudaError_t launch_init(const InitArgs& a, cudaStream_t s)
