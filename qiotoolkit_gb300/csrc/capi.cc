@@ -189,19 +189,24 @@ qio_status qio_model_destroy(qio_model* model)
 
 // Device scratch of a per-state call: the states' spin words, `extra` bytes
 // after them, and room for the states' own bytes, 256 MB of them at a time.  A
-// device without that room gets words packed on the host.
+// device without that room gets words packed on the host, and so do states of
+// `few` bytes in all, where a copy and a kernel more cost more than the loop.  From
+// the host and through the bytes (us), 64 variables: costs of 16 states 47 and 51,
+// of 64 states 50 and 48, cost differences of 64 35 and 39, of 128 40 and 44, of 256
+// 62 and 40.
 struct StateScratch
 {
   int nw;
   size_t words, chunk;  // bytes of the words; states of a copy
   DevBuf buf;
-  StateScratch(const HostModel& m, int64_t n, size_t extra)
+  StateScratch(const HostModel& m, int64_t n, size_t extra, size_t few)
   {
     nw = std::max(1, (int)((m.N + 31) / 32));
     words = ((size_t)n * nw * 4 + 255) & ~(size_t)255;
     extra = (extra + 255) & ~(size_t)255;
     chunk = std::min<size_t>((size_t)n, std::max<size_t>(1, ((size_t)256 << 20) / (size_t)std::max<int64_t>(1, m.N)));
     at = words + extra;
+    if ((size_t)n * (size_t)m.N <= few) chunk = 0;
     try
     {
       buf = DevBuf(at + chunk * (size_t)m.N);
@@ -255,7 +260,7 @@ qio_status qio_states_cost(const qio_model* model, int64_t n, const uint8_t* sta
     }
     ensure_device();
     const DevModel& dm = m.device();
-    StateScratch d(m, n, (size_t)n * 8);
+    StateScratch d(m, n, (size_t)n * 8, 2048);
     cudaStream_t s = as_stream(stream);
     d.pack(m, n, states, s);
     double* out = (double*)d.after();
@@ -330,7 +335,7 @@ qio_status qio_states_cost_difference(const qio_model* model, int64_t n, const u
         fail(1, "transition " + std::to_string(vars[q]) + " out of range [0, " + std::to_string(m.N) + ")");
     ensure_device();
     const DevModel& dm = m.device();
-    StateScratch d(m, n, (size_t)n * 16);
+    StateScratch d(m, n, (size_t)n * 16, 8192);
     cudaStream_t s = as_stream(stream);
     long long* dv = (long long*)d.after();
     double* out = (double*)(d.after() + (size_t)n * 8);

@@ -37,3 +37,19 @@ def test_state_costs(kind, coefs, n):
     v = rng.integers(0, n, len(states))
     np.testing.assert_array_equal(g.calculate_cost_difference(marked, v),
                                   [o.cost_difference(s, int(x)) for s, x in zip(states, v)])
+
+
+@pytest.mark.parametrize("n_states", [1, 31, 32, 33, 127, 128, 129])
+def test_few_states(n_states):
+    """Around 2 KB (costs) and 8 KB (differences) of 64 variables' state bytes, from
+    where the device packs them."""
+    rng = np.random.default_rng(n_states)
+    rows = [[v] for v in range(64)] + [sorted(rng.choice(64, 3, replace=False).tolist()) for _ in range(100)]
+    at = dict(zip(("off", "ids", "coef"), O.flatten_terms([(float(x), r) for x, r in zip(rng.standard_normal(164), rows)])))
+    g, o = q.Model("pubo", **at), O.Model("pubo", **at)
+    states = rng.integers(0, 2, (n_states, 64), dtype=np.uint8)
+    marked = states * rng.integers(1, 256, states.shape).astype(np.uint8)
+    np.testing.assert_array_equal(g.calculate_cost(marked), [o.cost(s) for s in states])
+    v = rng.integers(0, 64, n_states)
+    np.testing.assert_array_equal(g.calculate_cost_difference(marked, v),
+                                  [o.cost_difference(s, int(x)) for s, x in zip(states, v)])
