@@ -1412,7 +1412,8 @@ static const int kRing = 512;  // flip words, a power of two
 static const long long kPatience = 8000000000LL;  // cycles without progress
 struct Sync
 {
-  unsigned head, tail, abort, pad;
+  unsigned head, tail;  // variables decided, accounted for; published every 32
+  unsigned abort;
 };
 __device__ __forceinline__ unsigned acquire(const unsigned* p)
 {
@@ -1424,17 +1425,23 @@ __device__ __forceinline__ void release(unsigned* p, unsigned v)
 {
   asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
 }
-// waits until *p (counters wrap) reaches `want`; false: given up
+// waits until *p (counters wrap) reaches `want`; false: given up, as it stood still
 __device__ __noinline__ bool wait_for(const unsigned* p, unsigned want, unsigned* abort, int* err, unsigned& seen)
 {
   unsigned ok = 1;
   if ((threadIdx.x & 31) == 0)
   {
-    const long long t0 = clock64();
+    long long t0 = clock64();
+    unsigned last = acquire(p);
     while (true)
     {
       seen = acquire(p);
       if ((int)(seen - want) >= 0) break;
+      if (seen != last)
+      {
+        last = seen;
+        t0 = clock64();
+      }
       if (acquire(abort) || clock64() - t0 > kPatience)
       {
         if (err) atomicExch(err, 1);
@@ -1728,6 +1735,7 @@ __global__ void __launch_bounds__(64) qmc_sliced_kernel(const __grid_constant__ 
           __syncwarp();
         }
         tail++;
+        if ((tail & 31u) == 0u && lane == 0) release(&sync.tail, tail);
         R.shift();
       }
       // save_lowest: the first lowest slice
@@ -2150,9 +2158,14 @@ cudaError_t launch_qmc_levels(const QmcArgs& a, cudaStream_t s)
 template <int FL, bool I>
 static cudaError_t qmc_dispatch(const QmcArgs& a, cudaStream_t s)
 {
-  // a slice per lane where there are lanes and the variables' words fit
+  // A slice per lane where there are lanes and the variables' words fit.  Rows of
+  // more than 1024 incidences stay out: the screen's error bound grows with the
+  // row until it decides nothing (complete graphs of 500 variables, N(0, 1)
+  // couplings 118 ms here and there, of 1000, couplings of variance 1 / N, 332 here
+  // and 495 there, PUBO rows of 2400 102 and 93), and the work of the 32 variables
+  // between two signs of progress stays below what the warps' waits allow.
   const size_t words = ((size_t)a.m.n_vars * 3 + 1) * 4;  // two copies, the row bounds
-  if (a.trotter <= 32 && words <= 200 * 1024)
+  if (a.trotter <= 32 && words <= 200 * 1024 && a.m.max_deg <= 1024)
   {
     auto k = FL == F_PARITY && a.m.pair_only ? qmc_sliced_kernel<FL, I, FL == F_PARITY> : qmc_sliced_kernel<FL, I, false>;
     const cudaError_t allowed = allow_shared((const void*)k, (int)words);

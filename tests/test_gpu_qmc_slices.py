@@ -2,6 +2,8 @@
 for bit (GPU required): one to 32 slices and one more, a single variable, rows
 of more than 32 terms, terms of more members than are loaded ahead, negated
 literals, sweeps cut into launches of one."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -58,3 +60,34 @@ def test_lane_per_slice(name, trotter):
     for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
         np.testing.assert_array_equal(g[key], getattr(r, key), err_msg=key)
     assert s.stats().near_ties == 0
+
+
+def _solve(kind, inst, mode, sweeps, trotter):
+    params = {"seed": 5, "sweeps": sweeps, "restarts": 2, "trotter_number": trotter, "beta_start": 0.5, "beta_stop": 4.0,
+              "transverse_field_low": 0.1, "transverse_field_high": 2.0, "rng_mode": mode, "kernel": "warp"}
+    s = q.Solver(q.Model(kind, **inst), QMC, {"params": params}).init().run()
+    r = O.run(O.Model(kind, **inst), "qmc", seed=5, step_limit=sweeps, restarts=2, trotter_number=trotter,
+              sched=("linear", 0.5, 4.0), sched2=("linear", 0.1, 2.0), rng_mode=mode)
+    g = s.replicas()
+    for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
+        np.testing.assert_array_equal(g[key], getattr(r, key), err_msg=key)
+
+
+@pytest.mark.parametrize("mode", ["replay", "counter"])
+@pytest.mark.parametrize("n,trotter", [(511, 7), (700, 32)])
+def test_flip_ring_wraps(n, trotter, mode):
+    """Several sweeps in one launch: thousands of flip words through a ring of 512."""
+    inst = dict(zip(("off", "ids", "coef"), instance(n, [2], 3 * n, n)))
+    _solve("ising", inst, mode, 8, trotter)
+
+
+@pytest.mark.parametrize("mode", ["replay", "counter"])
+@pytest.mark.parametrize("n", [45, 46, 47])
+def test_rows_around_the_widest(n, mode):
+    """All terms of up to three variables: rows of 991 to 1082 incidences, around the
+    widest that a lane per slice takes."""
+    rows = [c for k in (1, 2, 3) for c in itertools.combinations(range(n), k)]
+    rng = np.random.default_rng(n)
+    inst = dict(zip(("off", "ids", "coef"), O.flatten_terms([(float(x), list(t)) for x, t in
+                                                             zip(rng.normal(size=len(rows)), rows)])))
+    _solve("pubo", inst, mode, 3, 5)
