@@ -534,7 +534,9 @@ static void build_fields(HostModel& m)
     rows[1] = (rows[1] + 1) & ~1;
     for (int l = 0; l < 32; l++) rows[0] = std::max(rows[0], left(l, 0));
     rows[0] = (rows[0] + 3) & ~3;
-    const size_t words = rec_at / 2 + 32 * (size_t)(rows[0] + rows[1] + rows[2] + rows[3]) + 16 * (size_t)rows[2];
+    const bool matrix = pair && kin > KI;
+    const size_t words = rec_at / 2 + 32 * (size_t)(rows[0] + rows[1] + rows[2] + rows[3]) + 16 * (size_t)rows[2] +
+                         (matrix ? 512 : 0);
     const size_t at = m.fc_tab.size();
     m.fc_tab.resize(at + ((2 * words + 3) & ~(size_t)3), 0u);
     uint32_t* tab = &m.fc_tab[at];
@@ -593,10 +595,22 @@ static void build_fields(HostModel& m)
         s3[(k * 32 + l) * 2] = have ? wide[l][k].w[0] | wide[l][k].w[2] << 29 : 1u << 30;
         s3[(k * 32 + l) * 2 + 1] = have ? wide[l][k].w[1] : 0u;
       }
+      if (matrix)
+      {
+        // one entry with the members' lanes and no value
+        for (const Entry& e : in[l])
+        {
+          tab[ent_at + l * ew] |= e.w[0];
+          uint32_t& w = s1[32 * __builtin_ctz(e.w[0]) + l];
+          w += e.w[1];
+        }
+        continue;
+      }
       for (size_t k = 0; k < in[l].size() && k < (size_t)KI; k++)
         memcpy(tab + ent_at + (k * 32 + l) * ew, in[l][k].w, ew * 4);
     }
-    if (kin > KI)
+    if (matrix) tab[1] |= 1u << 8;
+    else if (kin > KI)
     {
       const size_t more = m.fc_in.size() / ew;
       tab[1] |= (uint32_t)(kin - KI) << 8;

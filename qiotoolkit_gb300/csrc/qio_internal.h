@@ -89,8 +89,8 @@ struct DevModel
   // Block b's chunk begins at 8-byte word fc_desc[b].x of fc_tab:
   //   header, 32 bytes: rows of records of one literal / 4 | of two / 2 << 7 | of
   //     three / 2 << 15 | in-block entry rows (at most four) << 23 | the next
-  //     word is not 0 << 31; rows of wide terms | further entry rows << 8; first
-  //     further entry in fc_in;
+  //     word is not 0 << 31; rows of wide terms | further entry rows << 8 (pair-only
+  //     Ising: 1, a matrix); first further entry in fc_in;
   //   lane data, 8 bytes: the field with every record's op 0; degree; not pair: 16,
   //     the row's negated literals, its terms of v alone (counter models);
   //   in-block entries, four per lane (entry i of lane l at 32 i + l), one per
@@ -102,7 +102,10 @@ struct DevModel
   //   rows of 32 records, of the other terms' members: one literal (literal,
   //     weight); two (16 bits each, weight); three (the same, and the third's
   //     rows of 32 words behind them); wide terms (term | own literal negated <<
-  //     31, weight; 1 << 30: padding; 1 << 29: an entry holds its value).
+  //     31, weight; 1 << 30: padding; 1 << 29: an entry holds its value);
+  //   a pair-only Ising block of lanes with more than four entries: their only
+  //     entry has all earlier members' lanes and no value, and the values stand in
+  //     a matrix of 32-bit words, the member's lane by the own.
   // Weights and values of FP64 models that are not pair-only are multiples of 256,
   // the row position (modulo 32) beside them.  The field is the lane's value minus the weights whose op is 1: the literals'
   // OR (counter models) or XOR.  A literal 2u + n is variable u's, negated with n

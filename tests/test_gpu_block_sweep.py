@@ -106,3 +106,25 @@ def test_batches_of_every_form(kernel, mode):
     assert [b.run().result(i)["solutions"] for i in range(len(models))] == first
     pairs = q.Batch(models[:2], SA, {"params": dict(params, kernel=kernel)}).run()
     assert pairs.stats().kernel == 1 and [pairs.result(i)["solutions"] for i in range(2)] == first[:2]
+
+
+@pytest.mark.parametrize("mode", ["replay", "counter"])
+@pytest.mark.parametrize("integer", [True, False])
+@pytest.mark.parametrize("n", [5, 6, 32, 37, 64, 96, 200, 254])
+def test_dense_pair_blocks(n, integer, mode):
+    """Complete graphs, some couplings twice: a variable has four earlier members in
+    its block (n = 5), five, or all; staged blocks and ones too large for that."""
+    rng = np.random.default_rng(n)
+    rows = [[v] for v in range(n) if v % 3] + [[a, b] for a in range(n) for b in range(a + 1, n)]
+    rows += [rows[i] for i in rng.integers(0, len(rows), 3) if n < 250]
+    coef = rng.choice([-1.0, 1.0], len(rows)) if integer else rng.normal(size=len(rows))
+    off, ids, coef = O.flatten_terms([(float(c), r) for c, r in zip(coef, rows)])
+    params = {"seed": 4, "sweeps": 30, "restarts": 5, "beta_start": 0.02, "beta_stop": 1.0, "rng_mode": mode,
+              "kernel": "fields"}
+    s = q.Solver(q.Model("ising", off=off, ids=ids, coef=coef), SA, {"params": params}).init().run()
+    assert s.stats().sweep_kernel == 8
+    r = O.run(O.Model("ising", off=off, ids=ids, coef=coef), "sa", seed=4, step_limit=30, restarts=5,
+              sched=("linear", 0.02, 1.0), rng_mode=mode, threads=8)
+    out = s.replicas()
+    for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
+        np.testing.assert_array_equal(out[key], getattr(r, key), err_msg=key)
