@@ -22,8 +22,9 @@
 //
 // A second warp, the FEEDER, runs ahead of the decider: it fills a ring with
 // the walker's random draws as intervals of their ln-table values and brings
-// each block's chunk of the model (records, in-block entries) into one of three
-// or four shared-memory buffers by one TMA bulk copy.
+// each block's chunk of the model (records, in-block entries) into one of two to
+// four shared-memory buffers by one TMA bulk copy.  Walkers of a block whose
+// chunks are large have the same buffers, filled by the first one's feeder.
 //
 // FP64 models: a third warp, the ACCOUNTANT, consumes a log of the flips in
 // batches of up to 32: every lane recomputes one flip's exact FP64 cost
@@ -72,7 +73,8 @@ static const unsigned kFull = 0xffffffffu;
 static const int kIn = 4;         // in-block entries per lane of a staged block
 static const int kLogBytes = 1024;  // flip log per walker: 64 entries of 16 bytes, pair models 256 of 4
 static const int kRing = 128;     // draw intervals per walker (power of 2)
-static const int kCtrl = 64;      // per-walker control block: mbarriers, counters
+static const int kCtrl = 32;      // per-walker counters
+static const int kBars = 48;      // mbarriers and the abort flag, before chunk buffers
 static const int kTable = 4096;   // per block: screen row 0
 static const uint32_t kWideMask = 0x0003FFFFu;  // wide term of a record or entry
 static const uint32_t kNoWide = 0x40000000u;    // wide record: padding
@@ -180,6 +182,17 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 {
   for (int it = 0; it < (1 << 22); it++)
     if (mbar_try(bar, parity)) return true;
+  return false;
+}
+// the same for a chunk that may not have been issued yet, or never is once
+// `abort` is raised
+__device__ __forceinline__ bool chunk_wait(unsigned long long* bar, unsigned parity, const unsigned* abort)
+{
+  for (int it = 0; it < (1 << 22); it++)
+  {
+    if (mbar_try(bar, parity)) return true;
+    if (*(const volatile unsigned*)abort) return false;
+  }
   return false;
 }
 
@@ -357,16 +370,17 @@ struct Shape
   int nw;     // spin words of the population
   int zb;     // literal bytes and wide terms' bytes; pair models: a byte per variable
   int words;  // 8-byte words of a staged chunk (larger blocks read their records from HBM)
-  int bufs;   // chunk buffers: kBufs, or one less where another walker then fits
+  int bufs;   // chunk buffers, kBufs at most
+  int share;  // walkers that use the same ones (a block's, or 1)
   bool pair;
 };
 struct Region
 {
-  unsigned long long* bars;  // kBufs mbarriers
+  unsigned long long* bars;  // kBufs mbarriers, before the buffers
   unsigned* head;            // log entries published by the decider (with `used`, 8 bytes)
   unsigned* tail;            // log entries consumed by the accountant
   unsigned* done;            // the decider finished the walker
-  unsigned* abort;           // a wait gave up: all warps leave
+  unsigned* abort;           // a wait gave up: all warps leave (beside the mbarriers)
   unsigned* next;            // the walker taken from the queue
   unsigned* made;            // draws in the ring
   unsigned* used;            // draws taken by the decider
@@ -380,31 +394,43 @@ struct Region
   uint32_t* aspins;          // the accountant's spins (FP64 models), two copies for pair models
 };
 
-__host__ __device__ inline int region_bytes(const Shape& s, bool integer)
+// a walker's own part, and the chunk buffers', which a block's walkers may share
+__host__ __device__ inline int own_bytes(const Shape& s, bool integer)
 {
-  return kCtrl + kRing * 12 + (integer ? 0 : kLogBytes) + s.bufs * s.words * 8 + s.zb + 4 * (s.nw + 4) +
+  return kCtrl + kRing * 12 + (integer ? 0 : kLogBytes) + s.zb + 4 * (s.nw + 4) +
          (integer ? 0 : 4 * (s.nw + 4) * (s.pair ? 2 : 1));
 }
+__host__ __device__ inline int chunk_bytes(const Shape& s) { return kBars + s.bufs * s.words * 8; }
+__host__ __device__ inline int region_bytes(const Shape& s, bool integer)
+{
+  return own_bytes(s, integer) + (s.share > 1 ? 0 : chunk_bytes(s));
+}
+__host__ __device__ inline int common_bytes(const Shape& s) { return s.share > 1 ? chunk_bytes(s) : 0; }
 
+// Every pointer is one of two bases and little more: with a choice for each of
+// them an integer kernel, at its 128 registers, took 10 to 40 % longer.
 template <bool INT>
-__device__ __forceinline__ Region carve(unsigned char* base, const Shape& s)
+__device__ __forceinline__ Region carve(unsigned char* smem, int walker, const Shape& s)
 {
   Region R;
-  R.bars = (unsigned long long*)base;
-  unsigned* c = (unsigned*)(base + 32);
+  const int at = kTable + common_bytes(s) + walker * region_bytes(s, INT);
+  unsigned char* base = smem + at;
+  unsigned char* chunks = smem + (s.share > 1 ? kTable : at + own_bytes(s, INT));
+  R.bars = (unsigned long long*)chunks;
+  R.abort = (unsigned*)(chunks + 32);
+  R.tiles = (uint2*)(chunks + kBars);
+  unsigned* c = (unsigned*)base;
   R.head = c;
   R.used = c + 1;
   R.tail = c + 2;  // (tail, made: one 8-byte word)
   R.made = c + 3;
   R.done = c + 4;
-  R.abort = c + 5;
   R.next = c + 6;
   R.blocks = c + 7;
   R.ring = (float2*)(base + kCtrl);
   R.raw = (uint32_t*)(R.ring + kRing);
   R.log = (uint4*)(R.raw + kRing);
-  R.tiles = (uint2*)(R.log + (INT ? 0 : kLogBytes / 16));
-  R.z = (uint8_t*)(R.tiles + s.bufs * s.words);
+  R.z = (uint8_t*)(R.log + (INT ? 0 : kLogBytes / 16));
   R.spins = (uint32_t*)(R.z + s.zb);
   R.aspins = R.spins + s.nw + 4;
   return R;
@@ -472,12 +498,15 @@ __device__ __forceinline__ uint64_t stream_state(const Region& R, const Walk& W)
 // always accepts is (-inf, -inf).
 //
 // Chunks: a block's goes to the next buffer in turn (T, kept over the warp's
-// walkers) once the decider is done with the block `bufs` before.
+// walkers) once the decider is done with the block `bufs` before.  Where walkers
+// share the buffers, the first one's feeder brings the chunks, once all of them
+// are done with that block (`live` of them, 0 for the others' feeders; their
+// counters `stride` words apart).
 // ---------------------------------------------------------------------------
 template <int FM, bool REPLAY>
 __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int4* desc, const uint2* table, int tile_w,
                                   int cap, Turns& turns, int n_sweeps, uint64_t rs, uint64_t key, unsigned long long ctr,
-                                  int n_vars, int* err)
+                                  int n_vars, int live, int stride, int* err)
 {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -497,7 +526,9 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
     // what the decider has done
     const unsigned used = ld_acquire(R.used);
     const unsigned blocks = *(volatile unsigned*)R.blocks;
-    while (T.sweep < n_sweeps && in_flight(issued, blocks) < (unsigned)T.bufs)
+    unsigned held = in_flight(issued, blocks);  // chunks that the slowest walker needs yet
+    for (int k = 1; k < live; k++) held = max(held, in_flight(issued, ld_acquire(R.blocks + k * stride)));
+    for (; live > 0 && T.sweep < n_sweeps && held < (unsigned)T.bufs; held++)
     {
       if (lane == 0)
         tile_issue(R.tiles + T.buf * tile_w, table + d.x, (unsigned)min(d.y, cap) * 8u, &R.bars[T.buf]);
@@ -530,10 +561,11 @@ __device__ __noinline__ void feed(const Region R, const float4* s_scr, const int
         continue;
       }
       // the copies in flight land before the region is given up
-      if (lane == 0)
+      if (lane == 0 && live > 0)
       {
         Turns U = T;
-        const unsigned n = in_flight(issued, *(volatile unsigned*)R.blocks);
+        unsigned n = 0;
+        for (int k = 0; k < live; k++) n = max(n, in_flight(issued, *(volatile unsigned*)(R.blocks + k * stride)));
         U.back(n);
         for (unsigned x = 0; x < n; x++, U.next_buffer()) mbar_wait(&R.bars[U.buf], U.phase);
       }
@@ -828,7 +860,7 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
     // this block's chunk
     if (!__all_sync(kFull, mbar_try(&R.bars[T.buf], T.phase)))
     {
-      const bool landed = mbar_wait(&R.bars[T.buf], T.phase);
+      const bool landed = chunk_wait(&R.bars[T.buf], T.phase, R.abort);
       if (!__all_sync(kFull, landed))
       {
         raise_abort(R, a.err);
@@ -1500,6 +1532,16 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
   extern __shared__ __align__(128) unsigned char smem[];
   float4* s_scr = (float4*)smem;
   for (int t = threadIdx.x; t < 256; t += blockDim.x) s_scr[t] = g_scr[t];
+  if (sh.share > 1 && threadIdx.x == 0)
+  {
+    const Region R = carve<INT>(smem, 0, sh);
+    for (int i = 0; i < kBufs; i++) mbar_init(&R.bars[i]);
+    *R.abort = 0u;
+  }
+  const int stride = region_bytes(sh, INT);
+  // (blocks that the walkers have finished, before the first one's feeder looks)
+  if (sh.share > 1 && (int)threadIdx.x < wpc)
+    *carve<INT>(smem, (int)threadIdx.x, sh).blocks = 0u;
   // A chained launch: the kernel before is done from here on (this one's launch
   // and table overlap with it), and the one behind may start to.  PT on 3-SAT,
   // 200 steps of a 50 us sweep and its swaps: 12.8 and 11.9 ms.
@@ -1520,12 +1562,13 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
   const bool queued = a.queue != nullptr;
   if (!queued && ws0 >= a.n_streams) return;
   const int w = queued ? 0 : (a.order ? a.order[ws0] : ws0);
-  unsigned char* base = smem + kTable + (size_t)ws * region_bytes(sh, INT);
-  const Region R = carve<INT>(base, sh);
+  const Region R = carve<INT>(smem, ws, sh);
+  // the walkers whose chunks this one's feeder brings
+  const int live = sh.share <= 1 ? 1 : ws ? 0 : min(wpc, (a.n_streams - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x);
   const int bar_id = 1 + ws;
   const int me = role * 32 + lane, nme = kRoles * 32;  // thread of the walker
   // (the feeder's own barriers; the first walker_sync below shows them to the decider)
-  if (role == 1 && lane == 0)
+  if (sh.share <= 1 && role == 1 && lane == 0)
     for (int i = 0; i < kBufs; i++) mbar_init(&R.bars[i]);
   uint64_t rs = (REPLAY && !queued) ? a.rng[w] : 0;
   Turns turns(1, sh.bufs);
@@ -1551,7 +1594,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
       *R.head = 0u;
       *R.tail = 0u;
       *R.done = 0u;
-      *R.abort = 0u;
+      if (sh.share <= 1) *R.abort = 0u;
       *R.made = 0u;
       *R.used = 0u;
       *R.blocks = 0u;
@@ -1609,7 +1652,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     else if (role == 1)
     {
       feed<FM, REPLAY>(R, s_scr, m.fc_desc, m.fc_tab, sh.words, sh.words, turns, a.n_sweeps, rs, key,
-                       (unsigned long long)a.sweep_base * (unsigned long long)N, N, a.err);
+                       (unsigned long long)a.sweep_base * (unsigned long long)N, N, live, stride / 4, a.err);
       walker_sync<INT>(bar_id);
     }
     else
@@ -1647,7 +1690,7 @@ template <int FM, bool R, bool I>
 static cudaError_t go(const SweepArgs& a, cudaStream_t s, int wpc, const Shape& sh)
 {
   auto k = fc_sweep_kernel<FM, R, I>;
-  const int smem = kTable + wpc * region_bytes(sh, I);
+  const int smem = kTable + common_bytes(sh) + wpc * region_bytes(sh, I);
   const int threads = (I ? 64 : 96) * wpc;
   const cudaError_t allowed = allow_shared((const void*)k, smem);
   if (allowed != cudaSuccess) return allowed;
@@ -1688,20 +1731,26 @@ static cudaError_t go_fm(const SweepArgs& a, cudaStream_t s, int wpc, const Shap
 }
 
 // a walker's region for a model in a population of this stride
-static Shape shape_of(const DevModel& m, int nw)
+static Shape shape_of(const DevModel& m, int nw, int bufs, bool shared)
 {
   Shape s;
   s.pair = m.flavor == F_PARITY && m.pair_only;
   s.nw = nw;
   s.zb = s.pair ? nw * 32 : (64 * nw + 16 + m.fc_wide + 15) & ~15;
   s.words = m.fc_words;
-  s.bufs = kBufs;
+  s.bufs = bufs;
+  s.share = shared ? 2 : 1;
   // a state that leaves less room: smaller tiles (larger blocks read their
   // records from HBM)
   const int least = Chunk<COUNTER>::kRec;
-  const int room = (kMaxSmem - kTable - region_bytes(s, m.int_mode != 0)) / (8 * kBufs);
+  const int room = (kMaxSmem - kTable - common_bytes(s) - region_bytes(s, m.int_mode != 0)) / (8 * bufs);
   if (room < 0) s.words = std::max(least, (s.words + room - 1) & ~1);
   return s;
+}
+// walkers of a block, at most
+static int walkers_of(const Shape& s, bool integer)
+{
+  return std::min(integer ? 8 : 4, (kMaxSmem - kTable - common_bytes(s)) / region_bytes(s, integer));
 }
 }  // namespace fc
 
@@ -1709,26 +1758,40 @@ bool fc_fits(const DevModel& m, int nw)
 {
   if (!m.fc_desc || m.sweep_size != m.n_vars || m.n_vars <= 0) return false;
   if (!(m.flavor == F_PARITY || m.flavor == F_COUNTER)) return false;
-  return fc::kTable + fc::region_bytes(fc::shape_of(m, nw), m.int_mode != 0) <= fc::kMaxSmem;
+  // (the line as it has been; a launch may do with two buffers)
+  return fc::kTable + fc::region_bytes(fc::shape_of(m, nw, fc::kBufs, false), m.int_mode != 0) - 16 <= fc::kMaxSmem;
 }
 
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb)
 {
   if (!fc_fits(a.m, a.p.nw)) return cudaErrorInvalidValue;
-  fc::Shape sh = fc::shape_of(a.m, a.p.nw);
   const bool I = a.m.int_mode != 0;
-  auto fit = [&](int bufs) {
-    sh.bufs = bufs;
-    return std::min(I ? 8 : 4, (fc::kMaxSmem - fc::kTable) / fc::region_bytes(sh, I));
-  };
-  // Three chunk buffers where four would cost a wave of blocks: 512 tempering
-  // walkers of a 4096-variable PUBO, 100 sweeps: 61.3 ms at three walkers a block
-  // with four buffers, 43.7 at four with three.  Otherwise four: the third covers
-  // the copy's latency only just.
-  const int w3 = fit(fc::kBufs - 1), w4 = fit(fc::kBufs);
-  auto waves = [&](int w) { return (a.n_streams + w * fc::kSms - 1) / (w * fc::kSms); };
-  const int wmax = waves(w3) < waves(w4) ? w3 : w4;
-  if (wmax != w4) sh.bufs = fc::kBufs - 1;
+  // The first of these shapes with the fewest waves of blocks (twice as long where
+  // the largest blocks do not fit a buffer): four chunk buffers each, which cover
+  // the copy's latency best, three, or a block's walkers on the same ones, in
+  // step.  512 tempering walkers of a 4096-variable PUBO, 100 sweeps: 61.3 ms at
+  // three walkers a block with four buffers each, 43.7 at four with three.  608
+  // walkers of a 1000-spin model with 8 hubs of 200 couplings, 40 sweeps: 6.15 with
+  // buffers of their own, one walker a block, 1.99 with the same, four a block; of a
+  // complete +-1 graph of 200 spins, 100 sweeps: 5.8 and 1.75.
+  struct Choice { int bufs; bool shared; };
+  const Choice choices[] = {{4, false}, {3, false}, {4, true}, {3, true}, {2, false}, {2, true}};
+  fc::Shape sh{};
+  int wmax = 0;
+  long long least = LLONG_MAX;
+  for (const Choice& c : choices)
+  {
+    if (c.shared && (a.queue || a.n_streams != a.n_walkers)) continue;
+    const fc::Shape x = fc::shape_of(a.m, a.p.nw, c.bufs, c.shared);
+    const int w = fc::walkers_of(x, I);
+    if (w < 1) continue;
+    const long long waves = (a.n_streams + (long long)w * fc::kSms - 1) / ((long long)w * fc::kSms);
+    const long long cost = waves * (x.words < a.m.fc_words ? 2 : 1);
+    if (cost >= least) continue;
+    least = cost;
+    sh = x;
+    wmax = w;
+  }
   // spread the walkers over the SMs: as few per block as fills them
   int wpc = (a.n_streams + fc::kSms - 1) / fc::kSms;
   if (a.queue) wpc = std::min(wpc, wpb);

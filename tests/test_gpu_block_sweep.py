@@ -128,3 +128,29 @@ def test_dense_pair_blocks(n, integer, mode):
     out = s.replicas()
     for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
         np.testing.assert_array_equal(out[key], getattr(r, key), err_msg=key)
+
+
+SHARED = {  # models whose chunks are so large that a block's walkers share their buffers
+    "pair": ("ising", lambda: terms(200, [2], 16000, 31)),
+    "pair_int": ("ising", lambda: terms(130, [2], 7000, 32, integer=True)),
+    "hub": ("ising", lambda: terms(320, [2], 600, 33, hub=240)),
+    "pubo": ("pubo", lambda: terms(300, [2, 3], 500, 34, hub=240)),
+    "pubo_int": ("pubo", lambda: terms(96, [2], 3500, 35, integer=True)),
+}
+
+
+@pytest.mark.parametrize("mode", ["replay", "counter"])
+@pytest.mark.parametrize("restarts", [153, 305, 609, 1217])
+@pytest.mark.parametrize("name", list(SHARED))
+def test_shared_chunk_buffers(name, restarts, mode):
+    """Blocks of two to eight walkers on the same buffers, the last ones not full."""
+    kind, make = SHARED[name]
+    inst = dict(zip(("off", "ids", "coef"), make()))
+    params = {"seed": 9, "sweeps": 6, "restarts": restarts, "beta_start": 0.05, "beta_stop": 1.0, "rng_mode": mode,
+              "kernel": "fields"}
+    s = q.Solver(q.Model(kind, **inst), SA, {"params": params}).init().run()
+    r = O.run(O.Model(kind, **inst), "sa", seed=9, step_limit=6, restarts=restarts, sched=("linear", 0.05, 1.0),
+              rng_mode=mode, threads=8)
+    out = s.replicas()
+    for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
+        np.testing.assert_array_equal(out[key], getattr(r, key), err_msg=key)
