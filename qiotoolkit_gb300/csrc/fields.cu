@@ -15,8 +15,8 @@
 // mask of the last round, vote, and decide again where a member of a lane's
 // in-block terms changed; a mask that no longer changes any lane's terms is the
 // ordered sweep's, lane by lane from the first.  A field within its rounding
-// margin of zero, a comparison inside the FP32 screen's margin or a row too
-// wide for the log's masks ends the block early: the lanes before it are
+// margin of zero or a comparison inside the FP32 screen's margin
+// ends the block early: the lanes before it are
 // committed, the lane itself is tried alone with the reference's FP64 sum and
 // ln-table expression, and the rest of the block is decided after it.
 //
@@ -29,8 +29,9 @@
 // FP64 models: a third warp, the ACCOUNTANT, consumes a log of the flips in
 // batches of up to 32: every lane recomputes one flip's exact FP64 cost
 // difference (the reference's order and rounding, model/ising.h:108-117,
-// model/pubo.h:335-367) from the spins (pair-only Ising) or from the masks of
-// the contributing terms that the decider gathered beside the field, then the
+// model/pubo.h:335-367) from the spins (pair-only Ising, rows of more than 32
+// terms) or from the masks of the contributing terms that the decider gathered
+// beside the field, then the
 // running cost is accumulated in flip order exactly as cost_ += diff
 // (markov/walker.h:225) and the lowest state is taken at the first strict
 // improvement (markov/walker.h:269-280) from the accountant's own copy of the
@@ -191,7 +192,7 @@ __device__ __forceinline__ bool chunk_wait(unsigned long long* bar, unsigned par
   for (int it = 0; it < (1 << 22); it++)
   {
     if (mbar_try(bar, parity)) return true;
-    if (*(const volatile unsigned*)abort) return false;
+    if ((it & 255) == 255 && *(const volatile unsigned*)abort) return false;
   }
   return false;
 }
@@ -312,6 +313,37 @@ __device__ __forceinline__ double exact_dE(const DevModel& m, int v, int q, int 
   return FM == COUNTER ? d : neg2x(d);
 }
 
+// The accountant's batch of n flips where some rows are too wide for masks (this
+// lane's: `wide`): those are summed from the spins, in index order as pair models'
+// (account).  The differences, and the flips that are one sweep's.  (The decider
+// summing them itself, an accepted flip at a time: QUBO of 128 variables, complete,
+// 64 walkers, 200 sweeps 264 ms, here 16.5; 1000 variables of 40 terms, 100 sweeps
+// 301 and 31; the windowed sweep 212 and 177.)
+struct Summed
+{
+  double d;
+  int n;
+};
+template <int FM>
+__device__ __noinline__ Summed sum_rows(const DevModel& m, uint32_t* spins, int nw, int v, int q0, int q1, bool wide,
+                                        int n, double d)
+{
+  const int lane = threadIdx.x & 31;
+  if (__any_sync(kFull, wide))
+  {
+    const int prev = __shfl_up_sync(kFull, v, 1);
+    const unsigned wrap = __ballot_sync(kFull, lane > 0 && lane < n && v <= prev);
+    if (wrap) n = __ffs(wrap) - 1;
+    uint32_t* after = spins + nw + 4;
+    for (int q = lane; q < nw; q += 32) after[q] = spins[q];
+    __syncwarp();
+    if (lane < n) atomicXor(after + (v >> 5), 1u << (v & 31));
+    __syncwarp();
+    if (wide && lane < n) d = exact_dE<FM>(m, v, q0, q1, spins, after);
+  }
+  return {d, n};
+}
+
 // Exact cost difference from a log entry's masks (accountant): COUNTER: qm = the
 // contributing incidences, sm = their signs; PARITY: all contribute.
 template <int FM>
@@ -373,6 +405,7 @@ struct Shape
   int bufs;   // chunk buffers, kBufs at most
   int share;  // walkers that use the same ones (a block's, or 1)
   bool pair;
+  bool second;  // FP64: a second copy of the accountant's spins
 };
 struct Region
 {
@@ -391,14 +424,14 @@ struct Region
   uint2* tiles;              // the block chunks
   uint8_t* z;                // literals, a byte each, then the wide terms'; pair models: spins
   uint32_t* spins;           // nw + 4 words (words of zeros after the last)
-  uint32_t* aspins;          // the accountant's spins (FP64 models), two copies for pair models
+  uint32_t* aspins;          // the accountant's spins (FP64 models), two copies (Shape::second)
 };
 
 // a walker's own part, and the chunk buffers', which a block's walkers may share
 __host__ __device__ inline int own_bytes(const Shape& s, bool integer)
 {
   return kCtrl + kRing * 12 + (integer ? 0 : kLogBytes) + s.zb + 4 * (s.nw + 4) +
-         (integer ? 0 : 4 * (s.nw + 4) * (s.pair ? 2 : 1));
+         (integer ? 0 : 4 * (s.nw + 4) * (s.second ? 2 : 1));
 }
 __host__ __device__ inline int chunk_bytes(const Shape& s) { return kBars + s.bufs * s.words * 8; }
 __host__ __device__ inline int region_bytes(const Shape& s, bool integer)
@@ -1216,7 +1249,6 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
           const bool no = iv.x > __fadd_rn(thr, et);
           rare = rare || (up && !yes && !no);
           const bool acc = active && !rare && (!up || yes);
-          if (MASKS) rare = rare || (acc && deg > 32);  // its masks do not fit the log
           const unsigned An = __ballot_sync(kFull, acc) | done;
           const unsigned diff = An ^ A;
           A = An;
@@ -1388,9 +1420,9 @@ __device__ __forceinline__ void accumulate(double d, int n, double& cost, long l
 
 // ---------------------------------------------------------------------------
 // The accountant (FP64 models): running cost, lowest cost and lowest state
-// from the log.
+// from the log.  WIDE: a term model with rows of more than 32 terms.
 // ---------------------------------------------------------------------------
-template <int FM>
+template <int FM, bool WIDE>
 __device__ __noinline__ bool account(const SweepArgs& a, const DevModel& m, const Region R, double& cost,
                                         double& low, uint32_t* g_lsp)
 {
@@ -1473,12 +1505,19 @@ __device__ __noinline__ bool account(const SweepArgs& a, const DevModel& m, cons
         __syncwarp();
         if (lane < n) d = exact_dE<FM>(m, v, q0, q1, R.aspins, after);
       }
-      else if (lane < n)
+      else
       {
         const int deg = (int)((ent.x >> 16) & 255u);
-        if (ent.x & kExactF)
+        const bool exact = (ent.x & kExactF) != 0u;
+        if (lane < n && exact)
           d = __longlong_as_double((long long)((unsigned long long)ent.y | ((unsigned long long)ent.z << 32)));
-        else d = dE_from_masks<FM>(m.coef + q0, deg, ent.y, ent.z);
+        else if (lane < n && (!WIDE || deg <= 32)) d = dE_from_masks<FM>(m.coef + q0, deg, ent.y, ent.z);
+        if constexpr (WIDE)
+        {
+          const Summed x = sum_rows<FM>(m, R.aspins, nw, v, q0, q1, lane < n && !exact && deg > 32, n, d);
+          d = x.d;
+          n = x.n;
+        }
       }
       __syncwarp();
       tail += (unsigned)n;
@@ -1658,7 +1697,8 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     else
     {
       double cost = a.p.cost[slot], low = a.p.lowest[r];
-      const bool ok = account<FM>(a, m, R, cost, low, g_lsp);
+      const bool ok = FM != PAIR && m.max_deg > 32 ? account<FM, FM != PAIR>(a, m, R, cost, low, g_lsp)
+                                                   : account<FM, false>(a, m, R, cost, low, g_lsp);
       walker_sync<INT>(bar_id);
       if (ok && !*(volatile unsigned*)R.abort && lane == 0)
       {
@@ -1735,6 +1775,7 @@ static Shape shape_of(const DevModel& m, int nw, int bufs, bool shared)
 {
   Shape s;
   s.pair = m.flavor == F_PARITY && m.pair_only;
+  s.second = s.pair || m.max_deg > 32;
   s.nw = nw;
   s.zb = s.pair ? nw * 32 : (64 * nw + 16 + m.fc_wide + 15) & ~15;
   s.words = m.fc_words;
@@ -1758,8 +1799,12 @@ bool fc_fits(const DevModel& m, int nw)
 {
   if (!m.fc_desc || m.sweep_size != m.n_vars || m.n_vars <= 0) return false;
   if (!(m.flavor == F_PARITY || m.flavor == F_COUNTER)) return false;
-  // (the line as it has been; a launch may do with two buffers)
-  return fc::kTable + fc::region_bytes(fc::shape_of(m, nw, fc::kBufs, false), m.int_mode != 0) - 16 <= fc::kMaxSmem;
+  // (the line as it has been: a launch may do with two buffers, which saves more
+  // than a second copy of a term model's spins takes)
+  fc::Shape s = fc::shape_of(m, nw, fc::kBufs, false);
+  s.words = std::min(s.words, fc::Chunk<fc::COUNTER>::kRec);
+  s.second = s.pair;
+  return fc::kTable + fc::region_bytes(s, m.int_mode != 0) - 16 <= fc::kMaxSmem;
 }
 
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb)

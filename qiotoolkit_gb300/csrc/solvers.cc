@@ -2411,7 +2411,8 @@ class SABatch : public Batch
     int first, last;
     const HostModel* model;  // any member (flavour and coefficient kind)
     int max_block_inc;       // the members' largest 32-variable block
-    int fc_words, fc_wide;   // the same of the block-decided sweep's chunks and wide terms
+    int fc_words, fc_wide;   // the same of the block-decided sweep's chunks and wide terms,
+    int max_deg;             // and of their rows
     bool fields;             // runs on the block-decided sweep
   };
   // members of a group share the kernel's instance
@@ -2564,13 +2565,15 @@ class SABatch : public Batch
       const int first = (int)k * R;
       const int mb = m->device_view(full_sweep).max_block_inc;
       if (groups.empty() || kind(*groups.back().model) != kind(*m))
-        groups.push_back({first, first + R, m, mb, m->fc_words, (int)m->fc_wide.size(), block_decided(*m)});
+        groups.push_back({first, first + R, m, mb, m->fc_words, (int)m->fc_wide.size(),
+                          m->device_view(full_sweep).max_deg, block_decided(*m)});
       else
       {
         groups.back().last = first + R;
         groups.back().max_block_inc = std::max(groups.back().max_block_inc, mb);
         groups.back().fc_words = std::max(groups.back().fc_words, m->fc_words);
         groups.back().fc_wide = std::max(groups.back().fc_wide, (int)m->fc_wide.size());
+        groups.back().max_deg = std::max(groups.back().max_deg, m->device_view(full_sweep).max_deg);
       }
       if (groups.back().fields) continue;
       SweepArgs a{};
@@ -2636,6 +2639,7 @@ class SABatch : public Batch
     a.m.max_block_inc = G.max_block_inc;  // tiles sized for the group's largest block
     a.m.fc_words = G.fc_words;
     a.m.fc_wide = G.fc_wide;
+    a.m.max_deg = G.max_deg;
     a.fields = G.fields ? 1 : 0;
     cuda_check(launch_sweep(a, st, wpb), "sweep kernel");
   }

@@ -154,3 +154,51 @@ def test_shared_chunk_buffers(name, restarts, mode):
     out = s.replicas()
     for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
         np.testing.assert_array_equal(out[key], getattr(r, key), err_msg=key)
+
+
+def _rows_of(n, degree, sizes, seed, integer=False):
+    """Variables 0, 3, 6, ... with `degree` terms each, the others fewer."""
+    rng = np.random.default_rng(seed)
+    out = {(v,) for v in range(n)}
+    count = np.ones(n, int)
+    for v in range(0, n, 3):
+        while count[v] < degree:
+            others = rng.choice(np.setdiff1d(np.arange(n), np.arange(0, n, 3)), int(rng.choice(sizes)) - 1, replace=False)
+            t = tuple(sorted({v, *others.tolist()}))
+            if t not in out and count[list(others)].max() < 250:
+                out.add(t)
+                count[list(t)] += 1
+    out = sorted(out)
+    coef = rng.choice([-2.0, -1.0, 1.0, 3.0], len(out)) if integer else rng.normal(size=len(out))
+    return O.flatten_terms([(float(c), list(t)) for c, t in zip(coef, out)])
+
+
+@pytest.mark.parametrize("mode", ["replay", "counter"])
+@pytest.mark.parametrize("kind,n,degree,sizes", [
+    ("pubo", 40, 31, [3]), ("pubo", 40, 32, [3]), ("pubo", 40, 33, [3]), ("pubo", 33, 34, [3, 6]), ("pubo", 60, 90, [3, 4]),
+    ("pubo", 290, 190, [2]), ("ising", 40, 32, [3]), ("ising", 40, 33, [3]), ("ising", 70, 64, [3, 4, 7])])
+def test_rows_wider_than_the_masks(kind, n, degree, sizes, mode):
+    """FP64 rows around 32 terms, the widest that a flip's log entry has masks for."""
+    inst = dict(zip(("off", "ids", "coef"), _rows_of(n, degree, sizes, n + degree)))
+    for stop in (1.0, 6.0):
+        params = {"seed": 2, "sweeps": 40, "restarts": 7, "beta_start": 0.01, "beta_stop": stop, "rng_mode": mode,
+                  "kernel": "fields"}
+        s = q.Solver(q.Model(kind, **inst), SA, {"params": params}).init().run()
+        assert s.stats().sweep_kernel == 8
+        r = O.run(O.Model(kind, **inst), "sa", seed=2, step_limit=40, restarts=7, sched=("linear", 0.01, stop),
+                  rng_mode=mode, threads=8)
+        out = s.replicas()
+        for key in ("cost", "lowest", "attempts", "accepts", "states", "lowest_states"):
+            np.testing.assert_array_equal(out[key], getattr(r, key), err_msg=key)
+
+
+@pytest.mark.parametrize("mode", ["replay", "counter"])
+def test_batch_with_wide_and_narrow_rows(mode):
+    """One queue for models with rows that have masks and rows that have none."""
+    insts = [_rows_of(60, 8, [3], 1), _rows_of(64, 70, [3, 4], 2), _rows_of(200, 4, [2, 3], 3), _rows_of(45, 40, [3], 4)]
+    models = [q.Model("pubo", off=t[0], ids=t[1], coef=t[2]) for t in insts]
+    params = {"seed": 6, "sweeps": 12, "restarts": 9, "beta_start": 0.05, "beta_stop": 2.0, "rng_mode": mode}
+    b = q.Batch(models, SA, {"params": params}).run()
+    for i, m in enumerate(models):
+        plain = q.Solver(m, SA, {"params": dict(params, kernel="warp")}).init().run().result()
+        assert b.result(i)["solutions"] == plain["solutions"], i
