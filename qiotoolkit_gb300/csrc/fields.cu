@@ -861,7 +861,6 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
   // (read once: `m` may be the launch's parameter or lie in device memory)
   const uint2* table = m.fc_tab;
   const int4* descs = m.fc_desc;
-  const uint4* further = (const uint4*)m.fc_in;
   const int cap = sh.words;
   uint8_t* zw = R.z + 64 * sh.nw + 16;  // the wide terms' bytes
 
@@ -910,7 +909,8 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
     const int n0 = (int)(h0 & 127u) * 4, n1 = FM == PAIR ? 0 : (int)((h0 >> 7) & 255u) * 2;
     const int n2 = FM == PAIR ? 0 : (int)((h0 >> 15) & 255u) * 2, n3 = FM == PAIR ? 0 : (int)(h1 & 255u);
     const int ents = (int)((h0 >> 23) & 7u), xn = (int)(h1 >> 8);
-    const bool staged = C::kRec + 32 * (n0 + n1 + n2 + n3) + 16 * n2 + (FM == PAIR && xn ? 512 : 0) <= cap;
+    const int recs = C::kRec + 32 * (n0 + n1 + n2 + n3) + 16 * n2;  // words before the further entries
+    const bool staged = recs + (FM == PAIR ? (xn ? 512 : 0) : 64 * xn) <= cap;
     // The block itself.  SP: it has records or entries beyond its chunk, or wide
     // terms; the other form, most blocks', has a branch less for each of these
     // (a branch costs ten to twenty cycles of its warp): sparse Ising 23.6 and
@@ -1062,9 +1062,10 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
       int val[KI];
       unsigned bit[KI];  // its place in the mask
       unsigned em[KI], et[KI];
-      // further entries (rare): xn of them, in HBM
-      const uint4* xterm = further + (FM != PAIR && SP && xn ? (size_t)__shfl_sync(kFull, chunk[1].x, 0) + lane : 0);
-      const int* mat = (const int*)((!SP || staged ? chunk + C::kRec : far - lane) + 32 * n0) + lane;
+      // further entries, xn rows of them, or a pair block's matrix
+      const uint2* more = (!SP || staged ? chunk : far - lane - C::kRec) + recs;
+      const uint4* xterm = (const uint4*)more + lane;
+      const int* mat = (const int*)more + lane;
       unsigned done = 0;  // the block's flips so far
       // an entry's em and et; D: flips whose bytes are written already
       auto entry = [&](const uint4& e, unsigned D, unsigned& mm, unsigned& mt) {
@@ -1121,7 +1122,7 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
         take(3);
       }
       if (SP && FM != PAIR)
-        for (int i = 0; i < xn; i++) watch |= __ldg(&xterm[32 * i].x);
+        for (int i = 0; i < xn; i++) watch |= xterm[32 * i].x;
 
       // ---- the other warps: room for this block's flips and draws
       auto room = [&]() -> bool {
@@ -1201,7 +1202,7 @@ __device__ __forceinline__ bool decide_sweeps(const SweepArgs& a, const DevModel
           }
           for (int i = 0; FM != PAIR && SP && i < xn; i++)
           {
-            const uint4 e = __ldg(xterm + 32 * i);
+            const uint4 e = xterm[32 * i];
             unsigned mm, mt;
             entry(e, done, mm, mt);
             const bool on = e.x && holds(A, mm, mt);

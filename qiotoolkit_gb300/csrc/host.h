@@ -77,7 +77,7 @@ struct HostModel
   std::vector<unsigned int> rec_p;  // other << 8 | coefficient, when |coef| <= 127
   // block-decided sweep tables (see DevModel::fc_desc; empty: not eligible)
   std::vector<int> fc_desc;
-  std::vector<uint32_t> fc_tab, fc_in, fc_oth;
+  std::vector<uint32_t> fc_tab, fc_oth;
   std::vector<int> fc_wide;
   int fc_words = 0;
   int fc_S = 0;
@@ -115,7 +115,7 @@ struct HostModel
   template <class F> void device_arrays(F f) const
   {
     f(row), f(inc), f(coef), f(coef_i), f(nbr), f(trow), f(tvar), f(tcost), f(tcost_i), f(coef_f), f(near), f(other);
-    f(rec_i), f(rec_f), f(rec_p), f(lv_off), f(lv_ent), f(lv_pos), f(fc_tab), f(fc_desc), f(fc_in), f(fc_oth), f(fc_wide);
+    f(rec_i), f(rec_f), f(rec_p), f(lv_off), f(lv_ent), f(lv_pos), f(fc_tab), f(fc_desc), f(fc_oth), f(fc_wide);
   }
   size_t device_copy_bytes() const;
   void upload() const;

@@ -396,7 +396,6 @@ static void build_fields(HostModel& m)
 {
   m.fc_desc.clear();
   m.fc_tab.clear();
-  m.fc_in.clear();
   m.fc_oth.clear();
   m.fc_wide.clear();
   m.fc_words = 0;
@@ -536,7 +535,7 @@ static void build_fields(HostModel& m)
     rows[0] = (rows[0] + 3) & ~3;
     const bool matrix = pair && kin > KI;
     const size_t words = rec_at / 2 + 32 * (size_t)(rows[0] + rows[1] + rows[2] + rows[3]) + 16 * (size_t)rows[2] +
-                         (matrix ? 512 : 0);
+                         (matrix ? 512 : 64 * (size_t)std::max(0, kin - KI));
     const size_t at = m.fc_tab.size();
     m.fc_tab.resize(at + ((2 * words + 3) & ~(size_t)3), 0u);
     uint32_t* tab = &m.fc_tab[at];
@@ -544,13 +543,14 @@ static void build_fields(HostModel& m)
     m.fc_desc[(size_t)b * 4 + 1] = (int)((words + 1) & ~(size_t)1);
     m.fc_words = std::max(m.fc_words, m.fc_desc[(size_t)b * 4 + 1]);
     tab[0] = (uint32_t)(rows[0] / 4) | (uint32_t)(rows[1] / 2) << 7 | (uint32_t)(rows[2] / 2) << 15 |
-             (uint32_t)std::min(kin, KI) << 23 | (kin > KI || rows[3] ? 1u << 31 : 0u);
-    tab[1] = (uint32_t)rows[3];
+             (uint32_t)std::min(kin, KI) << 23;
+    tab[1] = (uint32_t)rows[3] | (uint32_t)(matrix ? 1 : std::max(0, kin - KI)) << 8;
     uint32_t* s0 = tab + rec_at;
     uint32_t* s1 = s0 + 64 * rows[0];
     uint32_t* s2 = s1 + 64 * rows[1];
     uint32_t* s2c = s2 + 64 * rows[2];
     uint32_t* s3 = s2c + 32 * rows[2];
+    uint32_t* more = s3 + 64 * rows[3];
     for (int l = 0; l < 32; l++)
     {
       uint32_t* own = tab + 8 + (pair ? 2 : 4) * l;
@@ -601,24 +601,12 @@ static void build_fields(HostModel& m)
         for (const Entry& e : in[l])
         {
           tab[ent_at + l * ew] |= e.w[0];
-          uint32_t& w = s1[32 * __builtin_ctz(e.w[0]) + l];
-          w += e.w[1];
+          more[32 * __builtin_ctz(e.w[0]) + l] += e.w[1];
         }
         continue;
       }
-      for (size_t k = 0; k < in[l].size() && k < (size_t)KI; k++)
-        memcpy(tab + ent_at + (k * 32 + l) * ew, in[l][k].w, ew * 4);
-    }
-    if (matrix) tab[1] |= 1u << 8;
-    else if (kin > KI)
-    {
-      const size_t more = m.fc_in.size() / ew;
-      tab[1] |= (uint32_t)(kin - KI) << 8;
-      tab[2] = (uint32_t)more;
-      m.fc_in.resize(m.fc_in.size() + (size_t)(kin - KI) * 32 * ew, 0u);
-      for (int l = 0; l < 32; l++)
-        for (size_t k = KI; k < in[l].size(); k++)
-          memcpy(&m.fc_in[(more + (k - KI) * 32 + l) * ew], in[l][k].w, ew * 4);
+      for (size_t k = 0; k < in[l].size(); k++)
+        memcpy(k < (size_t)KI ? tab + ent_at + (k * 32 + l) * ew : more + ((k - KI) * 32 + l) * ew, in[l][k].w, ew * 4);
     }
   }
 }
@@ -856,7 +844,7 @@ void HostModel::upload() const
 {
   ensure_device();
   std::vector<char> blob(device_copy_bytes());
-  std::array<size_t, 23> at;
+  std::array<size_t, 22> at;
   size_t n = 0, k = 0;
   device_arrays([&](const auto& v) {
     at[k++] = n = boundary(n);
@@ -864,7 +852,7 @@ void HostModel::upload() const
     n += v.size() * sizeof(v[0]);
   });
   const auto [o_row, o_inc, o_coef, o_ci, o_nbr, o_trow, o_tvar, o_tc, o_tci, o_cf, o_near, o_oth, o_ri, o_rf, o_rp,
-              o_lo, o_le, o_lp, o_ft, o_fd, o_fi, o_fo, o_fw] = at;
+              o_lo, o_le, o_lp, o_ft, o_fd, o_fo, o_fw] = at;
   dmem = DevBuf(blob.size());
   h2d(dmem.ptr, blob.data(), blob.size(), "model upload");
   char* b = (char*)dmem.ptr;
@@ -907,7 +895,6 @@ void HostModel::upload() const
   dev.lv_d8 = lv_d8 ? 1 : 0;
   dev.fc_desc = fc_desc.empty() ? nullptr : (const int4*)(b + o_fd);
   dev.fc_tab = (const uint2*)(b + o_ft);
-  dev.fc_in = (const void*)(b + o_fi);
   dev.fc_words = fc_words;
   dev.fc_oth = (const uint2*)(b + o_fo);
   dev.fc_wterm = (const int*)(b + o_fw);

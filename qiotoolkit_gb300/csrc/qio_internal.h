@@ -88,9 +88,8 @@ struct DevModel
   // block-decided sweep (fields.cu), blocks of 32 variables, a lane each.
   // Block b's chunk begins at 8-byte word fc_desc[b].x of fc_tab:
   //   header, 32 bytes: rows of records of one literal / 4 | of two / 2 << 7 | of
-  //     three / 2 << 15 | in-block entry rows (at most four) << 23 | the next
-  //     word is not 0 << 31; rows of wide terms | further entry rows << 8 (pair-only
-  //     Ising: 1, a matrix); first further entry in fc_in;
+  //     three / 2 << 15 | in-block entry rows (at most four) << 23; rows of wide
+  //     terms | further entry rows << 8 (pair-only Ising: 1, a matrix);
   //   lane data, 8 bytes: the field with every record's op 0; degree; not pair: 16,
   //     the row's negated literals, its terms of v alone (counter models);
   //   in-block entries, four per lane (entry i of lane l at 32 i + l), one per
@@ -103,17 +102,17 @@ struct DevModel
   //     weight); two (16 bits each, weight); three (the same, and the third's
   //     rows of 32 words behind them); wide terms (term | own literal negated <<
   //     31, weight; 1 << 30: padding; 1 << 29: an entry holds its value);
-  //   a pair-only Ising block of lanes with more than four entries: their only
-  //     entry has all earlier members' lanes and no value, and the values stand in
-  //     a matrix of 32-bit words, the member's lane by the own.
+  //   further entries, rows of 32.  Where a lane of a pair-only Ising block has
+  //     more than four, its only entry has all earlier members' lanes and no value,
+  //     and the values stand in a matrix of 32-bit words, the member's lane by the
+  //     own.
   // Weights and values of FP64 models that are not pair-only are multiples of 256,
-  // the row position (modulo 32) beside them.  The field is the lane's value minus the weights whose op is 1: the literals'
-  // OR (counter models) or XOR.  A literal 2u + n is variable u's, negated with n
-  // = 1; 2N is false; pair-only Ising uses u itself.  Further entries lie in
-  // fc_in, rows of 32.
+  // the row position (modulo 32) beside them.  The field is the lane's value minus
+  // the weights whose op is 1: the literals' OR (counter models) or XOR.  A literal
+  // 2u + n is variable u's, negated with n = 1; 2N is false; pair-only Ising uses u
+  // itself.
   const int4* fc_desc;     // (start, 8-byte words), or null when the model does not qualify
   const uint2* fc_tab;
-  const void* fc_in;
   const uint2* fc_oth;     // K (not pair-only): up to three other literals, 16 bits each (0xFFFF:
                            // none), own literal negated << 48, wide term << 49
   const int* fc_wterm;     // wide terms (more than four members)
