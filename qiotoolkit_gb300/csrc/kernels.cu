@@ -2202,9 +2202,13 @@ cudaError_t launch_qmc(const QmcArgs& a, cudaStream_t s)
 // ---------------------------------------------------------------------------
 __global__ void pt_swap_kernel(SwapArgs a)
 {
-  // launched while the sweep before it runs, and lets the next one's blocks in
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // Launched while the sweep before it runs; the next one's blocks come in once
+  // that is done.  (Let in before the wait, they held shared memory for the whole
+  // sweep that other solves had use for: 64 tempering requests of 128 walkers
+  // through a server 410 ms, so 339, 96 of 384 walkers 1433 and 1252; one solve
+  // alone, 3-SAT of 64 walkers, 200 steps, 10.55 and 10.39.)
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // one warp per restart: lanes over the ladder's walkers, then over the
   // step's pairs (pairs of one parity share no walker)
   const int lane = threadIdx.x & 31;
