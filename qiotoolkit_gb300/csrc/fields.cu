@@ -1711,18 +1711,7 @@ __global__ void __launch_bounds__(INT ? 512 : 384, 1) fc_sweep_kernel(const __gr
     if (*(volatile unsigned*)R.abort) return;
     copy16((uint4*)g_spins, (const uint4*)R.spins, a.p.nw >> 2, me, nme);
     walker_sync<INT>(bar_id);  // the region is reused by the next walker
-    if (!queued)
-    {
-      r += a.n_streams;
-      // a stream that serves several walkers goes on where the last one ended
-      if (REPLAY && r < a.n_walkers)
-      {
-        if (decider && lane == 0) a.rng[w] = rs;
-        __threadfence_block();
-        walker_sync<INT>(bar_id);
-        rs = *(volatile uint64_t*)(a.rng + w);
-      }
-    }
+    if (!queued) break;
   }
   if (REPLAY && !queued && decider && lane == 0) a.rng[w] = rs;
 }
@@ -1811,6 +1800,7 @@ bool fc_fits(const DevModel& m, int nw)
 cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb)
 {
   if (!fc_fits(a.m, a.p.nw)) return cudaErrorInvalidValue;
+  if (!a.queue && a.n_streams != a.n_walkers) return cudaErrorInvalidValue;  // (a stream to a walker)
   const bool I = a.m.int_mode != 0;
   // The first of these shapes with the fewest waves of blocks (twice as long where
   // the largest blocks do not fit a buffer): four chunk buffers each, which cover
@@ -1827,7 +1817,7 @@ cudaError_t launch_fc_sweep(const SweepArgs& a, cudaStream_t s, int wpb)
   long long least = LLONG_MAX;
   for (const Choice& c : choices)
   {
-    if (c.shared && (a.queue || a.n_streams != a.n_walkers)) continue;
+    if (c.shared && a.queue) continue;
     const fc::Shape x = fc::shape_of(a.m, a.p.nw, c.bufs, c.shared);
     const int w = fc::walkers_of(x, I);
     if (w < 1) continue;

@@ -899,8 +899,6 @@ void HostModel::upload() const
   dev.fc_oth = (const uint2*)(b + o_fo);
   dev.fc_wterm = (const int*)(b + o_fw);
   dev.fc_wide = (int)fc_wide.size();
-  dev.fc_S = fc_S;
-  dev.fc_pack = fc_pack ? 1 : 0;
   dev.fc_inv = std::ldexp(1.0, -fc_S);
   int ordinal = -1;
   cuda_check(cudaGetDevice(&ordinal), "cudaGetDevice");

@@ -118,9 +118,7 @@ struct DevModel
   const int* fc_wterm;     // wide terms (more than four members)
   int fc_wide;             // their number
   int fc_words;            // 8-byte words of the largest chunk
-  int fc_S;                // fixed-point scale exponent
-  int fc_pack;             // FP64 models that are not pair-only: field = fixed << 8
-  double fc_inv;           // 2^-fc_S
+  double fc_inv;           // fixed-point unit of the fields
 };
 
 // Walker population in HBM (structure of arrays).  Spins are bit-packed,
