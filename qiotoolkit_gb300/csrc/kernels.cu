@@ -2604,7 +2604,15 @@ cudaError_t launch_tabu(const TabuArgs& a, cudaStream_t s)
     const TabuFit f = tabu_fit(a.m, a.p.nw);
     // as few walkers a block as the SMs need
     const int wpb = std::min(f.warps, std::max(1, (a.n_walkers + 151) / 152));
-    if (wpb > 0)
+    // A wave of walkers takes the pair kernel 0.69 of a wave's time on the other one
+    // (integers 0.45), but that one's waves are 1216 walkers whatever the model (1.2
+    // of a small wave's time when full, in proportion from there on), this one's
+    // what fits beside the model.  Other / pair, 60 steps (ms): 1000 spins of 8000
+    // couplings, 152 walkers 4.9 / 2.9, 608 5.0 / 11.0; of 5000, 608 3.3 / 2.2, 912 4.0 /
+    // 4.2, 2432 10.0 / 8.2; 3000 spins, integers, 456 9.3 / 8.6, 912 11.4 / 13.0, 4096
+    // 30 / 57; 1000 spins of 3000, 4096 9.7 / 6.7.
+    const int waves = wpb > 0 ? (a.n_walkers + 152 * wpb - 1) / (152 * wpb) : 0;
+    if (wpb > 0 && waves * (I ? 0.45 : 0.69) <= (a.n_walkers <= 1216 ? 1.2 : a.n_walkers / 800.0))
     {
       const size_t smem = f.model + wpb * f.walker;
       auto k = I ? tabu_pair_kernel<true> : tabu_pair_kernel<false>;
