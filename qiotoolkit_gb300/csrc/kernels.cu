@@ -2163,9 +2163,15 @@ static cudaError_t qmc_dispatch(const QmcArgs& a, cudaStream_t s)
   // row until it decides nothing (complete graphs of 500 variables, N(0, 1)
   // couplings 118 ms here and there, of 1000, couplings of variance 1 / N, 332 here
   // and 495 there, PUBO rows of 2400 102 and 93), and the work of the 32 variables
-  // between two signs of progress stays below what the warps' waits allow.
+  // between two signs of progress stays below what the warps' waits allow.  Nor do
+  // launches of few decisions (partial MaxSat sweeps), as every variable's word is
+  // made and put back: 8000 variables, a decision a sweep, 30 sweeps 0.49 ms against
+  // 0.28, 100 0.63 against 0.79; 1000 variables 0.23 and 0.24, 0.45 and 0.68.  (The
+  // restarts are at most the host's threads or 16, so each has its SM, or nearly:
+  // 16000 variables, 16 restarts of 32 slices, 3 sweeps 49.9 ms against 165.)
   const size_t words = ((size_t)a.m.n_vars * 3 + 1) * 4;  // two copies, the row bounds
-  if (a.trotter <= 32 && words <= 200 * 1024 && a.m.max_deg <= 1024)
+  const bool few = (long long)a.n_steps * a.m.sweep_size < a.m.n_vars / 64;
+  if (a.trotter <= 32 && words <= 200 * 1024 && a.m.max_deg <= 1024 && !few)
   {
     auto k = FL == F_PARITY && a.m.pair_only ? qmc_sliced_kernel<FL, I, FL == F_PARITY> : qmc_sliced_kernel<FL, I, false>;
     const cudaError_t allowed = allow_shared((const void*)k, (int)words);
