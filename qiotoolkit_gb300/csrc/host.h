@@ -273,8 +273,8 @@ struct LaneRunner
 };
 bool lanes_eligible(const HostModel& m);
 // the lane kernel for this solver and walker count (params "kernel"; auto:
-// eligible models with at least 1024 walkers)
-// (blocks: the block-decided sweep runs the model)
+// eligible models from a number of walkers on; blocks: the block-decided sweep
+// runs the model)
 bool lanes_for(const Solver& s, const HostModel& m, int64_t walkers, bool blocks);
 bool levels_eligible(const HostModel& m);
 bool levels_for(const Solver& s, const HostModel& m);

@@ -213,6 +213,8 @@ cudaError_t launch_sweep(const SweepArgs& a, cudaStream_t s, int warps_per_block
 // one warp's walker state (term bytes, spins, lowest) fits shared memory
 // beside the windowed kernel's tables and tiles (required by batch queues)
 bool sweep_state_fits(const SweepArgs& a);
+// blocks of eight of its walkers that an SM's shared memory holds
+int sweep_blocks_fit(const SweepArgs& a);
 // block-decided sweep (fields.cu): whether it can run this model with this
 // population layout
 bool fc_fits(const DevModel& m, int nw);

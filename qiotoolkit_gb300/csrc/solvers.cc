@@ -403,13 +403,32 @@ bool lanes_eligible(const HostModel& m) { return m.flavor == F_PARITY && m.pair_
 
 // Kernel choice: one walker per lane when asked for, or when there are so many
 // walkers that the lane kernel's time, the same up to some tens of thousands of
-// them, is the shortest.  Measured, 20 sweeps (ms), lanes against the
-// block-decided sweep (`blocks`: it runs the model) -- sparse Ising N = 64: 4.2
-// / 8.4 at 65536 walkers, 1.5 / 2.1 at 16384, 1.4 / 0.56 at 4096; N = 1000: 66 /
-// 73, 23 / 18, 22 / 4.7; integer N = 1000: 23 / 36, 15 / 9.3, 15 / 2.7 -- and
-// against the windowed sweep: N = 1000 22 / 9.9 at 4096, 23 / 34 at 16384;
-// cubic lattice of 4096 76 / 19 at 1024, 77 / 73 at 4096, 86 / 255 at 16384.
-static int64_t lane_walkers(bool blocks) { return blocks ? 24576 : 4096; }
+// them, is the shortest.  Against the block-decided sweep (`blocks`: it runs the
+// model), lanes / blocks, 20 sweeps (ms): sparse Ising N = 64 1.44 / 1.16 at 8192
+// walkers, 1.46 / 1.70 at 12288, integer N = 128 2.01 / 1.65 at 16384, 2.18 / 2.45
+// at 24576, N = 250 7.49 / 6.89 at 24576, 10.7 / 13.6 at 49152, N = 1000 30.5 / 24.3
+// at 24576, 66 / 73 at 65536, cubic lattice of 4096 89.7 / 59.9 at 24576; long rows
+// cost a lane more, in FP64 above all (N = 1000, 17 terms a row, 10 sweeps 88 / 45 at
+// 65536, 89 / 68 at 98304, integer 13.6 / 12.4 at 40960, 16.0 / 19.7 at 65536, 40 terms
+// 198 / 95 and 37.7 / 38.3 at 98304; integer complete graphs of 64 spins 2.85 / 2.49 at
+// 32768).  Against the windowed sweep, whose walkers on an SM get fewer with N
+// and which reads rows 32 wide, lanes / windowed: integer N = 250 13.4 / 13.3 at 8192
+// (population annealing, 50 sweeps), N = 1000 62.3 / 63.3, integer 42.7 / 17.3 at
+// 4096, N = 10000 365 / 287 at 2048, 372 / 501 at 4096; 40000 spins (10 sweeps) 478 /
+// 374 at 1024, 476 / 746 at 2048, cubic lattice of 32768 299 / 647; complete graphs
+// of 300 spins 208 / 148 at 2048, 211 / 294 at 4096, integer 60.5 / 58.0 and 61.7 /
+// 107, of 600 831 / 539 at 1024, 835 / 1062 at 2048.
+static int64_t lane_walkers(const HostModel& m, bool blocks)
+{
+  const int64_t N = std::max<int64_t>(1, m.N), K = std::max<int64_t>(1, m.K);
+  if (blocks)
+  {
+    const int64_t line = N >= 512 ? 40000 : std::min<int64_t>(30000, std::max<int64_t>(10240, 160 * N));
+    return line * std::min<int64_t>(4, std::max<int64_t>(1, K / ((m.int_mode ? 16 : 5) * N)));
+  }
+  return std::min<int64_t>(m.int_mode ? 8192 : 4096,
+                           std::max<int64_t>(1024, std::min<int64_t>(20000000 / N, 220000000 / K)));
+}
 
 bool lanes_for(const Solver& s, const HostModel& m, int64_t walkers, bool blocks)
 {
@@ -421,7 +440,7 @@ bool lanes_for(const Solver& s, const HostModel& m, int64_t walkers, bool blocks
   }
   if (s.kernel == 1 || s.kernel == 3) return false;
   if (s.kernel == 4) return !blocks && lanes_eligible(m) && walkers >= 1024;
-  return lanes_eligible(m) && walkers >= lane_walkers(blocks);
+  return lanes_eligible(m) && walkers >= lane_walkers(m, blocks);
 }
 
 // The level kernel runs integer pair-only Ising models whose level schedule
@@ -480,15 +499,38 @@ bool levels_for(const Solver& s, const HostModel& m)
 
 // The block-decided sweep (fields.cu): Ising with the term cache or counter
 // models (PUBO, MaxSat with full sweeps) whose walker state and block chunks
-// fit a block's shared memory.  auto: wherever it runs.  20 sweeps, this
-// kernel against the windowed one (ms): sparse Ising N = 1000, 64 walkers 0.64
-// / 2.37; PUBO N = 4096, 64 walkers 5.5 / 21.1, 8192 walkers 114 / 239; 3-SAT
-// N = 1000, 64 walkers 1.25 / 2.95, 8192 walkers 20.1 / 22.1.  "warp" keeps the
-// windowed kernel.
+// fit a block's shared memory.  auto: wherever it runs, but for the models of
+// windowed_instead.  This kernel against the windowed one (ms), 20 sweeps: sparse
+// Ising N = 1000, 64 walkers 0.64 / 2.37; PUBO N = 4096, 64 walkers 5.5 / 21.1, 8192
+// walkers 114 / 239; 3-SAT N = 1000, 64 walkers 1.25 / 2.95, 8192 walkers 20.1 /
+// 22.1; dense models and models of a hub in every block are below the windowed
+// sweep's times too (500 variables, 20 to 240 terms a row; 512 to 4096 variables
+// with hubs of 60 to 200 couplings every 32 or 128; 8 to 2432 walkers).  "warp"
+// keeps the windowed kernel.
 bool fields_run(const Solver& s, const HostModel& m, const Population& P, bool full_maxsat_sweep)
 {
   return !m.empty() && !m.fc_desc.empty() && s.smem_state &&
          fc_fits(m.device_view(full_maxsat_sweep), P.pop.nw);
+}
+// Small FP64 models of short rows, with more walkers than one wave of the
+// block-decided sweep's blocks, four walkers an SM.  The windowed kernel has eight,
+// and sixteen where two of its blocks fit.  100 sweeps, windowed / block-decided
+// (ms): 3-SAT of 16 variables 0.77 / 1.33 at 1216 walkers, 3.1 / 8.7 at 8192, of 48
+// 1.41 / 1.79 and 8.8 / 11.6, of 96 15.5 / 15.8; PUBO of 16 variables 1.19 / 1.75 at
+// 2432, of 64 2.4 / 3.2, of 48, where two blocks do not fit, 4.2 / 3.2; sparse Ising of
+// 16 and 32 spins 0.48 / 0.61 and 0.72 / 0.90 at 2432, of 48 1.06 times as long;
+// complete graphs of 24 and 32 spins 1.3 and 3.9 times.
+static bool small_fp64(const HostModel& m) { return !m.int_mode && m.N <= 64; }
+static bool windowed_instead(const HostModel& m, const Population& P, bool full_maxsat_sweep, int64_t walkers)
+{
+  if (!small_fp64(m)) return false;
+  const bool pair = m.flavor == F_PARITY && m.pair_only;
+  SweepArgs a{};
+  a.m = m.device_view(full_maxsat_sweep);
+  a.p = P.pop;
+  if (a.m.max_deg > (pair ? 16 : 24)) return false;
+  if (pair) return m.N <= 32 && walkers > 1216;
+  return m.kind == K_MAXSAT ? walkers > 608 : walkers > 1216 && sweep_blocks_fit(a) > 1;
 }
 bool fields_for(const Solver& s, const HostModel& m, const Population& P, bool full_maxsat_sweep)
 {
@@ -501,7 +543,7 @@ bool fields_for(const Solver& s, const HostModel& m, const Population& P, bool f
               "and walker state that fits shared memory");
     return true;
   }
-  return s.kernel == 0 && ok;
+  return s.kernel == 0 && ok && !windowed_instead(m, P, full_maxsat_sweep, s.n_walkers());
 }
 
 // beta as Metropolis::set_beta / set_temperature store it
@@ -2476,10 +2518,11 @@ class SABatch : public Batch
     lanes = eligible && kernel != 1;
   }
 
+  bool windowed = false;  // the members run on the windowed kernel instead
   // the block-decided sweep runs the model's walkers in this population
   bool block_decided(const HostModel& m) const
   {
-    return smem && kernel != 1 && !m.fc_desc.empty() && fc_fits(m.device_view(full_sweep), P.pop.nw);
+    return smem && kernel != 1 && !windowed && !m.fc_desc.empty() && fc_fits(m.device_view(full_sweep), P.pop.nw);
   }
 
   int n_instances() const override { return (int)models.size(); }
@@ -2497,16 +2540,35 @@ class SABatch : public Batch
     P.alloc_sizes(N, M, W, W, false, std::max<int64_t>(1, steps));
     // every model on the device before any capture (uploads allocate)
     for (auto* m : models) m->device_view(full_sweep);
+    // Batches of such models throughout (one launch; mixed with others theirs would
+    // be one more), where rows are not long: 512 PUBO models of 16 variables, 16
+    // walkers each, windowed 7.2 ms, block-decided 10.0, of 12 to 64 13.1 and 16.0,
+    // 3-SAT 11.5 and 14.3.
+    int64_t some = 0;
+    windowed = kernel == 0;
+    for (auto* m : models)
+    {
+      windowed = windowed && small_fp64(*m) && m->device_view(full_sweep).max_deg <= 40;
+      if (windowed && windowed_instead(*m, P, full_sweep, W)) some++;
+    }
+    windowed = windowed && 2 * some >= (int64_t)models.size();
     // One walker per lane instead of the block-decided sweep's queue: for very
-    // many walkers (lane_walkers), and for batches of small models, which are
-    // a few ms either way and keep the kernel that their plan reports (96
-    // instances of 64 to 8000 spins, 16 walkers each, 100 sweeps: 518 ms on
-    // lanes, 162 on the windowed kernel's queue, 37 on this one's).
+    // many walkers (lane_walkers), and for lattices and graphs of fewer than 352
+    // spins, whose plans report that kernel.  Those would be faster on this sweep's
+    // queue (100 sweeps, ms, lanes and queue: 16 lattices of 27 to 64 spins, 16
+    // walkers each, 3.4 and 0.5, 512 of them 5.7 and 4.5, 96 of 343 spins 19.5 and
+    // 2.9, 512 21.2 and 11.6), which "kernel": "fields" asks for; 96 of 64 to 8000
+    // spins are 518 on lanes, 162 on the windowed kernel's queue, 37 on this one's.
     if (lanes && kernel != 2)
     {
       bool blocks = true;
-      for (auto* m : models) blocks = blocks && block_decided(*m);
-      lanes = !blocks || (kernel != 4 && (N < 352 || W >= lane_walkers(true)));
+      const HostModel* largest = models[0];
+      for (auto* m : models)
+      {
+        blocks = blocks && block_decided(*m);
+        if (m->N > largest->N) largest = m;
+      }
+      lanes = !blocks || (kernel != 4 && (N < 352 || W >= lane_walkers(*largest, true)));
     }
     order.resize(models.size());
     for (size_t i = 0; i < models.size(); i++) order[i] = (int)i;

@@ -1329,6 +1329,13 @@ bool sweep_state_fits(const SweepArgs& a)
   return sw::kTableBytes + sw::warp_region_bytes(b, true) <= 227 * 1024;
 }
 
+int sweep_blocks_fit(const SweepArgs& a)
+{
+  SweepArgs b = a;
+  if (b.tile_cap <= 0) b.tile_cap = sw::tile_cap_for(b.m);
+  return 228 * 1024 / (sw::kTableBytes + 8 * sw::warp_region_bytes(b, true) + 1024);
+}
+
 // Launch: warps per block chosen so that the grid spreads over the SMs;
 // walker state goes to shared memory when the per-warp region fits.
 cudaError_t launch_sweep(const SweepArgs& a_in, cudaStream_t s, int wpb)
