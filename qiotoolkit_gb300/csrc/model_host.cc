@@ -853,7 +853,22 @@ void HostModel::upload() const
   });
   const auto [o_row, o_inc, o_coef, o_ci, o_nbr, o_trow, o_tvar, o_tc, o_tci, o_cf, o_near, o_oth, o_ri, o_rf, o_rp,
               o_lo, o_le, o_lp, o_ft, o_fd, o_fo, o_fw] = at;
-  dmem = DevBuf(blob.size());
+  // The block-decided sweep's tables, the last arrays, stay away where the device
+  // has no room for them (hubs in every block make them most of a model); the
+  // windowed sweep runs the model then.
+  bool tables = !fc_desc.empty();
+  try
+  {
+    dmem = DevBuf(blob.size());
+  }
+  catch (const Error& e)
+  {
+    if (e.status != 2 || !tables) throw;
+    cudaGetLastError();  // (the refused allocation)
+    tables = false;
+    blob.resize(boundary(o_ft) + 256);
+    dmem = DevBuf(blob.size());
+  }
   h2d(dmem.ptr, blob.data(), blob.size(), "model upload");
   char* b = (char*)dmem.ptr;
   dev.flavor = flavor;
@@ -893,11 +908,11 @@ void HostModel::upload() const
   dev.n_levels = lv_ok ? n_levels : 0;
   dev.lv_recs = lv_ok ? lv_recs : 0;
   dev.lv_d8 = lv_d8 ? 1 : 0;
-  dev.fc_desc = fc_desc.empty() ? nullptr : (const int4*)(b + o_fd);
-  dev.fc_tab = (const uint2*)(b + o_ft);
+  dev.fc_desc = tables ? (const int4*)(b + o_fd) : nullptr;
+  dev.fc_tab = tables ? (const uint2*)(b + o_ft) : nullptr;
   dev.fc_words = fc_words;
-  dev.fc_oth = (const uint2*)(b + o_fo);
-  dev.fc_wterm = (const int*)(b + o_fw);
+  dev.fc_oth = tables ? (const uint2*)(b + o_fo) : nullptr;
+  dev.fc_wterm = tables ? (const int*)(b + o_fw) : nullptr;
   dev.fc_wide = (int)fc_wide.size();
   dev.fc_inv = std::ldexp(1.0, -fc_S);
   int ordinal = -1;
