@@ -759,6 +759,9 @@ __device__ __forceinline__ void block_rounds(const Smem& S, const DevModel& m, W
         if (g < total) apply_one(j, g - ej + (rj - rb), svj);
       }
     }
+    // the lanes' numbers of marks differ: the next round's looks at them come
+    // after the last one's
+    __syncwarp();
     const int wi = i0 >> 5;
     if (lane == 0 && flips) spins[wi] ^= flips;
     W.natt += (unsigned long long)adv;
