@@ -1405,7 +1405,8 @@ __global__ void __launch_bounds__(128) qmc_kernel(QmcArgs a)
 // 190), the accountant close behind.  N = 1000, 3000 couplings, 16 restarts of 32
 // slices, 50 sweeps: 145.4 ms with a lane per slice on spins, costs and streams in
 // HBM, 94 with w, costs and streams on the chip and every sum in FP64, 47.7 with
-// the exact sums off the way and the rows ahead in registers, 45.5 here.
+// the exact sums off the way and the rows ahead in registers, 45.5 here,
+// 45.9 with a sign of progress every 32 variables.
 namespace qs
 {
 static const int kRing = 512;  // flip words, a power of two
